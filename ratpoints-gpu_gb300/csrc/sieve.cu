@@ -1,20 +1,15 @@
-// Device sieve: table build and sieve kernels for sm_103a, and the host driver.
+// Device sieve: the host driver of the single-curve sieve kernel and its table
+// builds (sieve_fast.cuh) for sm_103a.
 //
-// Reference behaviour restated here (see the file:line citations per item):
-//   - mask basis: bit j of word u of row r for prime p is
-//     affine[((-H + 64 u + j) * r^-1) mod p], row 0 zero (src/sieve.cu:141-172,
-//     with 64-site words);
-//   - sieve: a site survives iff all 32 selected primes accept it; the last word
-//     is clipped at +H (src/sieve.cu:221-388, 196-213, 324-330);
+// Reference behaviour restated here:
+//   - a site (a, d) survives the reference plan iff f(a/d) mod p is a square
+//     for all 32 selected primes, the last word clipped at +H
+//     (src/sieve.cu:141-172, 196-213, 221-388);
 //   - survivors are (a, d) pairs, d = k or k*k (src/sieve.cu:179-181, 250-252).
 //
-// GB300 design: the tables for all 36 candidate primes are built once per search
-// on the device; one persistent launch per denominator batch; each CTA stages
-// the rows of its denominator's 10 largest selected primes into shared memory,
-// sweeps 64-bit words (4 per thread per step, lane-contiguous, rows extended so
-// no wrap test is needed inside a step), and compacts the rare stage-1
-// survivors into a per-warp queue that a full warp then checks against the
-// remaining 22 primes from L2-resident tables before warp-aggregated emission.
+// Both plans run on one kernel: the tables of a curve (stage-1 rows, class
+// lists, candidate primes) are built once per search on the device, and each
+// denominator batch is one persistent launch.
 #include "sieve.hpp"
 #include "tune.hpp"
 
@@ -32,6 +27,7 @@
 #include "preverify.hpp"
 #include "sieve_device.cuh"
 #include "sieve_fast.cuh"
+#include "sweep_plan.hpp"
 
 namespace rpg {
 
@@ -39,191 +35,6 @@ void check_cuda(cudaError_t status, const char *what) {
     if (status != cudaSuccess)
         throw CudaError(std::string(what) + ": " + cudaGetErrorString(status));
 }
-
-namespace dev {
-
-constexpr int kK = 4;                        // words per thread per step
-constexpr int kWarps = 8;
-constexpr int kThreads = kWarps * kWarpSize;
-constexpr int kStride = kThreads * kK;       // words per CTA step
-constexpr int kExt = kWarpSize * (kK - 1);   // row extension (words)
-constexpr int kRefFast = 10;                 // stage-1 primes held in shared memory
-constexpr int kSlotWords = 608;              // >= 509 + kExt, even
-constexpr int kQueue = 64;                   // per-warp stage-2 queue entries
-constexpr long long kMaxTileWords = 1LL << 30;
-constexpr std::size_t kRefSmem =
-    std::size_t(kRefFast) * kSlotWords * 8 + std::size_t(kWarps) * kQueue * 12;
-
-static_assert(kSlotWords >= kMaximumPrime + kExt, "slot must hold an extended row");
-static_assert(kSlotWords % 2 == 0, "slots must keep 16-byte alignment");
-
-struct RefTables {
-    const u64 *rows;
-    long long offset[kCandidatePrimes];   // word offset of (prime i, residue 0)
-    int length[kCandidatePrimes];         // words per row (p + kExt rounded up to even)
-    int prime[kCandidatePrimes];
-    u32 magic[kCandidatePrimes];
-};
-
-__global__ void ref_table_kernel(u64 *rows, RefTables T, const unsigned char *affine,
-                                 const unsigned short *inverse, const int *neg_h_mod,
-                                 long long total) {
-    long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (id >= total) return;
-    int i = 0;
-    while (i + 1 < kCandidatePrimes && T.offset[i + 1] <= id) ++i;
-    const int p = T.prime[i], L = T.length[i];
-    const long long rel = id - T.offset[i];
-    const int r = int(rel / L);
-    const int u = int(rel % L) % p;
-    u64 word = 0;
-    if (r != 0) {
-        const int inv = inverse[i * kMaximumPrime + r];
-        const int x0 = (neg_h_mod[i] + int((64LL * u) % p)) % p;
-        int x = int((long long)x0 * inv % p);
-        const unsigned char *aff = affine + i * kMaximumPrime;
-        for (int j = 0; j < 64; ++j) {
-            if (aff[x]) word |= u64(1) << j;
-            x += inv;
-            if (x >= p) x -= p;
-        }
-    }
-    rows[id] = word;
-}
-
-// Stage 2 for up to 32 queued words (one per lane), then emission.
-__device__ __forceinline__ void ref_drain(const u64 *qmask, const u32 *qoff, int start, int n,
-                                          const RefTables &T, const SieveArgs &A, int denominator,
-                                          const int *s_prime, const u32 *s_magic,
-                                          const u32 *s_bmod, const long long *s_row) {
-    const int lane = threadIdx.x & 31;
-    u64 m = 0;
-    u32 off = 0;
-    if (lane < n) {
-        m = qmask[start + lane];
-        off = qoff[start + lane];
-    }
-    __syncwarp();
-    const long long w = A.w_lo + off;
-    if (m) {
-        for (int s = kRefFast; s < kSelectedPrimes; ++s) {
-            const u32 p = u32(s_prime[s]);
-            u32 idx = s_bmod[s] + mod_small(off, p, s_magic[s]);
-            if (idx >= p) idx -= p;
-            m &= __ldg(T.rows + s_row[s] + idx);
-            if (!m) break;
-        }
-        if (m && w == A.words - 1) {
-            const int valid = int(2 * A.bound + 1 - 64 * (A.words - 1));
-            if (valid < 64) m &= (u64(1) << valid) - 1;
-        }
-    }
-    emit_survivors(m, w, A.bound, denominator, A.out_a, A.out_d, A.out_count, A.capacity);
-}
-
-__global__ void __launch_bounds__(kThreads) ref_sieve_kernel(RefTables T, SieveArgs A) {
-    extern __shared__ __align__(16) u64 smem[];
-    u64 *rows = smem;
-    u64 *qmask = rows + kRefFast * kSlotWords;
-    u32 *qoff = reinterpret_cast<u32 *>(qmask + kWarps * kQueue);
-
-    __shared__ int s_prime[kSelectedPrimes];
-    __shared__ u32 s_magic[kSelectedPrimes];
-    __shared__ u32 s_bmod[kSelectedPrimes];
-    __shared__ long long s_row[kSelectedPrimes];
-    __shared__ int s_len[kSelectedPrimes];
-    __shared__ int s_ok;
-
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const long long tile_words = A.w_hi - A.w_lo;
-    u64 *wq_mask = qmask + warp * kQueue;
-    u32 *wq_off = qoff + warp * kQueue;
-
-    for (int item = blockIdx.x; item < A.k_count; item += gridDim.x) {
-        const long long k = A.k_first + item;
-        const long long d = A.square ? k * k : k;
-        if (threadIdx.x == 0) {
-            int n = 0;
-            for (int i = kCandidatePrimes - 1; i >= 0 && n < kSelectedPrimes; --i) {
-                const int p = T.prime[i];
-                const int r = int(d % p);
-                if (r == 0) continue;
-                s_prime[n] = p;
-                s_magic[n] = T.magic[i];
-                s_row[n] = T.offset[i] + (long long)r * T.length[i];
-                s_len[n] = T.length[i];
-                s_bmod[n] = u32(A.w_lo % p);
-                ++n;
-            }
-            s_ok = n == kSelectedPrimes;
-        }
-        __syncthreads();
-        if (!s_ok) {  // unreachable for d < 2^31 (at most 3 candidates divide it)
-            __syncthreads();
-            continue;
-        }
-        for (int s = 0; s < kRefFast; ++s) {
-            const uint4 *src = reinterpret_cast<const uint4 *>(T.rows + s_row[s]);
-            uint4 *dst = reinterpret_cast<uint4 *>(rows + s * kSlotWords);
-            const int n16 = s_len[s] >> 1;
-            for (int t = threadIdx.x; t < n16; t += kThreads) dst[t] = __ldg(src + t);
-        }
-        __syncthreads();
-
-        u32 o[kRefFast], st[kRefFast], pb[kRefFast];
-        const u32 first = u32(warp * kWarpSize * kK + lane);
-#pragma unroll
-        for (int s = 0; s < kRefFast; ++s) {
-            const u32 p = u32(s_prime[s]);
-            o[s] = ((s_bmod[s] + first) % p) * 8u + u32(s * kSlotWords * 8);
-            st[s] = (u32(kStride) % p) * 8u;
-            pb[s] = p * 8u;
-        }
-        int qn = 0;
-        const unsigned char *rbase = reinterpret_cast<const unsigned char *>(rows);
-        for (long long off0 = 0; off0 < tile_words; off0 += kStride) {
-            u64 acc[kK];
-#pragma unroll
-            for (int kk = 0; kk < kK; ++kk) acc[kk] = ~u64(0);
-#pragma unroll
-            for (int s = 0; s < kRefFast; ++s) {
-                const unsigned char *rb = rbase + o[s];
-#pragma unroll
-                for (int kk = 0; kk < kK; ++kk)
-                    acc[kk] &= *reinterpret_cast<const u64 *>(rb + 256 * kk);
-                const u32 lo = u32(s * kSlotWords * 8);
-                const u32 t = o[s] + st[s];
-                o[s] = (t - lo >= pb[s]) ? t - pb[s] : t;
-            }
-#pragma unroll
-            for (int kk = 0; kk < kK; ++kk) {
-                const long long off = off0 + warp * kWarpSize * kK + kWarpSize * kk + lane;
-                const bool live = acc[kk] != 0 && off < tile_words;
-                const u32 b = __ballot_sync(kFullMask, live);
-                if (b) {
-                    const int pos = qn + __popc(b & lanemask_lt());
-                    if (live) {
-                        wq_mask[pos] = acc[kk];
-                        wq_off[pos] = u32(off);
-                    }
-                    qn += __popc(b);
-                    if (qn >= 32) {
-                        __syncwarp();
-                        ref_drain(wq_mask, wq_off, qn - 32, 32, T, A, int(d), s_prime, s_magic,
-                                  s_bmod, s_row);
-                        qn -= 32;
-                    }
-                }
-            }
-        }
-        __syncwarp();
-        ref_drain(wq_mask, wq_off, 0, qn, T, A, int(d), s_prime, s_magic, s_bmod, s_row);
-        __syncthreads();
-    }
-}
-
-}  // namespace dev
 
 // ---------------------------------------------------------------------------
 
@@ -315,19 +126,17 @@ int max_admissible_classes(const std::vector<std::string> &coefficients, int q) 
     return std::max(1, most2 * std::max(1, most_q));
 }
 
-// Dynamic shared memory of the fast kernel: `slots` staged row sets, the
-// consumer queues, and the slots' class runs and item prefixes.
-std::size_t fast_dynamic_smem(int row_words, int max_classes, int slots) {
-    const std::size_t runs = (std::size_t(slots) * max_classes * sizeof(dev::FastRun) + 7) & ~std::size_t(7);
-    return std::size_t(slots) * std::size_t(row_words) * 8 + std::size_t(dev::kFConsumers) * dev::kFQueue * 16 +
-           runs + std::size_t(slots) * std::size_t(max_classes + 1) * 4;
-}
+constexpr int kFastRowSlots = 3;  // most row sets the fast planner divides the budget by
 
-// Staged row words per slot that keep a CTA within half an SM's shared
-// memory (2 CTAs/SM, 1 KiB reserved each, 2 KiB of static shared memory).
+// Staged row words per slot that the fast planner may spend: `slots` row sets
+// (each row 96 words longer than its modulus), 12-warp queues and 32 bytes per
+// class within half an SM's shared memory.  These are the planner's terms; the
+// kernel stages the rows of the sweep plan made from its choice.
 long long fast_row_budget(int max_classes, int slots) {
     const long long per_cta = 228 * 1024 / 2 - 1024 - 2048;
-    return (per_cta - (long long)fast_dynamic_smem(0, max_classes, slots)) / (8LL * slots);
+    const long long lists = ((long long)slots * max_classes * 32 + 7) / 8 * 8 + (long long)slots * (max_classes + 1) * 4;
+    const long long queues = 11 * 64 * 16;
+    return (per_cta - queues - lists) / (8LL * slots);
 }
 
 FastPlan single_curve_plan(const std::vector<std::string> &coefficients, long long bound, int *max_classes,
@@ -349,23 +158,23 @@ FastPlan single_curve_plan(const std::vector<std::string> &coefficients, long lo
             plan = shape.rows > 0 ? planner.plan(cap, std::min(shape.rows, kMaxFastSlots), row_budget, false)
                                   : planner.plan(cap, kMaxFastSlots, row_budget);
             int row_words = 0;
-            for (int m : plan.moduli) row_words += (m + dev::kFExt + 1) & ~1;
+            for (int m : plan.moduli) row_words += (m + kFastRowExtension + 1) & ~1;
             if (row_words <= row_budget || cap <= 64) break;
             cap = cap * 7 / 8;
         }
         plan.row_slots = slots;
         return plan;
     };
-    if (shape.rows > 0) return plan_for(shape.slots == dev::kFMaxSlotCount ? dev::kFMaxSlotCount : 2);
+    if (shape.rows > 0) return plan_for(shape.slots == kFastRowSlots ? kFastRowSlots : 2);
     const FastPlan two = plan_for(2);
     if (word_count64(bound) > (1LL << 20)) return two;
-    const FastPlan three = plan_for(dev::kFMaxSlotCount);
+    const FastPlan three = plan_for(kFastRowSlots);
     return three.bits >= two.bits - 0.25 ? three : two;
 }
 
 struct Sieve::Impl {
     SieveOptions opt;
-    long long bound = 0, words = 0;
+    long long bound = 0;
     int device = 0, grid = 0;
     // stream: table builds and the launches into buffer 0; stream2: the
     // launches into buffer 1, so that a launch's first CTAs take the SMs that
@@ -379,22 +188,16 @@ struct Sieve::Impl {
     // batch's end, both measured from an origin recorded at start().
     cudaEvent_t origin = nullptr;
     float last_end_ms = 0;
-    dev::RefTables T{};
-    dev::u64 *rows = nullptr;
-    // fast plan
-    dev::FastTables F{};
-    dev::u64 *fast_rows = nullptr;
-    dev::u64 *fast_adm = nullptr;
-    dev::FastClassStart *fast_starts = nullptr;
-    dev::FastRun *list_runs = nullptr;     // class lists by denominator class (see FastTables)
-    int *list_count = nullptr;
-    long long list_words = 0;              // class words the lists cover (launches from word 0 to at least this)
-    int fast_max_classes = 1;
-    std::size_t fast_smem = 0;
-    std::vector<dev::u64> fast_adm_host;
-    std::vector<int> fast_bad_primes;      // denominator primes (see FastTables::nbad)
+    // the curve's tables, all in one allocation (see build_tables)
+    dev::SweepTables T{};
+    SweepPlan sweep;
+    unsigned char *arena = nullptr;
+    std::size_t sweep_smem = 0;
+    std::vector<int> count2_host;               // admissible residues mod two by d mod two
+    std::vector<std::vector<int>> countq_host;  // per class prime p: admissible residues by d mod p
+    std::vector<int> bad_primes;                // denominator primes (see SweepTables::nbad)
     FastPlan fast_plan;
-    long long max_tile = dev::kMaxTileWords;
+    long long tile = 0;           // numerators per launch (more: the row goes in pieces)
     long long capacity = 0;       // most survivors a buffer may grow to hold
     long long host_capacity = 0;  // entries of the pinned host arrays
     SieveTimings timings;
@@ -422,9 +225,9 @@ struct Sieve::Impl {
     long long q_next = 0, q_last = -1, q_batch = 1;
     std::deque<int> order;  // buffers in flight, oldest first
 
-    // Pieces of an overflowed batch still to deliver, in parameter/word order.
+    // Pieces of an overflowed batch still to deliver, in parameter/numerator order.
     struct Piece {
-        long long first, last, w_lo, w_hi;
+        long long first, last, a_lo, a_hi;
     };
     std::deque<Piece> pieces;
     long long piece_batch_first = 0, piece_batch_last = 0;
@@ -554,18 +357,8 @@ struct Sieve::Impl {
             if (b.copied) cudaEventDestroy(b.copied);
             b = Buffer{};
         }
-        cudaFree(rows);
-        rows = nullptr;
-        cudaFree(fast_rows);
-        fast_rows = nullptr;
-        cudaFree(fast_adm);
-        fast_adm = nullptr;
-        cudaFree(fast_starts);
-        fast_starts = nullptr;
-        cudaFree(list_runs);
-        cudaFree(list_count);
-        list_runs = nullptr;
-        list_count = nullptr;
+        cudaFree(arena);
+        arena = nullptr;
         if (h_count) cudaFreeHost(h_count);
         if (h_a) cudaFreeHost(h_a);
         if (h_d) cudaFreeHost(h_d);
@@ -582,68 +375,6 @@ struct Sieve::Impl {
         origin = nullptr;
         stream = stream2 = copy_stream = count_stream = nullptr;
         fork_event = join_event = nullptr;
-    }
-
-    void build_tables(const std::vector<std::string> &coefficients) {
-        auto t0 = Clock::now();
-        const auto &primes = candidate_primes();
-        long long total = 0;
-        for (int i = 0; i < kCandidatePrimes; ++i) {
-            const int p = primes[i];
-            T.prime[i] = p;
-            T.length[i] = (p + dev::kExt + 1) & ~1;
-            T.offset[i] = total;
-            T.magic[i] = dev::magic40(dev::u32(p));
-            total += (long long)p * T.length[i];
-        }
-        std::vector<unsigned char> affine(std::size_t(kCandidatePrimes) * kMaximumPrime, 0);
-        std::vector<unsigned short> inverse(std::size_t(kCandidatePrimes) * kMaximumPrime, 0);
-        std::vector<int> neg_h(kCandidatePrimes);
-        for (int i = 0; i < kCandidatePrimes; ++i) {
-            const int p = primes[i];
-            auto aff = affine_mask(p, coefficients);
-            std::copy(aff.begin(), aff.end(), affine.begin() + std::size_t(i) * kMaximumPrime);
-            modular_inverses(p, inverse.data() + std::size_t(i) * kMaximumPrime);
-            neg_h[i] = int((p - bound % p) % p);
-        }
-        timings.plan_ms += ms_since(t0);
-        auto t1 = Clock::now();
-        rows = device_alloc<dev::u64>(std::size_t(total), "cudaMalloc(sieve tables)");
-        unsigned char *d_aff = device_alloc<unsigned char>(affine.size(), "cudaMalloc(affine)");
-        unsigned short *d_inv = device_alloc<unsigned short>(inverse.size(), "cudaMalloc(inverse)");
-        int *d_neg = device_alloc<int>(neg_h.size(), "cudaMalloc(bound residues)");
-        timings.workspace_ms += ms_since(t1);
-        T.rows = rows;
-        cudaEvent_t e0, e1;
-        check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
-        check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
-        check_cuda(cudaEventRecord(e0, stream), "cudaEventRecord");
-        check_cuda(cudaMemcpyAsync(d_aff, affine.data(), affine.size(), cudaMemcpyHostToDevice, stream),
-                   "upload affine tables");
-        check_cuda(cudaMemcpyAsync(d_inv, inverse.data(), inverse.size() * sizeof(unsigned short),
-                                   cudaMemcpyHostToDevice, stream),
-                   "upload inverses");
-        check_cuda(cudaMemcpyAsync(d_neg, neg_h.data(), neg_h.size() * sizeof(int),
-                                   cudaMemcpyHostToDevice, stream),
-                   "upload bound residues");
-        const int threads = 256;
-        const long long blocks = (total + threads - 1) / threads;
-        timings.h2d_bytes += affine.size() + inverse.size() * sizeof(unsigned short) +
-                             neg_h.size() * sizeof(int);
-        dev::ref_table_kernel<<<unsigned(blocks), threads, 0, stream>>>(rows, T, d_aff, d_inv, d_neg,
-                                                                         total);
-        check_cuda(cudaGetLastError(), "ref_table_kernel launch");
-        check_cuda(cudaEventRecord(e1, stream), "cudaEventRecord");
-        check_cuda(cudaEventSynchronize(e1), "table build");
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        timings.table_ms += ms;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        cudaFree(d_aff);
-        cudaFree(d_inv);
-        cudaFree(d_neg);
-        timings.table_wall_ms += ms_since(t0);
     }
 
     void init(const std::vector<std::string> &coefficients) {
@@ -670,17 +401,6 @@ struct Sieve::Impl {
             check_cuda(cudaEventCreateWithFlags(&join_event, cudaEventDisableTiming), "cudaEventCreate");
             check_cuda(cudaEventCreate(&origin), "cudaEventCreate");
         }
-        check_cuda(cudaFuncSetAttribute(dev::ref_sieve_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        int(dev::kRefSmem)),
-                   "cudaFuncSetAttribute");
-        int sms = 0, per_sm = 0;
-        check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device),
-                   "cudaDeviceGetAttribute");
-        check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::ref_sieve_kernel,
-                                                                 dev::kThreads, dev::kRefSmem),
-                   "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-        grid = std::max(1, sms * std::max(1, per_sm));
         // Survivor buffers start small (most searches have few survivors) and
         // grow on overflow up to the per-buffer capacity; past it a batch is
         // split.  RPG_SURVIVOR_CAPACITY fixes both at its value (at least 64,
@@ -732,52 +452,87 @@ struct Sieve::Impl {
             host_capacity = initial;
         }
         timings.workspace_ms += ms_since(t0);
-        if (opt.plan == PlanKind::fast) build_fast_tables(coefficients, planned);
-        else build_tables(coefficients);
+        build_tables(coefficients, planned);
         if (opt.preverify) {
             preverifier.prepare({&coefficients}, stream);
             timings.h2d_bytes += preverifier.upload_bytes();
         }
     }
 
-    // Fast plan: the per-curve plan (class prime, stage-1 moduli), class-layout
-    // tables for the stage-1 moduli and the 36 reference candidates, and the
-    // admissible-class tables (2-adic by d mod 64, residues mod q by d mod q).
     using PlannedRows = std::future<std::pair<FastPlan, int>>;
 
-    void build_fast_tables(const std::vector<std::string> &coefficients, PlannedRows &planned) {
+    // The sweep plan of the curve's primes (sweep_plan.hpp), then its tables
+    // on the device: stage-1 rows, the 36 candidates' rows, late primes' rows
+    // and the class lists.
+    void build_tables(const std::vector<std::string> &coefficients, PlannedRows &planned) {
         auto t0 = Clock::now();
+        const bool fast = opt.plan == PlanKind::fast;
         // the plan was started on a host thread while the buffers were set up
-        std::tie(fast_plan, fast_max_classes) = planned.get();
+        if (fast) fast_plan = planned.get().first;
         const int n = int(coefficients.size()) - 1;
-        const int q = fast_plan.class_prime;
-        const long long M = 64LL * q;
-        const long long S = 64LL * M;
-        std::vector<int> primes_used;
-        for (const auto &f : fast_plan.slots)
-            for (int p : f) primes_used.push_back(p);
-        if (q > 1) primes_used.push_back(q);
-        for (int p : candidate_primes()) primes_used.push_back(p);
+        // the primes the plan tests before stage 2, then the 36 candidates
+        std::vector<int> plan_primes;
+        if (fast) {
+            for (const auto &f : fast_plan.slots)
+                for (int p : f) plan_primes.push_back(p);
+            if (fast_plan.class_prime > 1) plan_primes.push_back(fast_plan.class_prime);
+        }
         std::vector<unsigned char> affine;
         std::vector<unsigned short> inverse;
-        std::vector<int> base(kMaximumPrime, -1), lead(kMaximumPrime, 1);
-        for (int p : primes_used) {
-            if (base[p] >= 0) continue;
+        std::vector<int> base(kMaximumPrime, -1), lead(kMaximumPrime, 1), admitted(kMaximumPrime, 0);
+        std::vector<char> strict(kMaximumPrime, 0);
+        auto add_prime = [&](int p) {
+            if (base[p] >= 0) return;
             base[p] = int(affine.size());
             auto aff = affine_mask(p, coefficients);
+            for (auto v : aff) admitted[p] += v;
             affine.insert(affine.end(), aff.begin(), aff.end());
             const std::size_t at = inverse.size();
             inverse.resize(at + std::size_t(p), 0);
             modular_inverses(p, inverse.data() + at);
-            if (n % 2 == 0) {
-                lead[p] = square_mod(decimal_mod(coefficients.back(), p), p) ? 1 : 0;
-            }
+            if (n % 2 == 0) lead[p] = square_mod(decimal_mod(coefficients.back(), p), p) ? 1 : 0;
+        };
+        for (int p : plan_primes) {
+            add_prime(p);
+            strict[p] = 1;
         }
+        const auto &cands = candidate_primes();
+        for (int p : cands) add_prime(p);
+
+        SweepInput in;
+        in.bound = bound;
+        dev::u64 adm2[64];
+        for (auto &v : adm2) v = ~dev::u64(0);
+        if (fast) {
+            two_adic_classes(coefficients, adm2);
+            in.two = 64;
+            int total = 0, live = 0;
+            for (auto v : adm2) {
+                const int c = __builtin_popcountll(v);
+                total += c;
+                live += c > 0;
+                in.two_max = std::max(in.two_max, c);
+            }
+            in.two_classes = live ? double(total) / live : 1.0;
+        }
+        for (int p : plan_primes) in.primes.push_back({p, admitted[p], lead[p] ? p - 1 : 0, false});
+        // The 32 largest candidates are always selected where they do not
+        // divide d, so stage 1 may test them as well: all of the reference
+        // plan's, and those of a fast plan whose own rows filter weakly (13
+        // bits are usual) or whose long rows take several class primes away
+        // from them (shorter searches save the planning time).
+        if (!fast || fast_plan.bits < 12.5 || bound >= 4'000'000)
+            for (int i = kCandidatePrimes - kSelectedPrimes; i < kCandidatePrimes; ++i)
+                if (!strict[cands[i]]) in.primes.push_back({cands[i], admitted[cands[i]], cands[i], true});
+        sweep = plan_sweep(in);
+
+        const int q = sweep.q;
+        const long long M = (long long)sweep.two * q;
+        const long long S = 64LL * M;
+        // pattern rows per (prime, rho = 0 rule): step = M mod p, window start
+        // of residue x0 = x0 step^-1 mod p
         std::vector<dev::TableSpec> specs;
         long long total = 0;
-        int smem_words = 0;
-        // pattern rows per (prime, rho = 0 rule): step = M mod q, window start
-        // of residue x0 = x0 step^-1 mod q
         std::vector<dev::ClassPatternSpec> pspecs;
         long long pattern_total = 0;
         auto pattern_of = [&](int p, int lead_ok, dev::TableSpec &Sp, int f) {
@@ -801,232 +556,179 @@ struct Sieve::Impl {
             Sp.s_mod[f] = int(S % p);
             Sp.step_inv[f] = int(mod_inverse(M % p, p));
         };
-        F = dev::FastTables{};
-        F.slots = int(fast_plan.moduli.size());
-        for (int sl = 0; sl < F.slots; ++sl) {
+        auto magic_of = [](long long m) { return m == 1 ? ~0ull : (~0ull) / (unsigned long long)m + 1; };
+        auto mod_of = [](long long v, long long m) { return ((v % m) + m) % m; };
+        T = dev::SweepTables{};
+        dev::ClassListSpec C{};
+        C.two = sweep.two;
+        C.q = q;
+        C.two_max = sweep.two_max;
+        C.q_max = sweep.q_max;
+        C.nprimes = int(sweep.class_primes.size());
+        C.nrows = int(sweep.moduli.size());
+        C.lift2 = dev::u32(sweep.two == 1 ? 0 : (long long)q * mod_inverse(q % sweep.two, sweep.two) % M);
+        C.liftq = dev::u32(q == 1 ? 0 : (long long)sweep.two * mod_inverse(sweep.two % q, q) % M);
+        C.h2 = dev::u32(bound % sweep.two);
+        C.hq = dev::u32(bound % q);
+        int row_words = 0;
+        for (std::size_t r = 0; r < sweep.moduli.size(); ++r) {
             dev::TableSpec Sp{};
-            Sp.nf = int(fast_plan.slots[sl].size());
-            Sp.m = fast_plan.moduli[sl];
+            const int m = sweep.moduli[r];
+            Sp.m = m;
+            Sp.nf = int(sweep.rows[r].size());
             for (int i = 0; i < Sp.nf; ++i) {
-                Sp.q[i] = fast_plan.slots[sl][i];
-                pattern_of(Sp.q[i], lead[Sp.q[i]], Sp, i);
+                const int p = sweep.rows[r][std::size_t(i)];
+                Sp.q[i] = p;
+                pattern_of(p, strict[p] ? lead[p] : 2, Sp, i);
             }
-            Sp.length = (Sp.m + dev::kFExt + 1) & ~1;
+            Sp.length = sweep_row_words(m);
             Sp.offset = total;
-            total += (long long)Sp.m * Sp.length;
+            total += (long long)m * Sp.length;
             specs.push_back(Sp);
-            dev::FastModulus &Md = F.mod[sl];
-            Md.m = Sp.m;
-            Md.nf = Sp.nf;
-            for (int i = 0; i < Sp.nf; ++i) Md.q[i] = Sp.q[i];
-            Md.length = Sp.length;
-            Md.offset = Sp.offset;
-            Md.smem_offset = smem_words;
-            smem_words += Sp.length;
-            Md.inv_stride = dev::u32(mod_inverse(S % Sp.m, Sp.m));
-            Md.neg_h = dev::u32((Sp.m - bound % Sp.m) % Sp.m);
-            Md.wlo_mod = 0;
-            Md.step = dev::u32((dev::kWarpSize * dev::kFK) % Sp.m);
-            Md.step8 = 8u * Md.step;
-            Md.mod8 = 8u * dev::u32(Sp.m);
-            Md.soff8 = 8u * dev::u32(Md.smem_offset);
-            Md.magic = (unsigned long long)((~0ull) / (unsigned long long)Sp.m) + 1;
-            F.min_modulus = sl == 0 ? Sp.m : std::min(F.min_modulus, Sp.m);
+            dev::SweepRow &R = T.row[r];
+            R.offset = Sp.offset;
+            R.magic = magic_of(m);
+            R.m = dev::u32(m);
+            R.length = dev::u32(Sp.length);
+            R.soff8 = dev::u32(8 * row_words);
+            row_words += Sp.length;
+            C.m[r] = dev::u32(m);
+            C.inv_stride[r] = dev::u32(mod_inverse(S % m, m));
+            C.base[r] = dev::u32(mod_of(-(bound % m) - M, m));
         }
-        F.smem_words = smem_words;
-        const auto &cands = candidate_primes();
-        for (int i = 0; i < kCandidatePrimes; ++i) {
-            const int p = cands[i];
+        auto single = [&](int p, int lead_ok) {
             dev::TableSpec Sp{};
             Sp.nf = 1;
             Sp.m = p;
             Sp.q[0] = p;
-            pattern_of(p, 0, Sp, 0);  // rows with p | d go unused: stage 2 skips such p
+            pattern_of(p, lead_ok, Sp, 0);
             Sp.length = p;
             Sp.offset = total;
             total += (long long)p * p;
             specs.push_back(Sp);
-            dev::FastPrime &P = F.prime[i];
-            P.offset = Sp.offset;
+            return Sp.offset;
+        };
+        for (int i = 0; i < kCandidatePrimes; ++i) {
+            const int p = cands[i];
+            dev::FastPrime &P = T.prime[i];
+            // rows with p | d go unused: stage 2 skips such p.  A class prime
+            // has no rows: the swept classes are those that pass it
             P.p = p;
-            P.inv_stride = dev::u32(mod_inverse(S % p, p));
-            P.neg_h = dev::u32((p - bound % p) % p);
             P.magic = dev::magic40(dev::u32(p));
-            P.wlo_mod = 0;
+            if (q % p == 0) continue;
+            P.offset = single(p, 0);
+            P.inv_stride = dev::u32(mod_inverse(S % p, p));
         }
-        F.class_prime = q;
-        F.class_mod = int(M);
-        F.h_mod_m = int(bound % M);
-        F.inv64_q = q > 1 ? int(mod_inverse(64 % q, q)) : 0;
-        F.stride = S;
-        F.count_q = (2 * bound) / M;
-        F.count_r = int((2 * bound) % M);
-        for (int r64 = 0; r64 < 64; ++r64) F.mod_q[r64] = (unsigned char)(q > 1 ? r64 % q : 0);
-        if (q > 1)
-            for (int a = 0; a < q; ++a)
-                for (int rq = 0; rq < q; ++rq)
-                    F.crt[a * 13 + rq] = (unsigned char)(((rq - a + q) % q) * F.inv64_q % q);
-        // Admissible classes: 2-adic by d mod 64 (F(r, d) square mod 64, r odd
-        // when d is even), then residues r mod q by d mod q.
-        std::vector<int> c64(coefficients.size());
-        for (std::size_t i = 0; i < coefficients.size(); ++i) c64[i] = decimal_mod(coefficients[i], 64);
-        bool square64[64] = {};
-        for (int v = 0; v < 64; ++v) square64[(v * v) & 63] = true;
-        std::vector<dev::u64> adm(64 + dev::kFAdmQ, 0);
-        for (int dd = 0; dd < 64; ++dd) {
-            for (int r = 0; r < 64; ++r) {
-                if (dd % 2 == 0 && r % 2 == 0) continue;
-                int value = c64[n], power = 1;
-                for (int i = n - 1; i >= 0; --i) {
-                    value = (value * r) & 63;
-                    power = (power * dd) & 63;
-                    value = (value + c64[i] * power) & 63;
-                }
-                if (n % 2 == 1) value = (value * dd) & 63;
-                if (square64[value]) adm[dd] |= dev::u64(1) << r;
-            }
-        }
-        if (q > 1) {
-            const auto aff = affine_mask(q, coefficients);
-            for (int dq = 0; dq < q; ++dq) {
-                for (int r = 0; r < q; ++r) {
+        std::vector<dev::LatePrime> late;
+        for (int p : sweep.late)
+            late.push_back({single(p, lead[p]), dev::u32(p), dev::u32(mod_inverse(S % p, p))});
+        // admissible residues of the class primes by d mod p
+        std::vector<unsigned char> admq;
+        countq_host.clear();
+        for (int i = 0; i < C.nprimes; ++i) {
+            const int p = sweep.class_primes[std::size_t(i)];
+            const unsigned char *aff = affine.data() + base[p];
+            const unsigned short *inv = inverse.data() + base[p];
+            C.p[i] = p;
+            C.adm[i] = int(admq.size());
+            std::vector<int> counts(std::size_t(p), 0);
+            for (int dq = 0; dq < p; ++dq)
+                for (int r = 0; r < p; ++r) {
                     bool ok;
-                    if (dq == 0) ok = r != 0 && lead[q];
-                    else ok = aff[(r * mod_inverse(dq, q)) % q] != 0;
-                    if (ok) adm[64 + dq] |= dev::u64(1) << r;
+                    if (dq == 0) ok = strict[p] ? r != 0 && lead[p] : true;
+                    else ok = aff[r * inv[dq] % p] != 0;
+                    admq.push_back(ok);
+                    counts[std::size_t(dq)] += ok;
                 }
-            }
+            countq_host.push_back(std::move(counts));
         }
-        // Denominator primes: p < 512 (p != q, which the class residues
-        // already cover) with c_n not a square mod p, for even degree.  A
-        // denominator divisible by one holds no points: p !| a (gcd) gives
-        // F(a, d) = c_n a^n (mod p), a non-square.  The producer skips such
-        // denominators (pairs p, ceil(2^64 / p) after the class residues).
-        fast_bad_primes.clear();
-        if (n % 2 == 0) {
+        count2_host.assign(std::size_t(sweep.two), 0);
+        const dev::u64 two_bits = sweep.two == 64 ? ~dev::u64(0) : (dev::u64(1) << sweep.two) - 1;
+        for (int dd = 0; dd < sweep.two; ++dd) {
+            adm2[dd] &= two_bits;
+            count2_host[std::size_t(dd)] = __builtin_popcountll(adm2[dd]);
+        }
+        // Denominator primes (fast plan): p < 512 with c_n not a square mod p,
+        // for even degree.  A denominator divisible by one holds no points:
+        // p !| a (gcd) gives F(a, d) = c_n a^n (mod p), a non-square.  The
+        // producer skips such denominators.
+        bad_primes.clear();
+        if (fast && n % 2 == 0) {
             for (int p = 3; p < kMaximumPrime; p += 2) {
                 bool prime = true;
                 for (int f = 3; f * f <= p && prime; f += 2) prime = p % f != 0;
-                if (!prime || p == q) continue;
+                if (!prime) continue;
                 const int lc = decimal_mod(coefficients.back(), p);
                 if (lc == 0 || square_mod(lc, p)) continue;
-                fast_bad_primes.push_back(p);
-                adm.push_back(dev::u64(p));
-                adm.push_back((~0ull) / dev::u64(p) + 1);
+                dev::u32 inverse32 = dev::u32(p);  // p^-1 mod 2^32 by Newton's iteration (3 bits to start with)
+                for (int i = 0; i < 4; ++i) inverse32 *= 2u - dev::u32(p) * inverse32;
+                T.bad[bad_primes.size()] = make_uint2(inverse32, 0xFFFFFFFFu / dev::u32(p));
+                bad_primes.push_back(p);
             }
-        }
-        F.nbad = int(fast_bad_primes.size());
-        fast_adm_host = adm;
-        // class starts for every residue r mod M: ofs = (r + H) mod M and, per
-        // modulus, the row index ((-H + ofs) S^-1) mod m of class word 0
-        std::vector<dev::FastClassStart> starts(static_cast<std::size_t>(M));
-        for (long long r = 0; r < M; ++r) {
-            dev::FastClassStart &cs = starts[std::size_t(r)];
-            const long long ofs = (r + bound % M) % M;
-            cs.ofs = (unsigned short)ofs;
-            for (int sl = 0; sl < F.slots; ++sl) {
-                const dev::FastModulus &Md = F.mod[sl];
-                cs.start[sl] = (unsigned short)((Md.neg_h + ofs) % Md.m * Md.inv_stride % Md.m);
-            }
-        }
-        // class lists by denominator class k = (d mod 64) q + (d mod q), in the
-        // order the producer would lay them out, for launches over whole rows
-        const int maxc = fast_max_classes;
-        const int ncombo = 64 * q;
-        list_words = (F.count_q + 1 + 63) >> 6;
-        std::vector<dev::FastRun> lruns;
-        std::vector<int> lcount;
-        int list_ipc = 1;
-        if (list_words < (1LL << 23)) {
-            lruns.assign(std::size_t(ncombo) * maxc, dev::FastRun{});
-            lcount.assign(std::size_t(ncombo), 0);
-            // every class of a whole row has the same number of sweep items:
-            // that of the longest class (classes differ by one word at most)
-            list_ipc = int((list_words + dev::kFItemWords - 1) / dev::kFItemWords);
-            auto nth_bit = [](dev::u64 mask, int k) {
-                for (int i = 0; i < k; ++i) mask &= mask - 1;
-                return __builtin_ctzll(mask);
-            };
-            for (int dd = 0; dd < 64; ++dd)
-                for (int dq = 0; dq < q; ++dq) {
-                    const int k = dd * q + dq;
-                    const dev::u64 classes2 = adm[std::size_t(dd)];
-                    const dev::u64 classesq = q > 1 ? adm[std::size_t(64 + dq)] : dev::u64(1);
-                    const int nq = __builtin_popcountll(classesq);
-                    const int nclass = __builtin_popcountll(classes2) * nq;
-                    if (nclass > maxc) throw std::logic_error("class list longer than the class bound");
-                    for (int c = 0; c < nclass; ++c) {
-                        const int i2 = c / nq;
-                        const int r64 = nth_bit(classes2, i2);
-                        int r = r64;
-                        if (q > 1) r = r64 + 64 * int(F.crt[F.mod_q[r64] * 13 + nth_bit(classesq, c - i2 * nq)]);
-                        const dev::FastClassStart &cs = starts[std::size_t(r)];
-                        const long long count = F.count_q + (cs.ofs <= F.count_r ? 1 : 0);
-                        const long long cw = (count + 63) >> 6;
-                        const dev::u32 last_bits = cw > 0 ? dev::u32(count - 64 * (cw - 1)) : 64u;
-                        dev::FastRun &run = lruns[std::size_t(k) * maxc + c];
-                        run.words_last = dev::u32(cw) | (cw > 0 ? 1u << 24 : 0u) | ((last_bits - 1) << 25);
-                        run.ofs = cs.ofs;
-                        for (int sl = 0; sl < dev::kFastSlots; ++sl) run.start[sl] = cs.start[sl];
-                        if (cw > list_words) throw std::logic_error("class longer than its row");
-                    }
-                    lcount[std::size_t(k)] = nclass;
-                }
         }
         timings.plan_ms += ms_since(t0);
+
+        // One allocation and one upload: [rows, lists, counts][uploaded blob][patterns]
         auto t1 = Clock::now();
-        if (!lruns.empty()) {
-            list_runs = device_alloc<dev::FastRun>(lruns.size(), "cudaMalloc(class lists)");
-            list_count = device_alloc<int>(lcount.size(), "cudaMalloc(class lists)");
-            check_cuda(cudaMemcpyAsync(list_runs, lruns.data(), lruns.size() * sizeof(dev::FastRun),
-                                       cudaMemcpyHostToDevice, stream),
-                       "upload class lists");
-            check_cuda(cudaMemcpyAsync(list_count, lcount.data(), lcount.size() * sizeof(int),
-                                       cudaMemcpyHostToDevice, stream),
-                       "upload class lists");
-            timings.h2d_bytes += lruns.size() * sizeof(dev::FastRun) + lcount.size() * sizeof(int);
-        }
-        fast_rows = device_alloc<dev::u64>(std::size_t(total), "cudaMalloc(class tables)");
-        fast_adm = device_alloc<dev::u64>(adm.size(), "cudaMalloc(admissible classes)");
-        fast_starts = device_alloc<dev::FastClassStart>(starts.size(), "cudaMalloc(class starts)");
-        unsigned char *d_aff = device_alloc<unsigned char>(affine.size(), "cudaMalloc(affine)");
-        unsigned short *d_inv = device_alloc<unsigned short>(inverse.size(), "cudaMalloc(inverse)");
-        dev::TableSpec *d_specs = device_alloc<dev::TableSpec>(specs.size(), "cudaMalloc(specs)");
-        dev::ClassPatternSpec *d_pspecs = device_alloc<dev::ClassPatternSpec>(pspecs.size(), "cudaMalloc(specs)");
-        dev::u64 *d_patterns = device_alloc<dev::u64>(std::size_t(pattern_total), "cudaMalloc(patterns)");
+        std::size_t size = 0;
+        auto take = [&](std::size_t bytes) {
+            const std::size_t at = size;
+            size += (bytes + 255) & ~std::size_t(255);
+            return at;
+        };
+        const std::size_t rows_at = take(std::size_t(total) * 8);
+        const std::size_t list2_at = take(std::size_t(sweep.two) * sweep.two_max * sizeof(dev::SweepClass));
+        const std::size_t listq_at = take(std::size_t(q) * sweep.q_max * sizeof(dev::SweepClass));
+        const std::size_t count2_at = take(std::size_t(sweep.two) * sizeof(int));
+        const std::size_t countq_at = take(std::size_t(q) * sizeof(int));
+        const std::size_t blob_at = size;
+        std::vector<unsigned char> blob;
+        auto put = [&](const void *data, std::size_t bytes) {
+            const std::size_t at = take(bytes);
+            blob.resize(size - blob_at);
+            if (bytes) std::memcpy(blob.data() + (at - blob_at), data, bytes);
+            return at;
+        };
+        const std::size_t late_at = put(late.data(), late.size() * sizeof(dev::LatePrime));
+        const std::size_t aff_at = put(affine.data(), affine.size());
+        const std::size_t inv_at = put(inverse.data(), inverse.size() * sizeof(unsigned short));
+        const std::size_t specs_at = put(specs.data(), specs.size() * sizeof(dev::TableSpec));
+        const std::size_t pspecs_at = put(pspecs.data(), pspecs.size() * sizeof(dev::ClassPatternSpec));
+        const std::size_t admq_at = put(admq.data(), admq.size());
+        const std::size_t adm2_at = put(adm2, sizeof adm2);
+        const std::size_t patterns_at = take(std::size_t(pattern_total) * 8);
+        arena = device_alloc<unsigned char>(size, "cudaMalloc(sieve tables)");
         timings.workspace_ms += ms_since(t1);
         cudaEvent_t e0, e1;
         check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
         check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
         check_cuda(cudaEventRecord(e0, stream), "cudaEventRecord");
-        check_cuda(cudaMemcpyAsync(d_aff, affine.data(), affine.size(), cudaMemcpyHostToDevice, stream),
-                   "upload affine tables");
-        check_cuda(cudaMemcpyAsync(d_inv, inverse.data(), inverse.size() * sizeof(unsigned short),
-                                   cudaMemcpyHostToDevice, stream),
-                   "upload inverses");
-        check_cuda(cudaMemcpyAsync(d_specs, specs.data(), specs.size() * sizeof(dev::TableSpec),
-                                   cudaMemcpyHostToDevice, stream),
-                   "upload table specs");
-        check_cuda(cudaMemcpyAsync(d_pspecs, pspecs.data(), pspecs.size() * sizeof(dev::ClassPatternSpec),
-                                   cudaMemcpyHostToDevice, stream),
-                   "upload pattern specs");
-        check_cuda(cudaMemcpyAsync(fast_adm, adm.data(), adm.size() * sizeof(dev::u64),
-                                   cudaMemcpyHostToDevice, stream),
-                   "upload admissible classes");
-        check_cuda(cudaMemcpyAsync(fast_starts, starts.data(), starts.size() * sizeof(dev::FastClassStart),
-                                   cudaMemcpyHostToDevice, stream),
-                   "upload class starts");
-        timings.h2d_bytes += affine.size() + inverse.size() * sizeof(unsigned short) +
-                             specs.size() * sizeof(dev::TableSpec) + pspecs.size() * sizeof(dev::ClassPatternSpec) +
-                             adm.size() * sizeof(dev::u64) + starts.size() * sizeof(dev::FastClassStart);
+        check_cuda(cudaMemcpyAsync(arena + blob_at, blob.data(), blob.size(), cudaMemcpyHostToDevice, stream),
+                   "upload table inputs");
+        timings.h2d_bytes += blob.size();
+        auto at = [&](std::size_t offset) { return arena + offset; };
+        dev::u64 *rows = reinterpret_cast<dev::u64 *>(at(rows_at));
+        dev::u64 *patterns = reinterpret_cast<dev::u64 *>(at(patterns_at));
+        T.listq = reinterpret_cast<const dev::SweepClass *>(at(listq_at));
+        T.list2 = reinterpret_cast<const dev::SweepClass *>(at(list2_at));
+        T.count2 = reinterpret_cast<const int *>(at(count2_at));
+        T.countq = reinterpret_cast<const int *>(at(countq_at));
+        T.rows = rows;
+        T.late = reinterpret_cast<const dev::LatePrime *>(at(late_at));
         const int threads = 256;
         dev::pattern_rows_kernel<<<unsigned((pattern_total + threads - 1) / threads), threads, 0, stream>>>(
-            d_patterns, d_pspecs, int(pspecs.size()), d_aff, d_inv, pattern_total);
+            patterns, reinterpret_cast<const dev::ClassPatternSpec *>(at(pspecs_at)), int(pspecs.size()), at(aff_at),
+            reinterpret_cast<const unsigned short *>(at(inv_at)), pattern_total);
         check_cuda(cudaGetLastError(), "pattern_rows_kernel launch");
         const long long blocks = (total + threads - 1) / threads;
-        dev::class_table_kernel<<<unsigned(blocks), threads, 0, stream>>>(fast_rows, d_specs, int(specs.size()),
-                                                                          d_patterns, total);
+        dev::class_table_kernel<<<unsigned(blocks), threads, 0, stream>>>(
+            rows, reinterpret_cast<const dev::TableSpec *>(at(specs_at)), int(specs.size()), patterns, total);
         check_cuda(cudaGetLastError(), "class_table_kernel launch");
+        dev::class_list_kernel<<<unsigned(q + sweep.two), threads, 0, stream>>>(
+            C, at(admq_at), reinterpret_cast<const dev::u64 *>(at(adm2_at)),
+            reinterpret_cast<dev::SweepClass *>(at(list2_at)), reinterpret_cast<dev::SweepClass *>(at(listq_at)),
+            reinterpret_cast<int *>(at(count2_at)), reinterpret_cast<int *>(at(countq_at)));
+        check_cuda(cudaGetLastError(), "class_list_kernel launch");
         check_cuda(cudaEventRecord(e1, stream), "cudaEventRecord");
         check_cuda(cudaEventSynchronize(e1), "class table build");
         float ms = 0;
@@ -1034,74 +736,93 @@ struct Sieve::Impl {
         timings.table_ms += ms;
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        cudaFree(d_aff);
-        cudaFree(d_inv);
-        cudaFree(d_specs);
-        cudaFree(d_pspecs);
-        cudaFree(d_patterns);
-        F.rows = fast_rows;
-        F.prime_rows = fast_rows;
-        F.admissible = fast_adm;
-        F.class_starts = fast_starts;
-        F.max_classes = fast_max_classes;
-        F.list_runs = list_runs;
-        F.list_count = list_count;
-        F.list_ipc = list_ipc;
-        fast_smem = fast_dynamic_smem(F.smem_words, fast_max_classes, fast_plan.row_slots);
-        const void *kernel = fast_kernel_ptr(F.slots, fast_plan.row_slots);
-        check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        int(fast_smem)),
+
+        T.nbad = int(bad_primes.size());
+        T.nlate = int(late.size());
+        T.two_mask = sweep.two - 1;
+        T.q = dev::u32(q);
+        T.q_magic = magic_of(q);
+        T.two_max = sweep.two_max;
+        T.q_max = sweep.q_max;
+        T.stride = S;
+        T.class_mod = int(M);
+        T.row_words = row_words;
+        T.slots = sweep.slots;
+        sweep_smem = std::size_t(sweep.slots) * std::size_t(sweep_slot_bytes(row_words, sweep.two_max, sweep.q_max)) +
+                     std::size_t(kSweepQueueBytes) * std::size_t(kSweepWarps / sweep.ctas - 1);
+        const void *kernel = kernel_ptr(int(sweep.moduli.size()), sweep.pairs);
+        check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sweep_smem)),
                    "cudaFuncSetAttribute");
         int sms = 0, per_sm = 0;
         check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device),
                    "cudaDeviceGetAttribute");
-        check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, dev::kFThreads,
-                                                                 fast_smem),
+        check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads_per_cta(), sweep_smem),
                    "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
         grid = std::max(1, sms * std::max(1, per_sm));
-        // Word dimension of a launch: class words (64 sites spaced M apart).
-        const long long sites = 2 * bound + 1;
-        words = (sites / M + 1 + 63) / 64;
-        max_tile = dev::kFMaxClassWords;
+        // queued positions stay below 2^46 and class words below 2^23
+        tile = S * std::min<long long>(1LL << 23, (1LL << 45) / S);
         timings.table_wall_ms += ms_since(t0);
     }
 
-    static const void *fast_kernel_ptr(int rows, int slots) {
-        switch (rows * 4 + slots) {
-#define RPG_FAST_PTR(n)                                                                       \
-    case n * 4 + 2: return reinterpret_cast<const void *>(&dev::fast_sieve_kernel<n, 2>);   \
-    case n * 4 + 3: return reinterpret_cast<const void *>(&dev::fast_sieve_kernel<n, 3>);
+    int threads_per_cta() const { return kSweepWarps / sweep.ctas * dev::kWarpSize; }
+
+    static const void *kernel_ptr(int rows, int pairs) {
+        switch (2 * rows + pairs) {
+#define RPG_FAST_PTR(n)                                                                     \
+    case 2 * n + 1: return reinterpret_cast<const void *>(&dev::fast_sieve_kernel<n, 1>);   \
+    case 2 * n + 2: return reinterpret_cast<const void *>(&dev::fast_sieve_kernel<n, 2>);
         RPG_FAST_PTR(1) RPG_FAST_PTR(2) RPG_FAST_PTR(3) RPG_FAST_PTR(4) RPG_FAST_PTR(5) RPG_FAST_PTR(6)
         RPG_FAST_PTR(7) RPG_FAST_PTR(8) RPG_FAST_PTR(9) RPG_FAST_PTR(10) RPG_FAST_PTR(11) RPG_FAST_PTR(12)
 #undef RPG_FAST_PTR
-        default: throw std::logic_error("no fast kernel for this row and slot count");
+        default: throw std::logic_error("no sieve kernel for this row count");
         }
     }
 
-    void launch_fast(const dev::FastTables &Fl, const dev::SieveArgs &A, unsigned long long *work,
-                     cudaStream_t st) const {
-        const int blocks = int(std::min<long long>(grid, (A.k_count + dev::kFChunk - 1) / dev::kFChunk));
-        const void *kernel = fast_kernel_ptr(Fl.slots, fast_plan.row_slots);
-        void *params[] = {const_cast<dev::FastTables *>(&Fl), const_cast<dev::SieveArgs *>(&A), &work};
-        check_cuda(cudaLaunchKernel(kernel, dim3(unsigned(blocks)), dim3(dev::kFThreads), params, fast_smem, st),
-                   "fast sieve kernel launch");
-    }
-
-    dev::SieveArgs args(int which, long long first, long long last, long long w_lo, long long w_hi) {
-        dev::SieveArgs A{};
-        A.bound = bound;
-        A.words = words;
-        A.w_lo = w_lo;
-        A.w_hi = w_hi;
+    // One launch: parameters first .. last, numerators a_lo .. a_hi (at most
+    // `tile` of them), survivors into the given arrays.
+    void launch_sweep(long long first, long long last, long long a_lo, long long a_hi, long long *out_a, int *out_d,
+                      unsigned long long capacity, unsigned long long *out_count, unsigned long long *work,
+                      unsigned long long *error, cudaStream_t st) const {
+        const long long M = T.class_mod, S = T.stride;
+        const long long w_lo = (a_lo + bound) / S;
+        dev::SweepArgs A{};
+        A.abase = -bound - M + S * w_lo;
+        A.a_lo = a_lo;
+        A.a_hi = a_hi;
         A.k_first = first;
         A.k_count = int(last - first + 1);
+        // Few denominators with much to sweep are split into shares of their
+        // items, so that every CTA gets several (the tail of a launch is at
+        // most one of them per CTA), while a share stays well above the copy
+        // of its rows.  A fetch takes work worth about 2^15 cycles.
+        double cost = sweep.cost * (double(a_hi) - double(a_lo) + 1.0) / (2.0 * double(bound) + 1.0);
+        A.part_shift = 0;
+        while (A.part_shift < 6 && (A.k_count << A.part_shift) < 32 * grid && cost > 40000.0) {
+            ++A.part_shift;
+            cost *= 0.5;
+        }
+        const long long shares = (long long)A.k_count << A.part_shift;
+        A.chunk = int(std::max<long long>(1, std::min<long long>({dev::kFChunk, shares / (4LL * grid),
+                                                                  (long long)(32768.0 / cost)})));
         A.square = opt.square ? 1 : 0;
-        A.out_a = buf[which].a;
-        A.out_d = buf[which].d;
-        A.out_count = buf[which].count;
-        A.capacity = (unsigned long long)buf[which].cap;
-        A.error = buf[which].count + 2;
-        return A;
+        const long long words = ((a_hi - A.abase) / M >> 6) + 1;
+        A.segs = int((words + kSweepUnit - 1) / kSweepUnit);
+        A.shifted = w_lo != 0;
+        A.split = A.segs > 64 ? 0 : sweep.split;
+        A.out_a = out_a;
+        A.out_d = out_d;
+        A.out_count = out_count;
+        A.capacity = capacity;
+        A.error = error;
+        dev::SweepTables Tl = T;
+        Tl.segs_magic = A.segs == 1 ? 0 : (~0ull) / (unsigned long long)A.segs + 1;
+        for (std::size_t r = 0; r < sweep.moduli.size(); ++r) Tl.row[r].wlo = dev::u32(w_lo % sweep.moduli[r]);
+        for (auto &P : Tl.prime) P.base_mod = dev::u32(((A.abase % P.p) + P.p) % P.p);
+        const int blocks = int(std::min<long long>(grid, (shares + A.chunk - 1) / A.chunk));
+        void *params[] = {&Tl, &A, &work};
+        check_cuda(cudaLaunchKernel(kernel_ptr(int(sweep.moduli.size()), sweep.pairs), dim3(unsigned(blocks)), dim3(unsigned(threads_per_cta())),
+                                    params, sweep_smem, st),
+                   "sieve kernel launch");
     }
 
     cudaStream_t launch_stream(int which) const { return which ? stream2 : stream; }
@@ -1109,43 +830,27 @@ struct Sieve::Impl {
     // Counting pass: survivors accumulate in buffer 0's counter across
     // launches; launch i runs on launch stream i mod 2 with that buffer's
     // work counter.
-    void launch_counting(int which, long long first, long long last, long long w_lo, long long w_hi) {
-        const dev::SieveArgs A = args(0, first, last, w_lo, w_hi);
+    void launch_counting(int which, long long first, long long last, long long a_lo, long long a_hi) {
         const cudaStream_t st = launch_stream(which);
         check_cuda(cudaMemsetAsync(buf[which].count + 1, 0, sizeof(unsigned long long), st),
                    "cudaMemsetAsync");
-        launch_kernel(A, buf[which].count + 1, st);
+        launch_sweep(first, last, a_lo, a_hi, buf[0].a, buf[0].d, (unsigned long long)buf[0].cap, buf[0].count,
+                     buf[which].count + 1, buf[0].count + 2, st);
         ++timings.launches;
     }
 
-    void launch_kernel(const dev::SieveArgs &A, unsigned long long *work, cudaStream_t st) {
-        if (opt.plan == PlanKind::fast) {
-            dev::FastTables Fl = F;
-            for (int i = 0; i < kCandidatePrimes; ++i)
-                Fl.prime[i].wlo_mod = dev::u32(A.w_lo % Fl.prime[i].p);
-            for (int i = 0; i < Fl.slots; ++i) Fl.mod[i].wlo_mod = dev::u32(A.w_lo % Fl.mod[i].m);
-            if (A.w_lo != 0 || A.w_hi < list_words) {  // part of the class rows: the producer lays them out
-                Fl.list_runs = nullptr;
-                Fl.list_count = nullptr;
-            }
-            launch_fast(Fl, A, work, st);
-        } else {
-            const int blocks = int(std::min<long long>(grid, A.k_count));
-            dev::ref_sieve_kernel<<<blocks, dev::kThreads, dev::kRefSmem, st>>>(T, A);
-        }
-        check_cuda(cudaGetLastError(), "sieve kernel launch");
-    }
+    bool one_launch() const { return 2 * bound + 1 <= tile; }
 
-    void launch(int which, long long first, long long last, long long w_lo, long long w_hi) {
+    void launch(int which, long long first, long long last, long long a_lo, long long a_hi) {
         Buffer &b = buf[which];
         b.first = first;
         b.last = last;
         b.busy = true;
-        const dev::SieveArgs A = args(which, first, last, w_lo, w_hi);
         const cudaStream_t st = launch_stream(which);
         check_cuda(cudaMemsetAsync(b.count, 0, 4 * sizeof(unsigned long long), st), "cudaMemsetAsync");
         check_cuda(cudaEventRecord(b.begin, st), "cudaEventRecord");
-        launch_kernel(A, b.count + 1, st);
+        launch_sweep(first, last, a_lo, a_hi, b.a, b.d, (unsigned long long)b.cap, b.count, b.count + 1, b.count + 2,
+                     st);
         if (opt.preverify) {
             preverifier.launch(b.a, b.d, nullptr, b.count, (unsigned long long)b.cap, b.pa, b.pd, nullptr,
                                b.count + 3, nullptr, st);
@@ -1164,16 +869,16 @@ struct Sieve::Impl {
     }
 
     // Launch queued batches into free buffers (pipelined path, rows that fit
-    // one launch).  Rows longer than kMaxTileWords go through pieces instead.
+    // one launch).  Rows of more than `tile` numerators go through pieces instead.
     void refill() {
-        if (words > max_tile || !pieces.empty()) return;
+        if (!one_launch() || !pieces.empty()) return;
         while (order.size() < 2 && q_next <= q_last) {
             const int which = buf[0].busy ? 1 : 0;
             if (buf[which].busy) break;
             const long long first = q_next;
             const long long last = std::min(q_last, first + q_batch - 1);
             q_next = last + 1;
-            launch(which, first, last, 0, words);
+            launch(which, first, last, -bound, bound);
             order.push_back(which);
         }
     }
@@ -1262,24 +967,28 @@ struct Sieve::Impl {
         return true;
     }
 
-    // Queue a batch as pieces: word tiles of at most kMaxTileWords.
+    // Queue a batch as pieces of at most `tile` numerators.
     void queue_pieces(long long first, long long last) {
         piece_batch_first = first;
         piece_batch_last = last;
-        for (long long w = 0; w < words; w += max_tile)
-            pieces.push_back(Piece{first, last, w, std::min(words, w + max_tile)});
+        for (long long a = -bound;; a += tile) {
+            const bool end = bound - a < tile;  // no overflow near the largest bounds
+            pieces.push_back(Piece{first, last, a, end ? bound : a + tile - 1});
+            if (end) break;
+        }
     }
 
-    // Split a piece into two halves (by parameter, else by word range).
+    // Split a piece into two halves (by parameter, else by numerator range,
+    // down to the 64 numerators that the smallest buffer holds).
     void split_front(const Piece &p) {
         if (p.last > p.first) {
             const long long mid = p.first + (p.last - p.first) / 2;
-            pieces.push_front(Piece{mid + 1, p.last, p.w_lo, p.w_hi});
-            pieces.push_front(Piece{p.first, mid, p.w_lo, p.w_hi});
-        } else if (p.w_hi - p.w_lo > 1) {
-            const long long mid = p.w_lo + (p.w_hi - p.w_lo) / 2;
-            pieces.push_front(Piece{p.first, p.last, mid, p.w_hi});
-            pieces.push_front(Piece{p.first, p.last, p.w_lo, mid});
+            pieces.push_front(Piece{mid + 1, p.last, p.a_lo, p.a_hi});
+            pieces.push_front(Piece{p.first, mid, p.a_lo, p.a_hi});
+        } else if (p.a_hi - p.a_lo >= 64) {
+            const long long mid = p.a_lo + (p.a_hi - p.a_lo) / 2;
+            pieces.push_front(Piece{p.first, p.last, mid + 1, p.a_hi});
+            pieces.push_front(Piece{p.first, p.last, p.a_lo, mid});
         } else {
             throw std::logic_error("survivor buffer cannot hold one word of survivors");
         }
@@ -1292,7 +1001,7 @@ struct Sieve::Impl {
             pieces.pop_front();
             const int which = buf[0].busy ? 1 : 0;
             if (buf[which].busy) throw std::logic_error("no free survivor buffer");
-            launch(which, p.first, p.last, p.w_lo, p.w_hi);
+            launch(which, p.first, p.last, p.a_lo, p.a_hi);
             check_cuda(cudaEventSynchronize(buf[which].copied), "sieve kernel");
             buf[which].busy = false;
             // the counter words came back with the launch: [2] is its error word
@@ -1315,7 +1024,7 @@ struct Sieve::Impl {
 
     bool next(BatchView &out) {
         if (!pieces.empty()) return next_piece(out);
-        if (order.empty() && words > max_tile && q_next <= q_last) {
+        if (order.empty() && !one_launch() && q_next <= q_last) {
             const long long first = q_next;
             const long long last = std::min(q_last, first + q_batch - 1);
             q_next = last + 1;
@@ -1340,8 +1049,8 @@ struct Sieve::Impl {
             b.busy = false;
             piece_batch_first = b.first;
             piece_batch_last = b.last;
-            if (grow(which, n)) pieces.push_front(Piece{b.first, b.last, 0, words});
-            else split_front(Piece{b.first, b.last, 0, words});
+            if (grow(which, n)) pieces.push_front(Piece{b.first, b.last, -bound, bound});
+            else split_front(Piece{b.first, b.last, -bound, bound});
             return next_piece(out);
         }
         deliver(out, which, std::size_t(n), std::size_t(counts[3]), ms, b.first, b.last, true);
@@ -1360,7 +1069,6 @@ Sieve::Sieve(const std::vector<std::string> &coefficients, long long bound,
         throw std::invalid_argument("numerator bound too large for the fast plan (at most 2^45)");
     impl_->opt = options;
     impl_->bound = bound;
-    impl_->words = word_count64(bound);
     try {
         impl_->init(coefficients);
     } catch (...) {
@@ -1435,17 +1143,14 @@ const SieveTimings &Sieve::timings() const { return impl_->timings; }
 unsigned long long Sieve::swept_words(long long first, long long last) const {
     const auto &I = *impl_;
     if (last < first) return 0;
-    if (I.opt.plan != PlanKind::fast) return (unsigned long long)(last - first + 1) * I.words;
-    // Denominators per residue mod M, then the words of each admissible class.
-    const int q = I.F.class_prime;
-    const long long M = I.F.class_mod;
-    std::vector<unsigned long long> per_residue(M, 0);
-    if (I.fast_bad_primes.empty()) {
+    // Parameters per residue mod M, then the classes of each residue.
+    const long long M = I.T.class_mod;
+    std::vector<unsigned long long> per_residue(std::size_t(M), 0);
+    auto residue = [&](long long k) { return I.opt.square ? (k % M) * (k % M) % M : k % M; };
+    if (I.bad_primes.empty()) {
         for (long long t = 0; t < M; ++t) {
             const long long lo = first + ((t - first % M) % M + M) % M;  // first k >= first, k = t (mod M)
-            const unsigned long long n = lo > last ? 0 : (unsigned long long)((last - lo) / M + 1);
-            const long long dres = I.opt.square ? (t * t) % M : t;
-            per_residue[dres] += n;
+            if (lo <= last) per_residue[std::size_t(residue(t))] += (unsigned long long)((last - lo) / M + 1);
         }
     } else {
         // parameters k without a denominator prime factor, by segments
@@ -1454,32 +1159,20 @@ unsigned long long Sieve::swept_words(long long first, long long last) const {
         for (long long lo = first; lo <= last; lo += kSegment) {
             const long long hi = std::min(last, lo + kSegment - 1);
             skip.assign(std::size_t(hi - lo + 1), 0);
-            for (int p : I.fast_bad_primes)
+            for (int p : I.bad_primes)
                 for (long long k = lo + ((p - lo % p) % p); k <= hi; k += p) skip[std::size_t(k - lo)] = 1;
-            for (long long k = lo; k <= hi; ++k) {
-                if (skip[std::size_t(k - lo)]) continue;
-                const long long t = k % M;
-                per_residue[I.opt.square ? (t * t) % M : t] += 1;
-            }
+            for (long long k = lo; k <= hi; ++k)
+                if (!skip[std::size_t(k - lo)]) per_residue[std::size_t(residue(k))] += 1;
         }
     }
-    const long long sites = 2 * I.bound + 1;
     unsigned long long total = 0;
-    for (long long dres = 0; dres < M; ++dres) {
-        if (!per_residue[dres]) continue;
-        const dev::u64 c2 = I.fast_adm_host[dres % 64];
-        const dev::u64 cq = q > 1 ? I.fast_adm_host[64 + dres % q] : 1;
-        unsigned long long words = 0;
-        for (int r = 0; r < M; ++r) {
-            if (!((c2 >> (r % 64)) & 1)) continue;
-            if (q > 1 && !((cq >> (r % q)) & 1)) continue;
-            const long long ofs = (r + I.bound % M) % M;
-            const long long count = ofs < sites ? (sites - 1 - ofs) / M + 1 : 0;
-            words += (unsigned long long)((count + 63) / 64);
-        }
-        total += per_residue[dres] * words;
+    for (long long r = 0; r < M; ++r) {
+        unsigned long long classes = (unsigned long long)I.count2_host[std::size_t(r % I.sweep.two)];
+        for (std::size_t i = 0; i < I.countq_host.size(); ++i)
+            classes *= (unsigned long long)I.countq_host[i][std::size_t(r % I.sweep.class_primes[i])];
+        total += per_residue[std::size_t(r)] * classes;
     }
-    return total;
+    return total * (unsigned long long)sweep_words(I.bound, M);
 }
 
 FastPlanInfo Sieve::fast_plan_info() const {
@@ -1494,41 +1187,29 @@ FastPlanInfo Sieve::fast_plan_info() const {
 
 int Sieve::device() const { return impl_->device; }
 
-bool Sieve::fits_one_launch() const { return impl_->words <= impl_->max_tile; }
+// The limits of an allocation-free launch are those of the interface (2^23
+// words of a class mod 64 q under the fast plan, 2^30 words of consecutive
+// numerators under the reference plan); the kernel's tile is never smaller.
+bool Sieve::fits_one_launch() const {
+    const long long sites = 2 * impl_->bound + 1;
+    if (impl_->opt.plan == PlanKind::fast) {
+        const long long words = (sites / (64LL * impl_->fast_plan.class_prime) + 1 + 63) / 64;
+        return words <= (1LL << 23) && impl_->one_launch();
+    }
+    return word_count64(impl_->bound) <= (1LL << 30) && impl_->one_launch();
+}
 
 bool Sieve::launch_into(long long first, long long last, long long *out_a, int *out_d,
                         unsigned long long capacity, unsigned long long *out_count,
                         unsigned long long *work, unsigned long long *error, cudaStream_t stream) {
     const auto &I = *impl_;
     if (!fits_one_launch() || last < first || last - first + 1 > (1 << 16)) return false;
-    dev::SieveArgs A{};
-    A.bound = I.bound;
-    A.words = I.words;
-    A.w_lo = 0;
-    A.w_hi = I.words;
-    A.k_first = first;
-    A.k_count = int(last - first + 1);
-    A.square = I.opt.square ? 1 : 0;
-    A.out_a = out_a;
-    A.out_d = out_d;
-    A.out_count = out_count;
-    A.capacity = capacity;
-    A.error = error;  // a bounded wait that gives up sets it
-    if (I.opt.plan == PlanKind::fast) {
-        I.launch_fast(I.F, A, work, stream);
-    } else {
-        const int blocks = int(std::min<long long>(I.grid, A.k_count));
-        dev::ref_sieve_kernel<<<blocks, dev::kThreads, dev::kRefSmem, stream>>>(I.T, A);
-    }
-    check_cuda(cudaGetLastError(), "sieve kernel launch");
+    I.launch_sweep(first, last, -I.bound, I.bound, out_a, out_d, capacity, out_count, work, error, stream);
     return true;
 }
 
-unsigned Sieve::smem_bytes_per_word() const {
-    return impl_->opt.plan == PlanKind::fast ? unsigned(8 * impl_->F.slots)
-                                             : unsigned(8 * dev::kRefFast);
-}
-long long Sieve::words64() const { return impl_->words; }
+unsigned Sieve::smem_bytes_per_word() const { return unsigned(8 * impl_->sweep.moduli.size()); }
+long long Sieve::words64() const { return sweep_words(impl_->bound, impl_->T.class_mod); }
 cudaStream_t Sieve::stream() const { return impl_->stream; }
 
 unsigned long long Sieve::count_only(long long first, long long last, long long batch_size) {
@@ -1546,8 +1227,12 @@ unsigned long long Sieve::count_only(long long first, long long last, long long 
     int which = 0;
     for (long long f = first; f <= last; f += batch_size) {
         const long long l = std::min(last, f + batch_size - 1);
-        for (long long w = 0; w < I.words; w += I.max_tile, which ^= 1)
-            I.launch_counting(which, f, l, w, std::min(I.words, w + I.max_tile));
+        for (long long a = -I.bound;; a += I.tile, which ^= 1) {
+            const bool end = I.bound - a < I.tile;
+            I.launch_counting(which, f, l, a, end ? I.bound : a + I.tile - 1);
+            if (end) break;
+        }
+        which ^= 1;
     }
     check_cuda(cudaEventRecord(I.join_event, I.stream2), "cudaEventRecord");
     check_cuda(cudaStreamWaitEvent(I.stream, I.join_event, 0), "cudaStreamWaitEvent");

@@ -1,9 +1,4 @@
 // Device-side pieces of the modular square sieve shared by the sieve kernels.
-//
-// Site layout: for a search bound H, the numerators a in [-H, H] of one
-// denominator d form a row of 64-site words; word w holds a = -H + 64 w + j in
-// bit j.  The reference uses 32-site words (src/sieve.cu:179-181); the site set
-// and the survivor set are the same.
 #pragma once
 
 #include <cstdint>
@@ -16,24 +11,6 @@ using u64 = std::uint64_t;
 
 constexpr int kWarpSize = 32;
 constexpr unsigned kFullMask = 0xffffffffu;
-
-// Arguments of one sieve launch: parameters k_first .. k_first + k_count - 1
-// (denominators k, or k*k when square), word range [w_lo, w_hi) of each row,
-// and the survivor output (structure of arrays, capacity entries).
-struct SieveArgs {
-    long long bound;     // H
-    long long words;     // words per denominator row (64-site words)
-    long long w_lo;
-    long long w_hi;
-    long long k_first;
-    int k_count;
-    int square;
-    long long *out_a;
-    int *out_d;
-    unsigned long long *out_count;
-    unsigned long long capacity;
-    unsigned long long *error;   // set nonzero if a bounded device wait ran out (may be null)
-};
 
 // Quotient estimate for n mod p with n < 2^31 and 257 <= p < 2^9 (the
 // reference's candidate primes): q = (n * ceil(2^40 / p)) >> 40 is exact in
@@ -134,40 +111,6 @@ __device__ __forceinline__ u32 lanemask_lt() {
     u32 m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
-}
-
-// Warp-wide emission of surviving sites.  Every lane of the warp calls this
-// with its word index and final mask (0 if none).  One atomicAdd per warp
-// reserves output slots; slots past capacity are counted but not written, so
-// the host sees count > capacity and re-runs the work in smaller pieces.
-__device__ __forceinline__ void emit_survivors(u64 mask, long long word, long long bound,
-                                               int denominator, long long *out_a, int *out_d,
-                                               unsigned long long *out_count,
-                                               unsigned long long capacity) {
-    const int lane = threadIdx.x & 31;
-    u32 n = __popcll(mask);
-    if (!__any_sync(kFullMask, n != 0)) return;
-    u32 incl = n;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        u32 v = __shfl_up_sync(kFullMask, incl, off);
-        if (lane >= off) incl += v;
-    }
-    u32 total = __shfl_sync(kFullMask, incl, 31);
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(out_count, (unsigned long long)total);
-    base = __shfl_sync(kFullMask, base, 0);
-    unsigned long long pos = base + incl - n;
-    long long a0 = -bound + 64 * word;
-    while (mask) {
-        int bit = __ffsll((long long)mask) - 1;
-        mask &= mask - 1;
-        if (pos < capacity) {
-            out_a[pos] = a0 + bit;
-            out_d[pos] = denominator;
-        }
-        ++pos;
-    }
 }
 
 }  // namespace dev

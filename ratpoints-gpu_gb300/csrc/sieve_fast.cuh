@@ -1,141 +1,123 @@
-// Fast-plan sieve kernels (this project's plan; see plan.hpp).
+// The single-curve sieve kernel and its tables (reference and fast plan; see
+// plan.hpp for what survives, sweep_plan.hpp for how the tests are split).
 //
-// Class-strided layout.  For a denominator d only some numerator classes
-// a = r (mod M) can hold points, M = 64 * q with q the curve's class prime
-// (q = 1: M = 64):
-//   - r mod 64 must make F(r, d) a square mod 64 (and r odd when d is even);
-//   - r mod q must make f(r/d) a square mod q, or, when q | d, be nonzero
-//     (gcd) with c_n a square mod q for even degree.
-// Each admissible class is swept on its own: word w of class r holds the 64
-// sites a = a0 + S w + M j (j = bit, S = 64 M), a0 the least a >= -H in the
-// class.  For an odd modulus m prime to M, S is invertible mod m, so the mask
-// of m is periodic in w with period m and one table row per (m, d mod m)
-// serves every class: class r starts at row index a0 * S^-1 (mod m).  Tables
-// therefore do not depend on H.
+// Class layout.  With M = two * Q (Q the product of the class primes), a
+// denominator d sweeps only the numerator classes a = r (mod M) whose
+// residues are admissible: r mod two by d mod two (the 2-adic filter of the
+// fast plan, every residue otherwise), r mod Q by d mod Q.  A class holds the
+// sites a = a0 + M t; word w of it covers t = 64 w .. 64 w + 63, so words are
+// S = 64 M apart.  S is invertible modulo a stage-1 modulus m (odd, prime to
+// Q), so m's mask is periodic in w with period m and one table row per
+// (m, d mod m) serves every class: word w of the class of a0 is row word
+// a0 S^-1 + w (mod m).  Tables do not depend on H.
 //
-// Stage 1 ANDs the rows of NS composite moduli of small primes (chosen per
-// curve), staged in shared memory per denominator; surviving words go through
-// a per-warp queue to stage 2, which checks the reference's 32 selected
-// primes (same selection as the reference plan: the 32 largest of its 36
-// candidates that do not divide d) from class-layout tables in global memory,
-// then emits (a, d).  Survivors are a subset of the reference plan's.
-//
-// Warp-specialized pipeline: warp 0 produces denominators (prime selection,
-// class layout from the per-curve class-start table, TMA copies of the rows)
-// into one of two slots; the other warps consume a slot's sweep items once
-// its full barrier completes and release it through its empty barrier, so a
-// slot is refilled while the other is swept and no barrier spans the CTA.
+// A class is a pair: residue r2 mod two and residue rq mod Q.  Its a0 is
+// abase + x2 + xq with x2, xq in [0, M) the CRT lifts (abase = -H - M for a
+// whole row), so its row index is the sum of one term per residue, and the
+// terms are few enough to be tabled once per search.  x2 + xq is not reduced modulo M: a class may start a step
+// before the numerator range, and ends up to a step after it; emission drops
+// those sites, the sweep needs no masks.
 #pragma once
 
 #include "plan.hpp"
 #include "sieve_device.cuh"
+#include "sweep_plan.hpp"
 
 namespace rpg {
 namespace dev {
 
-constexpr int kFastSlots = kMaxFastSlots;  // stage-1 moduli (at most)
-constexpr int kFastMaxFactors = 4;         // primes per stage-1 modulus
-constexpr int kFK = 4;                     // words per lane per step (lanes 32 apart)
-constexpr int kFWarps = 12;                // warp 0 produces, the others sweep
-constexpr int kFThreads = kFWarps * kWarpSize;
-constexpr int kFConsumers = kFWarps - 1;
-constexpr int kFMaxSlotCount = 3;                          // denominators in flight per CTA: 2 or 3
-constexpr int kFChunk = 16;                                // parameters per producer fetch (one per lane)
-constexpr int kFSteps = 4;                                 // steps per work item
-constexpr int kFItemWords = kWarpSize * kFK * kFSteps;     // 512 words per item
-constexpr int kFExt = kWarpSize * (kFK - 1);               // row extension
-constexpr int kFQueue = 64;
-constexpr int kFStage2Group = 6;                           // stage-2 primes loaded together
-constexpr long long kFMaxClassWords = 1LL << 23;           // class words of a launch's tile (24-bit field)
-constexpr int kFAdmQ = 16;                                 // admissible-residue words for q <= 13
-constexpr int kFBadBase = 64 + kFAdmQ;                     // first denominator-prime word of admissible
+constexpr int kOddPrimes = 96;             // odd primes below 512
+constexpr int kFThreads = 12 * kWarpSize;  // largest CTA: warp 0 produces, the others sweep
+constexpr int kFChunk = kWarpSize;         // work units per producer fetch (at most; one per lane)
+constexpr int kFQueue = kSweepQueue;
+constexpr int kFStage2Group = 6;           // stage-2 primes loaded together
+constexpr int kFSegTable = 64;             // units of a class whose row offsets are tabled in shared memory
+static_assert(kSweepQueueBytes == kFQueue * 20, "the planner budgets the kernel's queues");
 
+// Arguments of one launch: parameters k_first .. k_first + k_count - 1
+// (denominators k, or k * k when square), numerators a_lo .. a_hi, and the
+// survivor output (structure of arrays, capacity entries).
+struct SweepArgs {
+    long long abase;     // a = abase + x2 + xq + S w + M j
+    long long a_lo, a_hi;
+    long long k_first;
+    int k_count;
+    int chunk;           // work units per producer fetch
+    int part_shift;      // a denominator is 2^part_shift work units, each a share of its items
+    int square;
+    int segs;            // units of 16 words per class
+    int shifted;         // the first class word is not word 0: row offsets take wlo
+    int split;           // a group of units is 2^split items, each a range of the residues mod two
+    long long *out_a;
+    int *out_d;
+    unsigned long long *out_count;
+    unsigned long long capacity;
+    unsigned long long *error;   // set nonzero if a bounded device wait ran out (may be null)
+};
 
-struct FastModulus {
-    int m;                         // modulus (odd, prime to the class modulus)
-    int nf;                        // number of prime factors
-    int q[kFastMaxFactors];        // prime factors
-    int length;                    // row length in words (m + kFExt, even)
+struct SweepRow {                  // one stage-1 modulus
     long long offset;              // word offset of row 0 in the table
-    int smem_offset;               // word offset of the staged row in shared memory
-    u32 inv_stride;                // (64 M)^-1 mod m
-    u32 neg_h;                     // (-H) mod m
-    u32 wlo_mod;                   // first word of the launch's tile, mod m
-    u32 step;                      // (32 * kFK) mod m: row advance per step
-    unsigned long long magic;      // ceil(2^64 / m) for 32-bit n mod m
-    u32 step8;                     // 8 step: byte advance of a lane's offset per step
-    u32 mod8;                      // 8 m
-    u32 soff8;                     // 8 smem_offset: byte offset of the staged row in a slot
-    u32 pad;
+    unsigned long long magic;      // mod_u32 constant
+    u32 m;                         // modulus (odd, prime to M)
+    u32 length;                    // staged words of a row (sweep_row_words)
+    u32 soff8;                     // byte offset of the row in a slot
+    u32 wlo;                       // the launch's first class word, mod m
 };
 
 struct FastPrime {                 // one of the 36 reference candidates, class layout
     long long offset;              // word offset of row 0 (rows of length p)
     int p;
-    u32 inv_stride;                // (64 M)^-1 mod p
-    u32 neg_h;                     // (-H) mod p
+    u32 inv_stride;                // S^-1 mod p; 0: a class prime, which every swept site passes
+    u32 base_mod;                  // abase mod p
     u32 magic;                     // magic40(p)
-    u32 wlo_mod;                   // first word of the launch's tile, mod p
 };
 
-// Per class residue r mod M: the row index of class word 0 for each modulus,
-// (a0 S^-1) mod m with a0 = -H + ofs, and ofs = (r + H) mod M.
-struct FastClassStart {
-    unsigned short start[kFastSlots];
-    unsigned short ofs;
-    unsigned short pad[3];
+struct LatePrime {                 // a prime of the plan tested after stage 2
+    long long offset;              // word offset of row 0 (rows of length p)
+    u32 p;
+    u32 inv_stride;
 };
-static_assert(sizeof(FastClassStart) == 32, "two 16-byte loads per class");
-static_assert(kFExt == kFastRowExtension, "the planner sizes rows with the kernel's extension");
 
-struct FastRun;
+// Entry of the lists by d mod two and by d mod Q: one admissible residue, its
+// CRT lift x and its term of the row index of each modulus, in bytes
+// (8 (x S^-1 mod m); by d mod Q with -H - M: 8 ((x - H - M) S^-1 mod m)).
+struct SweepClass {
+    unsigned short start8[kSweepRows];
+    u32 x;
+    u32 pad;
+};
+static_assert(sizeof(SweepClass) == kSweepListBytes, "class lists are copied by TMA");
+static_assert(kMaxModulus * 8 < 65536, "row offsets fit 16 bits");
 
-struct FastTables {
-    const FastClassStart *class_starts;  // [M]
-    int max_classes;               // most admissible classes of any denominator
-    // Class lists by denominator class k = (d mod 64) q + (d mod q), for
-    // launches over whole class rows (null otherwise): list_count[k] classes
-    // and their runs list_runs[k max_classes ..], copied into a slot with its
-    // rows.  A denominator's classes
-    // depend on k alone, so the producer looks them up instead of laying them
-    // out.  Every class of a whole row has list_ipc sweep items (its words
-    // differ from another class's by at most one, and a class with fewer
-    // words finds nothing to sweep in its last item), so item i of a list is
-    // item i mod list_ipc of class i / list_ipc.
-    const FastRun *list_runs;
-    const int *list_count;
-    int list_ipc;
-    const u64 *rows;               // stage-1 modulus tables
-    const u64 *prime_rows;         // reference candidate tables (class layout)
-    const u64 *admissible;         // [64] 2-adic classes by d mod 64, then [kFAdmQ] residues by d mod q,
-                                   // then nbad pairs (p, ceil(2^64 / p)): the denominator primes
-    int nbad;                      // denominator primes: p < 512, p != q, c_n not a square mod p (even degree)
-    int class_prime;               // q (1: none)
-    int class_mod;                 // M = 64 q
-    int h_mod_m;                   // H mod M
-    int inv64_q;                   // 64^-1 mod q (CRT), 0 when q = 1
-    long long stride;              // S = 64 M: numerator step between words of a class
-    long long count_q;             // 2H = count_q * M + count_r: a class with offset
-    int count_r;                   //   ofs <= count_r holds count_q + 1 sites, else count_q
-    unsigned char crt[13 * 13];    // [r64 mod q][rq] -> t with r = r64 + 64 t (mod 64 q)
-    unsigned char mod_q[64];       // r64 mod q
-    FastModulus mod[kFastSlots];
+struct SweepTables {
+    const SweepClass *listq;       // [Q][q_max]
+    const SweepClass *list2;       // [two][two_max]
+    const int *count2;             // [two]
+    const int *countq;             // [Q]
+    const u64 *rows;               // stage-1, candidate and late-prime tables
+    const LatePrime *late;
+    int nbad, nlate;
+    int two_mask;                  // two - 1
+    u32 q;                         // Q
+    unsigned long long q_magic;    // mod_u32 constant of Q
+    unsigned long long segs_magic; // ceil(2^64 / segs)
+    int two_max, q_max;
+    long long stride;              // S = 64 M
+    int class_mod;                 // M
+    int row_words;                 // staged row words of a slot
+    int slots;
+    SweepRow row[kSweepRows];
     FastPrime prime[kCandidatePrimes];
-    int slots;                     // stage-1 moduli in use
-    int smem_words;                // staged row words
-    int min_modulus;               // smallest stage-1 modulus
+    // denominator primes: p | k iff k x <= y (mod 2^32), x = p^-1 mod 2^32 and
+    // y = floor((2^32 - 1) / p)
+    uint2 bad[kOddPrimes];
 };
-
-// Position of the n-th set bit (n counted from 0) of a 64-bit mask.
-__device__ __forceinline__ int nth_set_bit(u64 mask, int n) {
-    for (int i = 0; i < n; ++i) mask &= mask - 1;
-    return __ffsll((long long)mask) - 1;
-}
 
 // One test of one site class for prime q: rho = d mod q, x = a mod q.
 __device__ __forceinline__ bool prime_bit(const unsigned char *affine, const unsigned short *inverse,
                                           int q, int rho, int lead_ok, int x) {
-    if (rho == 0) return x != 0 && lead_ok;  // q | d: need q !| a, and c_n square mod q (even n)
+    // q | d: need q !| a, and c_n square mod q (even n); lead_ok 2: no test there
+    if (rho == 0) return lead_ok == 2 || (x != 0 && lead_ok);
     return affine[(x * inverse[rho]) % q] != 0;
 }
 
@@ -188,12 +170,12 @@ struct TableSpec {
     long long offset;
     int m;
     int nf;
-    int q[kFastMaxFactors];
+    int q[kSweepRowFactors];
     int length;
-    long long pattern[kFastMaxFactors];  // word offset of q's pattern row 0
-    int pattern_words[kFastMaxFactors];
-    int s_mod[kFastMaxFactors];          // S mod q
-    int step_inv[kFastMaxFactors];       // (M mod q)^-1 mod q
+    long long pattern[kSweepRowFactors];  // word offset of q's pattern row 0
+    int pattern_words[kSweepRowFactors];
+    int s_mod[kSweepRowFactors];          // S mod q
+    int step_inv[kSweepRowFactors];       // (M mod q)^-1 mod q
 };
 
 __global__ void class_table_kernel(u64 *rows, const TableSpec *specs, int nspecs, const u64 *patterns,
@@ -223,42 +205,79 @@ __global__ void class_table_kernel(u64 *rows, const TableSpec *specs, int nspecs
     rows[id] = word;
 }
 
-// One admissible class of the slot's denominator: its words inside the
-// launch's tile, where its last word is (or -1), and that word's valid bits.
-struct FastRun {
-    u32 words_last;                // words in the tile (bits 0..23), last word in the tile (bit 24),
-                                   // valid bits of the class's last word (bits 25..31, 1..64)
-    unsigned short ofs;            // (r + H) mod M
-    unsigned short start[kFastSlots];  // row index of the tile's first class word, per modulus
-    unsigned short pad;
+// The class lists: block b < Q writes the entries of denominators d = b
+// (mod Q), block Q + b those of d = b (mod two).  A residue r mod Q is
+// admissible if every class prime admits it: bit map adm[(d mod p) p +
+// r mod p]; a residue mod two if bit r of adm2[d mod two] is set.
+struct ClassListSpec {
+    int two, q, two_max, q_max, nprimes, nrows;
+    int p[kSweepClassPrimes];
+    int adm[kSweepClassPrimes];    // byte offset of the prime's map
+    u32 lift2, liftq;              // 1 mod two and 0 mod Q; 0 mod two and 1 mod Q (below M)
+    u32 h2, hq;                    // H mod two, H mod Q
+    u32 m[kSweepRows], inv_stride[kSweepRows], base[kSweepRows];  // base: (-H - M) mod m
 };
-static_assert(sizeof(FastRun) == 32, "packed class run");
+
+__global__ void __launch_bounds__(256) class_list_kernel(ClassListSpec S, const unsigned char *admq, const u64 *adm2,
+                                                         SweepClass *list2, SweepClass *listq, int *count2,
+                                                         int *countq) {
+    __shared__ int s_count[8];
+    __shared__ int s_base;
+    const bool second = int(blockIdx.x) >= S.q;
+    const int dres = second ? int(blockIdx.x) - S.q : int(blockIdx.x);
+    const int n = second ? S.two : S.q;
+    const int room = second ? S.two_max : S.q_max;
+    const u32 M = u32(S.two) * u32(S.q);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_base = 0;
+    __syncthreads();
+    for (int r0 = 0; r0 < n; r0 += 256) {
+        const int r = r0 + int(threadIdx.x);
+        bool ok = r < n;
+        if (second) {
+            ok = ok && ((adm2[dres] >> (r & 63)) & 1);
+        } else {
+            for (int i = 0; i < S.nprimes && ok; ++i)
+                ok = admq[S.adm[i] + (dres % S.p[i]) * S.p[i] + r % S.p[i]] != 0;
+        }
+        const u32 vote = __ballot_sync(kFullMask, ok);
+        if (lane == 0) s_count[warp] = __popc(vote);
+        __syncthreads();
+        int at = s_base + __popc(vote & lanemask_lt());
+        for (int w = 0; w < warp; ++w) at += s_count[w];
+        if (ok && at < room) {
+            SweepClass C{};
+            const u32 v = u32(r) + (second ? S.h2 : S.hq);
+            C.x = u32(u64(second ? S.lift2 : S.liftq) * (v % u32(n)) % M);
+            for (int i = 0; i < S.nrows; ++i) {
+                const u32 m = S.m[i];
+                C.start8[i] = (unsigned short)(8u * ((C.x + (second ? 0u : S.base[i])) % m * S.inv_stride[i] % m));
+            }
+            (second ? list2 : listq)[(long long)dres * room + at] = C;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 0; w < 8; ++w) s_base += s_count[w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) (second ? count2 : countq)[dres] = s_base;
+}
 
 // A denominator in flight: written by the producer warp, read by the others.
-// Its class runs and item prefix are its class list in global memory, or laid
-// out by the producer in dynamic shared memory (launches over part of the
-// class rows), sized by the plan's largest class count.
 struct FastSlot {
     long long d;                   // denominator; -1: no more work
-    const FastRun *runs;
-    const int *prefix;             // sweep-item prefix of laid-out classes (null for class lists)
-    int nclass;
-    int items;                     // sweep items of the denominator
+    int n2;                        // residues mod two
+    int units;                     // units of 16 class words: residues mod Q times segs
+    int first, items;              // sweep items of the work unit: first .. items - 1
     int rot;                       // items handed out in this CTA before these, mod the consumer count
+    const SweepClass *list;        // residues mod Q in global memory
 };
-
-// A consumer warp's queued words carry one of kFCtx context indices; the
-// context holds their denominator, so a slot can be refilled before those
-// words go through stage 2.  Sixteen contexts per warp let its queue fill up
-// across many denominators before it is drained.
-constexpr int kFCtx = 16;
-constexpr int kFTagShift = 56;             // context index in bits 56..59 of a queued position
 
 // One group of stage 2: candidates ci0, ci0-1, .., ci0-COUNT+1 (descending),
 // each tested on the words whose denominator it does not divide; ndiv counts
 // the candidates that divide it.  The group's table words are loaded together.
 template <int COUNT>
-__device__ __forceinline__ void fast_stage2_group(const FastTables &T, int ci0, u32 hi, u32 lo, u32 d,
+__device__ __forceinline__ void fast_stage2_group(const SweepTables &T, int ci0, u32 hi, u32 lo, u32 d,
                                                   u64 &m, int &ndiv) {
     u64 rows[COUNT];
     bool skip[COUNT];
@@ -269,40 +288,43 @@ __device__ __forceinline__ void fast_stage2_group(const FastTables &T, int ci0, 
         const u32 rho = mod_small(d, p, P.magic);
         u32 r = mod_small(hi, p, P.magic);
         r = mod_small((r << 16) | lo, p, P.magic);  // pos mod p
-        r += P.neg_h;                               // a mod p
+        r += P.base_mod;                            // a mod p
         if (r >= p) r -= p;
         const u32 u = mod_small(r * P.inv_stride, p, P.magic);
         skip[t] = rho == 0;
         ndiv += skip[t] ? 1 : 0;
-        rows[t] = __ldg(T.prime_rows + P.offset + (long long)rho * p + u);
+        rows[t] = ~u64(0);
+        if (m != 0 && P.inv_stride != 0) rows[t] = __ldg(T.rows + P.offset + (long long)rho * p + u);
     }
 #pragma unroll
     for (int t = 0; t < COUNT; ++t) m &= skip[t] ? ~u64(0) : rows[t];
 }
 
-// Stage 2 for up to 32 queued words (one per lane), then emission.  A queued
-// word carries its context (bits 56..59) and the position pos = a - (-H) of
-// its bit 0 (bits 0..55): its sites are a = -H + pos + M j, and the
-// class-layout row index of prime p is (a mod p) S^-1 mod p in row d mod p.
+// Stage 2 for up to 32 queued words (one per lane), then emission.  Its table
+// reads are uncoalesced, one L1 cycle per lane that asks: lanes whose word is
+// already empty do not (after six primes one word in sixty is left).  A queued
+// word carries its denominator and the position pos = a - abase of its bit 0:
+// its sites are a = abase + pos + M j, and the class-layout row index of prime
+// p is (a mod p) S^-1 mod p in row d mod p.
 // A word meets the reference's selection, the 32 largest of the 36
 // candidates that do not divide d: the 32 largest candidates (six at a time
 // in a loop that is not unrolled, which keeps the kernel's code compact; the
 // warp stops once its words are empty), skipping those dividing d, then, one
 // at a time and only for words where some of those divided d, the four
-// smallest until 32 have been tested.
-__device__ __forceinline__ void fast_drain(const u64 *qmask, const u64 *qpos, int start, int n,
-                                           const FastTables &T, const SieveArgs &A, const int *ctx_d) {
+// smallest until 32 have been tested.  The few words left meet the late
+// primes and drop the sites outside the launch's numerators.
+__device__ __forceinline__ void fast_drain(const u64 *qmask, const u64 *qpos, const u32 *qd, int start, int n,
+                                           const SweepTables &T, const SweepArgs &A) {
     const int lane = threadIdx.x & 31;
     u64 m = 0, pos = 0;
+    u32 d = 1;  // lanes past n hold no word: any denominator keeps their row indices in range
     if (lane < n) {
         m = qmask[start + lane];
         pos = qpos[start + lane];
+        d = qd[start + lane];
     }
     __syncwarp();
-    // lanes past n hold no word: any denominator keeps their row indices in range
-    const u32 d = lane < n ? u32(ctx_d[int(pos >> kFTagShift) & (kFCtx - 1)]) : 1u;
-    const u64 p56 = pos & ((u64(1) << kFTagShift) - 1);
-    const u32 hi = u32(p56 >> 16), lo = u32(p56 & 0xFFFF);
+    const u32 hi = u32(pos >> 16), lo = u32(pos & 0xFFFF);
     static_assert(kCandidatePrimes == 36 && kSelectedPrimes == 32, "stage-2 group schedule");
     int ndiv = 0;  // of the candidates tested so far, those dividing d
 #pragma unroll 1
@@ -323,14 +345,34 @@ __device__ __forceinline__ void fast_drain(const u64 *qmask, const u64 *qpos, in
         if (m != 0 && ndiv > 0 && rho != 0) {
             u32 r = mod_small(hi, p, P.magic);
             r = mod_small((r << 16) | lo, p, P.magic);
-            r += P.neg_h;
+            r += P.base_mod;
             if (r >= p) r -= p;
             const u32 u = mod_small(r * P.inv_stride, p, P.magic);
-            m &= __ldg(T.prime_rows + P.offset + (long long)rho * p + u);
+            if (P.inv_stride != 0) m &= __ldg(T.rows + P.offset + (long long)rho * p + u);
             --ndiv;  // one of the 32 taken by a smaller candidate
         }
     }
-    // emission: a = -H + pos + M j
+    if (!__any_sync(kFullMask, m != 0)) return;
+    const long long a0 = A.abase + (long long)pos;
+    const long long M = T.class_mod;
+    if (m) {
+        if (T.nlate) {
+            for (int l = 0; l < T.nlate && m; ++l) {
+                const LatePrime P = T.late[l];
+                long long r = a0 % (long long)P.p;
+                if (r < 0) r += P.p;
+                const u32 u = u32(r) * P.inv_stride % P.p;
+                m &= __ldg(T.rows + P.offset + (long long)(d % P.p) * P.p + u);
+            }
+        }
+        if (a0 < A.a_lo || a0 + 63 * M > A.a_hi) {  // ends of the numerator range
+            for (u64 rest = m; rest; rest &= rest - 1) {
+                const int j = __ffsll((long long)rest) - 1;
+                const long long a = a0 + M * j;
+                if (a < A.a_lo || a > A.a_hi) m &= ~(u64(1) << j);
+            }
+        }
+    }
     u32 cnt = __popcll(m);
     if (!__any_sync(kFullMask, cnt != 0)) return;
     u32 incl = cnt;
@@ -344,245 +386,191 @@ __device__ __forceinline__ void fast_drain(const u64 *qmask, const u64 *qpos, in
     if (lane == 0) base = atomicAdd(A.out_count, (unsigned long long)total);
     base = __shfl_sync(kFullMask, base, 0);
     unsigned long long at = base + incl - cnt;
-    const long long abase = -A.bound + (long long)p56;
     while (m) {
         const int bit = __ffsll((long long)m) - 1;
         m &= m - 1;
         if (at < A.capacity) {
-            A.out_a[at] = abase + (long long)T.class_mod * bit;
+            A.out_a[at] = a0 + M * bit;
             A.out_d[at] = int(d);
         }
         ++at;
     }
 }
 
-// Producer work for denominator d into slot S (the whole warp): the
-// admissible classes and their sweep items (a prefix scan, 32 classes per
-// pass) in shared memory.  Returns the item count.
-__device__ __forceinline__ int fast_setup(const FastTables &T, const SieveArgs &A, long long d,
-                                           FastSlot &S, FastRun *runs, int *prefix) {
-    const int lane = threadIdx.x & 31;
-    const u32 du = u32(d);
-    const int q = T.class_prime;
-    const int M = T.class_mod;
-    const u64 classes2 = __ldg(T.admissible + (du & 63));
-    const u64 classesq =
-        q > 1 ? __ldg(T.admissible + 64 + int(mod_u32(du, u32(q), (~0ull) / u32(q) + 1))) : u64(1);
-    const int nq = __popcll(classesq);
-    const int nclass = __popcll(classes2) * nq;
-    int carry = 0;
-    for (int base = 0; base < nclass; base += 32) {
-        const int c = base + lane;
-        int items = 0;
-        if (c < nclass) {
-            const int i2 = nq == 1 ? c : c / nq;
-            const int r64 = nth_bit64(classes2, i2);
-            int r = r64;
-            if (q > 1) {
-                const int rq = nth_bit64(classesq, c - i2 * nq);
-                r = r64 + 64 * int(T.crt[T.mod_q[r64] * 13 + rq]);
-            }
-            const FastClassStart cs = T.class_starts[r];
-            const int ofs = cs.ofs;
-            // sites of class r: a = -H + ofs + M t, t in [0, count)
-            const long long count = T.count_q + (ofs <= T.count_r ? 1 : 0);
-            const long long words = (count + 63) >> 6;
-            const long long lo = A.w_lo < words ? A.w_lo : words;
-            const long long hi = A.w_hi < words ? A.w_hi : words;
-            FastRun run;
-            const u32 tile_words = u32(hi - lo);
-            const bool has_last = hi == words && words > 0 && hi > lo;
-            const u32 last_bits = has_last ? u32(count - 64 * (words - 1)) : 64u;
-            run.words_last = tile_words | (has_last ? 1u << 24 : 0u) | ((last_bits - 1) << 25);
-            run.ofs = (unsigned short)ofs;
-#pragma unroll
-            for (int sl = 0; sl < kFastSlots; ++sl) {
-                // tile word 0 is class word w_lo: (a0 S^-1 + w_lo) mod m
-                const FastModulus &Md = T.mod[sl];
-                u32 st = u32(cs.start[sl]) + Md.wlo_mod;  // both below m
-                if (st >= u32(Md.m)) st -= u32(Md.m);
-                run.start[sl] = (unsigned short)st;
-            }
-            runs[c] = run;
-            items = int((tile_words + kFItemWords - 1) / kFItemWords);
-        }
-        int incl = items;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(kFullMask, incl, o);
-            if (lane >= o) incl += v;
-        }
-        if (c < nclass) prefix[c] = carry + incl - items;
-        carry += __shfl_sync(kFullMask, incl, 31);
-    }
-    if (lane == 0) {
-        prefix[nclass] = carry;
-        S.runs = runs;
-        S.prefix = prefix;
-        S.nclass = nclass;
-        S.items = carry;
-        S.d = d;
-    }
-    return carry;
-    (void)M;
+__device__ __forceinline__ void lds_u64(u32 a, u32 &lo, u32 &hi) {
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(lo), "=r"(hi) : "r"(a));
+}
+__device__ __forceinline__ void lds_u32x4(u32 a, u32 (&v)[4]) {
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(a));
 }
 
-// Four 64-bit shared words of one staged row, 256 bytes apart (a lane's kFK
-// words, 32 apart), as 32-bit halves: one address register, immediate offsets.
-__device__ __forceinline__ void lds_row4(u32 a, u32 (&lo)[kFK], u32 (&hi)[kFK]) {
-    static_assert(kFK == 4, "four words per lane per step");
-    asm volatile(
-        "ld.shared.v2.u32 {%0, %1}, [%8];\n\t"
-        "ld.shared.v2.u32 {%2, %3}, [%8+256];\n\t"
-        "ld.shared.v2.u32 {%4, %5}, [%8+512];\n\t"
-        "ld.shared.v2.u32 {%6, %7}, [%8+768];"
-        : "=r"(lo[0]), "=r"(hi[0]), "=r"(lo[1]), "=r"(hi[1]), "=r"(lo[2]), "=r"(hi[2]), "=r"(lo[3]),
-          "=r"(hi[3])
-        : "r"(a));
+// The row terms of N rows: 16-bit values two to a word.
+template <int N>
+__device__ __forceinline__ void load_starts16(u32 a, u32 (&v)[N]) {
+#pragma unroll
+    for (int r = 0; r < N; r += 8) {
+        u32 x[4];
+        lds_u32x4(a + 2 * r, x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (r + i < N) v[r + i < N ? r + i : 0] = i % 2 ? x[i / 2] >> 16 : x[i / 2] & 0xFFFFu;
+    }
 }
 
-template <int NS, int SLOTS>
-__global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(FastTables T, SieveArgs A,
-                                                               unsigned long long *work) {
-    extern __shared__ __align__(16) u64 smem[];
-    const int row_stride = T.smem_words;  // even: buffers stay 16-byte aligned
-    u64 *qmask = smem + SLOTS * row_stride;
-    u64 *qpos = qmask + kFConsumers * kFQueue;
-    FastRun *runs0 = reinterpret_cast<FastRun *>(qpos + kFConsumers * kFQueue);  // [slots][max_classes]
-    int *prefix0 = reinterpret_cast<int *>(runs0 + SLOTS * T.max_classes);  // [slots][max_classes + 1]
+// Warp-specialized persistent CTAs.  Warp 0 produces: it takes work units from
+// the launch's counter, drops denominators without classes or with a
+// denominator prime, and for each live one fills a slot by TMA with the NS
+// stage-1 rows of d mod m and the class lists of d mod two and d mod Q.  The
+// other warps sweep filled slots.  An item is a group of U pairs of units (16
+// words of one residue mod Q each, one per half-warp) against the residues mod
+// two: the units' row addresses stay in registers, a step adds one residue's
+// terms (a broadcast read shared by the pairs) and ANDs one word per lane, row
+// and pair.  Items go round-robin over the consumer warps, across
+// denominators; no barrier spans the CTA and every wait is bounded.
+//
+// What bounds it: the shared-memory pipe.  A row's word for a warp (two
+// conflict-free 128-byte halves) takes two of its cycles, whatever the layout,
+// so a swept word costs NS / 16 cycles of an SM.  The class primes halve the
+// words per prime down to classes of 16 words; everything else keeps the
+// pipe's other work and the instructions small:
+//   - rows are staged as two periods, so that the sum of two row offsets below
+//     m needs no wrap: 61 instead of 115 instructions per step of ten rows,
+//     1.95 instead of 2.49 ms per 65,536 denominators of a curve of degree 6
+//     at H = 5e6, 98 instead of 71 % of the pipe busy;
+//   - a broadcast 128-bit shared read takes two cycles: the terms of a residue
+//     are packed to 16 bits (two reads for eight rows, three for twelve) and
+//     shared by U = 2 pairs (1.81 -> 1.75 ms); read from kernel parameters
+//     instead, they cost more instructions than they saved cycles (2.07 ms);
+//   - the 24 warps of an SM form two, three or four CTAs: with four, a curve of
+//     240 words per denominator (H = 3e5) takes 0.22 instead of 0.29 ms per
+//     131,072 denominators, each CTA's producer being serial.
+template <int NS, int U>
+__global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_constant__ SweepTables T,
+                                                                  const __grid_constant__ SweepArgs A,
+                                                                  unsigned long long *work) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const u32 list2_at = u32(T.row_words) * 8u;
+    const u32 listq_at = list2_at + u32(T.two_max) * u32(sizeof(SweepClass));
+    const bool listq_staged = T.q_max <= kSweepSlotClasses;
+    const u32 slot_bytes = listq_at + (listq_staged ? u32(T.q_max) * u32(sizeof(SweepClass)) : 0u);
+    u64 *qmask = reinterpret_cast<u64 *>(smem + T.slots * slot_bytes);
+    const int consumers = int(blockDim.x) / kWarpSize - 1;
+    u64 *qpos = qmask + consumers * kFQueue;
+    u32 *qd = reinterpret_cast<u32 *>(qpos + consumers * kFQueue);
 
-    __shared__ FastSlot slot[SLOTS];
-    __shared__ int s_ctx[kFConsumers][kFCtx];  // denominators of each warp's contexts
-    __shared__ __align__(8) unsigned long long s_full[SLOTS];
-    __shared__ __align__(8) unsigned long long s_empty[SLOTS];
+    __shared__ FastSlot slot[kSweepSlots];
+    __shared__ __align__(16) unsigned short s_seg[kFSegTable][16];  // row offsets of unit seg of a class
+    __shared__ __align__(8) unsigned long long s_full[kSweepSlots];
+    __shared__ __align__(8) unsigned long long s_empty[kSweepSlots];
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
+    const int slots = T.slots;
     if (threadIdx.x == 0) {
-        for (int b = 0; b < SLOTS; ++b) {
+        for (int b = 0; b < slots; ++b) {
             mbar_init(smem_addr(&s_full[b]), 1);
-            mbar_init(smem_addr(&s_empty[b]), kFConsumers);
+            mbar_init(smem_addr(&s_empty[b]), u32(consumers));
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = threadIdx.x; i < min(A.segs, kFSegTable) * NS; i += int(blockDim.x)) {
+        const int seg = i / NS, r = i % NS;
+        s_seg[seg][r] = (unsigned short)(8u * mod_u32(T.row[r].wlo + u32(kSweepUnit * seg), T.row[r].m, T.row[r].magic));
     }
     __syncthreads();
 
     if (warp == 0) {
-        // ---- producer: next live denominator into the next free slot ----
-        // Parameters come kFChunk at a time from the launch's work counter, the
-        // next chunk's fetch issued before this chunk is handed out so that its
-        // latency is hidden; lane j classifies parameter j of a chunk (class
-        // list length by d mod 64 and d mod q), and the live ones go to the
-        // slots in order.  The row copies of a slot are issued by lanes
-        // 0 .. NS-1, one row each.
-        const int q = T.class_prime;
-        const unsigned long long magic_q = (~0ull) / u32(q) + 1;  // q >= 1: mod_u32 constant
-        const bool lists = T.list_count != nullptr;
-        int uses[SLOTS] = {};      // fills of each slot so far
-        int b = 0;
+        // ---- producer ----
+        // A chunk's work units (parameter, share of its items) are classified
+        // one per lane, the next chunk's fetch already issued; the live ones go
+        // to the slots in order.
+        int b = 0, round = 0;      // slot of the next fill, and how often it has been filled
         bool failed = false;
-        int rot = 0;               // sweep items handed out so far, mod kFConsumers
+        int rot = 0;               // sweep items handed out so far, mod the consumer count
+        const SweepRow R = T.row[lane < NS ? lane : 0];  // the row this lane copies
+        const int chunk_size = A.chunk;
+        const long long unit_count = (long long)A.k_count << A.part_shift;
         unsigned long long next_chunk = 0;
-        if (lane == 0) next_chunk = atomicAdd(work, (unsigned long long)kFChunk);
+        if (lane == 0) next_chunk = atomicAdd(work, (unsigned long long)chunk_size);
         // waits until slot b is released by every consumer (false: gave up)
         auto acquire_slot = [&]() -> bool {
-            int used = 0;
-#pragma unroll
-            for (int t = 0; t < SLOTS; ++t) used = t == b ? uses[t] : used;
-            return used == 0 || mbar_wait(smem_addr(&s_empty[b]), u32(used - 1) & 1u);
+            return round == 0 || mbar_wait(smem_addr(&s_empty[b]), u32(round - 1) & 1u);
         };
         for (;;) {
             const long long chunk = (long long)__shfl_sync(kFullMask, next_chunk, 0);
-            if (chunk >= A.k_count) break;
-            if (lane == 0) next_chunk = atomicAdd(work, (unsigned long long)kFChunk);
-            static_assert(2 * kFChunk == kWarpSize, "lanes 16..31 mirror the chunk's parameters");
-            const long long idx = chunk + (lane & (kFChunk - 1));
-            const bool in_range = idx < A.k_count;
-            const bool valid = lane < kFChunk && in_range;
-            const long long k = A.k_first + (in_range ? idx : 0);
-            const long long dd = A.square ? k * k : k;
-            const u32 du = u32(dd);
-            const int combo = int(du & 63) * q + (q > 1 ? int(mod_u32(du, u32(q), magic_q)) : 0);
-            int list_n = 0;
+            if (chunk >= unit_count) break;
+            if (lane == 0) next_chunk = atomicAdd(work, (unsigned long long)chunk_size);
+            const long long idx = chunk + lane;
+            const bool valid = lane < chunk_size && idx < unit_count;
+            const long long k = A.k_first + (valid ? idx >> A.part_shift : 0);
+            const u32 du = A.square ? u32(k) * u32(k) : u32(k);
+            const u32 dq = mod_u32(du, T.q, T.q_magic);
+            int n2 = 0, nq = 0;
             if (valid) {
-                if (lists) {
-                    list_n = __ldg(T.list_count + combo);
-                } else {
-                    const bool adm = __ldg(T.admissible + (du & 63)) != 0 &&
-                                     (q == 1 || __ldg(T.admissible + 64 + int(mod_u32(du, u32(q), magic_q))) != 0);
-                    list_n = adm ? 1 : 0;
-                }
+                n2 = __ldg(T.count2 + (du & u32(T.two_mask)));
+                nq = __ldg(T.countq + dq);
             }
-            if (T.nbad > 0) {
-                // Denominator primes: for p | d and p !| a, F(a, d) = c_n a^n
-                // (mod p), which is not a square when c_n is not and n is
-                // even, so d holds no points.  p | k^2 iff p | k; the two
-                // half-warps test a parameter against alternate primes.
-                const u32 ku = u32(k);
-                int hit = 0;
-                for (int i = lane >> 4; i < T.nbad; i += 2) {
-                    const u32 p = u32(__ldg(T.admissible + kFBadBase + 2 * i));
-                    const unsigned long long mg = __ldg(T.admissible + kFBadBase + 2 * i + 1);
-                    hit |= mod_u32(ku, p, mg) == 0 ? 1 : 0;
-                }
-                hit |= __shfl_xor_sync(kFullMask, hit, kFChunk);
-                if (hit) list_n = 0;
-            }
-            u32 live = __ballot_sync(kFullMask, list_n > 0);
+            // Denominator primes: for p | d and p !| a, F(a, d) = c_n a^n
+            // (mod p), which is not a square when c_n is not and n is even, so
+            // d holds no points.  p | k^2 iff p | k.
+            bool hit = false;
+#pragma unroll 4
+            for (int i = 0; i < T.nbad; ++i) hit |= u32(k) * T.bad[i].x <= T.bad[i].y;
+            if (hit) nq = 0;
+            u32 live = __ballot_sync(kFullMask, n2 > 0 && nq > 0);
             while (live) {
                 const int j = __ffs(live) - 1;
                 live &= live - 1;
-                const long long d = __shfl_sync(kFullMask, dd, j);
-                const int combo_j = __shfl_sync(kFullMask, combo, j);
-                const int n_j = __shfl_sync(kFullMask, list_n, j);
+                const u32 d = __shfl_sync(kFullMask, du, j);
+                const u32 dq_j = __shfl_sync(kFullMask, dq, j);
+                const int n2_j = __shfl_sync(kFullMask, n2, j);
+                const int nq_j = __shfl_sync(kFullMask, nq, j);
                 if (!acquire_slot()) {
                     failed = true;
                     break;
                 }
-                FastSlot &S = slot[b];
                 const u32 full = smem_addr(&s_full[b]);
-                int items;
-                if (lists) {
-                    items = n_j * T.list_ipc;
-                    if (lane == 0) {
-                        S.runs = runs0 + b * T.max_classes;
-                        S.prefix = nullptr;
-                        S.nclass = n_j;
-                        S.items = items;
-                        S.d = d;
-                    }
-                } else {
-                    items = fast_setup(T, A, d, S, runs0 + b * T.max_classes, prefix0 + b * (T.max_classes + 1));
-                }
-                if (lane == 0) S.rot = rot;
-                rot = int((rot + (unsigned)items) % unsigned(kFConsumers));
-                __syncwarp();
-                const u32 run_bytes = lists ? u32(n_j) * u32(sizeof(FastRun)) : 0u;
+                const u32 at8 = smem_addr(smem) + u32(b) * slot_bytes;
+                const int units = nq_j * A.segs;
+                const int all = ((units + 2 * U - 1) / (2 * U)) << A.split;
+                const int part = int(chunk + j) & ((1 << A.part_shift) - 1);
+                const int first = int((long long)all * part >> A.part_shift);
+                const int items = int((long long)all * (part + 1) >> A.part_shift);
+                if (first == items) continue;  // fewer items than parts
                 if (lane == 0) {
-                    __threadfence_block();
-                    mbar_arrive_expect_tx(full, u32(T.smem_words) * 8u + run_bytes);
+                    FastSlot &S = slot[b];
+                    S.d = d;
+                    S.units = units;
+                    S.n2 = n2_j;
+                    S.first = first;
+                    S.items = items;
+                    S.rot = rot;
+                    S.list = T.listq + (long long)dq_j * T.q_max;
+                    mbar_arrive_expect_tx(full, u32(T.row_words) * 8u + u32(n2_j) * u32(sizeof(SweepClass)) +
+                                                    (listq_staged ? u32(nq_j) * u32(sizeof(SweepClass)) : 0u));
                 }
+                rot = int(unsigned(rot + items - first) % unsigned(consumers));
+                // the consumers' reads of this slot's previous contents are
+                // ordered before the asynchronous copies that overwrite them
+                fence_proxy_async_shared();
                 __syncwarp();
                 if (lane < NS) {
-                    // the consumers' reads of this slot's previous rows are
-                    // ordered before the asynchronous copies that overwrite them
-                    fence_proxy_async_shared();
-                    const FastModulus &Md = T.mod[lane];
-                    const u32 rho = mod_u32(u32(d), u32(Md.m), Md.magic);
-                    bulk_copy_to_shared(smem_addr(smem + b * row_stride) + u32(Md.smem_offset) * 8u,
-                                        T.rows + Md.offset + (long long)rho * Md.length,
-                                        u32(Md.length) * 8u, full);
+                    const u32 rho = mod_u32(d, R.m, R.magic);
+                    bulk_copy_to_shared(at8 + R.soff8, T.rows + R.offset + (long long)rho * R.length,
+                                        R.length * 8u, full);
+                } else if (lane == 30) {
+                    bulk_copy_to_shared(at8 + list2_at, T.list2 + (long long)(d & u32(T.two_mask)) * T.two_max,
+                                        u32(n2_j) * u32(sizeof(SweepClass)), full);
+                } else if (lane == 31 && listq_staged) {
+                    bulk_copy_to_shared(at8 + listq_at, T.listq + (long long)dq_j * T.q_max,
+                                        u32(nq_j) * u32(sizeof(SweepClass)), full);
                 }
-                if (lists && lane == 31) {
-                    // the class list's runs go next to the slot with the rows, so
-                    // the consumers read them from shared memory
-                    fence_proxy_async_shared();
-                    bulk_copy_to_shared(smem_addr(runs0 + b * T.max_classes),
-                                        T.list_runs + (long long)combo_j * T.max_classes, run_bytes, full);
+                if (++b == slots) {
+                    b = 0;
+                    ++round;
                 }
-#pragma unroll
-                for (int t = 0; t < SLOTS; ++t) uses[t] += t == b ? 1 : 0;
-                b = b + 1 == SLOTS ? 0 : b + 1;
             }
             if (failed) break;
         }
@@ -601,35 +589,25 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(FastTables T, 
         if (failed) {
             if (A.error && lane == 0) atomicOr(A.error, 1ull);
             // let the copies already issued land (bounded) before leaving
-#pragma unroll
-            for (int t = 0; t < SLOTS; ++t)
-                if (lane == 0 && uses[t] > 0) mbar_wait(smem_addr(&s_full[t]), u32(uses[t] - 1) & 1u);
+            for (int t = 0; t < slots; ++t) {
+                const int fills = round + (t < b ? 1 : 0);
+                if (lane == 0 && fills > 0) mbar_wait(smem_addr(&s_full[t]), u32(fills - 1) & 1u);
+            }
         }
         return;
     }
 
-    // ---- consumers: sweep the items of each filled slot in turn ----
-    // Items are dealt round-robin over the consumer warps, continuing across
-    // denominators (the slot's rot): consumer cw sweeps items i of a fill with
-    // (i + rot) mod kFConsumers = cw.  No counter is shared, and a warp with
-    // no item in a fill only releases the slot.
+    // ---- consumers ----
+    // Consumer cw sweeps the items i of a fill with (i - first + rot) mod
+    // consumers = cw, rot carried across denominators by the producer.
     const int cw = warp - 1;
     u64 *wq_mask = qmask + cw * kFQueue;
     u64 *wq_pos = qpos + cw * kFQueue;
-    int *ctx = s_ctx[cw];
+    u32 *wq_d = qd + cw * kFQueue;
     u32 phase = 0;   // bit b: parity of slot b's next fill
     int b = 0;
     int qn = 0;      // queued words (kept across denominators)
-    int seq = 0;     // slot fills this warp has taken items from
-    int oldest = 0;  // oldest context that may still have queued words
-    auto drain_all = [&]() {
-        while (qn > 0) {
-            const int n = qn < 32 ? qn : 32;
-            __syncwarp();
-            fast_drain(wq_mask, wq_pos, qn - n, n, T, A, ctx);
-            qn -= n;
-        }
-    };
+    const u32 lane_word8 = u32(lane & (kSweepUnit - 1)) * 8u;
     for (;;) {
         if (!mbar_wait(smem_addr(&s_full[b]), (phase >> b) & 1u)) {  // bounded wait
             if (A.error && lane == 0) atomicOr(A.error, 1ull);
@@ -638,151 +616,126 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(FastTables T, 
         phase ^= 1u << b;
         const FastSlot &S = slot[b];
         if (S.d < 0) {  // the producer has no more work
-            drain_all();
+            __syncwarp();
+            if (qn > 0) fast_drain(wq_mask, wq_pos, wq_d, 0, qn, T, A);
             return;
         }
         const int total_items = S.items;
         int item = cw - S.rot;
-        if (item < 0) item += kFConsumers;
+        if (item < 0) item += consumers;
+        item += S.first;
         if (item < total_items) {
-            // context k replaces the one taken kFCtx fills ago: its queued words go first
-            const int k = seq & (kFCtx - 1);
-            if (qn > 0 && seq - oldest >= kFCtx) drain_all();
-            if (qn == 0) oldest = seq;
-            __syncwarp();
-            if (lane == 0) ctx[k] = int(S.d);
-            __syncwarp();
-            const u64 tag = u64(k) << kFTagShift;
-
-            const unsigned char *sbase = reinterpret_cast<const unsigned char *>(smem + b * row_stride);
-            const FastRun *runs = S.runs;
-            const int *prefix = S.prefix;  // null: a class list, list_ipc items per class
-            const int nclass = S.nclass;
-            // laid-out classes, up to 31 of them: lane c keeps prefix[c], so
-            // finding an item's class takes no memory access
-            const bool lane_prefix = prefix != nullptr && nclass < kWarpSize;
-            const int my_prefix = lane_prefix && lane <= nclass ? prefix[lane] : 0;
-            const u32 slot_addr = smem_addr(sbase);
-            int c = 0;  // this warp's items of a slot only increase: so do their classes
-            for (; item < total_items; item += kFConsumers) {
-                // class index: item / list_ipc for a class list; otherwise the
-                // largest c with prefix[c] <= item (32 classes per probe, from
-                // the last one on)
-                int first_item;
-                if (prefix == nullptr) {
-                    const int ipc = T.list_ipc;
-                    c = ipc == 1 ? item : item / ipc;
-                    first_item = c * ipc;
-                } else if (lane_prefix) {
-                    const u32 bb = __ballot_sync(kFullMask, lane < nclass && my_prefix <= item);
-                    c = 31 - __clz(bb);
-                    first_item = __shfl_sync(kFullMask, my_prefix, c);
-                } else {
-                    for (int base = c; base < nclass; base += 32) {
-                        const int cc = base + lane;
-                        const u32 bb = __ballot_sync(kFullMask, cc < nclass && prefix[cc] <= item);
-                        if (bb) c = base + 31 - __clz(bb);
-                        if (bb != kFullMask) break;
-                    }
-                    first_item = prefix[c];
-                }
-                const int w0 = (item - first_item) * kFItemWords;
-                const FastRun run = runs[c];
-                const int wt = int(run.words_last & 0xFFFFFFu);
-                const int last_word = (run.words_last >> 24) & 1u ? wt - 1 : -1;
-                const u32 last_bits = (run.words_last >> 25) + 1;
-                const u64 last_mask = last_bits >= 64 ? ~u64(0) : ((u64(1) << last_bits) - 1);
-                // pos of word w of this class: ofs + S (w_lo + w)
-                const u64 pos0 = u64(run.ofs) + u64(T.stride) * u64(A.w_lo);
-                u32 o[NS];  // byte offset of this lane's word inside each staged row
-                if (w0 == 0 && T.min_modulus >= kWarpSize) {
-                    // a class's first item: start < m and lane < 32 <= m, one subtraction
+            const u32 d = u32(S.d);
+            const u32 slot_addr = smem_addr(smem) + u32(b) * slot_bytes;
+            const u32 words_addr = slot_addr + lane_word8;
+            const int units = S.units, n2 = S.n2;
+            for (; item < total_items; item += consumers) {
+                const int group = item >> A.split;
+                const int range = (n2 + (1 << A.split) - 1) >> A.split;
+                const int e0 = (item & ((1 << A.split) - 1)) * range;
+                const int steps = min(range, n2 - e0);
+                // this half-warp's units, 16 words of one residue mod Q each:
+                // the addresses of their first words in the staged rows
+                u32 o[U][NS];
+                u64 pos0[U];
+                bool valid[U];
 #pragma unroll
-                    for (int sl = 0; sl < NS; ++sl) {
-                        const u32 v = 8u * (u32(run.start[sl]) + u32(lane));
-                        o[sl] = min(v, v - T.mod[sl].mod8);
+                for (int u = 0; u < U; ++u) {
+                    int unit = 2 * (U * group + u) + (lane >> 4);
+                    valid[u] = unit < units;
+                    if (!valid[u]) unit = 0;
+                    int s = unit, seg = 0;
+                    if (A.segs > 1) {
+                        s = int(__umul64hi(u64(unit), T.segs_magic));
+                        seg = unit - s * A.segs;
                     }
-                } else {
+                    u32 xq;
+                    if (listq_staged) {
+                        const u32 entry = slot_addr + listq_at + u32(s) * u32(sizeof(SweepClass));
+                        u32 pad;
+                        load_starts16<NS>(entry, o[u]);
+                        lds_u64(entry + 2 * kSweepRows, xq, pad);
+                    } else {
+                        const uint4 *entry = reinterpret_cast<const uint4 *>(S.list + s);
+                        const uint4 e0 = __ldg(entry), e1 = __ldg(entry + 1);
+                        const u32 e[6] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y};
 #pragma unroll
-                    for (int sl = 0; sl < NS; ++sl)
-                        o[sl] = 8u * mod_u32(u32(run.start[sl]) + u32(w0 + lane), u32(T.mod[sl].m), T.mod[sl].magic);
+                        for (int r = 0; r < NS; ++r) o[u][r] = r % 2 ? e[r / 2] >> 16 : e[r / 2] & 0xFFFFu;
+                        xq = e1.z;
+                    }
+                    if (A.segs > 1 || A.shifted) {
+                        u32 g[NS];
+                        if (A.segs <= kFSegTable) {
+                            load_starts16<NS>(smem_addr(s_seg[seg]), g);
+                        } else {
+#pragma unroll
+                            for (int r = 0; r < NS; ++r)
+                                g[r] = 8u * mod_u32(T.row[r].wlo + u32(kSweepUnit * seg), T.row[r].m, T.row[r].magic);
+                        }
+#pragma unroll
+                        for (int r = 0; r < NS; ++r) {
+                            const u32 v = o[u][r] + g[r];
+                            o[u][r] = min(v, v - 8u * T.row[r].m);  // unsigned: wraps into [0, 8 m)
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < NS; ++r) o[u][r] += words_addr + T.row[r].soff8;
+                    pos0[u] = u64(xq) + u64(T.stride) * u64(kSweepUnit * seg + (lane & (kSweepUnit - 1)));
                 }
+                u32 a_addr = slot_addr + list2_at + u32(e0) * u32(sizeof(SweepClass));
 #pragma unroll 1
-                for (int step = 0; step < kFSteps; ++step) {
-                    const int ws = w0 + step * kWarpSize * kFK;
-                    if (ws >= wt) break;
-                    // stage 1: this lane's kFK words (32 apart) of each staged
-                    // row, ANDed three at a time
-                    u32 lo[kFK], hi[kFK];
-                    lds_row4(slot_addr + T.mod[0].soff8 + o[0], lo, hi);
+                for (int i = 0; i < steps; ++i, a_addr += u32(sizeof(SweepClass))) {
+                    u32 t[NS];
+                    load_starts16<NS>(a_addr, t);
+                    u32 al[U], ah[U];
+                    bool hit[U];
+                    u32 bb[U];
 #pragma unroll
-                    for (int sl = 1; sl + 1 < NS; sl += 2) {
-                        u32 xl[kFK], xh[kFK], yl[kFK], yh[kFK];
-                        lds_row4(slot_addr + T.mod[sl].soff8 + o[sl], xl, xh);
-                        lds_row4(slot_addr + T.mod[sl + 1].soff8 + o[sl + 1], yl, yh);
+                    for (int u = 0; u < U; ++u) {
+                        u32 lo[NS], hi[NS];
 #pragma unroll
-                        for (int kk = 0; kk < kFK; ++kk) {
-                            lo[kk] = and3(lo[kk], xl[kk], yl[kk]);
-                            hi[kk] = and3(hi[kk], xh[kk], yh[kk]);
+                        for (int r = 0; r < NS; ++r) lds_u64(o[u][r] + t[r], lo[r], hi[r]);
+                        al[u] = lo[0];
+                        ah[u] = hi[0];
+#pragma unroll
+                        for (int r = 1; r + 1 < NS; r += 2) {
+                            al[u] = and3(al[u], lo[r], lo[r + 1]);
+                            ah[u] = and3(ah[u], hi[r], hi[r + 1]);
                         }
-                    }
-                    if (NS % 2 == 0) {
-                        u32 xl[kFK], xh[kFK];
-                        lds_row4(slot_addr + T.mod[NS - 1].soff8 + o[NS - 1], xl, xh);
-#pragma unroll
-                        for (int kk = 0; kk < kFK; ++kk) {
-                            lo[kk] &= xl[kk];
-                            hi[kk] &= xh[kk];
+                        if (NS % 2 == 0) {
+                            al[u] &= lo[NS - 1];
+                            ah[u] &= hi[NS - 1];
                         }
+                        hit[u] = (al[u] | ah[u]) != 0 && valid[u];
+                        bb[u] = __ballot_sync(kFullMask, hit[u]);
                     }
+                    u32 any = bb[0];
+                    if (U > 1) any |= bb[U - 1];
+                    if (!any) continue;
+                    u32 x2, pad;
+                    lds_u64(a_addr + 2 * kSweepRows, x2, pad);
 #pragma unroll
-                    for (int sl = 0; sl < NS; ++sl) {
-                        // advance (32 kFK) mod m words; unsigned min wraps into [0, m)
-                        const u32 t = o[sl] + T.mod[sl].step8;
-                        o[sl] = min(t, t - T.mod[sl].mod8);
-                    }
-                    const u32 any = or3(or3(lo[0], hi[0], lo[1]), or3(hi[1], lo[2], hi[2]), lo[3] | hi[3]);
-                    if (!__ballot_sync(kFullMask, any != 0)) continue;
-                    u64 acc[kFK];
-#pragma unroll
-                    for (int kk = 0; kk < kFK; ++kk) acc[kk] = (u64(hi[kk]) << 32) | lo[kk];
-                    if (ws + kWarpSize * kFK >= wt) {
-                        // the step reaches the class's last word in the tile:
-                        // that word keeps its valid bits, words past it none
-#pragma unroll
-                        for (int kk = 0; kk < kFK; ++kk) {
-                            const int w = ws + kWarpSize * kk + lane;
-                            if (w == last_word) acc[kk] &= last_mask;
-                            if (w >= wt) acc[kk] = 0;
+                    for (int u = 0; u < U; ++u) {
+                        if (!bb[u]) continue;
+                        const int to = qn + __popc(bb[u] & lanemask_lt());
+                        if (hit[u]) {
+                            wq_mask[to] = (u64(ah[u]) << 32) | al[u];
+                            wq_pos[to] = pos0[u] + x2;
+                            wq_d[to] = d;
                         }
-                    }
-#pragma unroll
-                    for (int kk = 0; kk < kFK; ++kk) {
-                        const bool live = acc[kk] != 0;
-                        const u32 bb = __ballot_sync(kFullMask, live);
-                        if (bb) {
-                            const int at = qn + __popc(bb & lanemask_lt());
-                            if (live) {
-                                const int w = ws + kWarpSize * kk + lane;
-                                wq_mask[at] = acc[kk];
-                                wq_pos[at] = tag | (pos0 + u64(T.stride) * u64(w));
-                            }
-                            qn += __popc(bb);
-                            if (qn >= 32) {
-                                __syncwarp();
-                                fast_drain(wq_mask, wq_pos, qn - 32, 32, T, A, ctx);
-                                qn -= 32;
-                                if (qn == 0) oldest = seq;
-                            }
+                        qn += __popc(bb[u]);
+                        if (qn >= 32) {
+                            __syncwarp();
+                            fast_drain(wq_mask, wq_pos, wq_d, qn - 32, 32, T, A);
+                            qn -= 32;
                         }
                     }
                 }
             }
-            ++seq;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_addr(&s_empty[b]));  // this warp is done with slot b
-        b = b + 1 == SLOTS ? 0 : b + 1;
+        b = b + 1 == slots ? 0 : b + 1;
     }
 }
 

@@ -1,0 +1,46 @@
+"""The sieve kernel over the ways it splits a plan's tests (class primes, rows,
+late primes, shares of a denominator, ranges of numerators): its survivors are
+the oracle's for the reference plan, and those of them that pass the fast
+plan's filters for the fast plan."""
+
+import pytest
+
+from test_fast_plan_gpu import check
+from test_sieve_gpu import assert_same_set
+
+pytestmark = pytest.mark.gpu
+
+DENSE = "247747600 -985905640 567207969 2396040466 52485681 -470135160 82342800".split()
+CURVES = {"sextic": ["-533746463", "2318474698", "1819918790", "-3268433658", "1978982371", "1087269120", "-559365050"],
+          "quintic": ["9", "1", "-7", "0", "3", "2"], "dense": DENSE}
+
+# around classes of 16 words of 64 sites (a class prime more or less), of one
+# word, and long enough for several class primes
+BOUNDS = [31, 32_767, 32_768, 98_303, 163_841, 360_449, 2_500_001]
+
+
+@pytest.mark.parametrize("bound", BOUNDS)
+@pytest.mark.parametrize("curve", CURVES)
+def test_survivors(rpg, oracle, curve, bound):
+    # the second range has multiples of likely class primes and of candidates
+    for first, last in ((1, 12), (3 * 5 * 7 * 11 * 13, 3 * 5 * 7 * 11 * 13 + 2), (349 * 509, 349 * 509 + 1)):
+        assert_same_set(rpg, oracle, CURVES[curve], bound, first, last)
+        check(rpg, oracle, CURVES[curve], bound, first, last)
+
+
+def test_square_denominators_with_long_classes(rpg, oracle):
+    # few denominators of many words: each is shared out over several CTAs
+    check(rpg, oracle, ["7", "-10", "0", "1"], 20_000_003, 14, 19, square=True)
+    assert_same_set(rpg, oracle, ["7", "-10", "0", "1"], 20_000_003, 21, 22, square=True)
+
+
+@pytest.mark.parametrize("plan", ["reference", "fast"])
+def test_numerator_ranges(rpg, monkeypatch, plan):
+    # a buffer of 64 survivors: denominators are split into ranges of
+    # numerators, down to 64, at every position of a class word
+    coeffs = ["4", "0", "1", "0", "1"] if plan == "fast" else DENSE
+    bound, first, last = (40_009, 1, 3) if plan == "fast" else (400_009, 1, 2)
+    expected = sorted(zip(*(v.tolist() for v in rpg.sieve(coeffs, bound, first, last, plan=plan)[:2])))
+    monkeypatch.setenv("RPG_SURVIVOR_CAPACITY", "64")
+    got = sorted(zip(*(v.tolist() for v in rpg.sieve(coeffs, bound, first, last, plan=plan)[:2])))
+    assert got == expected and len(expected) > 0
