@@ -29,7 +29,7 @@ BIN_DIR = PACKAGE / "bin"
 LIBRARY = LIB_DIR / "librpgpu.so"
 EXECUTABLE = BIN_DIR / "ratpoints_gpu"
 
-CUDA_SOURCES = ["sieve.cu", "noalloc.cu", "batch.cu", "preverify.cu", "selftest.cu", "probe.cu"]
+CUDA_SOURCES = ["sweep.cu", "sieve.cu", "noalloc.cu", "batch.cu", "preverify.cu", "selftest.cu", "probe.cu"]
 CXX_SOURCES = ["bigint.cpp", "exact.cpp", "plan.cpp", "sweep_plan.cpp", "search.cpp", "cli.cpp", "point_format.cpp", "capi.cpp",
                "serve.cpp", "compat_sieve.cpp", "tune.cpp"]
 MAIN_SOURCE = "ratpoints_gpu_main.cpp"

@@ -169,6 +169,7 @@ rpg_status rpg_sieve_run(const char *const *coefficients, int32_t coefficient_co
         so.plan = (flags & RPG_SIEVE_FAST_PLAN) ? rpg::PlanKind::fast : rpg::PlanKind::reference;
         so.square = (flags & RPG_SIEVE_SQUARE_DENOMINATORS) != 0;
         so.device = device;
+        so.denominators = double(last) - double(first) + 1.0;
         if (so.square && last > 46340) return fail(RPG_E_ARG, "invalid denominator range");
         rpg::Sieve sieve(coeffs, numerator_bound, so);
         sieve.start(first, last, 1 << 16);

@@ -21,6 +21,7 @@ SieveResult run_modular_sieve(const Coefficients &coefficients, long long numera
     rpg::SieveOptions options;
     options.plan = rpg::PlanKind::reference;
     options.square = square_denominators;
+    options.denominators = double(denominators.last) - double(denominators.first) + 1.0;
     rpg::Sieve sieve(coefficients, numerator_bound, options);
     const auto started = Clock::now();
     sieve.start(denominators.first, denominators.last, denominators.count());

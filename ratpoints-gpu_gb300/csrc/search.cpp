@@ -218,6 +218,7 @@ SearchMetrics PointSearch::run(const PointCallback &callback) {
     so.capacity = options.capacity;
     so.device = devices.front().id;
     so.preverify = options.device_preverify;
+    so.denominators = double(options.last) - double(options.first) + 1.0;
     Sieve sieve(options.coefficients, options.numerator_bound, so);
     const int threads = options.verify_threads > 0
                             ? options.verify_threads

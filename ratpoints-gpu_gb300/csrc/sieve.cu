@@ -25,9 +25,7 @@
 
 #include "plan.hpp"
 #include "preverify.hpp"
-#include "sieve_device.cuh"
-#include "sieve_fast.cuh"
-#include "sweep_plan.hpp"
+#include "sweep.hpp"
 
 namespace rpg {
 
@@ -175,7 +173,7 @@ FastPlan single_curve_plan(const std::vector<std::string> &coefficients, long lo
 struct Sieve::Impl {
     SieveOptions opt;
     long long bound = 0;
-    int device = 0, grid = 0;
+    int device = 0;
     // stream: table builds and the launches into buffer 0; stream2: the
     // launches into buffer 1, so that a launch's first CTAs take the SMs that
     // the previous launch's last CTAs leave idle; copy_stream: survivor
@@ -188,16 +186,9 @@ struct Sieve::Impl {
     // batch's end, both measured from an origin recorded at start().
     cudaEvent_t origin = nullptr;
     float last_end_ms = 0;
-    // the curve's tables, all in one allocation (see build_tables)
-    dev::SweepTables T{};
-    SweepPlan sweep;
-    unsigned char *arena = nullptr;
-    std::size_t sweep_smem = 0;
-    std::vector<int> count2_host;               // admissible residues mod two by d mod two
-    std::vector<std::vector<int>> countq_host;  // per class prime p: admissible residues by d mod p
-    std::vector<int> bad_primes;                // denominator primes (see SweepTables::nbad)
+    std::unique_ptr<SweepCurve> curve;
+    unsigned char *arena = nullptr;  // its tables
     FastPlan fast_plan;
-    long long tile = 0;           // numerators per launch (more: the row goes in pieces)
     long long capacity = 0;       // most survivors a buffer may grow to hold
     long long host_capacity = 0;  // entries of the pinned host arrays
     SieveTimings timings;
@@ -461,274 +452,26 @@ struct Sieve::Impl {
 
     using PlannedRows = std::future<std::pair<FastPlan, int>>;
 
-    // The sweep plan of the curve's primes (sweep_plan.hpp), then its tables
-    // on the device: stage-1 rows, the 36 candidates' rows, late primes' rows
-    // and the class lists.
+    // The curve's sweep plan and its tables on the device.
     void build_tables(const std::vector<std::string> &coefficients, PlannedRows &planned) {
         auto t0 = Clock::now();
         const bool fast = opt.plan == PlanKind::fast;
         // the plan was started on a host thread while the buffers were set up
         if (fast) fast_plan = planned.get().first;
-        const int n = int(coefficients.size()) - 1;
-        // the primes the plan tests before stage 2, then the 36 candidates
-        std::vector<int> plan_primes;
-        if (fast) {
-            for (const auto &f : fast_plan.slots)
-                for (int p : f) plan_primes.push_back(p);
-            if (fast_plan.class_prime > 1) plan_primes.push_back(fast_plan.class_prime);
-        }
-        std::vector<unsigned char> affine;
-        std::vector<unsigned short> inverse;
-        std::vector<int> base(kMaximumPrime, -1), lead(kMaximumPrime, 1), admitted(kMaximumPrime, 0);
-        std::vector<char> strict(kMaximumPrime, 0);
-        auto add_prime = [&](int p) {
-            if (base[p] >= 0) return;
-            base[p] = int(affine.size());
-            auto aff = affine_mask(p, coefficients);
-            for (auto v : aff) admitted[p] += v;
-            affine.insert(affine.end(), aff.begin(), aff.end());
-            const std::size_t at = inverse.size();
-            inverse.resize(at + std::size_t(p), 0);
-            modular_inverses(p, inverse.data() + at);
-            if (n % 2 == 0) lead[p] = square_mod(decimal_mod(coefficients.back(), p), p) ? 1 : 0;
-        };
-        for (int p : plan_primes) {
-            add_prime(p);
-            strict[p] = 1;
-        }
-        const auto &cands = candidate_primes();
-        for (int p : cands) add_prime(p);
-
-        SweepInput in;
-        in.bound = bound;
-        dev::u64 adm2[64];
-        for (auto &v : adm2) v = ~dev::u64(0);
-        if (fast) {
-            two_adic_classes(coefficients, adm2);
-            in.two = 64;
-            int total = 0, live = 0;
-            for (auto v : adm2) {
-                const int c = __builtin_popcountll(v);
-                total += c;
-                live += c > 0;
-                in.two_max = std::max(in.two_max, c);
-            }
-            in.two_classes = live ? double(total) / live : 1.0;
-        }
-        for (int p : plan_primes) in.primes.push_back({p, admitted[p], lead[p] ? p - 1 : 0, false});
-        // The 32 largest candidates are always selected where they do not
-        // divide d, so stage 1 may test them as well: all of the reference
-        // plan's, and those of a fast plan whose own rows filter weakly (13
-        // bits are usual) or whose long rows take several class primes away
-        // from them (shorter searches save the planning time).
-        if (!fast || fast_plan.bits < 12.5 || bound >= 4'000'000)
-            for (int i = kCandidatePrimes - kSelectedPrimes; i < kCandidatePrimes; ++i)
-                if (!strict[cands[i]]) in.primes.push_back({cands[i], admitted[cands[i]], cands[i], true});
-        sweep = plan_sweep(in);
-
-        const int q = sweep.q;
-        const long long M = (long long)sweep.two * q;
-        const long long S = 64LL * M;
-        // pattern rows per (prime, rho = 0 rule): step = M mod p, window start
-        // of residue x0 = x0 step^-1 mod p
-        std::vector<dev::TableSpec> specs;
-        long long total = 0;
-        std::vector<dev::ClassPatternSpec> pspecs;
-        long long pattern_total = 0;
-        auto pattern_of = [&](int p, int lead_ok, dev::TableSpec &Sp, int f) {
-            int found = -1;
-            for (std::size_t i = 0; i < pspecs.size(); ++i)
-                if (pspecs[i].q == p && pspecs[i].lead_ok == lead_ok) found = int(i);
-            if (found < 0) {
-                dev::ClassPatternSpec P{};
-                P.out = pattern_total;
-                P.q = p;
-                P.words = (p + 64 + 63) / 64 + 1;
-                P.factor_base = base[p];
-                P.lead_ok = lead_ok;
-                P.step = int(M % p);
-                pattern_total += (long long)p * P.words;
-                pspecs.push_back(P);
-                found = int(pspecs.size()) - 1;
-            }
-            Sp.pattern[f] = pspecs[std::size_t(found)].out;
-            Sp.pattern_words[f] = pspecs[std::size_t(found)].words;
-            Sp.s_mod[f] = int(S % p);
-            Sp.step_inv[f] = int(mod_inverse(M % p, p));
-        };
-        auto magic_of = [](long long m) { return m == 1 ? ~0ull : (~0ull) / (unsigned long long)m + 1; };
-        auto mod_of = [](long long v, long long m) { return ((v % m) + m) % m; };
-        T = dev::SweepTables{};
-        dev::ClassListSpec C{};
-        C.two = sweep.two;
-        C.q = q;
-        C.two_max = sweep.two_max;
-        C.q_max = sweep.q_max;
-        C.nprimes = int(sweep.class_primes.size());
-        C.nrows = int(sweep.moduli.size());
-        C.lift2 = dev::u32(sweep.two == 1 ? 0 : (long long)q * mod_inverse(q % sweep.two, sweep.two) % M);
-        C.liftq = dev::u32(q == 1 ? 0 : (long long)sweep.two * mod_inverse(sweep.two % q, q) % M);
-        C.h2 = dev::u32(bound % sweep.two);
-        C.hq = dev::u32(bound % q);
-        int row_words = 0;
-        for (std::size_t r = 0; r < sweep.moduli.size(); ++r) {
-            dev::TableSpec Sp{};
-            const int m = sweep.moduli[r];
-            Sp.m = m;
-            Sp.nf = int(sweep.rows[r].size());
-            for (int i = 0; i < Sp.nf; ++i) {
-                const int p = sweep.rows[r][std::size_t(i)];
-                Sp.q[i] = p;
-                pattern_of(p, strict[p] ? lead[p] : 2, Sp, i);
-            }
-            Sp.length = sweep_row_words(m);
-            Sp.offset = total;
-            total += (long long)m * Sp.length;
-            specs.push_back(Sp);
-            dev::SweepRow &R = T.row[r];
-            R.offset = Sp.offset;
-            R.magic = magic_of(m);
-            R.m = dev::u32(m);
-            R.length = dev::u32(Sp.length);
-            R.soff8 = dev::u32(8 * row_words);
-            row_words += Sp.length;
-            C.m[r] = dev::u32(m);
-            C.inv_stride[r] = dev::u32(mod_inverse(S % m, m));
-            C.base[r] = dev::u32(mod_of(-(bound % m) - M, m));
-        }
-        auto single = [&](int p, int lead_ok) {
-            dev::TableSpec Sp{};
-            Sp.nf = 1;
-            Sp.m = p;
-            Sp.q[0] = p;
-            pattern_of(p, lead_ok, Sp, 0);
-            Sp.length = p;
-            Sp.offset = total;
-            total += (long long)p * p;
-            specs.push_back(Sp);
-            return Sp.offset;
-        };
-        for (int i = 0; i < kCandidatePrimes; ++i) {
-            const int p = cands[i];
-            dev::FastPrime &P = T.prime[i];
-            // rows with p | d go unused: stage 2 skips such p.  A class prime
-            // has no rows: the swept classes are those that pass it
-            P.p = p;
-            P.magic = dev::magic40(dev::u32(p));
-            if (q % p == 0) continue;
-            P.offset = single(p, 0);
-            P.inv_stride = dev::u32(mod_inverse(S % p, p));
-        }
-        std::vector<dev::LatePrime> late;
-        for (int p : sweep.late)
-            late.push_back({single(p, lead[p]), dev::u32(p), dev::u32(mod_inverse(S % p, p))});
-        // admissible residues of the class primes by d mod p
-        std::vector<unsigned char> admq;
-        countq_host.clear();
-        for (int i = 0; i < C.nprimes; ++i) {
-            const int p = sweep.class_primes[std::size_t(i)];
-            const unsigned char *aff = affine.data() + base[p];
-            const unsigned short *inv = inverse.data() + base[p];
-            C.p[i] = p;
-            C.adm[i] = int(admq.size());
-            std::vector<int> counts(std::size_t(p), 0);
-            for (int dq = 0; dq < p; ++dq)
-                for (int r = 0; r < p; ++r) {
-                    bool ok;
-                    if (dq == 0) ok = strict[p] ? r != 0 && lead[p] : true;
-                    else ok = aff[r * inv[dq] % p] != 0;
-                    admq.push_back(ok);
-                    counts[std::size_t(dq)] += ok;
-                }
-            countq_host.push_back(std::move(counts));
-        }
-        count2_host.assign(std::size_t(sweep.two), 0);
-        const dev::u64 two_bits = sweep.two == 64 ? ~dev::u64(0) : (dev::u64(1) << sweep.two) - 1;
-        for (int dd = 0; dd < sweep.two; ++dd) {
-            adm2[dd] &= two_bits;
-            count2_host[std::size_t(dd)] = __builtin_popcountll(adm2[dd]);
-        }
-        // Denominator primes (fast plan): p < 512 with c_n not a square mod p,
-        // for even degree.  A denominator divisible by one holds no points:
-        // p !| a (gcd) gives F(a, d) = c_n a^n (mod p), a non-square.  The
-        // producer skips such denominators.
-        bad_primes.clear();
-        if (fast && n % 2 == 0) {
-            for (int p = 3; p < kMaximumPrime; p += 2) {
-                bool prime = true;
-                for (int f = 3; f * f <= p && prime; f += 2) prime = p % f != 0;
-                if (!prime) continue;
-                const int lc = decimal_mod(coefficients.back(), p);
-                if (lc == 0 || square_mod(lc, p)) continue;
-                dev::u32 inverse32 = dev::u32(p);  // p^-1 mod 2^32 by Newton's iteration (3 bits to start with)
-                for (int i = 0; i < 4; ++i) inverse32 *= 2u - dev::u32(p) * inverse32;
-                T.bad[bad_primes.size()] = make_uint2(inverse32, 0xFFFFFFFFu / dev::u32(p));
-                bad_primes.push_back(p);
-            }
-        }
+        curve.reset(new SweepCurve(coefficients, bound, opt.square, fast ? &fast_plan : nullptr, opt.denominators));
+        SweepBuilder builder;
+        builder.add(*curve);
         timings.plan_ms += ms_since(t0);
-
-        // One allocation and one upload: [rows, lists, counts][uploaded blob][patterns]
         auto t1 = Clock::now();
-        std::size_t size = 0;
-        auto take = [&](std::size_t bytes) {
-            const std::size_t at = size;
-            size += (bytes + 255) & ~std::size_t(255);
-            return at;
-        };
-        const std::size_t rows_at = take(std::size_t(total) * 8);
-        const std::size_t list2_at = take(std::size_t(sweep.two) * sweep.two_max * sizeof(dev::SweepClass));
-        const std::size_t listq_at = take(std::size_t(q) * sweep.q_max * sizeof(dev::SweepClass));
-        const std::size_t count2_at = take(std::size_t(sweep.two) * sizeof(int));
-        const std::size_t countq_at = take(std::size_t(q) * sizeof(int));
-        const std::size_t blob_at = size;
-        std::vector<unsigned char> blob;
-        auto put = [&](const void *data, std::size_t bytes) {
-            const std::size_t at = take(bytes);
-            blob.resize(size - blob_at);
-            if (bytes) std::memcpy(blob.data() + (at - blob_at), data, bytes);
-            return at;
-        };
-        const std::size_t late_at = put(late.data(), late.size() * sizeof(dev::LatePrime));
-        const std::size_t aff_at = put(affine.data(), affine.size());
-        const std::size_t inv_at = put(inverse.data(), inverse.size() * sizeof(unsigned short));
-        const std::size_t specs_at = put(specs.data(), specs.size() * sizeof(dev::TableSpec));
-        const std::size_t pspecs_at = put(pspecs.data(), pspecs.size() * sizeof(dev::ClassPatternSpec));
-        const std::size_t admq_at = put(admq.data(), admq.size());
-        const std::size_t adm2_at = put(adm2, sizeof adm2);
-        const std::size_t patterns_at = take(std::size_t(pattern_total) * 8);
-        arena = device_alloc<unsigned char>(size, "cudaMalloc(sieve tables)");
+        arena = device_alloc<unsigned char>(builder.bytes(), "cudaMalloc(sieve tables)");
         timings.workspace_ms += ms_since(t1);
         cudaEvent_t e0, e1;
         check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
         check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
         check_cuda(cudaEventRecord(e0, stream), "cudaEventRecord");
-        check_cuda(cudaMemcpyAsync(arena + blob_at, blob.data(), blob.size(), cudaMemcpyHostToDevice, stream),
-                   "upload table inputs");
-        timings.h2d_bytes += blob.size();
-        auto at = [&](std::size_t offset) { return arena + offset; };
-        dev::u64 *rows = reinterpret_cast<dev::u64 *>(at(rows_at));
-        dev::u64 *patterns = reinterpret_cast<dev::u64 *>(at(patterns_at));
-        T.listq = reinterpret_cast<const dev::SweepClass *>(at(listq_at));
-        T.list2 = reinterpret_cast<const dev::SweepClass *>(at(list2_at));
-        T.count2 = reinterpret_cast<const int *>(at(count2_at));
-        T.countq = reinterpret_cast<const int *>(at(countq_at));
-        T.rows = rows;
-        T.late = reinterpret_cast<const dev::LatePrime *>(at(late_at));
-        const int threads = 256;
-        dev::pattern_rows_kernel<<<unsigned((pattern_total + threads - 1) / threads), threads, 0, stream>>>(
-            patterns, reinterpret_cast<const dev::ClassPatternSpec *>(at(pspecs_at)), int(pspecs.size()), at(aff_at),
-            reinterpret_cast<const unsigned short *>(at(inv_at)), pattern_total);
-        check_cuda(cudaGetLastError(), "pattern_rows_kernel launch");
-        const long long blocks = (total + threads - 1) / threads;
-        dev::class_table_kernel<<<unsigned(blocks), threads, 0, stream>>>(
-            rows, reinterpret_cast<const dev::TableSpec *>(at(specs_at)), int(specs.size()), patterns, total);
-        check_cuda(cudaGetLastError(), "class_table_kernel launch");
-        dev::class_list_kernel<<<unsigned(q + sweep.two), threads, 0, stream>>>(
-            C, at(admq_at), reinterpret_cast<const dev::u64 *>(at(adm2_at)),
-            reinterpret_cast<dev::SweepClass *>(at(list2_at)), reinterpret_cast<dev::SweepClass *>(at(listq_at)),
-            reinterpret_cast<int *>(at(count2_at)), reinterpret_cast<int *>(at(countq_at)));
-        check_cuda(cudaGetLastError(), "class_list_kernel launch");
+        builder.place(arena, stream);
+        timings.h2d_bytes += builder.upload_bytes();
+        builder.enqueue(stream);
         check_cuda(cudaEventRecord(e1, stream), "cudaEventRecord");
         check_cuda(cudaEventSynchronize(e1), "class table build");
         float ms = 0;
@@ -736,93 +479,24 @@ struct Sieve::Impl {
         timings.table_ms += ms;
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-
-        T.nbad = int(bad_primes.size());
-        T.nlate = int(late.size());
-        T.two_mask = sweep.two - 1;
-        T.q = dev::u32(q);
-        T.q_magic = magic_of(q);
-        T.two_max = sweep.two_max;
-        T.q_max = sweep.q_max;
-        T.stride = S;
-        T.class_mod = int(M);
-        T.row_words = row_words;
-        T.slots = sweep.slots;
-        sweep_smem = std::size_t(sweep.slots) * std::size_t(sweep_slot_bytes(row_words, sweep.two_max, sweep.q_max)) +
-                     std::size_t(kSweepQueueBytes) * std::size_t(kSweepWarps / sweep.ctas - 1);
-        const void *kernel = kernel_ptr(int(sweep.moduli.size()), sweep.pairs);
-        check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sweep_smem)),
-                   "cudaFuncSetAttribute");
-        int sms = 0, per_sm = 0;
-        check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device),
-                   "cudaDeviceGetAttribute");
-        check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads_per_cta(), sweep_smem),
-                   "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-        grid = std::max(1, sms * std::max(1, per_sm));
-        // queued positions stay below 2^46 and class words below 2^23
-        tile = S * std::min<long long>(1LL << 23, (1LL << 45) / S);
         timings.table_wall_ms += ms_since(t0);
     }
 
-    int threads_per_cta() const { return kSweepWarps / sweep.ctas * dev::kWarpSize; }
-
-    static const void *kernel_ptr(int rows, int pairs) {
-        switch (2 * rows + pairs) {
-#define RPG_FAST_PTR(n)                                                                     \
-    case 2 * n + 1: return reinterpret_cast<const void *>(&dev::fast_sieve_kernel<n, 1>);   \
-    case 2 * n + 2: return reinterpret_cast<const void *>(&dev::fast_sieve_kernel<n, 2>);
-        RPG_FAST_PTR(1) RPG_FAST_PTR(2) RPG_FAST_PTR(3) RPG_FAST_PTR(4) RPG_FAST_PTR(5) RPG_FAST_PTR(6)
-        RPG_FAST_PTR(7) RPG_FAST_PTR(8) RPG_FAST_PTR(9) RPG_FAST_PTR(10) RPG_FAST_PTR(11) RPG_FAST_PTR(12)
-#undef RPG_FAST_PTR
-        default: throw std::logic_error("no sieve kernel for this row count");
-        }
-    }
-
-    // One launch: parameters first .. last, numerators a_lo .. a_hi (at most
-    // `tile` of them), survivors into the given arrays.
     void launch_sweep(long long first, long long last, long long a_lo, long long a_hi, long long *out_a, int *out_d,
-                      unsigned long long capacity, unsigned long long *out_count, unsigned long long *work,
+                      unsigned long long cap, unsigned long long *out_count, unsigned long long *work,
                       unsigned long long *error, cudaStream_t st) const {
-        const long long M = T.class_mod, S = T.stride;
-        const long long w_lo = (a_lo + bound) / S;
-        dev::SweepArgs A{};
-        A.abase = -bound - M + S * w_lo;
-        A.a_lo = a_lo;
-        A.a_hi = a_hi;
-        A.k_first = first;
-        A.k_count = int(last - first + 1);
-        // Few denominators with much to sweep are split into shares of their
-        // items, so that every CTA gets several (the tail of a launch is at
-        // most one of them per CTA), while a share stays well above the copy
-        // of its rows.  A fetch takes work worth about 2^15 cycles.
-        double cost = sweep.cost * (double(a_hi) - double(a_lo) + 1.0) / (2.0 * double(bound) + 1.0);
-        A.part_shift = 0;
-        while (A.part_shift < 6 && (A.k_count << A.part_shift) < 32 * grid && cost > 40000.0) {
-            ++A.part_shift;
-            cost *= 0.5;
-        }
-        const long long shares = (long long)A.k_count << A.part_shift;
-        A.chunk = int(std::max<long long>(1, std::min<long long>({dev::kFChunk, shares / (4LL * grid),
-                                                                  (long long)(32768.0 / cost)})));
-        A.square = opt.square ? 1 : 0;
-        const long long words = ((a_hi - A.abase) / M >> 6) + 1;
-        A.segs = int((words + kSweepUnit - 1) / kSweepUnit);
-        A.shifted = w_lo != 0;
-        A.split = A.segs > 64 ? 0 : sweep.split;
-        A.out_a = out_a;
-        A.out_d = out_d;
-        A.out_count = out_count;
-        A.capacity = capacity;
-        A.error = error;
-        dev::SweepTables Tl = T;
-        Tl.segs_magic = A.segs == 1 ? 0 : (~0ull) / (unsigned long long)A.segs + 1;
-        for (std::size_t r = 0; r < sweep.moduli.size(); ++r) Tl.row[r].wlo = dev::u32(w_lo % sweep.moduli[r]);
-        for (auto &P : Tl.prime) P.base_mod = dev::u32(((A.abase % P.p) + P.p) % P.p);
-        const int blocks = int(std::min<long long>(grid, (shares + A.chunk - 1) / A.chunk));
-        void *params[] = {&Tl, &A, &work};
-        check_cuda(cudaLaunchKernel(kernel_ptr(int(sweep.moduli.size()), sweep.pairs), dim3(unsigned(blocks)), dim3(unsigned(threads_per_cta())),
-                                    params, sweep_smem, st),
-                   "sieve kernel launch");
+        SweepLaunch l;
+        l.first = first;
+        l.last = last;
+        l.a_lo = a_lo;
+        l.a_hi = a_hi;
+        l.out_a = out_a;
+        l.out_d = out_d;
+        l.capacity = cap;
+        l.out_count = out_count;
+        l.work = work;
+        l.error = error;
+        curve->launch(l, st);
     }
 
     cudaStream_t launch_stream(int which) const { return which ? stream2 : stream; }
@@ -839,7 +513,7 @@ struct Sieve::Impl {
         ++timings.launches;
     }
 
-    bool one_launch() const { return 2 * bound + 1 <= tile; }
+    bool one_launch() const { return 2 * bound + 1 <= curve->tile(); }
 
     void launch(int which, long long first, long long last, long long a_lo, long long a_hi) {
         Buffer &b = buf[which];
@@ -967,10 +641,11 @@ struct Sieve::Impl {
         return true;
     }
 
-    // Queue a batch as pieces of at most `tile` numerators.
+    // Queue a batch as pieces of at most a tile of numerators.
     void queue_pieces(long long first, long long last) {
         piece_batch_first = first;
         piece_batch_last = last;
+        const long long tile = curve->tile();
         for (long long a = -bound;; a += tile) {
             const bool end = bound - a < tile;  // no overflow near the largest bounds
             pieces.push_back(Piece{first, last, a, end ? bound : a + tile - 1});
@@ -1141,38 +816,7 @@ void Sieve::cancel() {
 const SieveTimings &Sieve::timings() const { return impl_->timings; }
 
 unsigned long long Sieve::swept_words(long long first, long long last) const {
-    const auto &I = *impl_;
-    if (last < first) return 0;
-    // Parameters per residue mod M, then the classes of each residue.
-    const long long M = I.T.class_mod;
-    std::vector<unsigned long long> per_residue(std::size_t(M), 0);
-    auto residue = [&](long long k) { return I.opt.square ? (k % M) * (k % M) % M : k % M; };
-    if (I.bad_primes.empty()) {
-        for (long long t = 0; t < M; ++t) {
-            const long long lo = first + ((t - first % M) % M + M) % M;  // first k >= first, k = t (mod M)
-            if (lo <= last) per_residue[std::size_t(residue(t))] += (unsigned long long)((last - lo) / M + 1);
-        }
-    } else {
-        // parameters k without a denominator prime factor, by segments
-        constexpr long long kSegment = 1LL << 22;
-        std::vector<unsigned char> skip;
-        for (long long lo = first; lo <= last; lo += kSegment) {
-            const long long hi = std::min(last, lo + kSegment - 1);
-            skip.assign(std::size_t(hi - lo + 1), 0);
-            for (int p : I.bad_primes)
-                for (long long k = lo + ((p - lo % p) % p); k <= hi; k += p) skip[std::size_t(k - lo)] = 1;
-            for (long long k = lo; k <= hi; ++k)
-                if (!skip[std::size_t(k - lo)]) per_residue[std::size_t(residue(k))] += 1;
-        }
-    }
-    unsigned long long total = 0;
-    for (long long r = 0; r < M; ++r) {
-        unsigned long long classes = (unsigned long long)I.count2_host[std::size_t(r % I.sweep.two)];
-        for (std::size_t i = 0; i < I.countq_host.size(); ++i)
-            classes *= (unsigned long long)I.countq_host[i][std::size_t(r % I.sweep.class_primes[i])];
-        total += per_residue[std::size_t(r)] * classes;
-    }
-    return total * (unsigned long long)sweep_words(I.bound, M);
+    return impl_->curve->swept_words(first, last);
 }
 
 FastPlanInfo Sieve::fast_plan_info() const {
@@ -1208,8 +852,8 @@ bool Sieve::launch_into(long long first, long long last, long long *out_a, int *
     return true;
 }
 
-unsigned Sieve::smem_bytes_per_word() const { return unsigned(8 * impl_->sweep.moduli.size()); }
-long long Sieve::words64() const { return sweep_words(impl_->bound, impl_->T.class_mod); }
+unsigned Sieve::smem_bytes_per_word() const { return unsigned(8 * impl_->curve->plan().moduli.size()); }
+long long Sieve::words64() const { return sweep_words(impl_->bound, (long long)impl_->curve->plan().two * impl_->curve->plan().q); }
 cudaStream_t Sieve::stream() const { return impl_->stream; }
 
 unsigned long long Sieve::count_only(long long first, long long last, long long batch_size) {
@@ -1227,9 +871,10 @@ unsigned long long Sieve::count_only(long long first, long long last, long long 
     int which = 0;
     for (long long f = first; f <= last; f += batch_size) {
         const long long l = std::min(last, f + batch_size - 1);
-        for (long long a = -I.bound;; a += I.tile, which ^= 1) {
-            const bool end = I.bound - a < I.tile;
-            I.launch_counting(which, f, l, a, end ? I.bound : a + I.tile - 1);
+        const long long tile = I.curve->tile();
+        for (long long a = -I.bound;; a += tile, which ^= 1) {
+            const bool end = I.bound - a < tile;
+            I.launch_counting(which, f, l, a, end ? I.bound : a + tile - 1);
             if (end) break;
         }
         which ^= 1;

@@ -45,6 +45,7 @@ struct SieveOptions {
     bool square = false;            // parameters k give denominators k*k
     long long capacity = 1 << 22;   // survivors per device buffer
     int device = -1;                // -1: current device
+    double denominators = 0;        // about how many the search has (0: not known)
     // Drop survivors that cannot be points on the device before the copy
     // (gcd and residue tests; see preverify.hpp).  Deliveries then hold a
     // subset of the modular survivors that still contains every point.
@@ -131,8 +132,8 @@ public:
     FastPlanInfo fast_plan_info() const;
 
     // Whether a whole row (all numerators of a denominator) fits one launch:
-    // false only for very large H (fast plan: more than 2^23 class words,
-    // reference plan: more than 2^30 words).
+    // false only for very large H (fast plan: more than 2^23 words of a class mod
+    // 64 q, reference plan: more than 2^30 words).
     bool fits_one_launch() const;
     // Enqueue one sieve launch for parameters [first, last] (at most one batch
     // of 65536) on `stream`, writing survivors into caller-owned device arrays

@@ -50,9 +50,12 @@ struct SweepArgs {
     int split;           // a group of units is 2^split items, each a range of the residues mod two
     long long *out_a;
     int *out_d;
+    int *out_curve;              // curve tags (may be null)
+    int curve;
     unsigned long long *out_count;
     unsigned long long capacity;
     unsigned long long *error;   // set nonzero if a bounded device wait ran out (may be null)
+    unsigned long long *swept;   // class words swept (may be null)
 };
 
 struct SweepRow {                  // one stage-1 modulus
@@ -64,18 +67,23 @@ struct SweepRow {                  // one stage-1 modulus
     u32 wlo;                       // the launch's first class word, mod m
 };
 
-struct FastPrime {                 // one of the 36 reference candidates, class layout
-    long long offset;              // word offset of row 0 (rows of length p)
+struct FastPrime {                 // one of the 36 reference candidates
+    long long pattern;             // word offset of its pattern row 0
+    long long offset;              // word offset of its class-layout row 0 (rows of length p), if tabled
     int p;
     u32 inv_stride;                // S^-1 mod p; 0: a class prime, which every swept site passes
+    u32 inv_mod;                   // M^-1 mod p
     u32 base_mod;                  // abase mod p
     u32 magic;                     // magic40(p)
+    int words;                     // words per pattern row
 };
 
 struct LatePrime {                 // a prime of the plan tested after stage 2
-    long long offset;              // word offset of row 0 (rows of length p)
+    long long pattern;
     u32 p;
-    u32 inv_stride;
+    u32 inv_mod;
+    int words;
+    int pad;
 };
 
 // Entry of the lists by d mod two and by d mod Q: one admissible residue, its
@@ -94,9 +102,10 @@ struct SweepTables {
     const SweepClass *list2;       // [two][two_max]
     const int *count2;             // [two]
     const int *countq;             // [Q]
-    const u64 *rows;               // stage-1, candidate and late-prime tables
+    const u64 *rows;               // stage-1 and candidate tables, pattern rows
     const LatePrime *late;
     int nbad, nlate;
+    int tabled;                    // the largest candidates have class-layout tables
     int two_mask;                  // two - 1
     u32 q;                         // Q
     unsigned long long q_magic;    // mod_u32 constant of Q
@@ -111,157 +120,8 @@ struct SweepTables {
     // denominator primes: p | k iff k x <= y (mod 2^32), x = p^-1 mod 2^32 and
     // y = floor((2^32 - 1) / p)
     uint2 bad[kOddPrimes];
+    uint2 need;                    // d has survivors only if d x <= y (mod 2^32): a divisor d must have
 };
-
-// One test of one site class for prime q: rho = d mod q, x = a mod q.
-__device__ __forceinline__ bool prime_bit(const unsigned char *affine, const unsigned short *inverse,
-                                          int q, int rho, int lead_ok, int x) {
-    // q | d: need q !| a, and c_n square mod q (even n); lead_ok 2: no test there
-    if (rho == 0) return lead_ok == 2 || (x != 0 && lead_ok);
-    return affine[(x * inverse[rho]) % q] != 0;
-}
-
-// Bit patterns of one prime q used by the class-layout tables: for each
-// rho in [0, q), bit k of row rho is prime_bit(.., rho, (k step) mod q) for
-// k in [0, q + 64), step = M mod q (k taken mod q), `words` words per row.
-// Bit j of a table word whose first site has residue x0 is then bit
-// (x0 step^-1 mod q) + j of the row: one 64-bit window instead of 64 tests.
-struct ClassPatternSpec {
-    long long out;                 // word offset of row 0
-    int q;
-    int words;                     // words per row: ceil((q + 64) / 64) + 1
-    int factor_base;               // offset of q's affine/inverse arrays
-    int lead_ok;
-    int step;                      // M mod q
-    int pad;
-};
-
-__global__ void pattern_rows_kernel(u64 *patterns, const ClassPatternSpec *specs, int nspecs,
-                                    const unsigned char *affine, const unsigned short *inverse,
-                                    long long total) {
-    const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (id >= total) return;
-    int lo = 0, hi = nspecs - 1;  // last spec with out <= id
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (specs[mid].out <= id) lo = mid;
-        else hi = mid - 1;
-    }
-    const ClassPatternSpec &P = specs[lo];
-    const long long rel = id - P.out;
-    const int rho = int(rel / P.words);
-    const int wi = int(rel % P.words);
-    const unsigned char *aff = affine + P.factor_base;
-    const unsigned short *inv = inverse + P.factor_base;
-    u64 word = 0;
-    int k = (64 * wi) % P.q;
-    for (int j = 0; j < 64; ++j) {
-        const int x = int((long long)k * P.step % P.q);
-        if (prime_bit(aff, inv, P.q, rho, P.lead_ok, x)) word |= u64(1) << j;
-        if (++k == P.q) k = 0;
-    }
-    patterns[id] = word;
-}
-
-// Description of one class-layout table: m rows of `length` words, bit j of
-// word u of row rho = AND over the prime factors q of
-// prime_bit(.., rho mod q, (S u + M j) mod q), read from q's pattern rows.
-struct TableSpec {
-    long long offset;
-    int m;
-    int nf;
-    int q[kSweepRowFactors];
-    int length;
-    long long pattern[kSweepRowFactors];  // word offset of q's pattern row 0
-    int pattern_words[kSweepRowFactors];
-    int s_mod[kSweepRowFactors];          // S mod q
-    int step_inv[kSweepRowFactors];       // (M mod q)^-1 mod q
-};
-
-__global__ void class_table_kernel(u64 *rows, const TableSpec *specs, int nspecs, const u64 *patterns,
-                                   long long total) {
-    const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (id >= total) return;
-    int lo = 0, hi = nspecs - 1;  // last spec with offset <= id
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (specs[mid].offset <= id) lo = mid;
-        else hi = mid - 1;
-    }
-    const TableSpec &S = specs[lo];
-    const long long rel = id - S.offset;
-    const int rho = int(rel / S.length);
-    const int u = int(rel % S.length) % S.m;
-    u64 word = ~u64(0);
-    for (int f = 0; f < S.nf; ++f) {
-        const int q = S.q[f];
-        const int x0 = int((long long)S.s_mod[f] * u % q);
-        const int k0 = int((long long)x0 * S.step_inv[f] % q);
-        const u64 *row = patterns + S.pattern[f] + (long long)(rho % q) * S.pattern_words[f];
-        const int w = k0 >> 6, sh = k0 & 63;
-        const u64 lo_word = __ldg(row + w), hi_word = __ldg(row + w + 1);
-        word &= sh ? (lo_word >> sh) | (hi_word << (64 - sh)) : lo_word;
-    }
-    rows[id] = word;
-}
-
-// The class lists: block b < Q writes the entries of denominators d = b
-// (mod Q), block Q + b those of d = b (mod two).  A residue r mod Q is
-// admissible if every class prime admits it: bit map adm[(d mod p) p +
-// r mod p]; a residue mod two if bit r of adm2[d mod two] is set.
-struct ClassListSpec {
-    int two, q, two_max, q_max, nprimes, nrows;
-    int p[kSweepClassPrimes];
-    int adm[kSweepClassPrimes];    // byte offset of the prime's map
-    u32 lift2, liftq;              // 1 mod two and 0 mod Q; 0 mod two and 1 mod Q (below M)
-    u32 h2, hq;                    // H mod two, H mod Q
-    u32 m[kSweepRows], inv_stride[kSweepRows], base[kSweepRows];  // base: (-H - M) mod m
-};
-
-__global__ void __launch_bounds__(256) class_list_kernel(ClassListSpec S, const unsigned char *admq, const u64 *adm2,
-                                                         SweepClass *list2, SweepClass *listq, int *count2,
-                                                         int *countq) {
-    __shared__ int s_count[8];
-    __shared__ int s_base;
-    const bool second = int(blockIdx.x) >= S.q;
-    const int dres = second ? int(blockIdx.x) - S.q : int(blockIdx.x);
-    const int n = second ? S.two : S.q;
-    const int room = second ? S.two_max : S.q_max;
-    const u32 M = u32(S.two) * u32(S.q);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_base = 0;
-    __syncthreads();
-    for (int r0 = 0; r0 < n; r0 += 256) {
-        const int r = r0 + int(threadIdx.x);
-        bool ok = r < n;
-        if (second) {
-            ok = ok && ((adm2[dres] >> (r & 63)) & 1);
-        } else {
-            for (int i = 0; i < S.nprimes && ok; ++i)
-                ok = admq[S.adm[i] + (dres % S.p[i]) * S.p[i] + r % S.p[i]] != 0;
-        }
-        const u32 vote = __ballot_sync(kFullMask, ok);
-        if (lane == 0) s_count[warp] = __popc(vote);
-        __syncthreads();
-        int at = s_base + __popc(vote & lanemask_lt());
-        for (int w = 0; w < warp; ++w) at += s_count[w];
-        if (ok && at < room) {
-            SweepClass C{};
-            const u32 v = u32(r) + (second ? S.h2 : S.hq);
-            C.x = u32(u64(second ? S.lift2 : S.liftq) * (v % u32(n)) % M);
-            for (int i = 0; i < S.nrows; ++i) {
-                const u32 m = S.m[i];
-                C.start8[i] = (unsigned short)(8u * ((C.x + (second ? 0u : S.base[i])) % m * S.inv_stride[i] % m));
-            }
-            (second ? list2 : listq)[(long long)dres * room + at] = C;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0)
-            for (int w = 0; w < 8; ++w) s_base += s_count[w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) (second ? count2 : countq)[dres] = s_base;
-}
 
 // A denominator in flight: written by the producer warp, read by the others.
 struct FastSlot {
@@ -273,10 +133,18 @@ struct FastSlot {
     const SweepClass *list;        // residues mod Q in global memory
 };
 
+// The 64 bits from position k of a pattern row.
+__device__ __forceinline__ u64 pattern_window(const u64 *row, u32 k) {
+    const u64 lo = __ldg(row + (k >> 6)), hi = __ldg(row + (k >> 6) + 1);
+    const u32 sh = k & 63u;
+    return sh ? (lo >> sh) | (hi << (64 - sh)) : lo;
+}
+
 // One group of stage 2: candidates ci0, ci0-1, .., ci0-COUNT+1 (descending),
 // each tested on the words whose denominator it does not divide; ndiv counts
-// the candidates that divide it.  The group's table words are loaded together.
-template <int COUNT>
+// the candidates that divide it.  The group's words are loaded together, from
+// class-layout tables (TABLED) or as windows of the pattern rows.
+template <int COUNT, bool TABLED>
 __device__ __forceinline__ void fast_stage2_group(const SweepTables &T, int ci0, u32 hi, u32 lo, u32 d,
                                                   u64 &m, int &ndiv) {
     u64 rows[COUNT];
@@ -290,11 +158,13 @@ __device__ __forceinline__ void fast_stage2_group(const SweepTables &T, int ci0,
         r = mod_small((r << 16) | lo, p, P.magic);  // pos mod p
         r += P.base_mod;                            // a mod p
         if (r >= p) r -= p;
-        const u32 u = mod_small(r * P.inv_stride, p, P.magic);
+        const u32 u = mod_small(r * (TABLED ? P.inv_stride : P.inv_mod), p, P.magic);
         skip[t] = rho == 0;
         ndiv += skip[t] ? 1 : 0;
         rows[t] = ~u64(0);
-        if (m != 0 && P.inv_stride != 0) rows[t] = __ldg(T.rows + P.offset + (long long)rho * p + u);
+        if (m != 0 && P.inv_stride != 0)
+            rows[t] = TABLED ? __ldg(T.rows + P.offset + (long long)rho * p + u)
+                             : pattern_window(T.rows + P.pattern + (long long)rho * P.words, u);
     }
 #pragma unroll
     for (int t = 0; t < COUNT; ++t) m &= skip[t] ? ~u64(0) : rows[t];
@@ -304,14 +174,16 @@ __device__ __forceinline__ void fast_stage2_group(const SweepTables &T, int ci0,
 // reads are uncoalesced, one L1 cycle per lane that asks: lanes whose word is
 // already empty do not (after six primes one word in sixty is left).  A queued
 // word carries its denominator and the position pos = a - abase of its bit 0:
-// its sites are a = abase + pos + M j, and the class-layout row index of prime
-// p is (a mod p) S^-1 mod p in row d mod p.
+// its sites are a = abase + pos + M j.  For prime p they are the 64 bits from
+// position (a mod p) M^-1 mod p of pattern row d mod p, or, tabled, the word
+// (a mod p) S^-1 mod p of class-layout row d mod p.
 // A word meets the reference's selection, the 32 largest of the 36
-// candidates that do not divide d: the 32 largest candidates (six at a time
-// in a loop that is not unrolled, which keeps the kernel's code compact; the
-// warp stops once its words are empty), skipping those dividing d, then, one
-// at a time and only for words where some of those divided d, the four
-// smallest until 32 have been tested.  The few words left meet the late
+// candidates that do not divide d: the 32 largest candidates (the first six,
+// which nearly every word meets, from tables when the curve has them; the
+// others four at a time in a loop that is not unrolled, which keeps the
+// kernel's code compact; the warp stops once its words are empty), skipping
+// those dividing d, then, one at a time and only for words where some of those
+// divided d, the four smallest until 32 have been tested.  The few words left meet the late
 // primes and drop the sites outside the launch's numerators.
 __device__ __forceinline__ void fast_drain(const u64 *qmask, const u64 *qpos, const u32 *qd, int start, int n,
                                            const SweepTables &T, const SweepArgs &A) {
@@ -327,14 +199,22 @@ __device__ __forceinline__ void fast_drain(const u64 *qmask, const u64 *qpos, co
     const u32 hi = u32(pos >> 16), lo = u32(pos & 0xFFFF);
     static_assert(kCandidatePrimes == 36 && kSelectedPrimes == 32, "stage-2 group schedule");
     int ndiv = 0;  // of the candidates tested so far, those dividing d
-#pragma unroll 1
-    for (int g = 0; g + kFStage2Group <= kSelectedPrimes; g += kFStage2Group) {
-        if (!__any_sync(kFullMask, m != 0)) break;
-        fast_stage2_group<kFStage2Group>(T, kCandidatePrimes - 1 - g, hi, lo, d, m, ndiv);
+    int g = 0;
+    if (T.tabled) {
+        fast_stage2_group<kFStage2Group, true>(T, kCandidatePrimes - 1, hi, lo, d, m, ndiv);
+        g = kFStage2Group;
     }
-    constexpr int kRest = kSelectedPrimes % kFStage2Group;
-    if (kRest > 0 && __any_sync(kFullMask, m != 0))
-        fast_stage2_group<kRest>(T, kCandidatePrimes - 1 - (kSelectedPrimes - kRest), hi, lo, d, m, ndiv);
+    constexpr int kLater = 4;  // primes per later group
+    static_assert((kSelectedPrimes - kFStage2Group) % kLater == 2 && kSelectedPrimes % kLater == 0, "group schedule");
+    if (T.tabled && __any_sync(kFullMask, m != 0)) {
+        fast_stage2_group<2, false>(T, kCandidatePrimes - 1 - g, hi, lo, d, m, ndiv);
+        g += 2;
+    }
+#pragma unroll 1
+    for (; g < kSelectedPrimes; g += kLater) {
+        if (!__any_sync(kFullMask, m != 0)) break;
+        fast_stage2_group<kLater, false>(T, kCandidatePrimes - 1 - g, hi, lo, d, m, ndiv);
+    }
     // candidates 3, 2, 1, 0 make up for the larger ones that divide d
 #pragma unroll
     for (int ci = 3; ci >= 0; --ci) {
@@ -347,8 +227,8 @@ __device__ __forceinline__ void fast_drain(const u64 *qmask, const u64 *qpos, co
             r = mod_small((r << 16) | lo, p, P.magic);
             r += P.base_mod;
             if (r >= p) r -= p;
-            const u32 u = mod_small(r * P.inv_stride, p, P.magic);
-            if (P.inv_stride != 0) m &= __ldg(T.rows + P.offset + (long long)rho * p + u);
+            const u32 u = mod_small(r * P.inv_mod, p, P.magic);
+            if (P.inv_stride != 0) m &= pattern_window(T.rows + P.pattern + (long long)rho * P.words, u);
             --ndiv;  // one of the 32 taken by a smaller candidate
         }
     }
@@ -361,8 +241,8 @@ __device__ __forceinline__ void fast_drain(const u64 *qmask, const u64 *qpos, co
                 const LatePrime P = T.late[l];
                 long long r = a0 % (long long)P.p;
                 if (r < 0) r += P.p;
-                const u32 u = u32(r) * P.inv_stride % P.p;
-                m &= __ldg(T.rows + P.offset + (long long)(d % P.p) * P.p + u);
+                const u32 u = u32(r) * P.inv_mod % P.p;
+                m &= pattern_window(T.rows + P.pattern + (long long)(d % P.p) * P.words, u);
             }
         }
         if (a0 < A.a_lo || a0 + 63 * M > A.a_hi) {  // ends of the numerator range
@@ -392,6 +272,7 @@ __device__ __forceinline__ void fast_drain(const u64 *qmask, const u64 *qpos, co
         if (at < A.capacity) {
             A.out_a[at] = a0 + M * bit;
             A.out_d[at] = int(d);
+            if (A.out_curve) A.out_curve[at] = A.curve;
         }
         ++at;
     }
@@ -488,6 +369,7 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
         // to the slots in order.
         int b = 0, round = 0;      // slot of the next fill, and how often it has been filled
         bool failed = false;
+        unsigned long long swept = 0;  // class words handed out
         int rot = 0;               // sweep items handed out so far, mod the consumer count
         const SweepRow R = T.row[lane < NS ? lane : 0];  // the row this lane copies
         const int chunk_size = A.chunk;
@@ -518,7 +400,7 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
             bool hit = false;
 #pragma unroll 4
             for (int i = 0; i < T.nbad; ++i) hit |= u32(k) * T.bad[i].x <= T.bad[i].y;
-            if (hit) nq = 0;
+            if (hit || du * T.need.x > T.need.y) nq = 0;
             u32 live = __ballot_sync(kFullMask, n2 > 0 && nq > 0);
             while (live) {
                 const int j = __ffs(live) - 1;
@@ -548,6 +430,7 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
                     S.items = items;
                     S.rot = rot;
                     S.list = T.listq + (long long)dq_j * T.q_max;
+                    if (part == 0) swept += (unsigned long long)units * unsigned(n2_j) * kSweepUnit;
                     mbar_arrive_expect_tx(full, u32(T.row_words) * 8u + u32(n2_j) * u32(sizeof(SweepClass)) +
                                                     (listq_staged ? u32(nq_j) * u32(sizeof(SweepClass)) : 0u));
                 }
@@ -574,6 +457,7 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
             }
             if (failed) break;
         }
+        if (A.swept && lane == 0) atomicAdd(A.swept, swept);
         if (!failed) {
             // no more work: an empty slot fill tells the consumers to finish
             if (acquire_slot()) {

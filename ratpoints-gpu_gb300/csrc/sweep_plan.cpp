@@ -76,7 +76,7 @@ SweepPlan plan_sweep(const SweepInput &in) {
     std::vector<Weighed> primes;
     for (const auto &s : in.primes)
         primes.push_back({s.p, s.admitted, s.divided, s.optional,
-                          s.admitted > 0 ? -std::log2(double(s.admitted) / s.p) : 8.0});
+                          -std::log2(double(s.admitted) / s.p)});
     std::sort(primes.begin(), primes.end(), [](const Weighed &a, const Weighed &b) {
         const double da = a.bits / std::log2(double(a.p)), db = b.bits / std::log2(double(b.p));
         return da != db ? da > db : a.p < b.p;
@@ -109,7 +109,7 @@ SweepPlan plan_sweep(const SweepInput &in) {
         if (c.count == kSweepClassPrimes) return;
         for (int i = from; i < n; ++i) {
             const Weighed &w = primes[std::size_t(i)];
-            if (w.bits < 0.3 || w.admitted == 0) continue;
+            if (w.bits < 0.3) continue;
             const long long q = (long long)c.q * w.p;
             if (sites / (double(c.two) * double(q)) < 640.0) continue;  // classes of ten words at least
             const long long q_max = (long long)c.q_max * std::max(w.admitted, w.divided);
@@ -197,7 +197,15 @@ SweepPlan plan_sweep(const SweepInput &in) {
                     ctas = n_ctas;
                     slots = int(std::min<long long>(kSweepSlots, room / slot));
                 }
-                if (!ctas || (found && cost >= out.cost)) continue;
+                if (!ctas) continue;
+                // the rows' build, about three words per SM cycle over the
+                // device, shared by the denominators
+                if (in.denominators > 0) {
+                    double build = 0;
+                    for (int i = 0; i < p.count; ++i) build += double(p.modulus[i]) * sweep_row_words(p.modulus[i]);
+                    cost += build / 3.0 / in.denominators;
+                }
+                if (found && cost >= out.cost) continue;
                 found = true;
                 out.cost = cost;
                 out.two = c.two;

@@ -26,13 +26,14 @@ constexpr long long kSweepListBytes = 32; // bytes of a class-list entry
 
 struct SweepPrime {
     int p = 0;
-    int admitted = 0;       // residues x with f(x) a square mod p
+    int admitted = 0;       // residues x with f(x) a square mod p (at least one)
     int divided = 0;        // residues admitted where p | d
     bool optional = false;  // stage 2 tests it as well: it may be left out before
 };
 
 struct SweepInput {
     long long bound = 0;
+    double denominators = 0;  // about how many the search has (0: not known)
     int two = 0;            // power of two whose classes the plan filters (0: no such filter, any may be used)
     double two_classes = 1; // mean classes mod two of a denominator that has any
     int two_max = 1;        // most of them

@@ -44,3 +44,17 @@ def test_numerator_ranges(rpg, monkeypatch, plan):
     monkeypatch.setenv("RPG_SURVIVOR_CAPACITY", "64")
     got = sorted(zip(*(v.tolist() for v in rpg.sieve(coeffs, bound, first, last, plan=plan)[:2])))
     assert got == expected and len(expected) > 0
+
+
+def test_primes_without_squares(rpg, oracle):
+    # 2 + 3 (..) is no square mod 3: only denominators divisible by 3 keep
+    # survivors (odd degree), or none at all (even degree, leading coefficient
+    # not a square mod 3)
+    for coeffs in (["2", "3", "-6", "9"], ["5", "3", "-6", "9", "2"], ["2", "15", "-30", "45", "4"]):
+        for first, last in ((1, 40), (13 * 15, 13 * 15 + 3)):
+            assert_same_set(rpg, oracle, coeffs, 50_003, first, last)
+            check(rpg, oracle, coeffs, 50_003, first, last)
+    # modulo a candidate of the reference plan
+    coeffs = ["2", "509", "0", "-1018"]  # 2 is not a square mod 509
+    assert_same_set(rpg, oracle, coeffs, 20_011, 500, 520)
+    check(rpg, oracle, coeffs, 20_011, 500, 520)
