@@ -17,6 +17,7 @@
 #include "preverify.hpp"
 #include "sieve.hpp"
 #include "sieve_device.cuh"
+#include "sweep.hpp"
 #include "tune.hpp"
 
 namespace rpg {
@@ -74,11 +75,6 @@ struct WideCurve {
     long long count_q;             // 2H = count_q M + count_r
     long long aff;                 // u64 offset of the 36 candidate bitmasks
     long long cls;                 // index of the curve's ClassStart[M] block
-    // class lists by denominator class k = (d mod 64) q + (d mod q): counts at
-    // list_count + k, runs at list_runs + k list_max, item prefixes at
-    // list_prefix + k (list_max + 1); list_count = -1 for curves with x
-    // intervals (their classes are clipped per denominator)
-    long long list_count, list_runs, list_prefix;
     Modulus mod[kWideSlots];
     u64 admissible[64 + kAdmQ];    // 2-adic classes by d mod 64, residues mod q by d mod q
     int count_r;
@@ -87,13 +83,9 @@ struct WideCurve {
     int h_mod_m;                   // H mod M
     int inv64_q;                   // 64^-1 mod q (CRT)
     int smem_words;
-    int list_max;                  // class-list stride: most classes of one denominator
-    int list_steps;                // classes of at most 128 words: 32-word steps per class
-                                   // (their items are kWK classes swept side by side); else 0
     int square;
     int index;                     // position in the caller's curve list
     int rows;                      // stage-1 moduli in use (the others are padding)
-    int pad0;
     u64 denom_primes[2];           // bit i: odd prime i of the OddPrime table is a denominator prime
     unsigned short neg_h[kCandidatePrimes];   // (-H) mod p
     unsigned short s_mod[kCandidatePrimes];   // S mod p
@@ -403,17 +395,15 @@ __device__ __forceinline__ bool has_denominator_prime(u32 k, u64 mask0, u64 mask
 }
 
 // ---------------------------------------------------------------------------
-// Wide rows: class layout, warp-specialized like the single-curve fast
-// kernel.  Warp 0 produces denominators into two slots: it takes work items
-// (curve, parameter range, numerator range) from the device queue, skips
-// parameters without admissible classes or with a denominator prime, points
-// the slot at the curve's class list for the
-// denominator's class k = (d mod 64) q + (d mod q) (or, for curves with x
-// intervals, lays out the classes clipped to the numerator range in shared
-// memory), and copies the curve's stage-1 rows into the slot by TMA.  The
-// other warps sweep each filled slot's items and release it; queued words
-// carry a private context (curve, d), so they wait past later
-// denominators and curves.  No barrier spans the CTA.
+// Wide rows with x intervals: class layout, warp-specialized like the
+// single-curve kernel (which sweeps the wide rows without intervals).  Warp 0
+// produces denominators into two slots: it takes work items (curve, parameter
+// range, numerator range) from the device queue, skips parameters without
+// admissible classes or with a denominator prime, lays out the classes clipped
+// to the numerator range in shared memory, and copies the curve's stage-1 rows
+// into the slot by TMA.  The other warps sweep each filled slot's items and
+// release it; queued words carry a private context (curve, d), so they wait
+// past later denominators and curves.  No barrier spans the CTA.
 
 // One class of one denominator in the numerator range being swept: class
 // words [wbase, wbase + words); the first word drops its `first` low bits,
@@ -426,13 +416,7 @@ struct WideRun {
     unsigned char first;
     unsigned char last;            // 1..64
     unsigned short start[kWideSlots];
-    unsigned int pad[2];           // 32 bytes: class lists are copied by TMA in whole 16-byte units
 };
-static_assert(sizeof(WideRun) == 32, "packed class run");
-
-// Item prefixes of a class list are stored at a stride of whole 16-byte
-// units, so that a list's prefix row starts 16-byte aligned.
-__host__ __device__ inline int wide_prefix_stride(int max_classes) { return (max_classes + 1 + 3) & ~3; }
 
 // Per curve and class residue r mod M (precomputed on the host): the row
 // index of class word 0 for each modulus, (a0 S^-1) mod m with a0 = -H + ofs.
@@ -455,7 +439,6 @@ struct WideSlot {
     int curve;
     int nclass;
     int next;                      // sweep-item counter
-    int steps;                     // > 0: items are groups of kWK short classes, this many steps
 };
 
 // A denominator a consumer warp still has queued words of.
@@ -590,9 +573,7 @@ __device__ __forceinline__ int wide_layout(const WideCurve &C, const ClassStart 
 __global__ void __launch_bounds__(kWThreads, 2)
     wide_kernel(const WideCurve *__restrict__ curves, const BatchItem *__restrict__ items,
                 int nitems, const u64 *__restrict__ pool, const u64 *__restrict__ affine,
-                const ClassStart *__restrict__ class_starts, const WideRun *__restrict__ list_runs,
-                const int *__restrict__ list_prefix, const int *__restrict__ list_count,
-                const unsigned short *__restrict__ inv_table, const OddPrime *__restrict__ odd,
+                const ClassStart *__restrict__ class_starts, const unsigned short *__restrict__ inv_table, const OddPrime *__restrict__ odd,
                 Candidates cand, BatchOut out, int row_stride, int max_classes, unsigned long long *work,
                 unsigned long long *swept) {
     extern __shared__ __align__(16) u64 smem[];
@@ -600,7 +581,7 @@ __global__ void __launch_bounds__(kWThreads, 2)
     u64 *qpos = qmask + kWConsumers * kQueue;
     WideRun *runs0 = reinterpret_cast<WideRun *>(qpos + kWConsumers * kQueue);  // [slots][max_classes]
     int *prefix0 = reinterpret_cast<int *>(runs0 + kWSlotCount * max_classes);  // [slots][prefix stride]
-    const int pstride = wide_prefix_stride(max_classes);
+    const int pstride = (max_classes + 1);
     __shared__ WideSlot slot[kWSlotCount];
     __shared__ WideCtx s_ctx[kWConsumers][kWCtx];
     __shared__ unsigned long long s_swept[kWConsumers][2];
@@ -627,7 +608,7 @@ __global__ void __launch_bounds__(kWThreads, 2)
         // Work items come from the device queue with the next item's index
         // fetched ahead; lane j classifies parameter j of each 32 of an item,
         // and the live denominators go to the slots in order.  Lanes
-        // 0 .. kWideSlots-1 copy one row each, lanes 30 and 31 the class list.
+        // 0 .. kWideSlots-1 copy one row each.
         int b = 0;
         int uses[kWSlotCount] = {};  // fills of each slot so far
         bool failed = false;
@@ -646,7 +627,6 @@ __global__ void __launch_bounds__(kWThreads, 2)
             const BatchItem item = items[idx];
             const WideCurve &C = curves[item.curve];
             const int q = C.class_prime;
-            const long long lists = C.list_count;  // -1: classes laid out here
             const unsigned long long magic_q = (~0ull) / u32(q) + 1;
             const u64 bad0 = C.denom_primes[0], bad1 = C.denom_primes[1];
             for (int base = 0; base < item.count && !failed; base += kWarpSize) {
@@ -655,25 +635,16 @@ __global__ void __launch_bounds__(kWThreads, 2)
                 const long long dd = C.square ? k * k : k;
                 const u32 dv = u32(dd);
                 const int dq = q > 1 ? int(mod_u32(dv, u32(q), magic_q)) : 0;
-                const int combo = int(dv & 63) * q + dq;
-                int nlist = 0;
                 bool live = false;
                 if (valid) {
-                    if (lists >= 0) {
-                        nlist = __ldg(list_count + lists + combo);
-                        live = nlist > 0;
-                    } else {
-                        long long L, U;
-                        live = C.admissible[dv & 63] != 0 && (q == 1 || C.admissible[64 + dq] != 0) &&
-                               (C.nint == 0 || x_range(C.lo, C.hi, C.nint, C.bound, dd, item.range, L, U));
-                    }
+                    long long L, U;
+                    live = C.admissible[dv & 63] != 0 && (q == 1 || C.admissible[64 + dq] != 0) &&
+                           x_range(C.lo, C.hi, C.nint, C.bound, dd, item.range, L, U);
                 }
                 if (bad0 | bad1) live = live && !has_denominator_prime(u32(k), bad0, bad1, odd);
                 for (u32 todo = __ballot_sync(kFullMask, live); todo; todo &= todo - 1) {
                     const int j = __ffs(todo) - 1;
                     const long long d = __shfl_sync(kFullMask, dd, j);
-                    const int combo_j = __shfl_sync(kFullMask, combo, j);
-                    const int nlist_j = __shfl_sync(kFullMask, nlist, j);
                     if (!acquire_slot()) {
                         failed = true;
                         break;
@@ -690,26 +661,17 @@ __global__ void __launch_bounds__(kWThreads, 2)
                     }
                     WideRun *runs = runs0 + b * max_classes;
                     int *prefix = prefix0 + b * pstride;
-                    // a class list goes next to the slot by TMA with the rows
-                    u32 list_bytes = 0, prefix_bytes = 0;
-                    int nclass = nlist_j;
-                    if (lists >= 0) {
-                        list_bytes = u32(nlist_j) * u32(sizeof(WideRun));
-                        prefix_bytes = u32(wide_prefix_stride(nlist_j)) * 4u;  // within the list's stride
-                    } else {
-                        nclass = wide_layout(C, class_starts + C.cls, du, d, item.range, runs, prefix);
-                    }
+                    const int nclass = wide_layout(C, class_starts + C.cls, du, d, item.range, runs, prefix);
                     __syncwarp();
                     if (lane == 0) {
                         S.runs = runs;
                         S.prefix = prefix;
                         S.nclass = nclass;
-                        S.steps = lists >= 0 ? C.list_steps : 0;
                         S.d = d;
                         S.curve = item.curve;
                         S.next = 0;
                         __threadfence_block();
-                        mbar_arrive_expect_tx(full, u32(C.smem_words) * 8u + list_bytes + prefix_bytes);
+                        mbar_arrive_expect_tx(full, u32(C.smem_words) * 8u);
                     }
                     __syncwarp();
                     if (lane < kWideSlots) {
@@ -721,16 +683,6 @@ __global__ void __launch_bounds__(kWThreads, 2)
                         bulk_copy_to_shared(smem_addr(smem + b * row_stride) + u32(Md.smem_offset) * 8u,
                                             pool + Md.offset + (long long)rho * Md.length,
                                             u32(Md.length) * 8u, full);
-                    } else if (list_bytes && lane >= kWarpSize - 2) {
-                        fence_proxy_async_shared();
-                        const int lm = C.list_max;
-                        if (lane == kWarpSize - 2)
-                            bulk_copy_to_shared(smem_addr(runs), list_runs + C.list_runs + (long long)combo_j * lm,
-                                                list_bytes, full);
-                        else
-                            bulk_copy_to_shared(smem_addr(prefix),
-                                                list_prefix + C.list_prefix + (long long)combo_j * wide_prefix_stride(lm),
-                                                prefix_bytes, full);
                     }
 #pragma unroll
                     for (int t = 0; t < kWSlotCount; ++t) uses[t] += t == b ? 1 : 0;
@@ -816,172 +768,89 @@ __global__ void __launch_bounds__(kWThreads, 2)
         const WideRun *runs = S.runs;
         const int *prefix = S.prefix;
         const int nclass = S.nclass;
-        const int nsteps = S.steps;
-        if (nsteps > 0) {
-            // Short classes (at most 128 words): an item is kWK classes side
-            // by side, group kk of a lane's words taken from class kk, so a
-            // step covers 32 words of each; a lane's word w of a class is row
-            // word (start + lane) mod m + 32 s, inside the row's 96-word
-            // extension.  o holds byte offsets from the slot's row base.
-            for (;;) {
-                int g = 0;
-                if (lane == 0) g = atomicAdd(const_cast<int *>(&S.next), 1);
-                g = __shfl_sync(kFullMask, g, 0);
-                if (g * kWK >= nclass) break;
-                u32 o[kWideSlots][kWK];
-                u32 meta[kWK];  // class words (bits 0..7), valid bits of its last word (8..15), ofs (16..31)
+        u32 step8[kWideSlots], mod8[kWideSlots];
+        const unsigned char *slot_base[kWideSlots];
+#pragma unroll
+        for (int sl = 0; sl < kWideSlots; ++sl) {
+            step8[sl] = S.step8[sl];
+            mod8[sl] = 8u * S.m[sl];
+            slot_base[sl] = sbase + S.soff[sl];
+        }
+        const int total_items = prefix[nclass];
+        int c = 0;  // this warp's items of a slot only increase: so do their classes
+        for (;;) {
+            int sweep = 0;
+            if (lane == 0) sweep = atomicAdd(const_cast<int *>(&S.next), 1);
+            sweep = __shfl_sync(kFullMask, sweep, 0);
+            if (sweep >= total_items) break;
+            // class index: largest c with prefix[c] <= sweep, from the last one on
+            for (int base = c; base < nclass; base += 32) {
+                const int cc = base + lane;
+                const u32 bb = __ballot_sync(kFullMask, cc < nclass && prefix[cc] <= sweep);
+                if (bb) c = base + 31 - __clz(bb);
+                if (bb != kFullMask) break;
+            }
+            const int w0 = (sweep - prefix[c]) * kWItemWords;
+            const WideRun run = runs[c];
+            const int wt = run.words;
+            if (lane == 0) {
+                const u32 words = u32(min(kWItemWords, wt - w0));
+                my_swept[0] += words;
+                my_swept[1] += 8ull * words * rows;
+            }
+            const u64 first_mask = ~u64(0) << run.first;
+            const u64 last_mask = run.last >= 64 ? ~u64(0) : ((u64(1) << run.last) - 1);
+            const u64 pos0 = u64(run.ofs) + stride * u64(run.wbase);
+            u32 o[kWideSlots];
+#pragma unroll
+            for (int sl = 0; sl < kWideSlots; ++sl)
+                o[sl] = 8u * mod_u32(u32(run.start[sl]) + u32(w0 + lane), S.m[sl], S.magic[sl]);
+#pragma unroll 1
+            for (int step = 0; step < kWSteps; ++step) {
+                const int ws = w0 + step * kWarpSize * kWK;
+                if (ws >= wt) break;
+                // a class's last step often covers fewer than kWK groups of
+                // 32 words (short rows): the groups past its end are skipped
+                const int nk = min(kWK, (wt - ws + kWarpSize - 1) / kWarpSize);
+                u64 acc[kWK];
+#pragma unroll
+                for (int kk = 0; kk < kWK; ++kk)
+                    acc[kk] = kk < nk ? *reinterpret_cast<const u64 *>(slot_base[0] + o[0] + 256 * kk) : 0;
+#pragma unroll
+                for (int sl = 1; sl < kWideSlots; ++sl) {
+#pragma unroll
+                    for (int kk = 0; kk < kWK; ++kk)
+                        if (kk < nk) acc[kk] &= *reinterpret_cast<const u64 *>(slot_base[sl] + o[sl] + 256 * kk);
+                }
+#pragma unroll
+                for (int sl = 0; sl < kWideSlots; ++sl) {
+                    // advance (32 kWK) mod m words; unsigned min wraps into [0, m)
+                    const u32 t = o[sl] + step8[sl];
+                    o[sl] = min(t, t - mod8[sl]);
+                }
+                const u64 any = acc[0] | acc[1] | acc[2] | acc[3];
+                if (!__ballot_sync(kFullMask, any != 0)) continue;
 #pragma unroll
                 for (int kk = 0; kk < kWK; ++kk) {
-                    const int cc = g * kWK + kk;
-                    meta[kk] = 0;
-#pragma unroll
-                    for (int sl = 0; sl < kWideSlots; ++sl) o[sl][kk] = S.soff[sl];
-                    if (cc < nclass) {
-                        const WideRun run = runs[cc];
-                        meta[kk] = u32(run.words) | (u32(run.last) << 8) | (u32(run.ofs) << 16);
-#pragma unroll
-                        for (int sl = 0; sl < kWideSlots; ++sl) {
-                            const u32 m = S.m[sl];
-                            const u32 v = u32(run.start[sl]) + u32(lane);
-                            o[sl][kk] += 8u * (m >= 32 ? (v >= m ? v - m : v) : mod_u32(v, m, S.magic[sl]));
+                    if (kk >= nk) break;
+                    const int w = ws + kWarpSize * kk + lane;
+                    u64 a = acc[kk];
+                    if (w == 0) a &= first_mask;
+                    if (w == wt - 1) a &= last_mask;
+                    const bool live_word = a != 0 && w < wt;
+                    const u32 bb = __ballot_sync(kFullMask, live_word);
+                    if (bb) {
+                        const int at = qn + __popc(bb & lanemask_lt());
+                        if (live_word) {
+                            wq_mask[at] = a;
+                            wq_pos[at] = tag | (pos0 + stride * u64(w));
                         }
-                    }
-                }
-                if (lane == 0) {
-                    const u32 words = (meta[0] & 0xFFu) + (meta[1] & 0xFFu) + (meta[2] & 0xFFu) + (meta[3] & 0xFFu);
-                    my_swept[0] += words;
-                    my_swept[1] += 8ull * words * rows;
-                }
-#pragma unroll 1
-                for (int step = 0; step < nsteps; ++step) {
-                    u64 acc[kWK];
-#pragma unroll
-                    for (int kk = 0; kk < kWK; ++kk)
-                        acc[kk] = *reinterpret_cast<const u64 *>(sbase + o[0][kk] + 256 * step);
-#pragma unroll
-                    for (int sl = 1; sl < kWideSlots; ++sl) {
-#pragma unroll
-                        for (int kk = 0; kk < kWK; ++kk)
-                            acc[kk] &= *reinterpret_cast<const u64 *>(sbase + o[sl][kk] + 256 * step);
-                    }
-                    const int w = kWarpSize * step + lane;
-#pragma unroll
-                    for (int kk = 0; kk < kWK; ++kk) {
-                        const int wk = int(meta[kk] & 0xFFu);
-                        if (w == wk - 1) {
-                            const u32 last = (meta[kk] >> 8) & 0xFFu;
-                            if (last < 64) acc[kk] &= (u64(1) << last) - 1;
-                        }
-                        if (w >= wk) acc[kk] = 0;
-                    }
-                    const u64 any = acc[0] | acc[1] | acc[2] | acc[3];
-                    if (!__ballot_sync(kFullMask, any != 0)) continue;
-#pragma unroll
-                    for (int kk = 0; kk < kWK; ++kk) {
-                        const bool live_word = acc[kk] != 0;
-                        const u32 bb = __ballot_sync(kFullMask, live_word);
-                        if (bb) {
-                            const int at = qn + __popc(bb & lanemask_lt());
-                            if (live_word) {
-                                wq_mask[at] = acc[kk];
-                                wq_pos[at] = tag | (u64(meta[kk] >> 16) + stride * u64(w));
-                            }
-                            qn += __popc(bb);
-                            if (qn >= 32) {
-                                __syncwarp();
-                                wide_drain(wq_mask, wq_pos, qn - 32, 32, curves, affine, cand, inv_table, ctx, out);
-                                qn -= 32;
-                                if (qn == 0) oldest = seq;
-                            }
-                        }
-                    }
-                }
-            }
-        } else {
-            u32 step8[kWideSlots], mod8[kWideSlots];
-            const unsigned char *slot_base[kWideSlots];
-#pragma unroll
-            for (int sl = 0; sl < kWideSlots; ++sl) {
-                step8[sl] = S.step8[sl];
-                mod8[sl] = 8u * S.m[sl];
-                slot_base[sl] = sbase + S.soff[sl];
-            }
-            const int total_items = prefix[nclass];
-            int c = 0;  // this warp's items of a slot only increase: so do their classes
-            for (;;) {
-                int sweep = 0;
-                if (lane == 0) sweep = atomicAdd(const_cast<int *>(&S.next), 1);
-                sweep = __shfl_sync(kFullMask, sweep, 0);
-                if (sweep >= total_items) break;
-                // class index: largest c with prefix[c] <= sweep, from the last one on
-                for (int base = c; base < nclass; base += 32) {
-                    const int cc = base + lane;
-                    const u32 bb = __ballot_sync(kFullMask, cc < nclass && prefix[cc] <= sweep);
-                    if (bb) c = base + 31 - __clz(bb);
-                    if (bb != kFullMask) break;
-                }
-                const int w0 = (sweep - prefix[c]) * kWItemWords;
-                const WideRun run = runs[c];
-                const int wt = run.words;
-                if (lane == 0) {
-                    const u32 words = u32(min(kWItemWords, wt - w0));
-                    my_swept[0] += words;
-                    my_swept[1] += 8ull * words * rows;
-                }
-                const u64 first_mask = ~u64(0) << run.first;
-                const u64 last_mask = run.last >= 64 ? ~u64(0) : ((u64(1) << run.last) - 1);
-                const u64 pos0 = u64(run.ofs) + stride * u64(run.wbase);
-                u32 o[kWideSlots];
-#pragma unroll
-                for (int sl = 0; sl < kWideSlots; ++sl)
-                    o[sl] = 8u * mod_u32(u32(run.start[sl]) + u32(w0 + lane), S.m[sl], S.magic[sl]);
-#pragma unroll 1
-                for (int step = 0; step < kWSteps; ++step) {
-                    const int ws = w0 + step * kWarpSize * kWK;
-                    if (ws >= wt) break;
-                    // a class's last step often covers fewer than kWK groups of
-                    // 32 words (short rows): the groups past its end are skipped
-                    const int nk = min(kWK, (wt - ws + kWarpSize - 1) / kWarpSize);
-                    u64 acc[kWK];
-#pragma unroll
-                    for (int kk = 0; kk < kWK; ++kk)
-                        acc[kk] = kk < nk ? *reinterpret_cast<const u64 *>(slot_base[0] + o[0] + 256 * kk) : 0;
-#pragma unroll
-                    for (int sl = 1; sl < kWideSlots; ++sl) {
-#pragma unroll
-                        for (int kk = 0; kk < kWK; ++kk)
-                            if (kk < nk) acc[kk] &= *reinterpret_cast<const u64 *>(slot_base[sl] + o[sl] + 256 * kk);
-                    }
-#pragma unroll
-                    for (int sl = 0; sl < kWideSlots; ++sl) {
-                        // advance (32 kWK) mod m words; unsigned min wraps into [0, m)
-                        const u32 t = o[sl] + step8[sl];
-                        o[sl] = min(t, t - mod8[sl]);
-                    }
-                    const u64 any = acc[0] | acc[1] | acc[2] | acc[3];
-                    if (!__ballot_sync(kFullMask, any != 0)) continue;
-#pragma unroll
-                    for (int kk = 0; kk < kWK; ++kk) {
-                        if (kk >= nk) break;
-                        const int w = ws + kWarpSize * kk + lane;
-                        u64 a = acc[kk];
-                        if (w == 0) a &= first_mask;
-                        if (w == wt - 1) a &= last_mask;
-                        const bool live_word = a != 0 && w < wt;
-                        const u32 bb = __ballot_sync(kFullMask, live_word);
-                        if (bb) {
-                            const int at = qn + __popc(bb & lanemask_lt());
-                            if (live_word) {
-                                wq_mask[at] = a;
-                                wq_pos[at] = tag | (pos0 + stride * u64(w));
-                            }
-                            qn += __popc(bb);
-                            if (qn >= 32) {
-                                __syncwarp();
-                                wide_drain(wq_mask, wq_pos, qn - 32, 32, curves, affine, cand, inv_table, ctx, out);
-                                qn -= 32;
-                                if (qn == 0) oldest = seq;
-                            }
+                        qn += __popc(bb);
+                        if (qn >= 32) {
+                            __syncwarp();
+                            wide_drain(wq_mask, wq_pos, qn - 32, 32, curves, affine, cand, inv_table, ctx, out);
+                            qn -= 32;
+                            if (qn == 0) oldest = seq;
                         }
                     }
                 }
@@ -1320,12 +1189,6 @@ void denominator_prime_mask(const std::vector<std::string> &coefficients, int sk
     }
 }
 
-// Position of the k-th set bit (k counted from 0) of a 64-bit mask.
-int nth_bit_host(dev::u64 mask, int k) {
-    for (int i = 0; i < k; ++i) mask &= mask - 1;
-    return __builtin_ctzll(mask);
-}
-
 bool lead_is_square(const std::vector<std::string> &coefficients, int q) {
     const int n = int(coefficients.size()) - 1;
     if (n % 2) return true;  // odd degree: F(a, d) = d (...) vanishes mod q | d
@@ -1390,6 +1253,7 @@ struct CurveWork {
     dev::u64 adm2[64] = {};    // 2-adic admissible classes by d mod 64
     int classes = 1;           // wide curves: most numerator classes of one denominator
     std::unique_ptr<FastPlanner> planner;  // wide curves, until planned
+    std::unique_ptr<SweepCurve> sweep;     // curves swept by launches of their own
     std::vector<unsigned short> cand_residues;  // c_i mod p for the 36 candidates, candidate-major
     dev::u64 denom_primes[2] = {};             // the curve's denominator primes (no class prime removed)
 };
@@ -1409,6 +1273,20 @@ long long swept_row_words(const BatchCurveSpec &c, long long words) {
         total += std::min(double(words), len * d / 64.0 + 2.0);
     }
     return std::min(words, (long long)std::ceil(total));
+}
+
+// Whether a curve gets sieve launches of its own (sweep.hpp) instead of work
+// items of the batched kernels.  Rows of at least kBatchWideWords words always
+// do; shorter ones when the narrow kernel's time for them, 0.45 ns per
+// denominator and 1.85e-3 ns per row word, exceeds the sweep's (0.9 to 1.1 ns
+// per denominator up to H = 65,504) by more than building the curve's tables
+// takes (400,000 denominators of sextics, narrow and sweep: H = 5,000 0.35 and
+// 0.40 ms, 10,000 0.45 and 0.38, 20,000 0.66 and 0.38, 65,000 1.7 and 0.40).
+// Curves with x intervals stay in the kernels that sweep only those.
+bool swept_alone(const BatchCurveSpec &c, const CurveWork &cw) {
+    if (!c.intervals.empty() && c.intervals.size() <= std::size_t(dev::kMaxIntervals)) return false;
+    if (cw.wide) return true;
+    return double(cw.count) * (1.85e-3 * double(cw.words) - 0.6) > 20000.0;
 }
 
 // Narrow plan: every odd prime up to kBatchNarrowModulus that filters at
@@ -1469,8 +1347,8 @@ long long wide_row_budget(int max_classes) {
     const long long per_cta = 228 * 1024 / 2 - 1024;
     const long long fixed = 6 * 1024 +  // static shared memory of the kernel (5 KB) and slack
                             (long long)dev::kWConsumers * dev::kQueue * 16 +
-                            (long long)dev::kWSlotCount * max_classes * (long long)sizeof(dev::WideRun) +
-                            (long long)dev::kWSlotCount * dev::wide_prefix_stride(max_classes) * 4;
+                            (long long)dev::kWSlotCount * max_classes * 32 +
+                            (long long)dev::kWSlotCount * ((max_classes + 4) & ~3) * 4;
     return std::max(2LL * 64, (per_cta - fixed) / 8);
 }
 
@@ -1530,6 +1408,7 @@ namespace {
 // and work items, built on the host from the curves' plans.
 struct BatchPlan {
     std::vector<CurveWork> work;
+    std::vector<std::size_t> sweeps;           // curves with launches of their own
     std::vector<dev::WideCurve> wide;
     std::vector<dev::NarrowCurve> narrow;
     std::vector<dev::AffineSpec> aspecs;
@@ -1538,8 +1417,6 @@ struct BatchPlan {
     std::vector<dev::CompositeSpec> cspecs;
     std::vector<dev::BatchItem> wide_items, narrow_items;
     std::vector<dev::ClassStart> class_starts;
-    std::vector<dev::WideRun> list_runs;       // class lists of wide curves without x intervals
-    std::vector<int> list_prefix, list_count;
     long long aff_words = 0, pattern_words = 0, row_words = 0;
     int wide_smem_words = 0;
     int wide_max_classes = 1;   // most classes of a denominator of any wide curve
@@ -1572,6 +1449,12 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
             cw.count = c.last >= c.first ? c.last - c.first + 1 : 0;
             cw.swept = swept_row_words(c, cw.words);
             cw.wide = cw.swept >= kBatchWideWords;
+            if (cw.count > 0 && swept_alone(c, cw)) {
+                cw.plan = single_curve_plan(c.coefficients, c.bound, nullptr);
+                cw.sweep.reset(new SweepCurve(c.coefficients, c.bound, c.square, &cw.plan, double(cw.count)));
+                cw.ok = true;
+                return;
+            }
             two_adic_classes(c.coefficients, cw.adm2);
             if (cw.wide) {
                 cw.planner.reset(new FastPlanner(c.coefficients, c.bound, true, kFastPrimeLimit));
@@ -1597,11 +1480,11 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
     // of its curves (each slot holds its denominator's classes)
     int max_classes = 1;
     for (std::size_t i = 0; i < curves.size(); ++i)
-        if (P.work[i].ok && P.work[i].wide) max_classes = std::max(max_classes, P.work[i].classes);
+        if (P.work[i].ok && P.work[i].wide && !P.work[i].sweep) max_classes = std::max(max_classes, P.work[i].classes);
     parallel_for(curves.size(), [&](std::size_t i) {
         CurveWork &cw = P.work[i];
         if (!cw.ok) return;
-        if (cw.wide) {
+        if (cw.wide && !cw.sweep) {
             cw.plan = wide_plan(*cw.planner, (long double)cw.words * cw.count, max_classes);
             cw.planner.reset();
         }
@@ -1624,13 +1507,28 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
     };
     // largest work first, so that the persistent kernels end on small items
     std::vector<std::size_t> order;
-    for (std::size_t i = 0; i < curves.size(); ++i)
-        if (P.work[i].ok && P.work[i].count > 0) order.push_back(i);
+    for (std::size_t i = 0; i < curves.size(); ++i) {
+        const CurveWork &cw = P.work[i];
+        if (!cw.ok || cw.count <= 0) continue;
+        if (!cw.sweep) {
+            order.push_back(i);
+            continue;
+        }
+        P.sweeps.push_back(i);
+        stats.rectangle_sites += (long double)(2 * curves[i].bound + 1) * (long double)cw.count;
+        stats.denominators += (unsigned long long)cw.count;
+        stats.words += (unsigned long long)(cw.words * cw.count);
+        stats.curves += 1;
+        stats.wide_curves += cw.wide ? 1 : 0;
+    }
+    // the longest first, so that the device is shared to the end
+    std::stable_sort(P.sweeps.begin(), P.sweeps.end(), [&](std::size_t a, std::size_t b) {
+        return P.work[a].sweep->cost(double(P.work[a].count)) > P.work[b].sweep->cost(double(P.work[b].count));
+    });
     std::stable_sort(order.begin(), order.end(), [&](std::size_t a, std::size_t b) {
         return (long double)P.work[a].words * P.work[a].count >
                (long double)P.work[b].words * P.work[b].count;
     });
-    std::vector<std::pair<std::size_t, std::size_t>> list_curves;  // (descriptor, curve) with class lists
     // items: large enough that building and fetching them stays cheap, small
     // enough that a small batch still spreads over the device (about
     // items_per_kernel items per kernel): up to 2^21 row words (wide) and 2^18
@@ -1663,7 +1561,6 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
         P.wide_items.reserve(wide_items);
         P.narrow_items.reserve(narrow_items);
     }
-    long long list_count_total = 0, list_runs_total = 0, list_prefix_total = 0;
     for (std::size_t i : order) {
         const BatchCurveSpec &c = curves[i];
         CurveWork &cw = P.work[i];
@@ -1791,25 +1688,6 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
                 C.m_mod[ci] = (unsigned short)(M % p);
             }
             device_intervals(c.intervals, C.nint, C.lo, C.hi);
-            C.list_max = std::max(1, cw.classes);
-            if (C.nint == 0) {
-                // room for the curve's class lists (64 q denominator classes)
-                const int lm = C.list_max;
-                const std::size_t ncombo = std::size_t(64) * std::size_t(q);
-                C.list_count = list_count_total;
-                C.list_runs = list_runs_total;
-                C.list_prefix = list_prefix_total;  // a multiple of 4: rows start 16-byte aligned
-                list_count_total += (long long)ncombo;
-                list_runs_total += (long long)ncombo * lm;
-                list_prefix_total += (long long)ncombo * dev::wide_prefix_stride(lm);
-                list_curves.push_back({P.wide.size(), i});  // filled below, in parallel
-                // classes of at most 128 words are swept kWK at a time
-                const long long max_words = (C.count_q + 1 + 63) >> 6;
-                C.list_steps = max_words <= 4 * dev::kWarpSize ? int((max_words + dev::kWarpSize - 1) / dev::kWarpSize) : 0;
-            } else {
-                C.list_steps = 0;
-                C.list_count = -1;
-            }
             P.wide_max_classes = std::max(P.wide_max_classes, cw.classes);
             const long long chunk = item_chunk(cw);
             for (int range = 0; range < std::max(1, C.nint); ++range)
@@ -1868,48 +1746,6 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
         }
         stats.curves += 1;
     }
-    // class lists by denominator class k = (d mod 64) q + (d mod q), in the
-    // order the producer lays out classes for interval curves
-    P.list_count.resize(std::size_t(list_count_total));
-    P.list_runs.resize(std::size_t(list_runs_total));
-    P.list_prefix.resize(std::size_t(list_prefix_total));
-    parallel_for(list_curves.size(), [&](std::size_t j) {
-        const dev::WideCurve &C = P.wide[list_curves[j].first];
-        const CurveWork &cw = P.work[list_curves[j].second];
-        const int q = C.class_prime;
-        const int lm = C.list_max;
-        for (int dd = 0; dd < 64; ++dd)
-            for (int dq = 0; dq < q; ++dq) {
-                const std::size_t k = std::size_t(dd) * std::size_t(q) + std::size_t(dq);
-                const dev::u64 classes2 = cw.adm2[dd];
-                const dev::u64 classesq = q > 1 ? C.admissible[64 + dq] : dev::u64(1);
-                const int nq = __builtin_popcountll(classesq);
-                const int nclass = __builtin_popcountll(classes2) * nq;
-                if (nclass > lm) throw std::logic_error("class list longer than its stride");
-                dev::WideRun *runs = P.list_runs.data() + C.list_runs + k * std::size_t(lm);
-                int *prefix = P.list_prefix.data() + C.list_prefix + k * std::size_t(dev::wide_prefix_stride(lm));
-                int items = 0;
-                for (int cidx = 0; cidx < nclass; ++cidx) {
-                    const int r64 = nth_bit_host(classes2, cidx / nq);
-                    int r = r64;
-                    if (q > 1) r = r64 + 64 * int(C.crt[C.mod_q[r64] * 13 + nth_bit_host(classesq, cidx % nq)]);
-                    const dev::ClassStart &cs = P.class_starts[std::size_t(C.cls + r)];
-                    const long long count = C.count_q + (cs.ofs <= C.count_r ? 1 : 0);
-                    const long long words = (count + 63) >> 6;
-                    dev::WideRun &run = runs[cidx];
-                    run.wbase = 0;
-                    run.words = int(words);
-                    run.ofs = cs.ofs;
-                    run.first = 0;
-                    run.last = (unsigned char)(words > 0 ? count - 64 * (words - 1) : 64);
-                    for (int sl = 0; sl < dev::kWideSlots; ++sl) run.start[sl] = cs.start[sl];
-                    prefix[cidx] = items;
-                    items += int((words + dev::kWItemWords - 1) / dev::kWItemWords);
-                }
-                prefix[nclass] = items;
-                P.list_count[std::size_t(C.list_count) + k] = nclass;
-            }
-    });
     stats.wide_items = P.wide_items.size();
     stats.narrow_items = P.narrow_items.size();
     stats.table_words = (unsigned long long)P.row_words;
@@ -1921,6 +1757,11 @@ struct BatchEngine::Impl {
     int device = 0;
     int sms = 0;
     cudaStream_t stream = nullptr, side = nullptr;
+    // the sweeps' launches go round-robin over these and `stream`, so that
+    // the short ones share the device
+    static constexpr int kSweepStreams = 7;
+    cudaStream_t sweep_stream[kSweepStreams] = {};
+    cudaEvent_t sweep_join[kSweepStreams] = {};
     cudaEvent_t ev[6] = {};    // tables, wide kernel, narrow kernel (start, end)
     cudaEvent_t fork = nullptr, join = nullptr;
     // device counters of a run: survivors, wide and narrow work items, error
@@ -1937,13 +1778,13 @@ struct BatchEngine::Impl {
     DeviceArray<dev::PatternSpec> d_pspecs;
     DeviceArray<dev::CompositeSpec> d_cspecs;
     DeviceArray<dev::ClassStart> d_cls;
-    DeviceArray<dev::WideRun> d_lruns;
-    DeviceArray<int> d_lprefix, d_lcount;
     DeviceArray<unsigned short> d_res, d_inv;
     DeviceArray<dev::u64> d_sq, d_aff, d_patterns, d_rows;
     DeviceArray<dev::OddPrime> d_odd;
     // [0] survivors [1] wide work [2] narrow work [3] error [4] pre-verified survivors
+    // [5] swept words [6] their row bytes, then a work counter per sweep
     DeviceArray<unsigned long long> d_counters;
+    DeviceArray<unsigned char> d_sweep_tables;
     DeviceArray<long long> d_a, d_pa;        // survivors, and those kept by pre-verification
     DeviceArray<int> d_d, d_c, d_pd, d_pc;
     DeviceArray<unsigned long long> d_curve_modular;  // per-curve modular survivors
@@ -1956,6 +1797,8 @@ struct BatchEngine::Impl {
                    "cudaDeviceGetAttribute");
         check_cuda(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
         check_cuda(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "cudaStreamCreate");
+        for (auto &s : sweep_stream) check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
+        for (auto &e : sweep_join) check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         for (auto &e : ev) check_cuda(cudaEventCreate(&e), "cudaEventCreate");
         check_cuda(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "cudaEventCreate");
         check_cuda(cudaEventCreateWithFlags(&join, cudaEventDisableTiming), "cudaEventCreate");
@@ -1997,6 +1840,13 @@ struct BatchEngine::Impl {
     ~Impl() {
         if (stream) cudaStreamSynchronize(stream);
         if (side) cudaStreamSynchronize(side);
+        for (auto &s : sweep_stream)
+            if (s) {
+                cudaStreamSynchronize(s);
+                cudaStreamDestroy(s);
+            }
+        for (auto &e : sweep_join)
+            if (e) cudaEventDestroy(e);
         for (auto &e : ev)
             if (e) cudaEventDestroy(e);
         if (fork) cudaEventDestroy(fork);
@@ -2095,7 +1945,7 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
             }
         });
 
-    if (!P.wide.empty() || !P.narrow.empty()) {
+    if (!P.wide.empty() || !P.narrow.empty() || !P.sweeps.empty()) {
         d_wide.upload(P.wide, stream, stats.h2d_bytes, "upload wide curves");
         d_narrow.upload(P.narrow, stream, stats.h2d_bytes, "upload narrow curves");
         d_witems.upload(P.wide_items, stream, stats.h2d_bytes, "upload work items");
@@ -2105,12 +1955,17 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
         d_cspecs.upload(P.cspecs, stream, stats.h2d_bytes, "upload table specs");
         d_res.upload(P.residues, stream, stats.h2d_bytes, "upload residues");
         d_cls.upload(P.class_starts, stream, stats.h2d_bytes, "upload class starts");
-        d_lruns.upload(P.list_runs, stream, stats.h2d_bytes, "upload class lists");
-        d_lprefix.upload(P.list_prefix, stream, stats.h2d_bytes, "upload class lists");
-        d_lcount.upload(P.list_count, stream, stats.h2d_bytes, "upload class lists");
         d_aff.ensure(std::size_t(P.aff_words), "cudaMalloc(batch bitmasks)");
         d_patterns.ensure(std::size_t(P.pattern_words), "cudaMalloc(batch patterns)");
         d_rows.ensure(std::size_t(P.row_words), "cudaMalloc(batch tables)");
+        SweepBuilder sweep_tables;
+        for (std::size_t i : P.sweeps) sweep_tables.add(*work[i].sweep);
+        if (!P.sweeps.empty()) {
+            d_sweep_tables.ensure(sweep_tables.bytes(), "cudaMalloc(sieve tables)");
+            sweep_tables.place(d_sweep_tables.p, stream);
+            stats.h2d_bytes += sweep_tables.upload_bytes();
+        }
+        d_counters.ensure(kCounters + P.sweeps.size(), "cudaMalloc(batch counters)");
         if (preverify) {
             std::vector<const std::vector<std::string> *> coefs(curves.size(), nullptr);
             for (std::size_t i = 0; i < curves.size(); ++i)
@@ -2126,7 +1981,7 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
                                       std::size_t(dev::kWConsumers) * dev::kQueue * 16 +
                                       std::size_t(dev::kWSlotCount) * std::size_t(wide_max_classes) *
                                           sizeof(dev::WideRun) +
-                                      std::size_t(dev::kWSlotCount) * std::size_t(dev::wide_prefix_stride(wide_max_classes)) * 4;
+                                      std::size_t(dev::kWSlotCount) * std::size_t(wide_max_classes + 1) * 4;
         const std::size_t narrow_smem = std::size_t(dev::kNarrowTableWords + dev::kAffWords) * 8 +
                                         std::size_t(dev::kNWarps) * dev::kQueue * 12;
         int wide_grid = 0, narrow_grid = 0;
@@ -2160,7 +2015,8 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
         };
         auto enqueue_sieve = [&]() {
             const dev::BatchOut out{d_a.p, d_d.p, d_c.p, d_counters.p, capacity, d_counters.p + 3};
-            check_cuda(cudaMemsetAsync(d_counters.p, 0, kCounters * sizeof(unsigned long long), stream),
+            check_cuda(cudaMemsetAsync(d_counters.p, 0, (kCounters + P.sweeps.size()) * sizeof(unsigned long long),
+                                       stream),
                        "cudaMemsetAsync");
             if (preverify)
                 check_cuda(cudaMemsetAsync(d_curve_modular.p, 0, curves.size() * sizeof(unsigned long long), stream),
@@ -2170,10 +2026,35 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
             record(ev[2], stream);
             if (wide_grid) {
                 dev::wide_kernel<<<wide_grid, dev::kWThreads, wide_smem, stream>>>(
-                    d_wide.p, d_witems.p, int(P.wide_items.size()), d_rows.p, d_aff.p, d_cls.p, d_lruns.p,
-                    d_lprefix.p, d_lcount.p, d_inv.p, d_odd.p, cand, out, wide_smem_words, wide_max_classes,
+                    d_wide.p, d_witems.p, int(P.wide_items.size()), d_rows.p, d_aff.p, d_cls.p, d_inv.p, d_odd.p, cand, out, wide_smem_words, wide_max_classes,
                     d_counters.p + 1, d_counters.p + 5);
                 check_cuda(cudaGetLastError(), "wide_kernel launch");
+            }
+            const int streams = int(std::min<std::size_t>(kSweepStreams, P.sweeps.size()));
+            for (int k = 0; k < streams; ++k)
+                check_cuda(cudaStreamWaitEvent(sweep_stream[k], fork, 0), "cudaStreamWaitEvent");
+            for (std::size_t j = 0; j < P.sweeps.size(); ++j) {
+                const std::size_t i = P.sweeps[j];
+                SweepLaunch l;
+                l.first = curves[i].first;
+                l.last = curves[i].last;
+                l.a_lo = -curves[i].bound;
+                l.a_hi = curves[i].bound;
+                l.out_a = d_a.p;
+                l.out_d = d_d.p;
+                l.out_curve = d_c.p;
+                l.curve = int(i);
+                l.capacity = capacity;
+                l.out_count = d_counters.p;
+                l.work = d_counters.p + kCounters + j;
+                l.error = d_counters.p + 3;
+                l.swept = d_counters.p + 5;
+                const int k = int(j % std::size_t(kSweepStreams + 1));
+                work[i].sweep->launch(l, k < streams ? sweep_stream[k] : stream);
+            }
+            for (int k = 0; k < streams; ++k) {
+                check_cuda(cudaEventRecord(sweep_join[k], sweep_stream[k]), "cudaEventRecord");
+                check_cuda(cudaStreamWaitEvent(stream, sweep_join[k], 0), "cudaStreamWaitEvent");
             }
             record(ev[3], stream);
             record(ev[4], side);
@@ -2215,6 +2096,7 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
                     d_cspecs.p, int(P.cspecs.size()), d_patterns.p, d_rows.p, P.row_words);
                 check_cuda(cudaGetLastError(), "composite_kernel launch");
             }
+            if (!P.sweeps.empty()) sweep_tables.enqueue(stream);
             record(ev[1], stream);
             enqueue_sieve();
         };
@@ -2248,7 +2130,8 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
             check_cuda(cudaStreamSynchronize(stream), "batch sieve");
         }
         stats.launches += (P.aspecs.empty() ? 0 : 1) + (P.pattern_words ? 1 : 0) + (P.row_words ? 1 : 0) +
-                          (wide_grid ? 1 : 0) + (narrow_grid ? 1 : 0) + (preverify ? 1 : 0);
+                          (wide_grid ? 1 : 0) + (narrow_grid ? 1 : 0) + (preverify ? 1 : 0) +
+                          (P.sweeps.empty() ? 0 : 3 + P.sweeps.size());
         auto elapsed = [&](int a, int b) {
             float ms = 0;
             cudaEventElapsedTime(&ms, ev[a], ev[b]);
@@ -2265,7 +2148,7 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
             enqueue_sieve();
             check_cuda(cudaStreamSynchronize(stream), "batch sieve");
             stats.sieve_ms += std::max(elapsed(2, 3), elapsed(2, 5));
-            stats.launches += (wide_grid ? 1 : 0) + (narrow_grid ? 1 : 0) + (preverify ? 1 : 0);
+            stats.launches += (wide_grid ? 1 : 0) + (narrow_grid ? 1 : 0) + (preverify ? 1 : 0) + P.sweeps.size();
             if (h_counters[3]) throw DeviceTimeout("batched sieve: a bounded wait timed out");
         }
         stats.survivors = h_counters[0];
@@ -2378,6 +2261,8 @@ unsigned long long BatchEngine::estimate_bytes(const BatchCurveSpec &c) {
     } else {
         table = dev::kNarrowTableWords;
     }
+    // curves with launches of their own: pattern rows and candidate tables
+    if (words >= 512 && c.intervals.empty()) table = std::max(table, 1700000LL);
     // tables, bitmasks, patterns, descriptor and items (8-byte words)
     return (unsigned long long)(table + 2 * dev::kAffWords + 6 * 127 * 127 + 1024 +
                                 std::max(1LL, count * std::max(1LL, (long long)c.intervals.size()) /

@@ -55,7 +55,7 @@ struct SweepArgs {
     unsigned long long *out_count;
     unsigned long long capacity;
     unsigned long long *error;   // set nonzero if a bounded device wait ran out (may be null)
-    unsigned long long *swept;   // class words swept (may be null)
+    unsigned long long *swept;   // class words swept and the row bytes they read (may be null)
 };
 
 struct SweepRow {                  // one stage-1 modulus
@@ -457,7 +457,10 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
             }
             if (failed) break;
         }
-        if (A.swept && lane == 0) atomicAdd(A.swept, swept);
+        if (A.swept && lane == 0) {
+            atomicAdd(A.swept, swept);
+            atomicAdd(A.swept + 1, swept * 8ull * NS);
+        }
         if (!failed) {
             // no more work: an empty slot fill tells the consumers to finish
             if (acquire_slot()) {

@@ -24,7 +24,8 @@ struct ListJob;
 // One launch: parameters first .. last (at most 2^31 / 64), numerators
 // a_lo .. a_hi (at most SweepCurve::tile() of them).  Device pointers: the
 // survivor arrays (curve tags only with out_curve), their count, a zeroed work
-// counter, the error word, and (optional) the count of swept words.
+// counter, the error word, and (optional) the counts of swept words and of the
+// row bytes they read.
 struct SweepLaunch {
     long long first = 0, last = 0;
     long long a_lo = 0, a_hi = 0;
@@ -50,6 +51,8 @@ public:
     SweepCurve &operator=(const SweepCurve &) = delete;
 
     const SweepPlan &plan() const { return plan_; }
+    // Modelled work of a pass over `denominators` of them (SM cycles).
+    double cost(double denominators) const { return plan_.cost * denominators / double(need_); }
     // Most numerators of one launch.
     long long tile() const { return tile_; }
     // Words a pass over parameters first .. last sweeps (64 sites each).

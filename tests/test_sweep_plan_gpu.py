@@ -58,3 +58,23 @@ def test_primes_without_squares(rpg, oracle):
     coeffs = ["2", "509", "0", "-1018"]  # 2 is not a square mod 509
     assert_same_set(rpg, oracle, coeffs, 20_011, 500, 520)
     check(rpg, oracle, coeffs, 20_011, 500, 520)
+
+
+def test_batched_curves_with_launches_of_their_own(rpg):
+    # either side of the batch's rule: wide rows whatever the denominators,
+    # shorter ones only with many; such a curve's points and survivors are
+    # those of its own search
+    curves = [{"coefficients": CURVES[name], "bound": bound, "first": first, "last": last}
+              for name in CURVES
+              for bound, first, last in ((65_503, 1, 50), (65_504, 1, 50), (300_000, 7, 7), (20_011, 1, 36_000),
+                                         (20_011, 5, 30_000), (9_001, 1, 60_000))]
+    points, status, survivors, stats = rpg.batch_search(curves)
+    assert status == [0] * len(curves)
+    alone = 0
+    for c, got, n in zip(curves, points, survivors):
+        expected, st = rpg.point_search(c["coefficients"], c["bound"], c["first"], c["last"])
+        assert got == expected, c
+        alone += n == st["survivor_count"]
+        if c["bound"] >= 65_504 or c["last"] == 36_000:
+            assert n == st["survivor_count"], c
+    assert alone >= 9 and stats["wide_curves"] == 6
