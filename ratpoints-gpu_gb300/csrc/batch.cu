@@ -38,8 +38,9 @@ constexpr int kQueue = 64;
 constexpr long long kMaxClassWords = 1LL << 23;         // class words of a row (sweep-item arithmetic)
 constexpr int kAdmQ = 16;                               // residue words for class primes <= 13
 constexpr int kNarrowSlots = 8;
-constexpr int kNK = 4;                                  // consecutive row words per lane
-constexpr int kND = 4;                                  // consecutive parameters per warp fetch
+constexpr int kNK = 4;                                  // consecutive row words per lane (long ranges)
+constexpr int kNShortWords = 96;                        // ranges up to this many words: one word per lane
+constexpr int kNarrowQueue = 64;                        // queued words per warp
 constexpr int kNWarps = 8;
 constexpr int kNThreads = kNWarps * kWarpSize;
 constexpr int kNarrowTableWords = 7680;                 // sum of m (m + kNK - 1) per curve
@@ -54,7 +55,7 @@ constexpr int kMaxIntervals = 8;                        // more: sweep the whole
 constexpr int kOddPrimes = 96;
 struct OddPrime {
     u32 p;
-    u32 pad;
+    u32 inverse;                   // p^-1 mod 2^32: p | n iff n inverse <= (2^32 - 1) / p (mod 2^32)
     unsigned long long magic;
 };
 
@@ -126,7 +127,7 @@ struct BatchItem {
     long long first;               // first parameter k
     int curve;                     // descriptor index
     int count;                     // parameters in this item
-    int range;                     // which numerator range of each denominator (see x_ranges)
+    int range;                     // which numerator range of each denominator (wide items, see x_range)
     int pad;
 };
 
@@ -134,8 +135,31 @@ struct BatchItem {
 // interval [lo, hi] gives a in [floor(lo d) - 1, ceil(hi d) + 1] (widened by
 // one so that double rounding never drops a site; the host applies the exact
 // interval test), clipped to [-H, H]; overlapping ranges are merged.  Sets
-// [L, U] to the want-th of the disjoint ascending ranges and returns false if
-// there are not that many.  Without intervals the one range is [-H, H].
+// [L, U] to the first of the disjoint ascending ranges from interval i on, and
+// i to the interval after it; false if there is none.
+__device__ __forceinline__ bool next_x_range(const double *lo, const double *hi, int nint, long long H, double d,
+                                             int &i, long long &L, long long &U) {
+    const double h = double(H);
+    bool any = false;
+    for (; i < nint; ++i) {
+        const double x = floor(lo[i] * d) - 1.0;
+        const double y = ceil(hi[i] * d) + 1.0;
+        const long long l = !(x > -h) ? -H : (x > h ? H + 1 : (long long)x);
+        const long long u = !(y < h) ? H : (y < -h ? -H - 1 : (long long)y);
+        if (l > u) continue;
+        if (any && l > U + 1) break;
+        if (!any) {
+            any = true;
+            L = l;
+            U = u;
+        } else if (u > U) {
+            U = u;
+        }
+    }
+    return any;
+}
+
+// The want-th of them.  Without intervals the one range is [-H, H].
 __device__ __forceinline__ bool x_range(const double *lo, const double *hi, int nint, long long H,
                                         long long d, int want, long long &L, long long &U) {
     if (nint == 0) {
@@ -143,28 +167,9 @@ __device__ __forceinline__ bool x_range(const double *lo, const double *hi, int 
         U = H;
         return want == 0;
     }
-    const double dd = double(d), h = double(H);
-    int n = -1;
-    long long cl = 0, cu = -1;
-    for (int i = 0; i < nint; ++i) {
-        const double x = floor(lo[i] * dd) - 1.0;
-        const double y = ceil(hi[i] * dd) + 1.0;
-        const long long l = !(x > -h) ? -H : (x > h ? H + 1 : (long long)x);
-        const long long u = !(y < h) ? H : (y < -h ? -H - 1 : (long long)y);
-        if (l > u) continue;
-        if (n >= 0 && l <= cu + 1) {
-            if (u > cu) cu = u;
-            continue;
-        }
-        if (n == want) break;
-        ++n;
-        cl = l;
-        cu = u;
-    }
-    if (n != want) return false;
-    L = cl;
-    U = cu;
-    return true;
+    for (int i = 0, n = 0; next_x_range(lo, hi, nint, H, double(d), i, L, U); ++n)
+        if (n == want) return true;
+    return false;
 }
 
 struct AffineSpec {                // bitmask of x in [0, p) with f(x) a square mod p
@@ -300,57 +305,6 @@ __global__ void composite_kernel(const CompositeSpec *specs, int nspecs, const u
 
 // ---------------------------------------------------------------------------
 // Stage 2 and emission
-
-// The 32 largest candidates not dividing d with 1/d mod p, by one warp: lane
-// l tests candidate 35 - l, lanes 0..3 also candidate 3 - l.
-__device__ __forceinline__ void select_warp(u32 du, const Candidates &cand,
-                                            const unsigned short *inv_table, int *s_ci, u32 *s_dinv) {
-    const int lane = threadIdx.x & 31;
-    const int ch = kCandidatePrimes - 1 - lane;
-    const u32 rh = mod_small(du, u32(cand.p[ch]), cand.magic[ch]);
-    const u32 hi_div = __ballot_sync(kFullMask, rh == 0);
-    const int cl = kCandidatePrimes - 1 - 32 - lane;
-    const u32 rl = lane < kCandidatePrimes - 32 ? mod_small(du, u32(cand.p[cl]), cand.magic[cl]) : 1u;
-    const u32 lo_div = __ballot_sync(kFullMask, rl == 0);
-    const u32 below = lanemask_lt();
-    const int rank_h = lane - __popc(hi_div & below);
-    if (rh != 0 && rank_h < kSelectedPrimes) {
-        s_ci[rank_h] = ch;
-        s_dinv[rank_h] = __ldg(inv_table + cand.p[ch] * kMaximumPrime + rh);
-    }
-    const int rank_l = 32 - __popc(hi_div) + lane - __popc(lo_div & below);
-    if (lane < kCandidatePrimes - 32 && rl != 0 && rank_l < kSelectedPrimes) {
-        s_ci[rank_l] = cl;
-        s_dinv[rank_l] = __ldg(inv_table + cand.p[cl] * kMaximumPrime + rl);
-    }
-    __syncwarp();
-}
-
-// Clears the bits j of m whose site a = base + step j fails one of the 32
-// selected primes: f(a/d) mod p must be a square.  residue(ci, p, magic)
-// returns base mod p; step_mod(ci) returns step mod p; aff holds the curve's
-// 36 candidate bitmasks in shared memory.
-template <typename Residue, typename StepMod, typename Index, typename Inverse>
-__device__ __forceinline__ u64 stage2(u64 m, const Index *s_ci, const Inverse *s_dinv,
-                                      const Candidates &cand, const u64 *aff, Residue residue,
-                                      StepMod step_mod) {
-    for (int s = 0; s < kSelectedPrimes && m; ++s) {
-        const int ci = s_ci[s];
-        const u32 p = u32(cand.p[ci]), magic = cand.magic[ci];
-        const u32 dinv = s_dinv[s];
-        const u32 x0 = mod_small(residue(ci, p, magic) * dinv, p, magic);
-        const u32 dx = mod_small(step_mod(ci) * dinv, p, magic);
-        const u64 *bits = aff + ci * kRefWords;
-        u64 rest = m;
-        while (rest) {
-            const int j = __ffsll((long long)rest) - 1;
-            rest &= rest - 1;
-            const u32 x = mod_small(x0 + u32(j) * dx, p, magic);
-            if (!((bits[x >> 6] >> (x & 63)) & 1)) m &= ~(u64(1) << j);
-        }
-    }
-    return m;
-}
 
 // Warp-collective emission of sites a = base + step j for the set bits j of m.
 __device__ __forceinline__ void emit(u64 m, long long base, long long step, long long d, int curve,
@@ -866,30 +820,59 @@ __global__ void __launch_bounds__(kWThreads, 2)
 // ---------------------------------------------------------------------------
 // Narrow rows: dense layout, one warp per denominator, whole tables in shared memory.
 
-__device__ __forceinline__ void narrow_drain(const u64 *qmask, const u32 *qword, int start, int n,
-                                             const NarrowCurve &C, const Candidates &cand,
-                                             const u64 *s_aff, const int *s_ci, const u32 *s_dinv,
-                                             long long d, const BatchOut &out) {
+// Stage 2 and emission for up to 32 queued words of one curve, each with its
+// denominator: the 32 largest of the 36 candidates that do not divide it,
+// largest first, until every word has met 32 or is empty.
+__device__ __forceinline__ void narrow_drain(const u64 *qmask, const u32 *qword, const u32 *qd, int start, int n,
+                                             const NarrowCurve &C, const Candidates &cand, const u64 *s_aff,
+                                             const unsigned short *inv_table, const BatchOut &out) {
     const int lane = threadIdx.x & 31;
     u64 m = 0;
-    u32 w = 0;
+    u32 w = 0, d = 1;
     if (lane < n) {
         m = qmask[start + lane];
         w = qword[start + lane];
+        d = qd[start + lane];
     }
     __syncwarp();
-    if (m) {
-        m = stage2(
-            m, s_ci, s_dinv, cand, s_aff,
-            [&](int ci, u32 p, u32 magic) {
-                const u32 r = C.neg_h[ci] + mod_small(64u * mod_small(w, p, magic), p, magic);
-                return r >= p ? r - p : r;
-            },
-            [&](int) { return 1u; });
+    int tested = 0;
+    for (int ci = kCandidatePrimes - 1; ci >= 0; --ci) {
+        if (!__any_sync(kFullMask, m != 0 && tested < kSelectedPrimes)) break;
+        const u32 p = u32(cand.p[ci]), magic = cand.magic[ci];
+        const u32 rho = mod_small(d, p, magic);
+        if (m != 0 && tested < kSelectedPrimes && rho != 0) {
+            ++tested;
+            const u32 dinv = __ldg(inv_table + p * kMaximumPrime + rho);
+            u32 r = C.neg_h[ci] + mod_small(64u * mod_small(w, p, magic), p, magic);  // a mod p
+            if (r >= p) r -= p;
+            const u32 x0 = mod_small(r * dinv, p, magic);
+            const u64 *bits = s_aff + ci * kRefWords;
+            u64 rest = m;
+            while (rest) {
+                const int j = __ffsll((long long)rest) - 1;
+                rest &= rest - 1;
+                const u32 x = mod_small(x0 + u32(j) * dinv, p, magic);
+                if (!((bits[x >> 6] >> (x & 63)) & 1)) m &= ~(u64(1) << j);
+            }
+        }
     }
-    emit(m, -C.bound + 64LL * w, 1, d, C.index, out);
+    emit(m, -C.bound + 64LL * w, 1, (long long)d, C.index, out);
 }
 
+// A CTA takes items (curve, parameters; all numerator ranges) and keeps the curve's
+// stage-1 tables in shared memory.  A warp fetches up to 32 parameters and
+// classifies one per lane (2-adic masks, denominator primes, numerator range),
+// then sweeps the live ones in turn; live words of all of them share its
+// queue, so that stage 2 runs with full warps.
+//
+// What bounds it is what a denominator costs besides its words: with the range
+// of x (fp64, 16 cycles an instruction on this chip), the denominator primes
+// and the selection of stage 2's primes worked out by a whole warp per
+// denominator, 96 curves of degree 12 to 40, 1e5 denominators in three
+// intervals each, took 41.5 ms, now 20.1 (470 instructions for a denominator
+// and interval of 90 words, 58 % of the issue slots); 400,000 denominators of
+// sextics 0.20 -> 0.08 ms at H = 1,000, 0.35 -> 0.27 at 5,000.  The curve's
+// constants stay in shared memory: held in registers they spill (+10 %).
 __global__ void __launch_bounds__(kNThreads, 3)
     narrow_kernel(const NarrowCurve *__restrict__ curves, const BatchItem *__restrict__ items,
                   int nitems, const u64 *__restrict__ pool, const u64 *__restrict__ affine,
@@ -900,23 +883,30 @@ __global__ void __launch_bounds__(kNThreads, 3)
     __shared__ int s_item;
     __shared__ int s_next;
     __shared__ int s_abort;
-    __shared__ int s_ci[kNWarps][kSelectedPrimes];
-    __shared__ u32 s_dinv[kNWarps][kSelectedPrimes];
-    __shared__ unsigned char s_lane_at[kNarrowSlots][kWarpSize];  // (shift + kNK lane) mod m
+    __shared__ int s_nbad;
+    __shared__ uint2 s_bad[kOddPrimes];  // the curve's denominator primes: p^-1 mod 2^32, (2^32 - 1) / p
+    // (k lane) mod m for k = 1 and kNK, 32 mod m
+    __shared__ unsigned char s_lane1[kNarrowSlots][kWarpSize], s_lane4[kNarrowSlots][kWarpSize];
+    __shared__ u32 s_step32[kNarrowSlots];
     __shared__ __align__(8) unsigned long long s_bar;
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const u64 *tab = smem;
     const u64 *s_aff = smem + kNarrowTableWords;  // the curve's 36 candidate bitmasks
-    u64 *wq_mask = smem + kNarrowTableWords + kAffWords + warp * kQueue;
-    u32 *wq_word =
-        reinterpret_cast<u32 *>(smem + kNarrowTableWords + kAffWords + kNWarps * kQueue) + warp * kQueue;
+    u64 *queues = smem + kNarrowTableWords + kAffWords;
+    u64 *wq_mask = queues + warp * kNarrowQueue;
+    u32 *wq_word = reinterpret_cast<u32 *>(queues + kNWarps * kNarrowQueue) + warp * kNarrowQueue;
+    u32 *wq_d = wq_word + kNWarps * kNarrowQueue;
     const u32 bar = smem_addr(&s_bar);
     u32 phase = 0;
     int cur = -1;
     // row words this warp sweeps and the stage-1 shared-memory bytes they read
-    unsigned long long swept_words = 0, swept_bytes = 0;
+    unsigned long long swept_words = 0, swept_bytes = 0, counted = 0;
+    // lane s mod 8 works out modulus s of a denominator: its constants
+    const int my = lane & (kNarrowSlots - 1);
+    u32 my_m = 1, my_shift = 0, my_off = 0, my_len = 1;
+    unsigned long long my_magic = ~0ull;
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         s_abort = 0;
@@ -939,12 +929,27 @@ __global__ void __launch_bounds__(kNThreads, 3)
             for (int i = threadIdx.x; i < int(sizeof(NarrowCurve) / 4); i += kNThreads) dst[i] = src[i];
             cur = item.curve;
             __syncthreads();
-            // each lane's first table word per modulus for rows swept from word 0
             for (int t = threadIdx.x; t < kNarrowSlots * kWarpSize; t += kNThreads) {
                 const int s = t / kWarpSize, l = t % kWarpSize;
-                s_lane_at[s][l] = (unsigned char)((C.shift[s] + u32(kNK * l)) % u32(C.m[s]));
+                s_lane1[s][l] = (unsigned char)(u32(l) % u32(C.m[s]));
+                s_lane4[s][l] = (unsigned char)(u32(kNK * l) % u32(C.m[s]));
             }
+            if (threadIdx.x < kNarrowSlots) s_step32[threadIdx.x] = u32(kWarpSize) % u32(C.m[threadIdx.x]);
+            const u64 bad0 = C.denom_primes[0], bad1 = C.denom_primes[1];
+            if (int(threadIdx.x) < kOddPrimes) {
+                const int i = int(threadIdx.x), b = i & 63;
+                if (((i < 64 ? bad0 : bad1) >> b) & 1) {
+                    const int rank = __popcll((i < 64 ? bad0 : bad1) & ((u64(1) << b) - 1)) + (i < 64 ? 0 : __popcll(bad0));
+                    s_bad[rank] = make_uint2(odd[i].inverse, 0xFFFFFFFFu / odd[i].p);
+                }
+            }
+            my_m = u32(C.m[my]);
+            my_magic = C.magic[my];
+            my_shift = C.shift[my];
+            my_off = u32(C.off[my]);
+            my_len = u32(C.len[my]);
             if (threadIdx.x == 0) {
+                s_nbad = __popcll(bad0) + __popcll(bad1);
                 fence_proxy_async_shared();
                 mbar_arrive_expect_tx(bar, u32(C.table_words + kAffWords) * 8u);
                 bulk_copy_to_shared(smem_addr(smem), pool + C.tables, u32(C.table_words) * 8u, bar);
@@ -962,114 +967,137 @@ __global__ void __launch_bounds__(kNThreads, 3)
                 return;
             }
         }
-        int *w_ci = s_ci[warp];
-        u32 *w_dinv = s_dinv[warp];
+        // parameters per fetch: a lane each, but every warp gets some
+        const int fetch = max(1, min(kWarpSize, (item.count + 2 * kNWarps - 1) / (2 * kNWarps)));
+        const int nbad = s_nbad;
+        int qn = 0;
         for (;;) {
             int idx0 = 0;
-            if (lane == 0) idx0 = atomicAdd(&s_next, kND);
+            if (lane == 0) idx0 = atomicAdd(&s_next, fetch);
             idx0 = __shfl_sync(kFullMask, idx0, 0);
             if (idx0 >= item.count) break;
-            const int jn = min(kND, item.count - idx0);
-            u32 rho[kNarrowSlots];
-            for (int j = 0; j < jn; ++j) {
-                const long long k = item.first + idx0 + j;
-                const long long d = C.square ? k * k : k;
-                const u32 du = u32(d);
-                // d mod m for every modulus: reduced for the first parameter of the
-                // fetch (and for square denominators), else advanced by one
-#pragma unroll
-                for (int s = 0; s < kNarrowSlots; ++s) {
-                    if (j == 0 || C.square) {
-                        rho[s] = mod_u32(du, u32(C.m[s]), C.magic[s]);
-                    } else {
-                        rho[s] += 1;
-                        if (rho[s] == u32(C.m[s])) rho[s] = 0;
-                    }
-                }
-                const u64 mask2 = C.dense2[du & 63];
-                if (!mask2) continue;
-                // denominator primes (see has_denominator_prime), split over the lanes
-                bool hit = false;
-                for (int i = lane; i < kOddPrimes; i += kWarpSize)
-                    if ((C.denom_primes[i >> 6] >> (i & 63)) & 1)
-                        hit |= mod_u32(u32(k), __ldg(&odd[i].p), __ldg(&odd[i].magic)) == 0;
-                if (__any_sync(kFullMask, hit)) continue;
-                // words [w_lo, w_hi] hold the numerator range of this item: a in [L, U]
+            const bool valid = lane < fetch && idx0 + lane < item.count;
+            const long long k = item.first + idx0 + (valid ? lane : 0);
+            const u32 dd = C.square ? u32(k) * u32(k) : u32(k);
+            bool live = valid && C.dense2[dd & 63] != 0;
+            bool hit = false;
+#pragma unroll 4
+            for (int i = 0; i < nbad; ++i) hit |= u32(k) * s_bad[i].x <= s_bad[i].y;
+            live = live && !hit;
+            for (int interval = 0;;) {
+                // the denominators' next numerator range, a in [L, U]: words
+                // [w_lo, w_hi], the first keeping its bits from L on, the last up to U
                 long long L = -C.bound, U = C.bound;
-                if (C.nint > 0 && !x_range(C.lo, C.hi, C.nint, C.bound, d, item.range, L, U)) continue;
-                const int w_lo = int((L + C.bound) >> 6), w_hi = int((U + C.bound) >> 6);
-                swept_words += u32(w_hi - w_lo + 1);
-                swept_bytes += 8ull * u32(C.rows) * u32(w_hi - w_lo + 1);
-                const u64 first_mask = ~u64(0) << ((L + C.bound) & 63);
-                const int last_bits = int((U + C.bound) & 63) + 1;
-                const u64 last_mask = last_bits >= 64 ? ~u64(0) : ((u64(1) << last_bits) - 1);
-                // lane l takes words w0 + kNK l .. w0 + kNK l + kNK - 1 of each
-                // 128-word step: rows repeat their first kNK - 1 words, so the kNK
-                // words of a lane never wrap and one index per modulus advances
-                u32 base[kNarrowSlots], at[kNarrowSlots], mods[kNarrowSlots], steps[kNarrowSlots];
-#pragma unroll
-                for (int s = 0; s < kNarrowSlots; ++s) {
-                    const u32 m = u32(C.m[s]);
-                    mods[s] = m;
-                    steps[s] = C.step[s];
-                    base[s] = u32(C.off[s]) + rho[s] * u32(C.len[s]);
-                    at[s] = w_lo == 0 ? u32(s_lane_at[s][lane])
-                                      : mod_u32(C.shift[s] + u32(w_lo + kNK * lane), m, C.magic[s]);
-                }
-                bool selected = false;
-                int qn = 0;
-                for (int w0 = w_lo; w0 <= w_hi; w0 += kWarpSize * kNK) {
-                    u64 acc[kNK];
-#pragma unroll
-                    for (int k = 0; k < kNK; ++k) acc[k] = mask2;
+                bool here = live;
+                if (C.nint > 0)
+                    here = live && next_x_range(C.lo, C.hi, C.nint, C.bound, double(dd), interval, L, U);
+                u32 todo = __ballot_sync(kFullMask, here);
+                if (!todo) break;
+                const u32 first = u32(L + C.bound), last = u32(U + C.bound);
+                for (; todo; todo &= todo - 1) {
+                    const int j = __ffs(todo) - 1;
+                    const u32 d = __shfl_sync(kFullMask, dd, j);
+                    const u32 lo_j = __shfl_sync(kFullMask, first, j), hi_j = __shfl_sync(kFullMask, last, j);
+                    const int w_lo = int(lo_j >> 6), w_hi = int(hi_j >> 6);
+                    const u64 first_mask = ~u64(0) << (lo_j & 63), last_mask = ~u64(0) >> (63 - (hi_j & 63));
+                    const u64 mask2 = C.dense2[d & 63];
+                    swept_words += u32(w_hi - w_lo + 1);
+                    // per modulus: the table word of row d mod m and the row index of word w_lo
+                    const u32 mine = (my_off + mod_u32(d, my_m, my_magic) * my_len) |
+                                     (mod_u32(my_shift + u32(w_lo), my_m, my_magic) << 16);
+                    static_assert(kNarrowTableWords < 65536, "table words fit 16 bits");
+                    u32 base[kNarrowSlots], at[kNarrowSlots];
 #pragma unroll
                     for (int s = 0; s < kNarrowSlots; ++s) {
-                        const u64 *row = tab + base[s] + at[s];
-#pragma unroll
-                        for (int k = 0; k < kNK; ++k) acc[k] &= row[k];
-                        const u32 t = at[s] + steps[s];  // advance 32 kNK words mod m
-                        at[s] = min(t, t - mods[s]);
+                        const u32 v = __shfl_sync(kFullMask, mine, s);
+                        base[s] = v & 0xFFFFu;
+                        at[s] = v >> 16;
                     }
-                    const int wl = w0 + kNK * lane;
-                    if (w0 == w_lo || w0 + kWarpSize * kNK - 1 > w_hi) {  // the range's first or last step
-#pragma unroll
-                        for (int k = 0; k < kNK; ++k) {
-                            const int w = wl + k;
-                            if (w > w_hi) acc[k] = 0;
-                            if (w == w_lo) acc[k] &= first_mask;
-                            if (w == w_hi) acc[k] &= last_mask;
-                        }
-                    }
-                    if (!__ballot_sync(kFullMask, (acc[0] | acc[1] | acc[2] | acc[3]) != 0)) continue;
-#pragma unroll
-                    for (int k = 0; k < kNK; ++k) {
-                        const u32 b = __ballot_sync(kFullMask, acc[k] != 0);
-                        if (!b) continue;
+                    // queues the live words of a 32-lane step
+                    auto push = [&](u64 word, int w) {
+                        const u32 b = __ballot_sync(kFullMask, word != 0);
+                        if (!b) return;
                         const int pos = qn + __popc(b & lanemask_lt());
-                        if (acc[k]) {
-                            wq_mask[pos] = acc[k];
-                            wq_word[pos] = u32(wl + k);
+                        if (word) {
+                            wq_mask[pos] = word;
+                            wq_word[pos] = u32(w);
+                            wq_d[pos] = d;
                         }
                         qn += __popc(b);
                         if (qn >= 32) {
-                            if (!selected) {
-                                select_warp(du, cand, inv_table, w_ci, w_dinv);
-                                selected = true;
-                            }
                             __syncwarp();
-                            narrow_drain(wq_mask, wq_word, qn - 32, 32, C, cand, s_aff, w_ci, w_dinv, d,
-                                         out);
+                            narrow_drain(wq_mask, wq_word, wq_d, qn - 32, 32, C, cand, s_aff, inv_table, out);
                             qn -= 32;
+                        }
+                    };
+                    if (w_hi - w_lo < kNShortWords) {
+                        // lane l takes word w0 + l of each 32-word step
+#pragma unroll
+                        for (int s = 0; s < kNarrowSlots; ++s) {
+                            const u32 t = at[s] + u32(s_lane1[s][lane]);
+                            at[s] = min(t, t - u32(C.m[s]));
+                        }
+                        for (int w0 = w_lo;;) {
+                            u64 acc = mask2;
+#pragma unroll
+                            for (int s = 0; s < kNarrowSlots; ++s) acc &= tab[base[s] + at[s]];
+                            const int w = w0 + lane;
+                            if (w > w_hi) acc = 0;
+                            if (w == w_lo) acc &= first_mask;
+                            if (w == w_hi) acc &= last_mask;
+                            push(acc, w);
+                            w0 += kWarpSize;
+                            if (w0 > w_hi) break;
+#pragma unroll
+                            for (int s = 0; s < kNarrowSlots; ++s) {
+                                const u32 t = at[s] + s_step32[s];
+                                at[s] = min(t, t - u32(C.m[s]));
+                            }
+                        }
+                    } else {
+                        // lane l takes words w0 + kNK l .. w0 + kNK l + kNK - 1 of each
+                        // 128-word step: rows repeat their first kNK - 1 words, so the
+                        // kNK words of a lane never wrap and one index per modulus advances
+#pragma unroll
+                        for (int s = 0; s < kNarrowSlots; ++s) {
+                            const u32 t = at[s] + u32(s_lane4[s][lane]);
+                            at[s] = min(t, t - u32(C.m[s]));
+                        }
+                        for (int w0 = w_lo; w0 <= w_hi; w0 += kWarpSize * kNK) {
+                            u64 acc[kNK];
+#pragma unroll
+                            for (int k4 = 0; k4 < kNK; ++k4) acc[k4] = mask2;
+#pragma unroll
+                            for (int s = 0; s < kNarrowSlots; ++s) {
+                                const u64 *row = tab + base[s] + at[s];
+#pragma unroll
+                                for (int k4 = 0; k4 < kNK; ++k4) acc[k4] &= row[k4];
+                                const u32 t = at[s] + C.step[s];
+                                at[s] = min(t, t - u32(C.m[s]));
+                            }
+                            const int wl = w0 + kNK * lane;
+                            if (w0 == w_lo || w0 + kWarpSize * kNK - 1 > w_hi) {  // the range's first or last step
+#pragma unroll
+                                for (int k4 = 0; k4 < kNK; ++k4) {
+                                    if (wl + k4 > w_hi) acc[k4] = 0;
+                                    if (wl + k4 == w_lo) acc[k4] &= first_mask;
+                                    if (wl + k4 == w_hi) acc[k4] &= last_mask;
+                                }
+                            }
+                            if (!__ballot_sync(kFullMask, (acc[0] | acc[1] | acc[2] | acc[3]) != 0)) continue;
+#pragma unroll
+                            for (int k4 = 0; k4 < kNK; ++k4) push(acc[k4], wl + k4);
                         }
                     }
                 }
-                if (qn) {
-                    if (!selected) select_warp(du, cand, inv_table, w_ci, w_dinv);
-                    __syncwarp();
-                    narrow_drain(wq_mask, wq_word, 0, qn, C, cand, s_aff, w_ci, w_dinv, d, out);
-                }
+                if (C.nint == 0) break;
             }
         }
+        // the queue's words are this curve's: stage 2 before the next item
+        __syncwarp();
+        if (qn) narrow_drain(wq_mask, wq_word, wq_d, 0, qn, C, cand, s_aff, inv_table, out);
+        swept_bytes += 8ull * u32(C.rows) * (swept_words - counted);
+        counted = swept_words;
         __syncthreads();
     }
     if (lane == 0) {
@@ -1277,16 +1305,17 @@ long long swept_row_words(const BatchCurveSpec &c, long long words) {
 
 // Whether a curve gets sieve launches of its own (sweep.hpp) instead of work
 // items of the batched kernels.  Rows of at least kBatchWideWords words always
-// do; shorter ones when the narrow kernel's time for them, 0.45 ns per
-// denominator and 1.85e-3 ns per row word, exceeds the sweep's (0.9 to 1.1 ns
-// per denominator up to H = 65,504) by more than building the curve's tables
-// takes (400,000 denominators of sextics, narrow and sweep: H = 5,000 0.35 and
-// 0.40 ms, 10,000 0.45 and 0.38, 20,000 0.66 and 0.38, 65,000 1.7 and 0.40).
+// do; shorter ones when the narrow kernel's time for them, about 0.1 ns per
+// denominator and 2.8e-3 ns per row word, exceeds the sweep's (1 ns per
+// denominator up to H = 65,504) by more than building the curve's tables takes
+// (400,000 denominators of sextics, narrow and sweep: H = 5,000 0.28 and 0.40
+// ms, 10,000 0.40 and 0.38; with the narrow kernel before it shared stage 2
+// among denominators, 20,000 0.66 and 0.38, 65,000 1.7 and 0.40).
 // Curves with x intervals stay in the kernels that sweep only those.
 bool swept_alone(const BatchCurveSpec &c, const CurveWork &cw) {
     if (!c.intervals.empty() && c.intervals.size() <= std::size_t(dev::kMaxIntervals)) return false;
     if (cw.wide) return true;
-    return double(cw.count) * (1.85e-3 * double(cw.words) - 0.6) > 20000.0;
+    return double(cw.count) * (2.8e-3 * double(cw.words) - 0.9) > 20000.0;
 }
 
 // Narrow plan: every odd prime up to kBatchNarrowModulus that filters at
@@ -1556,7 +1585,9 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
             const std::size_t n = curves[i].intervals.size();
             const long long ranges = n > 0 && n <= std::size_t(dev::kMaxIntervals) ? (long long)n : 1;
             const long long chunk = item_chunk(cw);
-            (cw.wide ? wide_items : narrow_items) += std::size_t(ranges * ((cw.count + chunk - 1) / chunk));
+            const std::size_t parts = std::size_t((cw.count + chunk - 1) / chunk);
+            if (cw.wide) wide_items += std::size_t(ranges) * parts;
+            else narrow_items += parts;
         }
         P.wide_items.reserve(wide_items);
         P.narrow_items.reserve(narrow_items);
@@ -1738,10 +1769,8 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
             }
             device_intervals(c.intervals, C.nint, C.lo, C.hi);
             const long long chunk = item_chunk(cw);
-            for (int range = 0; range < std::max(1, C.nint); ++range)
-                for (long long f = c.first; f <= c.last; f += chunk)
-                    P.narrow_items.push_back({f, int(P.narrow.size()),
-                                              int(std::min(chunk, c.last - f + 1)), range, 0});
+            for (long long f = c.first; f <= c.last; f += chunk)
+                P.narrow_items.push_back({f, int(P.narrow.size()), int(std::min(chunk, c.last - f + 1)), 0, 0});
             P.narrow.push_back(C);
         }
         stats.curves += 1;
@@ -1826,7 +1855,11 @@ struct BatchEngine::Impl {
         }
         std::vector<dev::OddPrime> odd;
         for (int p = 3; p < kMaximumPrime; p += 2)
-            if (is_small_prime(p)) odd.push_back({dev::u32(p), 0, host_magic(p)});
+            if (is_small_prime(p)) {
+                dev::u32 inverse = dev::u32(p);  // Newton's iteration, right in 3 bits to start with
+                for (int i = 0; i < 4; ++i) inverse *= 2u - dev::u32(p) * inverse;
+                odd.push_back({dev::u32(p), inverse, host_magic(p)});
+            }
         if (odd.size() != std::size_t(dev::kOddPrimes)) throw std::logic_error("odd prime table");
         unsigned long long bytes = 0;
         d_inv.upload(inv_table, stream, bytes, "upload inverses");
@@ -1983,7 +2016,7 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
                                           sizeof(dev::WideRun) +
                                       std::size_t(dev::kWSlotCount) * std::size_t(wide_max_classes + 1) * 4;
         const std::size_t narrow_smem = std::size_t(dev::kNarrowTableWords + dev::kAffWords) * 8 +
-                                        std::size_t(dev::kNWarps) * dev::kQueue * 12;
+                                        std::size_t(dev::kNWarps) * dev::kNarrowQueue * 16;
         int wide_grid = 0, narrow_grid = 0;
         if (!P.wide.empty()) {
             int per_sm = 0;

@@ -78,3 +78,24 @@ def test_batched_curves_with_launches_of_their_own(rpg):
         if c["bound"] >= 65_504 or c["last"] == 36_000:
             assert n == st["survivor_count"], c
     assert alone >= 9 and stats["wide_curves"] == 6
+
+
+@pytest.mark.parametrize("last", [1, 7, 33, 700])
+def test_narrow_rows(rpg, last):
+    # rows and x ranges either side of the one-word-per-lane steps (32 and 96
+    # words), a word's first and last bit, overlapping, empty and many
+    # intervals, with few and many denominators per work item
+    several = [(f"{i - 3.5:.2f}", f"{i - 3.5 + 0.3 * i:.2f}") for i in range(8)]
+    curves = []
+    for bound in (1, 31, 32, 1_023, 1_024, 3_071, 3_103, 9_000):
+        for intervals in ((), [("-0.5", "0.5")], [("0", "0"), ("-2", "1.75"), ("1.5", "3"), ("5", "4")], several):
+            for coeffs, square in ((["1", "0", "0", "1"], False), (["4", "-3", "0", "0", "1"], False),
+                                   (["1", "-1", "0", "1"], True)):
+                curves.append({"coefficients": coeffs, "bound": bound, "first": 1, "last": last,
+                               "intervals": intervals, "square": square})
+    points, status, _, stats = rpg.batch_search(curves)
+    assert status == [0] * len(curves) and stats["wide_curves"] == 0
+    for c, got in zip(curves, points):
+        expected, _ = rpg.point_search(c["coefficients"], c["bound"], 1, last, intervals=c["intervals"],
+                                       square=c["square"])
+        assert got == expected, c
