@@ -104,17 +104,39 @@ __host__ __device__ inline bool square_mod_2_64(u64 x) {
     return v == 62 ? (odd & 3u) == 1u : (odd & 7u) == 1u;
 }
 
-// F(a, d) mod m by Horner in a with the powers of d accumulated; slot
-// selects the coefficients' residues mod m.
-__host__ __device__ inline u32 value_mod(const PreCoef *c, int n, int slot, u32 am, u32 dm, u32 m, u64 magic) {
-    u32 v = c[n - 1].r[slot], pw = 1u % m;
-    for (int i = n - 2; i >= 0; --i) {
-        v = mul_mod(v, am, m, magic);
-        pw = mul_mod(pw, dm, m, magic);
-        v = add_mod(v, mul_mod(c[i].r[slot], pw, m, magic), m);
+// F(a, d) mod the four moduli of one kind (slots base .. base + 3) by Horner in
+// a with the powers of d accumulated.  The four chains are independent: a
+// launch of few survivors is bound by their latency (24 us for the points
+// of a small search, every test in turn).
+struct FourValues {
+    u32 v[4];
+};
+__host__ __device__ inline FourValues values_mod(const PreCoef *c, int n, int base, const u32 (&m)[4], long long a,
+                                                 long long d) {
+    FourValues out;
+    u32 am[4], dm[4], pw[4];
+    u64 magic[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        magic[i] = ~0ull / m[i];
+        am[i] = signed_mod(a, m[i]);
+        dm[i] = signed_mod(d, m[i]);
+        pw[i] = 1u % m[i];
+        out.v[i] = c[n - 1].r[base + i];
     }
-    if ((n & 1) == 0) v = mul_mod(v, dm, m, magic);
-    return v;
+    for (int k = n - 2; k >= 0; --k) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            out.v[i] = mul_mod(out.v[i], am[i], m[i], magic[i]);
+            pw[i] = mul_mod(pw[i], dm[i], m[i], magic[i]);
+            out.v[i] = add_mod(out.v[i], mul_mod(c[k].r[base + i], pw[i], m[i], magic[i]), m[i]);
+        }
+    }
+    if ((n & 1) == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) out.v[i] = mul_mod(out.v[i], dm[i], m[i], magic[i]);
+    }
+    return out;
 }
 
 __host__ __device__ inline bool may_be_point(long long a, long long d, const PreCoef *c, int n,
@@ -131,32 +153,39 @@ __host__ __device__ inline bool may_be_point(long long a, long long d, const Pre
         if ((n & 1) == 0) v *= ud;
         if (!square_mod_2_64(v)) return false;
     }
+    {
+        static_assert(kGroups == 4 && kLarge == 4, "four moduli of each kind");
+        const u32 m[4] = {group_modulus(0), group_modulus(1), group_modulus(2), group_modulus(3)};
+        const FourValues f = values_mod(c, n, 0, m, a, d);
+        bool square = true;
 #pragma unroll
-    for (int g = 0; g < kGroups; ++g) {
-        const u32 m = group_modulus(g);
-        const u64 magic = ~0ull / m;
-        const u32 v = value_mod(c, n, g, signed_mod(a, m), signed_mod(d, m), m, magic);
+        for (int g = 0; g < kGroups; ++g)
 #pragma unroll
-        for (int i = group_first(g); i < group_first(g + 1); ++i) {
-            const u32 r = v % small_prime(i);
-            if (!((masks.bits[i][r >> 6] >> (r & 63)) & 1u)) return false;
-        }
+            for (int i = group_first(g); i < group_first(g + 1); ++i) {
+                const u32 r = f.v[g] % small_prime(i);
+                square = square && ((masks.bits[i][r >> 6] >> (r & 63)) & 1u);
+            }
+        if (!square) return false;
     }
+    const u32 p[4] = {large_prime(0), large_prime(1), large_prime(2), large_prime(3)};
+    const FourValues f = values_mod(c, n, kGroups, p, a, d);
+    // Euler's criterion: v^((p-1)/2) is 1 for a nonzero square, p - 1 otherwise.
+    // (p-1)/2 has 30 bits for each of the four primes.
+    u32 base[4], acc[4] = {1, 1, 1, 1};
+#pragma unroll
+    for (int l = 0; l < kLarge; ++l) base[l] = f.v[l];
 #pragma unroll 1
-    for (int l = 0; l < kLarge; ++l) {
-        const u32 p = large_prime(l);
-        const u64 magic = ~0ull / p;
-        const u32 v = value_mod(c, n, kGroups + l, signed_mod(a, p), signed_mod(d, p), p, magic);
-        if (v == 0) continue;
-        // Euler's criterion: v^((p-1)/2) is 1 for a nonzero square, p - 1 otherwise
-        u32 e = (p - 1) / 2, base = v, acc = 1;
-        while (e) {
-            if (e & 1u) acc = mul_mod(acc, base, p, magic);
-            base = mul_mod(base, base, p, magic);
-            e >>= 1;
+    for (int bit = 0; bit < 30; ++bit) {
+#pragma unroll
+        for (int l = 0; l < kLarge; ++l) {
+            const u64 magic = ~0ull / p[l];
+            if (((p[l] - 1) / 2 >> bit) & 1u) acc[l] = mul_mod(acc[l], base[l], p[l], magic);
+            base[l] = mul_mod(base[l], base[l], p[l], magic);
         }
-        if (acc != 1) return false;
     }
+#pragma unroll
+    for (int l = 0; l < kLarge; ++l)
+        if (f.v[l] != 0 && acc[l] != 1) return false;
     return true;
 }
 

@@ -80,11 +80,14 @@ struct FastPrime {                 // one of the 36 reference candidates
 
 struct LatePrime {                 // a prime of the plan tested after stage 2
     long long pattern;
+    unsigned long long magic;      // mod_u32 constant
     u32 p;
     u32 inv_mod;
+    u32 base_mod;                  // abase mod p
     int words;
-    int pad;
 };
+constexpr int kLatePrimes = kSweepRows * kSweepRowFactors + 1;  // every prime of a fast plan
+constexpr int kFLateGroup = 4;     // late primes loaded together
 
 // Entry of the lists by d mod two and by d mod Q: one admissible residue, its
 // CRT lift x and its term of the row index of each modulus, in bytes
@@ -103,7 +106,6 @@ struct SweepTables {
     const int *count2;             // [two]
     const int *countq;             // [Q]
     const u64 *rows;               // stage-1 and candidate tables, pattern rows
-    const LatePrime *late;
     int nbad, nlate;
     int tabled;                    // the largest candidates have class-layout tables
     int two_mask;                  // two - 1
@@ -120,6 +122,7 @@ struct SweepTables {
     // denominator primes: p | k iff k x <= y (mod 2^32), x = p^-1 mod 2^32 and
     // y = floor((2^32 - 1) / p)
     uint2 bad[kOddPrimes];
+    LatePrime late[kLatePrimes + kFLateGroup];  // padded with its last
     uint2 need;                    // d has survivors only if d x <= y (mod 2^32): a divisor d must have
 };
 
@@ -236,14 +239,21 @@ __device__ __forceinline__ void fast_drain(const u64 *qmask, const u64 *qpos, co
     const long long a0 = A.abase + (long long)pos;
     const long long M = T.class_mod;
     if (m) {
-        if (T.nlate) {
-            for (int l = 0; l < T.nlate && m; ++l) {
-                const LatePrime P = T.late[l];
-                long long r = a0 % (long long)P.p;
-                if (r < 0) r += P.p;
-                const u32 u = u32(r) * P.inv_mod % P.p;
-                m &= pattern_window(T.rows + P.pattern + (long long)(d % P.p) * P.words, u);
+        // four at a time: the chain of one is long, and the survivors of a
+        // small search all meet every late prime (padded with repeats)
+        for (int l = 0; l < T.nlate && m; l += kFLateGroup) {
+            u64 rows[kFLateGroup];
+#pragma unroll
+            for (int t = 0; t < kFLateGroup; ++t) {
+                const LatePrime &P = T.late[l + t];
+                u32 r = mod_u32(hi, P.p, P.magic);
+                r = mod_u32((r << 16) | lo, P.p, P.magic) + P.base_mod;
+                if (r >= P.p) r -= P.p;
+                const u32 k = mod_u32(r * P.inv_mod, P.p, P.magic);
+                rows[t] = pattern_window(T.rows + P.pattern + (long long)mod_u32(d, P.p, P.magic) * P.words, k);
             }
+#pragma unroll
+            for (int t = 0; t < kFLateGroup; ++t) m &= rows[t];
         }
         if (a0 < A.a_lo || a0 + 63 * M > A.a_hi) {  // ends of the numerator range
             for (u64 rest = m; rest; rest &= rest - 1) {

@@ -433,12 +433,13 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
             P.offset = (long long)(K.out / 8);
         }
     }
-    std::vector<dev::LatePrime> late;
+    if (late_primes.size() > std::size_t(dev::kLatePrimes)) throw std::logic_error("more late primes than a plan has");
     for (int p : late_primes) {
         const dev::PatternJob &J = pattern_of(p, lead_of(p));
-        late.push_back({(long long)(J.out / 8), dev::u32(p), dev::u32(mod_inverse(M % p, p)), J.words, 0});
+        T.late[T.nlate++] = {(long long)(J.out / 8), magic_of(p), dev::u32(p), dev::u32(mod_inverse(M % p, p)), 0, J.words};
     }
-    late_at_ = put(late.data(), late.size() * sizeof(dev::LatePrime));
+    if (T.nlate)
+        for (int t = 0; t < dev::kFLateGroup; ++t) T.late[T.nlate + t] = T.late[T.nlate - 1];
     // admissible residues of the class primes by d mod p
     for (int i = 0; i < L.nprimes; ++i) {
         const int p = plan_.class_primes[std::size_t(i)];
@@ -482,7 +483,6 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
     dev::u32 inverse = dev::u32(need_);
     for (int i = 0; i < 4; ++i) inverse *= 2u - dev::u32(need_) * inverse;
     T.need = make_uint2(inverse, dev::u32(0xFFFFFFFFull / need_));
-    T.nlate = int(late.size());
     T.two_mask = plan_.two - 1;
     T.q = dev::u32(q);
     T.q_magic = magic_of(q);
@@ -572,6 +572,8 @@ void SweepCurve::launch(const SweepLaunch &l, cudaStream_t stream) const {
     T.segs_magic = A.segs == 1 ? 0 : magic_of(A.segs);
     for (std::size_t r = 0; r < plan_.moduli.size(); ++r) T.row[r].wlo = dev::u32(w_lo % plan_.moduli[r]);
     for (auto &P : T.prime) P.base_mod = dev::u32(mod_of(A.abase, P.p));
+    for (int l = 0; T.nlate && l < T.nlate + dev::kFLateGroup; ++l)
+        T.late[l].base_mod = dev::u32(mod_of(A.abase, (long long)T.late[l].p));
     const int blocks = int(std::min<long long>(grid, (shares + A.chunk - 1) / A.chunk));
     unsigned long long *work = l.work;
     void *params[] = {&T, &A, &work};
@@ -644,7 +646,6 @@ void SweepBuilder::place(unsigned char *arena, cudaStream_t stream) {
         T.listq = reinterpret_cast<const dev::SweepClass *>(arena + block + c.listq_at_);
         T.count2 = reinterpret_cast<const int *>(arena + block + c.count2_at_);
         T.countq = reinterpret_cast<const int *>(arena + block + c.countq_at_);
-        T.late = reinterpret_cast<const dev::LatePrime *>(arena + input + c.late_at_);
     }
     auto append = [&](const void *data, std::size_t bytes) {
         blob_.resize(aligned(blob_.size()));

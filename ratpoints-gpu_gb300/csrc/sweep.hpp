@@ -70,12 +70,11 @@ private:
     std::size_t smem_ = 0;
     std::unique_ptr<dev::SweepTables> tables_;  // pointers set by SweepBuilder::place
     // build inputs, offsets from the curve's table block (rows, patterns,
-    // lists) or from its input block (residues, maps, late primes)
+    // lists) or from its input block (residues, maps)
     std::vector<dev::PatternJob> patterns_;
     std::vector<dev::TableJob> jobs_;
     std::unique_ptr<dev::ListJob> list_;
     std::vector<unsigned char> input_;
-    std::size_t late_at_ = 0;
     std::size_t list2_at_ = 0, listq_at_ = 0, count2_at_ = 0, countq_at_ = 0, rows_at_ = 0;
     std::vector<int> count2_;               // admissible residues mod two by d mod two
     std::vector<std::vector<int>> countq_;  // per class prime p: by d mod p
