@@ -415,11 +415,14 @@ rpg_status rpg_smem_read_probe(int32_t device, int32_t iterations, double *gbs,
                                double *bytes_per_clock_per_sm, double *ms);
 
 /* A finished rpg_sieve_run or rpg_point_search leaves its streams, events,
- * survivor buffers (up to 262,144 survivors) and pinned staging for the next
- * search on the same device (at most four such sets per process, about 16 MB
- * each).  This call frees them for `device` (-1: every device); a caller that
- * resets a device (cudaDeviceReset) calls it first.  Searches still running
- * are not affected.  No reference counterpart. */
+ * survivor buffers (up to 262,144 survivors), pinned staging and table memory
+ * for the next search on the same device (at most four such sets per process,
+ * up to 80 MB each; mostly 20), and a finished rpg_batch_search or server the
+ * resources of its engines (at most four, up to 512 MB of device memory each).
+ * An allocation that finds no memory frees them all and is tried again.  This
+ * call frees them for `device` (-1: every device); a caller that resets a
+ * device (cudaDeviceReset) calls it first.  Searches still running are not
+ * affected.  No reference counterpart. */
 rpg_status rpg_release_cached_resources(int32_t device);
 
 int32_t rpg_device_count(void);

@@ -101,7 +101,7 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False) -
     if force or _stale(LIBRARY, objects):
         tmp = LIBRARY.with_name(f"librpgpu.{os.getpid()}.tmp.so")
         _run([nvcc, GENCODE, "-shared", "-o", str(tmp), *map(str, objects),
-              "-Xcompiler", "-pthread"])
+              "-Xcompiler", "-pthread", "-Xlinker", "-z,nodelete"])
         os.replace(tmp, LIBRARY)
     main_obj = BUILD / (MAIN_SOURCE + ".o")
     if force or _stale(EXECUTABLE, [main_obj, LIBRARY]):

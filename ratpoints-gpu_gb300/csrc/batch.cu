@@ -1,15 +1,21 @@
 // Batched many-curve sieve (batch.hpp): device kernels and host driver.
 #include "batch.hpp"
 
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cmath>
+#include <condition_variable>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <stdexcept>
+#include <system_error>
 #include <thread>
 
 #include "exact.hpp"
@@ -1134,8 +1140,14 @@ struct DeviceArray {
         cudaFree(p);
         p = nullptr;
         cap = 0;
-        check_cuda(cudaMalloc(&p, count * sizeof(T)), what);
+        p = static_cast<T *>(device_malloc(count * sizeof(T), what));
         cap = count;
+    }
+    std::size_t bytes() const { return cap * sizeof(T); }
+    void free() {
+        cudaFree(p);
+        p = nullptr;
+        cap = 0;
     }
     void upload(const std::vector<T> &v, cudaStream_t s, unsigned long long &bytes, const char *what) {
         ensure(v.size(), what);
@@ -1146,32 +1158,105 @@ struct DeviceArray {
     }
 };
 
+// Host threads that share the per-curve work of batched runs (any number of
+// runs at a time).  They are started as work arrives, wait for more, and end
+// after a second without any: starting 16 threads for each of a run's four
+// loops took longer than the loops of a small batch.
+class Workers {
+public:
+    struct Job {
+        std::function<void(std::size_t)> fn;
+        std::size_t n = 0;
+        std::atomic<std::size_t> next{0};
+        int running = 0;  // threads inside, the caller apart (guarded by the mutex)
+        std::exception_ptr error;
+    };
+
+    // The process's instance; a child made by fork, which has none of its
+    // threads, gets a new one.  Never destroyed: its threads may outlive main.
+    static Workers &get() {
+        static std::mutex *creation = new std::mutex();
+        static Workers *instance = nullptr;
+        std::lock_guard<std::mutex> lock(*creation);
+        if (!instance || instance->pid_ != getpid()) instance = new Workers();
+        return *instance;
+    }
+
+    // fn(i) for i in [0, n), the caller taking part; rethrows the first exception.
+    void run(std::size_t n, std::function<void(std::size_t)> fn) {
+        const auto job = std::make_shared<Job>();
+        job->fn = std::move(fn);
+        job->n = n;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            jobs_.push_back(job);
+            const std::size_t wanted = std::min<std::size_t>(n - 1, limit_);
+            try {
+                while (threads_ < wanted) {
+                    std::thread(&Workers::loop, this).detach();
+                    ++threads_;
+                }
+            } catch (const std::system_error &) {
+                // no more threads to be had: those there are, and the caller, do the work
+            }
+        }
+        wake_.notify_all();
+        work(*job);
+        std::unique_lock<std::mutex> lock(mutex_);
+        const auto it = std::find(jobs_.begin(), jobs_.end(), job);
+        if (it != jobs_.end()) jobs_.erase(it);
+        done_.wait(lock, [&] { return job->running == 0; });
+        if (job->error) std::rethrow_exception(job->error);
+    }
+
+private:
+    Workers() : pid_(getpid()), limit_(std::min(std::max(std::thread::hardware_concurrency(), 1u), 64u) - 1) {}
+
+    void work(Job &job) {
+        for (std::size_t i; (i = job.next.fetch_add(1)) < job.n;) {
+            try {
+                job.fn(i);
+            } catch (...) {
+                std::lock_guard<std::mutex> lock(mutex_);
+                if (!job.error) job.error = std::current_exception();
+            }
+        }
+    }
+
+    void loop() {
+        std::unique_lock<std::mutex> lock(mutex_);
+        while (wake_.wait_for(lock, std::chrono::seconds(1), [&] { return !jobs_.empty(); })) {
+            const std::shared_ptr<Job> job = jobs_.front();
+            if (job->next.load() >= job->n) {
+                jobs_.pop_front();  // nothing of it left to take
+                continue;
+            }
+            ++job->running;
+            lock.unlock();
+            work(*job);
+            lock.lock();
+            --job->running;
+            done_.notify_all();
+        }
+        --threads_;
+    }
+
+    const pid_t pid_;
+    const std::size_t limit_;
+    std::size_t threads_ = 0;
+    std::mutex mutex_;
+    std::condition_variable wake_, done_;
+    std::deque<std::shared_ptr<Job>> jobs_;
+};
+
 // Runs fn(i) for i in [0, n) on the host's threads; rethrows the first exception.
 template <typename F>
 void parallel_for(std::size_t n, F &&fn) {
-    const unsigned threads = std::max(1u, std::min<unsigned>(std::thread::hardware_concurrency(), 64));
-    if (n < 2 || threads == 1) {
+    if (n < 2 || std::thread::hardware_concurrency() <= 1) {
         for (std::size_t i = 0; i < n; ++i) fn(i);
         return;
     }
-    std::atomic<std::size_t> next{0};
-    std::vector<std::thread> pool;
-    std::exception_ptr error;
-    std::mutex error_mutex;
-    for (unsigned t = 0; t < std::min<std::size_t>(threads, n); ++t) {
-        pool.emplace_back([&] {
-            for (std::size_t i; (i = next.fetch_add(1)) < n;) {
-                try {
-                    fn(i);
-                } catch (...) {
-                    std::lock_guard<std::mutex> lock(error_mutex);
-                    if (!error) error = std::current_exception();
-                }
-            }
-        });
-    }
-    for (auto &th : pool) th.join();
-    if (error) std::rethrow_exception(error);
+    Workers::get().run(n, std::function<void(std::size_t)>(std::ref(fn)));
 }
 
 long long gcd_ll(long long a, long long b) {
@@ -1289,9 +1374,9 @@ struct CurveWork {
 // Words of one denominator's row that the sieve sweeps: the whole row, or with
 // x intervals the interval numerators at a middle denominator (each interval
 // [lo, hi] covers about (hi - lo) d / 64 words).  Picks the kernel shape.
-long long swept_row_words(const BatchCurveSpec &c, long long words) {
+long long swept_row_words(const BatchCurveSpec &c, long long first, long long last, long long words) {
     if (c.intervals.empty() || c.intervals.size() > std::size_t(dev::kMaxIntervals)) return words;
-    const double dmid = 0.5 * double(c.first) + 0.5 * double(std::max(c.first, c.last));
+    const double dmid = 0.5 * double(first) + 0.5 * double(std::max(first, last));
     const double d = c.square ? dmid * dmid : dmid;
     double total = 0;
     for (const auto &iv : c.intervals) {
@@ -1388,8 +1473,9 @@ void class_prime_residues(const std::vector<std::string> &coefficients, int q, d
     const bool lead = lead_is_square(coefficients, q);
     for (int dq = 0; dq < q; ++dq) {
         out[dq] = 0;
+        const int inverse = dq == 0 ? 0 : int(mod_inverse(dq, q));
         for (int r = 0; r < q; ++r) {
-            const bool ok = dq == 0 ? (r != 0 && lead) : aff[(r * mod_inverse(dq, q)) % q] != 0;
+            const bool ok = dq == 0 ? (r != 0 && lead) : aff[(r * inverse) % q] != 0;
             if (ok) out[dq] |= dev::u64(1) << r;
         }
     }
@@ -1449,22 +1535,38 @@ struct BatchPlan {
     long long aff_words = 0, pattern_words = 0, row_words = 0;
     int wide_smem_words = 0;
     int wide_max_classes = 1;   // most classes of a denominator of any wide curve
+
+    // Empty, with the arrays' memory kept for the next run.
+    void clear() {
+        work.clear(), sweeps.clear(), wide.clear(), narrow.clear(), aspecs.clear(), residues.clear();
+        pspecs.clear(), cspecs.clear(), wide_items.clear(), narrow_items.clear(), class_starts.clear();
+        aff_words = pattern_words = row_words = 0;
+        wide_smem_words = 0;
+        wide_max_classes = 1;
+    }
+    std::size_t bytes() const {
+        auto of = [](const auto &v) { return v.capacity() * sizeof(v[0]); };
+        return of(work) + of(sweeps) + of(wide) + of(narrow) + of(aspecs) + of(residues) + of(pspecs) + of(cspecs) +
+               of(wide_items) + of(narrow_items) + of(class_starts);
+    }
 };
 
 // Validation and per-curve plans (one curve per task), then descriptors,
-// table specs and work items in the order the kernels take them.
-void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurveResult> &results,
-                BatchPlan &P, BatchStats &stats, int items_per_kernel) {
+// table specs and work items in the order the kernels take them.  Curves
+// marked in `solo` are validated and planned, but given no denominators.
+void build_plan(const std::vector<BatchCurveSpec> &curves, const std::vector<char> &solo,
+                std::vector<BatchCurveResult> &results, BatchPlan &P, BatchStats &stats, int items_per_kernel) {
     P.work.resize(curves.size());
     parallel_for(curves.size(), [&](std::size_t i) {
         const BatchCurveSpec &c = curves[i];
         BatchCurveResult &r = results[i];
         CurveWork &cw = P.work[i];
+        const long long first = solo[i] ? 1 : c.first, last = solo[i] ? 0 : c.last;
         try {
             if (c.coefficients.size() < 2) throw std::invalid_argument("polynomial must have degree >= 1");
             if (c.bound < 1) throw std::invalid_argument("numerator bound must be positive");
-            if (c.first < 1) throw std::invalid_argument("denominators start at 1");
-            if (c.last > (c.square ? 46340LL : 2147483647LL))
+            if (first < 1) throw std::invalid_argument("denominators start at 1");
+            if (last > (c.square ? 46340LL : 2147483647LL))
                 throw std::invalid_argument("denominator range too large for 32-bit denominators");
             if (c.bound > (1LL << 33))
                 throw std::invalid_argument("numerator bound too large for the batched search");
@@ -1475,8 +1577,8 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
                 return;
             }
             cw.words = word_count64(c.bound);
-            cw.count = c.last >= c.first ? c.last - c.first + 1 : 0;
-            cw.swept = swept_row_words(c, cw.words);
+            cw.count = last >= first ? last - first + 1 : 0;
+            cw.swept = swept_row_words(c, first, last, cw.words);
             cw.wide = cw.swept >= kBatchWideWords;
             if (cw.count > 0 && swept_alone(c, cw)) {
                 cw.plan = single_curve_plan(c.coefficients, c.bound, nullptr);
@@ -1523,17 +1625,6 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
     });
 
     const auto &cands = candidate_primes();
-    auto add_affine = [&](int p, const std::vector<std::string> &coeffs) {
-        dev::AffineSpec A{};
-        A.out = P.aff_words;
-        A.residues = (long long)P.residues.size();
-        A.p = p;
-        A.n = int(coeffs.size()) - 1;
-        for (const auto &c : coeffs) P.residues.push_back((unsigned short)decimal_mod(c, p));
-        P.aspecs.push_back(A);
-        P.aff_words += dev::kRefWords;
-        return A.out;
-    };
     // largest work first, so that the persistent kernels end on small items
     std::vector<std::size_t> order;
     for (std::size_t i = 0; i < curves.size(); ++i) {
@@ -1577,63 +1668,114 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
                        : std::max<long long>(dev::kNWarps,
                                              std::min<long long>(1 << 16, narrow_item / std::max(1LL, cw.swept)));
     };
+    // Where each curve's part of every array begins, so that the curves are
+    // described in parallel (one after another they took half the planning of
+    // a batch of 384 small searches).
+    struct Place {
+        std::size_t curve, aspec, residue, pspec, cspec, item, descriptor, cls;
+        long long aff, pattern, row;
+    };
+    std::vector<Place> places;
+    places.reserve(order.size());
     {
-        // sizes first, so that the vectors grow once
-        std::size_t wide_items = 0, narrow_items = 0;
+        std::size_t pspecs = 0, cspecs = 0, wide_items = 0, narrow_items = 0, wide = 0, narrow = 0, cls = 0;
+        std::size_t aspecs = 0, residues = 0;
         for (std::size_t i : order) {
             const CurveWork &cw = P.work[i];
-            const std::size_t n = curves[i].intervals.size();
-            const long long ranges = n > 0 && n <= std::size_t(dev::kMaxIntervals) ? (long long)n : 1;
+            places.push_back({i, aspecs, residues, pspecs, cspecs, cw.wide ? wide_items : narrow_items,
+                              cw.wide ? wide : narrow, cls, P.aff_words, P.pattern_words, P.row_words});
+            std::size_t primes = 0;
+            for (const auto &slot : cw.plan.slots)
+                for (int q : slot) {
+                    ++primes;
+                    P.pattern_words += (long long)q * q;
+                }
+            const int slots = cw.wide ? dev::kWideSlots : dev::kNarrowSlots;
+            for (int sl = 0; sl < slots; ++sl) {
+                const long long m = sl < int(cw.plan.moduli.size()) ? cw.plan.moduli[std::size_t(sl)] : 1;
+                P.row_words += m * (cw.wide ? round_even(m + dev::kWExt) : m + dev::kNK - 1);
+            }
+            P.row_words += P.row_words % 2;  // 16-byte aligned bulk copies
+            P.aff_words += (long long)(std::size_t(kCandidatePrimes) + primes) * dev::kRefWords;
+            aspecs += std::size_t(kCandidatePrimes) + primes;
+            residues += (std::size_t(kCandidatePrimes) + primes) * curves[i].coefficients.size();
+            pspecs += primes;
+            cspecs += std::size_t(slots);
             const long long chunk = item_chunk(cw);
             const std::size_t parts = std::size_t((cw.count + chunk - 1) / chunk);
-            if (cw.wide) wide_items += std::size_t(ranges) * parts;
-            else narrow_items += parts;
+            if (cw.wide) {
+                if ((2 * curves[i].bound) / (64LL * cw.plan.class_prime) / 64 + 2 >= dev::kMaxClassWords)
+                    throw std::invalid_argument("numerator bound too large for the batched search");
+                const std::size_t n = curves[i].intervals.size();
+                wide_items += parts * (n > 0 && n <= std::size_t(dev::kMaxIntervals) ? n : 1);
+                cls += 64 * std::size_t(cw.plan.class_prime);
+                ++wide;
+            } else {
+                narrow_items += parts;
+                ++narrow;
+            }
+            stats.rectangle_sites += (long double)(2 * curves[i].bound + 1) * (long double)cw.count;
+            stats.denominators += (unsigned long long)cw.count;
+            stats.words += (unsigned long long)(cw.words * cw.count);
+            stats.curves += 1;
+            stats.wide_curves += cw.wide ? 1 : 0;
         }
-        P.wide_items.reserve(wide_items);
-        P.narrow_items.reserve(narrow_items);
+        P.wide.resize(wide);
+        P.narrow.resize(narrow);
+        P.aspecs.resize(aspecs);
+        P.residues.resize(residues);
+        P.pspecs.resize(pspecs);
+        P.cspecs.resize(cspecs);
+        P.wide_items.resize(wide_items);
+        P.narrow_items.resize(narrow_items);
+        P.class_starts.resize(cls);
     }
-    for (std::size_t i : order) {
+    parallel_for(places.size(), [&](std::size_t k) {
+        Place at = places[k];
+        const std::size_t i = at.curve;
         const BatchCurveSpec &c = curves[i];
         CurveWork &cw = P.work[i];
         const FastPlan &plan = cw.plan;
+        auto add_affine = [&](int p, const unsigned short *residues) {
+            dev::AffineSpec A{};
+            A.out = at.aff;
+            A.residues = (long long)at.residue;
+            A.p = p;
+            A.n = int(c.coefficients.size()) - 1;
+            std::copy(residues, residues + c.coefficients.size(), &P.residues[at.residue]);
+            at.residue += c.coefficients.size();
+            P.aspecs[at.aspec++] = A;
+            at.aff += dev::kRefWords;
+            return A.out;
+        };
         const long long H = c.bound;
-        const long long aff_base = P.aff_words;
-        {
-            // the 36 candidate bitmasks, residues computed in the parallel phase
-            const std::size_t nc = c.coefficients.size();
-            for (int ci = 0; ci < kCandidatePrimes; ++ci) {
-                dev::AffineSpec A{};
-                A.out = P.aff_words;
-                A.residues = (long long)P.residues.size();
-                A.p = cands[ci];
-                A.n = int(nc) - 1;
-                P.residues.insert(P.residues.end(), cw.cand_residues.begin() + std::ptrdiff_t(ci * nc),
-                                  cw.cand_residues.begin() + std::ptrdiff_t((ci + 1) * nc));
-                P.aspecs.push_back(A);
-                P.aff_words += dev::kRefWords;
-            }
-        }
+        const long long aff_base = at.aff;
+        // the 36 candidate bitmasks, residues computed with the plan
+        for (int ci = 0; ci < kCandidatePrimes; ++ci)
+            add_affine(cands[ci], &cw.cand_residues[std::size_t(ci) * c.coefficients.size()]);
         // per-prime patterns of this curve's stage-1 factors
         const long long M = cw.wide ? 64LL * plan.class_prime : 1;
         const long long S = cw.wide ? 64LL * M : 64;
-        std::vector<long long> pattern_of(kFastPrimeLimit, -1);
+        long long pattern_of[kFastPrimeLimit];
+        std::vector<unsigned short> residues(c.coefficients.size());
         for (const auto &slot : plan.slots)
             for (int q : slot) {
-                if (pattern_of[q] >= 0) continue;
+                for (std::size_t j = 0; j < residues.size(); ++j)
+                    residues[j] = (unsigned short)decimal_mod(c.coefficients[j], q);
                 dev::PatternSpec Q{};
-                Q.offset = P.pattern_words;
-                Q.aff = add_affine(q, c.coefficients);
+                Q.offset = at.pattern;
+                Q.aff = add_affine(q, residues.data());
                 Q.q = q;
                 Q.lead_ok = lead_is_square(c.coefficients, q) ? 1 : 0;
                 Q.s = int(S % q);
                 Q.t = int(M % q);
-                P.pspecs.push_back(Q);
-                pattern_of[q] = P.pattern_words;
-                P.pattern_words += (long long)q * q;
+                P.pspecs[at.pspec++] = Q;
+                pattern_of[q] = at.pattern;
+                at.pattern += (long long)q * q;
             }
         auto add_composite = [&](int sl, int length) {
             dev::CompositeSpec T{};
-            T.offset = P.row_words;
+            T.offset = at.row;
             if (sl < int(plan.moduli.size())) {
                 T.m = plan.moduli[sl];
                 T.nf = int(plan.slots[sl].size());
@@ -1646,13 +1788,10 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
                 T.nf = 0;
             }
             T.length = length < 0 ? T.m : length;
-            P.cspecs.push_back(T);
-            P.row_words += (long long)T.m * T.length;
+            P.cspecs[at.cspec++] = T;
+            at.row += (long long)T.m * T.length;
             return T;
         };
-        stats.rectangle_sites += (long double)(2 * H + 1) * (long double)cw.count;
-        stats.denominators += (unsigned long long)cw.count;
-        stats.words += (unsigned long long)(cw.words * cw.count);
         if (cw.wide) {
             dev::WideCurve C{};
             const int q = plan.class_prime;
@@ -1671,8 +1810,6 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
             C.denom_primes[0] = cw.denom_primes[0] & ~(q > 1 ? dev::u64(1) << odd_prime_index(q) : 0);
             C.denom_primes[1] = cw.denom_primes[1];
             C.aff = aff_base;
-            if (C.count_q / 64 + 2 >= dev::kMaxClassWords)
-                throw std::invalid_argument("numerator bound too large for the batched search");
             int smem = 0;
             for (int sl = 0; sl < dev::kWideSlots; ++sl) {
                 const int m = sl < int(plan.moduli.size()) ? plan.moduli[sl] : 1;
@@ -1689,7 +1826,6 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
                 Md.step = dev::u32((dev::kWarpSize * dev::kWK) % m);
             }
             C.smem_words = smem;
-            P.wide_smem_words = std::max(P.wide_smem_words, round_even(smem));
             std::copy(cw.adm2, cw.adm2 + 64, C.admissible);
             if (q > 1) {
                 class_prime_residues(c.coefficients, q, C.admissible + 64);
@@ -1700,7 +1836,7 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
             for (int r64 = 0; r64 < 64; ++r64) C.mod_q[r64] = (unsigned char)(q > 1 ? r64 % q : 0);
             // class starts for every residue r mod M: ofs = (r + H) mod M, and per
             // modulus the row index ((-H + ofs) S^-1) mod m of class word 0
-            C.cls = (long long)P.class_starts.size();
+            C.cls = (long long)at.cls;
             for (long long r = 0; r < M; ++r) {
                 dev::ClassStart cs{};
                 const long long ofs = (r + H % M) % M;
@@ -1710,7 +1846,7 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
                     const long long m = Md.m;
                     cs.start[sl] = (unsigned short)((Md.neg_h + ofs) % m * Md.inv_stride % m);
                 }
-                P.class_starts.push_back(cs);
+                P.class_starts[at.cls++] = cs;
             }
             for (int ci = 0; ci < kCandidatePrimes; ++ci) {
                 const int p = cands[ci];
@@ -1719,16 +1855,13 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
                 C.m_mod[ci] = (unsigned short)(M % p);
             }
             device_intervals(c.intervals, C.nint, C.lo, C.hi);
-            P.wide_max_classes = std::max(P.wide_max_classes, cw.classes);
             const long long chunk = item_chunk(cw);
             for (int range = 0; range < std::max(1, C.nint); ++range)
                 for (long long f = c.first; f <= c.last; f += chunk)
-                    P.wide_items.push_back({f, int(P.wide.size()), int(std::min(chunk, c.last - f + 1)),
-                                            range, 0});
-            P.wide.push_back(C);
-            stats.wide_curves += 1;
+                    P.wide_items[at.item++] = {f, int(at.descriptor), int(std::min(chunk, c.last - f + 1)), range, 0};
+            P.wide[at.descriptor] = C;
         } else {
-            dev::NarrowCurve C{};
+            dev::NarrowCurve &C = P.narrow[at.descriptor];
             C.bound = H;
             C.words = cw.words;
             C.square = c.square ? 1 : 0;
@@ -1737,8 +1870,7 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
             C.denom_primes[0] = cw.denom_primes[0];
             C.denom_primes[1] = cw.denom_primes[1];
             C.aff = aff_base;
-            if (P.row_words % 2) P.row_words += 1;  // 16-byte aligned bulk copy
-            C.tables = P.row_words;
+            C.tables = at.row;
             int used = 0;
             for (int sl = 0; sl < dev::kNarrowSlots; ++sl) {
                 const int m = sl < int(plan.moduli.size()) ? plan.moduli[sl] : 1;
@@ -1752,10 +1884,7 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
                 C.shift[sl] = dev::u32(((m - H % m) % m) * inv64 % m);
                 C.step[sl] = dev::u32((dev::kWarpSize * dev::kNK) % m);
             }
-            if (used % 2) {
-                P.row_words += 1;
-                used += 1;
-            }
+            used += used % 2;
             if (used > dev::kNarrowTableWords) throw std::logic_error("narrow tables exceed shared memory");
             C.table_words = used;
             // dense layout: bit j of a word holds a = -H + 64 w + j, so a = j - H (mod 64)
@@ -1770,14 +1899,51 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, std::vector<BatchCurv
             device_intervals(c.intervals, C.nint, C.lo, C.hi);
             const long long chunk = item_chunk(cw);
             for (long long f = c.first; f <= c.last; f += chunk)
-                P.narrow_items.push_back({f, int(P.narrow.size()), int(std::min(chunk, c.last - f + 1)), 0, 0});
-            P.narrow.push_back(C);
+                P.narrow_items[at.item++] = {f, int(at.descriptor), int(std::min(chunk, c.last - f + 1)), 0, 0};
         }
-        stats.curves += 1;
-    }
+    });
+    for (const auto &C : P.wide) P.wide_smem_words = std::max(P.wide_smem_words, round_even(C.smem_words));
+    for (const auto &at : places)
+        if (P.work[at.curve].wide) P.wide_max_classes = std::max(P.wide_max_classes, P.work[at.curve].classes);
     stats.wide_items = P.wide_items.size();
     stats.narrow_items = P.narrow_items.size();
     stats.table_words = (unsigned long long)P.row_words;
+}
+
+}  // namespace
+
+namespace {
+
+// Curve-independent tables: inverses and squares modulo every prime below
+// 512, made once per process.
+struct FixedTables {
+    std::vector<unsigned short> inverses;
+    std::vector<dev::u64> squares;
+    std::vector<dev::OddPrime> odd;
+};
+const FixedTables &fixed_tables() {
+    static const FixedTables tables = [] {
+        FixedTables t;
+        t.inverses.assign(std::size_t(kMaximumPrime) * kMaximumPrime, 0);
+        t.squares.assign(std::size_t(kMaximumPrime) * dev::kRefWords, 0);
+        for (int p = 2; p < kMaximumPrime; ++p) {
+            if (!is_small_prime(p)) continue;
+            modular_inverses(p, &t.inverses[std::size_t(p) * kMaximumPrime]);
+            for (int v = 0; v < p; ++v) {
+                const int sq = v * v % p;
+                t.squares[std::size_t(p) * dev::kRefWords + sq / 64] |= dev::u64(1) << (sq % 64);
+            }
+        }
+        for (int p = 3; p < kMaximumPrime; p += 2)
+            if (is_small_prime(p)) {
+                dev::u32 inverse = dev::u32(p);  // Newton's iteration, right in 3 bits to start with
+                for (int i = 0; i < 4; ++i) inverse *= 2u - dev::u32(p) * inverse;
+                t.odd.push_back({dev::u32(p), inverse, host_magic(p)});
+            }
+        if (t.odd.size() != std::size_t(dev::kOddPrimes)) throw std::logic_error("odd prime table");
+        return t;
+    }();
+    return tables;
 }
 
 }  // namespace
@@ -1798,7 +1964,9 @@ struct BatchEngine::Impl {
     // shared-memory bytes read
     static constexpr int kCounters = 7;
     unsigned long long *h_counters = nullptr;
-    unsigned long long capacity = 1ull << 20;
+    unsigned long long capacity = 0;  // survivors of a run (grows)
+    BatchPlan plan;                   // of the run; its memory is kept
+    bool failed = false;              // a run is under way, or ended with an exception
     dev::Candidates cand{};
     DeviceArray<dev::WideCurve> d_wide;
     DeviceArray<dev::NarrowCurve> d_narrow;
@@ -1819,8 +1987,7 @@ struct BatchEngine::Impl {
     DeviceArray<unsigned long long> d_curve_modular;  // per-curve modular survivors
     Preverifier pre;
 
-    explicit Impl(int dev_ordinal) {
-        if (dev_ordinal >= 0) check_cuda(cudaSetDevice(dev_ordinal), "cudaSetDevice");
+    Impl() {  // on the current device
         check_cuda(cudaGetDevice(&device), "cudaGetDevice");
         check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device),
                    "cudaDeviceGetAttribute");
@@ -1832,42 +1999,59 @@ struct BatchEngine::Impl {
         check_cuda(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "cudaEventCreate");
         check_cuda(cudaEventCreateWithFlags(&join, cudaEventDisableTiming), "cudaEventCreate");
         check_cuda(cudaMallocHost(&h_counters, 8 * sizeof(unsigned long long)), "cudaMallocHost");
-        // RPG_BATCH_CAPACITY overrides the first survivor capacity (tests use a
-        // small one to exercise the rerun after an overflow)
-        if (const char *env = std::getenv("RPG_BATCH_CAPACITY"))
-            capacity = (unsigned long long)std::max(1LL, std::atoll(env));
         const auto &cands = candidate_primes();
         for (int ci = 0; ci < kCandidatePrimes; ++ci) {
             cand.p[ci] = cands[ci];
             cand.magic[ci] = dev::magic40(dev::u32(cands[ci]));
         }
-        // curve-independent tables: inverses and squares modulo every prime below 512
-        std::vector<unsigned short> inv_table(std::size_t(kMaximumPrime) * kMaximumPrime, 0);
-        std::vector<dev::u64> square_masks(std::size_t(kMaximumPrime) * dev::kRefWords, 0);
-        for (int p = 2; p < kMaximumPrime; ++p) {
-            if (!is_small_prime(p)) continue;
-            for (int r = 1; r < p; ++r)
-                inv_table[std::size_t(p) * kMaximumPrime + r] = (unsigned short)mod_inverse(r, p);
-            for (long long v = 0; v < p; ++v) {
-                const int sq = int(v * v % p);
-                square_masks[std::size_t(p) * dev::kRefWords + sq / 64] |= dev::u64(1) << (sq % 64);
-            }
-        }
-        std::vector<dev::OddPrime> odd;
-        for (int p = 3; p < kMaximumPrime; p += 2)
-            if (is_small_prime(p)) {
-                dev::u32 inverse = dev::u32(p);  // Newton's iteration, right in 3 bits to start with
-                for (int i = 0; i < 4; ++i) inverse *= 2u - dev::u32(p) * inverse;
-                odd.push_back({dev::u32(p), inverse, host_magic(p)});
-            }
-        if (odd.size() != std::size_t(dev::kOddPrimes)) throw std::logic_error("odd prime table");
+        const FixedTables &fixed = fixed_tables();
         unsigned long long bytes = 0;
-        d_inv.upload(inv_table, stream, bytes, "upload inverses");
-        d_sq.upload(square_masks, stream, bytes, "upload squares");
-        d_odd.upload(odd, stream, bytes, "upload odd primes");
+        d_inv.upload(fixed.inverses, stream, bytes, "upload inverses");
+        d_sq.upload(fixed.squares, stream, bytes, "upload squares");
+        d_odd.upload(fixed.odd, stream, bytes, "upload odd primes");
         d_counters.ensure(kCounters, "cudaMalloc(batch counters)");
-        ensure_output(capacity);
         check_cuda(cudaStreamSynchronize(stream), "batch engine setup");
+    }
+
+    // The survivor capacity of an engine's first run.  RPG_BATCH_CAPACITY
+    // overrides it (tests use a small one to exercise the rerun after an
+    // overflow).
+    static unsigned long long first_capacity() {
+        if (const char *env = std::getenv("RPG_BATCH_CAPACITY"))
+            return (unsigned long long)std::max(1LL, std::atoll(env));
+        return 1ull << 20;
+    }
+
+    // True if nothing of it is in flight and every stream finished without error.
+    bool idle() {
+        if (failed) return false;
+        for (cudaStream_t s : {stream, side})
+            if (cudaStreamSynchronize(s) != cudaSuccess) return false;
+        for (cudaStream_t s : sweep_stream)
+            if (cudaStreamSynchronize(s) != cudaSuccess) return false;
+        return true;
+    }
+
+    // Frees the largest arrays until at most `limit` bytes are held on the
+    // device, and the host's plan if it holds more than an eighth of that.
+    void trim(std::size_t limit) {
+        plan.clear();
+        if (plan.bytes() > limit / 8) plan = BatchPlan{};
+        std::vector<std::pair<std::size_t, std::function<void()>>> arrays;
+        std::size_t total = 0;
+        auto add = [&](auto &x) {
+            arrays.push_back({x.bytes(), [&x] { x.free(); }});
+            total += x.bytes();
+        };
+        add(d_wide), add(d_narrow), add(d_witems), add(d_nitems), add(d_aspecs), add(d_pspecs), add(d_cspecs);
+        add(d_cls), add(d_res), add(d_aff), add(d_patterns), add(d_rows), add(d_counters), add(d_sweep_tables);
+        add(d_a), add(d_pa), add(d_d), add(d_c), add(d_pd), add(d_pc), add(d_curve_modular);
+        std::sort(arrays.begin(), arrays.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
+        for (auto &x : arrays) {
+            if (total <= limit) break;
+            x.second();
+            total -= x.first;
+        }
     }
 
     ~Impl() {
@@ -1915,12 +2099,12 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
     stats.items_per_kernel = items_per_kernel;
     std::vector<BatchCurveResult> results(curves.size());
     check_cuda(cudaSetDevice(device), "cudaSetDevice");
+    failed = true;  // until the end
     // Curves with huge rows fill the device on their own: batching gains them
     // nothing, and the single-curve kernel (row count compiled in, stage 2
     // from class-layout tables) sweeps them faster.  They are validated with
     // the others, then searched one by one in a thread beside the batched
     // kernels.
-    std::vector<BatchCurveSpec> batched(curves);
     std::vector<std::size_t> solo;
     std::vector<char> is_solo(curves.size(), 0);
     for (std::size_t i = 0; i < curves.size(); ++i)
@@ -1928,12 +2112,11 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
             word_count64(curves[i].bound) >= kBatchSoloWords) {
             solo.push_back(i);
             is_solo[i] = 1;
-            batched[i].first = 1;
-            batched[i].last = 0;
         }
-    BatchPlan P;
+    BatchPlan &P = plan;
+    P.clear();
     const auto t_plan = Clock::now();
-    build_plan(batched, results, P, stats, items_per_kernel);
+    build_plan(curves, is_solo, results, P, stats, items_per_kernel);
     stats.plan_ms = ms_since(t_plan);
     const std::vector<CurveWork> &work = P.work;
     std::exception_ptr solo_error;
@@ -1998,12 +2181,15 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
             sweep_tables.place(d_sweep_tables.p, stream);
             stats.h2d_bytes += sweep_tables.upload_bytes();
         }
+        ensure_output(capacity);
         d_counters.ensure(kCounters + P.sweeps.size(), "cudaMalloc(batch counters)");
         if (preverify) {
             std::vector<const std::vector<std::string> *> coefs(curves.size(), nullptr);
             for (std::size_t i = 0; i < curves.size(); ++i)
                 if (work[i].ok) coefs[i] = &curves[i].coefficients;
-            pre.prepare(coefs, stream);
+            pre.prepare(coefs, stream, [](std::size_t n, const std::function<void(std::size_t)> &fn) {
+                parallel_for(n, fn);
+            });
             stats.h2d_bytes += pre.upload_bytes();
             d_curve_modular.ensure(std::max<std::size_t>(1, curves.size()), "cudaMalloc(batch counters)");
         }
@@ -2267,14 +2453,72 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
         if (work[i].poly->square_root(1, 0, root))
             results[i].points.insert(results[i].points.begin(), PointPair{1, root, 0});
     });
+    failed = false;
     for (const auto &r : results) stats.points += r.points.size();
     stats.wall_ms = ms_since(started);
     if (stats_out) *stats_out = stats;
     return results;
 }
 
-BatchEngine::BatchEngine(int device) : impl_(new Impl(device)) {}
-BatchEngine::~BatchEngine() = default;
+// The device resources of engines that are gone, kept for the next engine on
+// the same device: creating and freeing nine streams, the events and some
+// twenty arrays took about 3 of the 13 ms of a batch of 384 small searches.  Every
+// run uploads, clears or builds all that it reads but the tables that are the
+// same for all curves.  Never destroyed: static destructors may run after the
+// CUDA runtime is gone.
+struct BatchEnginePool {
+    static constexpr std::size_t kEngines = 4;                     // per process
+    static constexpr std::size_t kBytes = std::size_t(512) << 20;  // device memory kept by each
+    std::mutex mutex;
+    std::vector<std::unique_ptr<BatchEngine::Impl>> idle;
+
+    static BatchEnginePool &get() {
+        static auto *pool = new BatchEnginePool();
+        return *pool;
+    }
+    std::unique_ptr<BatchEngine::Impl> take(int device) {
+        std::lock_guard<std::mutex> lock(mutex);
+        for (auto it = idle.rbegin(); it != idle.rend(); ++it)
+            if ((*it)->device == device) {
+                std::unique_ptr<BatchEngine::Impl> engine = std::move(*it);
+                idle.erase(std::next(it).base());
+                return engine;
+            }
+        return nullptr;
+    }
+    // Destroys what it does not keep (outside the lock).
+    void give(std::unique_ptr<BatchEngine::Impl> engine) {
+        if (!engine->idle()) return;
+        engine->trim(kBytes);
+        std::lock_guard<std::mutex> lock(mutex);
+        if (idle.size() < kEngines) idle.push_back(std::move(engine));
+    }
+};
+
+BatchEngine::BatchEngine(int device) {
+    if (device >= 0) check_cuda(cudaSetDevice(device), "cudaSetDevice");
+    int current = 0;
+    check_cuda(cudaGetDevice(&current), "cudaGetDevice");
+    impl_ = BatchEnginePool::get().take(current);
+    if (!impl_) impl_.reset(new Impl());
+    impl_->capacity = Impl::first_capacity();
+}
+
+BatchEngine::~BatchEngine() {
+    try {
+        if (impl_) BatchEnginePool::get().give(std::move(impl_));
+    } catch (...) {  // no memory for the pool's list: the engine is freed
+    }
+}
+
+void release_pooled_engines(int device) {
+    std::vector<std::unique_ptr<BatchEngine::Impl>> taken;
+    auto &pool = BatchEnginePool::get();
+    std::lock_guard<std::mutex> lock(pool.mutex);
+    for (auto &engine : pool.idle)
+        if (device < 0 || engine->device == device) taken.push_back(std::move(engine));
+    pool.idle.erase(std::remove(pool.idle.begin(), pool.idle.end(), nullptr), pool.idle.end());
+}
 
 std::vector<BatchCurveResult> BatchEngine::run(const std::vector<BatchCurveSpec> &curves,
                                                BatchStats *stats, bool use_graph, bool preverify,

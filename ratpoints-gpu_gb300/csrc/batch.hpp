@@ -78,7 +78,9 @@ struct BatchStats {
 // Device resources of batched runs kept across runs: streams, events, the
 // curve-independent tables and grow-only device buffers (tables, bitmasks,
 // descriptors, work items, survivors), so that a run allocates nothing once
-// the buffers are large enough.  One engine serves one thread at a time.
+// the buffers are large enough.  One engine serves one thread at a time; when
+// it goes, a bounded part of its resources stays for the process's next engine
+// on the device.
 class BatchEngine {
 public:
     explicit BatchEngine(int device);  // -1: the calling thread's current device
@@ -98,16 +100,20 @@ public:
     std::vector<BatchCurveResult> run(const std::vector<BatchCurveSpec> &curves, BatchStats *stats,
                                       bool use_graph = true, bool preverify = true, int items_per_kernel = 0);
     int device() const;
+    struct Impl;
 
     // Upper estimate of the device bytes a curve adds to a run (admission).
     static unsigned long long estimate_bytes(const BatchCurveSpec &curve);
 
 private:
-    struct Impl;
     std::unique_ptr<Impl> impl_;
 };
 
-// One batched pass on a fresh engine on `device` (-1: current).
+// Frees what engines that are gone left for reuse on `device` (-1: every
+// device).
+void release_pooled_engines(int device);
+
+// One batched pass on an engine on `device` (-1: current).
 std::vector<BatchCurveResult> batch_search(const std::vector<BatchCurveSpec> &curves, int device,
                                            BatchStats *stats, bool use_graph = true, bool preverify = true);
 

@@ -66,16 +66,14 @@ bool coefficients_from(const char *const *c, int32_t n, std::vector<std::string>
         }
         std::string s(c[i]);
         if (!s.empty() && s.front() == '+') s.erase(0, 1);
-        rpg::BigInt probe;
-        if (!rpg::BigInt::parse(s, probe)) {
+        const std::size_t digits = s.find_first_not_of("+-") == 0 ? 0 : 1;  // after at most one sign
+        if (s.size() <= digits || s.find_first_not_of("0123456789", digits) != std::string::npos) {
             error = "coefficients must be decimal integers";
             return false;
         }
-        out.push_back(s);
+        out.push_back(std::move(s));
     }
-    rpg::BigInt lead;
-    rpg::BigInt::parse(out.back(), lead);
-    if (lead.is_zero()) {
+    if (out.back().find_first_of("123456789") == std::string::npos) {
         error = "leading coefficient must be nonzero";
         return false;
     }
@@ -360,6 +358,7 @@ rpg_status rpg_session_create(const char *const *coefficients, int32_t coefficie
         so.device = device;
         std::unique_ptr<rpg_session> s(new rpg_session);
         s->sieve.reset(new rpg::Sieve(coeffs, numerator_bound, so));
+        s->sieve->wait_tables();  // allocation-free launches come on the callers' streams
         rpg::check_cuda(cudaEventCreate(&s->begin), "cudaEventCreate");
         rpg::check_cuda(cudaEventCreate(&s->end), "cudaEventCreate");
         *session = s.release();
@@ -426,13 +425,13 @@ void batch_specs_from(const rpg_search_options *curves, int32_t curve_count, std
             continue;
         }
         rpg::BatchCurveSpec b;
-        b.coefficients = s.coefficients;
+        b.coefficients = std::move(s.coefficients);
         b.bound = s.numerator_bound;
         b.first = s.first;
         b.last = s.last;
         b.square = s.square;
         b.include_infinity = s.include_infinity;
-        b.intervals = s.intervals;
+        b.intervals = std::move(s.intervals);
         valid.push_back(std::size_t(i));
         run.push_back(std::move(b));
     }
@@ -567,13 +566,13 @@ rpg_status rpg_server_submit(rpg_server *server, const rpg_search_options *reque
         std::string error;
         if (!options_from(*request, s, error)) return fail(RPG_E_ARG, error);
         rpg::BatchCurveSpec b;
-        b.coefficients = s.coefficients;
+        b.coefficients = std::move(s.coefficients);
         b.bound = s.numerator_bound;
         b.first = s.first;
         b.last = s.last;
         b.square = s.square;
         b.include_infinity = s.include_infinity;
-        b.intervals = s.intervals;
+        b.intervals = std::move(s.intervals);
         *request_id = server->server->submit(b, first_point_only != 0);
         return RPG_OK;
     });
@@ -618,6 +617,7 @@ int32_t rpg_abi_version(void) { return RPG_ABI_VERSION; }
 rpg_status rpg_release_cached_resources(int32_t device) {
     return guarded([&]() -> rpg_status {
         rpg::release_pooled_pipelines(device < 0 ? -1 : device);
+        rpg::release_pooled_engines(device < 0 ? -1 : device);
         return RPG_OK;
     });
 }

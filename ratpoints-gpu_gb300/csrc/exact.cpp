@@ -205,7 +205,8 @@ bool ExactPolynomial::is_squarefree() const {
     long long needed = (long long)(bound_bits / 60.0) + 2;
     long long tested = 0;
     for (u64 p = (u64(1) << 61) - 1; tested < needed; p -= 2) {
-        if (!is_prime_u64(p)) continue;
+        // 2^61 - 1, with which nearly every call ends, is a Mersenne prime
+        if (p != (u64(1) << 61) - 1 && !is_prime_u64(p)) continue;
         if (coeffs_.back().mod(p) == 0 || u64(n) % p == 0) continue;
         std::vector<u64> f(coeffs_.size()), g(coeffs_.size() - 1);
         for (std::size_t i = 0; i < coeffs_.size(); ++i) f[i] = coeffs_[i].mod(p);

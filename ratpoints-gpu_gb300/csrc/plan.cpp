@@ -24,10 +24,16 @@ const std::array<int, kCandidatePrimes> &candidate_primes() {
 
 int decimal_mod(const std::string &text, int modulus) {
     std::size_t i = 0;
-    bool negative = i < text.size() && text[i] == '-';
+    const bool negative = i < text.size() && text[i] == '-';
     if (i < text.size() && (text[i] == '-' || text[i] == '+')) ++i;
+    // nine digits per division: value * 10^9 + chunk < 2^31 (10^9 + 1)
     long long value = 0;
-    for (; i < text.size(); ++i) value = (10 * value + (text[i] - '0')) % modulus;
+    while (i < text.size()) {
+        const std::size_t end = std::min(text.size(), i + 9);
+        long long chunk = 0, scale = 1;
+        for (; i < end; ++i, scale *= 10) chunk = 10 * chunk + (text[i] - '0');
+        value = (value * scale + chunk) % modulus;
+    }
     return negative && value ? int(modulus - value) : int(value);
 }
 
@@ -55,55 +61,101 @@ void modular_inverses(int p, unsigned short *out) {
     }
 }
 
+namespace {
+
+// squares[p][v]: v is a square mod p, for the primes p below 512 (made once).
+struct SquareTable {
+    std::vector<std::uint8_t> bits[kMaximumPrime];
+    SquareTable() {
+        for (int p = 3; p < kMaximumPrime; p += 2) {
+            bool prime = true;
+            for (int f = 3; f * f <= p && prime; f += 2) prime = p % f != 0;
+            if (!prime) continue;
+            bits[p].assign(std::size_t(p), 0);
+            for (int v = 0; 2 * v <= p; ++v) bits[p][std::size_t(v * v % p)] = 1;
+        }
+    }
+};
+const SquareTable &square_table() {
+    static const SquareTable table;
+    return table;
+}
+
+}  // namespace
+
 bool square_mod(long long value, int p) {
     long long v = value % p;
     if (v < 0) v += p;
     if (v == 0 || p == 2) return true;
+    if (p < kMaximumPrime) {
+        const auto &squares = square_table().bits[p];
+        if (!squares.empty()) return squares[std::size_t(v)] != 0;
+    }
     long long result = 1;  // Euler's criterion: v^((p-1)/2) = 1
     for (long long e = (p - 1) / 2, b = v; e; e >>= 1, b = b * b % p)
         if (e & 1) result = result * b % p;
     return result == 1;
 }
 
-std::vector<std::uint8_t> affine_mask(int prime, const std::vector<std::string> &coefficients) {
-    std::vector<int> residues(coefficients.size());
-    for (std::size_t i = 0; i < coefficients.size(); ++i)
-        residues[i] = decimal_mod(coefficients[i], prime);
-    std::vector<std::uint8_t> square(prime, 0);
-    // v^2 mod p for v <= p / 2 (the rest repeat them): (v + 1)^2 = v^2 + 2v + 1
-    for (long long v = 0, sq = 0; 2 * v <= prime; ++v) {
-        square[sq] = 1;
-        sq += 2 * v + 1;
-        while (sq >= prime) sq -= prime;
+namespace {
+
+// out[x] = 1 iff f(x) mod p is a square (0 included); returns how many are.
+// p an odd prime < 512: n mod p for n < 2^19 is n - p floor(n ceil(2^32 / p) / 2^32).
+int affine_into(int prime, const std::vector<std::string> &coefficients, std::uint8_t *out) {
+    const unsigned p = unsigned(prime);
+    const unsigned long long magic = ((1ull << 32) + p - 1) / p;
+    auto mod = [&](unsigned n) { return n - unsigned((n * magic) >> 32) * p; };
+    const std::uint8_t *square = square_table().bits[prime].data();
+    const int degree = int(coefficients.size()) - 1;
+    // the coefficients mod p; c_k with k >= p joins c_(k mod (p - 1)), as
+    // x^p = x, so that at most p coefficients are left
+    unsigned residues[kMaximumPrime] = {};
+    int n = 0;
+    for (int k = 0; k <= degree; ++k) {
+        const int at = k < prime ? k : (k - 1) % (prime - 1) + 1;
+        residues[at] = mod(residues[at] + unsigned(decimal_mod(coefficients[std::size_t(k)], prime)));
+        n = std::max(n, at);
     }
-    std::vector<std::uint8_t> affine(prime, 0);
-    auto evaluate = [&](long long x) {
-        long long value = 0;
-        for (std::size_t i = residues.size(); i-- > 0;) value = (value * x + residues[i]) % prime;
+    auto evaluate = [&](unsigned x) {
+        unsigned value = 0;
+        for (int k = n; k >= 0; --k) value = mod(value * x + residues[k]);
         return value;
     };
-    const int degree = int(residues.size()) - 1;
-    if (prime <= 2 * (degree + 1)) {
-        for (int x = 0; x < prime; ++x) affine[x] = square[evaluate(x)];
-        return affine;
+    int count = 0;
+    if (prime <= 2 * (n + 1)) {
+        for (unsigned x = 0; x < p; ++x) count += out[x] = square[evaluate(x)];
+        return count;
     }
-    // Forward differences: f(x + 1) from f(x) with degree additions mod p
-    // instead of a Horner evaluation (a division per coefficient) at every x.
-    std::vector<long long> diff(std::size_t(degree) + 1);
-    for (int x = 0; x <= degree; ++x) diff[std::size_t(x)] = evaluate(x);
-    for (int k = 1; k <= degree; ++k)  // diff[k] = k-th difference at 0
-        for (int x = degree; x >= k; --x) {
-            long long v = diff[std::size_t(x)] - diff[std::size_t(x) - 1];
-            diff[std::size_t(x)] = v < 0 ? v + prime : v;
+    // Forward differences: f(x + 1) from f(x) with n additions mod p instead
+    // of a Horner evaluation at every x.
+    unsigned diff[kMaximumPrime];
+    for (int x = 0; x <= n; ++x) diff[x] = evaluate(unsigned(x));
+    for (int k = 1; k <= n; ++k)  // diff[k] = k-th difference at 0
+        for (int x = n; x >= k; --x) {
+            const unsigned v = diff[x] + p - diff[x - 1];
+            diff[x] = v >= p ? v - p : v;
         }
-    for (int x = 0; x < prime; ++x) {
-        affine[x] = square[diff[0]];
-        for (int k = 0; k < degree; ++k) {
-            long long v = diff[std::size_t(k)] + diff[std::size_t(k) + 1];
-            diff[std::size_t(k)] = v >= prime ? v - prime : v;
+    for (unsigned x = 0; x < p; ++x) {
+        count += out[x] = square[diff[0]];
+        for (int k = 0; k < n; ++k) {
+            const unsigned v = diff[k] + diff[k + 1];
+            diff[k] = std::min(v, v - p);  // unsigned: wraps below p
         }
     }
+    return count;
+}
+
+}  // namespace
+
+std::vector<std::uint8_t> affine_mask(int prime, const std::vector<std::string> &coefficients) {
+    std::vector<std::uint8_t> affine(static_cast<std::size_t>(prime), 0);
+    affine_into(prime, coefficients, affine.data());
     return affine;
+}
+
+int admitted_residues(int prime, const std::vector<std::string> &coefficients) {
+    std::uint8_t affine[kMaximumPrime];
+    return affine_into(prime, coefficients, affine);
 }
 
 bool select_primes(long long denominator, int *indices) {
@@ -121,31 +173,29 @@ long long word_count64(long long bound) {
 long long word_count32(long long bound) { return (2 * bound + 32) / 32; }
 
 double pass_rate(int q, const std::vector<std::string> &coefficients) {
-    const auto aff = affine_mask(q, coefficients);
-    int n = 0;
-    for (auto v : aff) n += v;
-    return double(n) / q;
+    return double(admitted_residues(q, coefficients)) / q;
 }
 
 void two_adic_classes(const std::vector<std::string> &coefficients, std::uint64_t out[64]) {
     const int n = int(coefficients.size()) - 1;
-    std::vector<int> c64(coefficients.size());
-    for (std::size_t i = 0; i < coefficients.size(); ++i) c64[i] = decimal_mod(coefficients[i], 64);
-    bool square64[64] = {};
-    for (int v = 0; v < 64; ++v) square64[(v * v) & 63] = true;
+    std::vector<std::uint8_t> c(coefficients.size());
+    for (std::size_t i = 0; i < c.size(); ++i) c[i] = std::uint8_t(decimal_mod(coefficients[i], 64));
+    // Horner for all residues r at once, in bytes: sums and products mod 256
+    // are right mod 64
+    std::uint8_t square[64] = {}, value[64];
+    for (int v = 0; v < 64; ++v) square[(v * v) & 63] = 1;
     for (int dd = 0; dd < 64; ++dd) {
-        out[dd] = 0;
-        for (int r = 0; r < 64; ++r) {
-            if (dd % 2 == 0 && r % 2 == 0) continue;
-            int value = c64[n], power = 1;
-            for (int i = n - 1; i >= 0; --i) {
-                value = (value * r) & 63;
-                power = (power * dd) & 63;
-                value = (value + c64[i] * power) & 63;
-            }
-            if (n % 2 == 1) value = (value * dd) & 63;
-            if (square64[value]) out[dd] |= std::uint64_t(1) << r;
+        std::uint8_t power = 1;
+        std::fill(value, value + 64, c[std::size_t(n)]);
+        for (int i = n - 1; i >= 0; --i) {
+            power = std::uint8_t(power * dd);
+            const std::uint8_t term = std::uint8_t(c[std::size_t(i)] * power);
+            for (int r = 0; r < 64; ++r) value[r] = std::uint8_t(value[r] * r + term);
         }
+        std::uint64_t mask = 0;
+        for (int r = 0; r < 64; ++r)
+            mask |= std::uint64_t(square[(n % 2 ? value[r] * dd : value[r]) & 63]) << r;
+        out[dd] = dd % 2 ? mask : mask & 0xAAAAAAAAAAAAAAAAull;
     }
 }
 
@@ -318,6 +368,15 @@ FastPlan FastPlanner::plan(int max_modulus, int max_slots, long long row_budget,
         plan.moduli.push_back(pair[0] * pair[1]);
         plan.slots.push_back(pair);
     }
+    // counts back from the strengths (8 bits stand for none)
+    auto count_of = [&](int q) {
+        for (const auto &s : strength_)
+            if (s.second == q) return s.first >= 8.0 ? 0 : int(std::lround(std::exp2(-s.first) * q));
+        return -1;  // not a prime of the planner: left to the caller
+    };
+    for (const auto &f : plan.slots)
+        for (int q : f) plan.admitted.push_back({q, count_of(q)});
+    if (plan.class_prime > 1) plan.admitted.push_back({plan.class_prime, count_of(plan.class_prime)});
     return plan;
 }
 

@@ -39,7 +39,10 @@ void modular_inverses(int p, unsigned short *out);
 bool square_mod(long long value, int p);
 
 // affine[x] = 1 iff f(x) mod p is a square (0 included), for x in [0, p).
+// An odd prime below 512.
 std::vector<std::uint8_t> affine_mask(int prime, const std::vector<std::string> &coefficients);
+// How many such x there are.
+int admitted_residues(int prime, const std::vector<std::string> &coefficients);
 
 // Indices into candidate_primes() of the 32 largest candidates not dividing
 // denominator, largest first.  Returns false if fewer than 32 qualify.
@@ -83,6 +86,8 @@ struct FastPlan {
     std::vector<std::vector<int>> slots;   // prime factors of each stage-1 modulus
     std::vector<int> moduli;               // their products
     double bits = 0;                       // expected filtering of the stage-1 rows (bits)
+    // (p, residues x with f(x) a square mod p) of the plan's primes, class prime included
+    std::vector<std::pair<int, int>> admitted;
     int row_slots = 2;                     // single-curve kernel: denominators staged per CTA (2 or 3)
 };
 // max_modulus caps each stage-1 modulus (table size grows as its square);

@@ -246,34 +246,28 @@ const PreMasks &host_masks() {
     return masks;
 }
 
-// c mod m for decimal text c (sign folded in), m < 2^32.
-u32 text_mod(const std::string &text, u32 m) {
-    std::size_t i = 0;
-    const bool negative = !text.empty() && text[0] == '-';
-    if (!text.empty() && (text[0] == '-' || text[0] == '+')) i = 1;
-    u64 r = 0;
-    for (; i < text.size(); ++i) {
-        if (text[i] < '0' || text[i] > '9') throw std::invalid_argument("coefficients must be decimal integers");
-        r = (r * 10 + u64(text[i] - '0')) % m;
-    }
-    return u32(negative && r ? m - r : r);
-}
-
-// c mod 2^64 (two's complement of the signed value).
-u64 text_wrap(const std::string &text) {
-    std::size_t i = 0;
-    const bool negative = !text.empty() && text[0] == '-';
-    if (!text.empty() && (text[0] == '-' || text[0] == '+')) i = 1;
-    u64 r = 0;
-    for (; i < text.size(); ++i) r = r * 10 + u64(text[i] - '0');
-    return negative ? u64(0) - r : r;
-}
-
 PreCoef coef_residues(const std::string &text) {
     PreCoef c{};
-    c.wrap = text_wrap(text);
-    for (int g = 0; g < kGroups; ++g) c.r[g] = text_mod(text, group_modulus(g));
-    for (int l = 0; l < kLarge; ++l) c.r[kGroups + l] = text_mod(text, large_prime(l));
+    const bool negative = !text.empty() && text[0] == '-';
+    std::size_t i = !text.empty() && (text[0] == '-' || text[0] == '+') ? 1 : 0;
+    // nine digits at a time: r 10^9 + chunk < 2^62 for residues below 2^32
+    while (i < text.size()) {
+        const std::size_t end = std::min(text.size(), i + 9);
+        u64 chunk = 0, scale = 1;
+        for (; i < end; ++i, scale *= 10) {
+            if (text[i] < '0' || text[i] > '9') throw std::invalid_argument("coefficients must be decimal integers");
+            chunk = chunk * 10 + u64(text[i] - '0');
+        }
+        c.wrap = c.wrap * scale + chunk;
+        for (int g = 0; g < kGroups; ++g) c.r[g] = u32((c.r[g] * scale + chunk) % group_modulus(g));
+        for (int l = 0; l < kLarge; ++l) c.r[kGroups + l] = u32((c.r[kGroups + l] * scale + chunk) % large_prime(l));
+    }
+    if (negative) {
+        c.wrap = u64(0) - c.wrap;
+        for (int g = 0; g < kGroups; ++g) c.r[g] = c.r[g] ? group_modulus(g) - c.r[g] : 0;
+        for (int l = 0; l < kLarge; ++l)
+            c.r[kGroups + l] = c.r[kGroups + l] ? large_prime(l) - c.r[kGroups + l] : 0;
+    }
     return c;
 }
 
@@ -288,34 +282,42 @@ void Preverifier::release() {
     curves_cap_ = coefs_cap_ = 0;
 }
 
-void Preverifier::prepare(const std::vector<const std::vector<std::string> *> &curves, cudaStream_t stream) {
+void Preverifier::prepare(const std::vector<const std::vector<std::string> *> &curves, cudaStream_t stream,
+                          const Parallel &parallel) {
     std::vector<pre::PreCurve> hc(curves.size());
-    std::vector<pre::PreCoef> hk;
+    std::size_t total = 0;
     for (std::size_t i = 0; i < curves.size(); ++i) {
-        hc[i].coef = (long long)hk.size();
+        hc[i].coef = (long long)total;
         hc[i].n = curves[i] ? int(curves[i]->size()) : 0;
-        if (curves[i])
-            for (const auto &t : *curves[i]) hk.push_back(pre::coef_residues(t));
+        total += std::size_t(hc[i].n);
     }
-    if (hk.empty()) hk.push_back(pre::PreCoef{});
+    std::vector<pre::PreCoef> hk(std::max<std::size_t>(total, 1));
+    auto reduce = [&](std::size_t i) {
+        for (int j = 0; j < hc[i].n; ++j)
+            hk[std::size_t(hc[i].coef + j)] = pre::coef_residues((*curves[i])[std::size_t(j)]);
+    };
+    if (parallel) {
+        parallel(curves.size(), reduce);
+    } else {
+        for (std::size_t i = 0; i < curves.size(); ++i) reduce(i);
+    }
     auto grow = [](void *&p, std::size_t &cap, std::size_t bytes) {
         if (cap >= bytes) return;
         cudaFree(p);
         p = nullptr;
         cap = 0;
-        check_cuda(cudaMalloc(&p, bytes), "cudaMalloc(pre-verification tables)");
+        p = device_malloc(bytes, "cudaMalloc(pre-verification tables)");
         cap = bytes;
     };
     grow(curves_, curves_cap_, std::max<std::size_t>(1, hc.size()) * sizeof(pre::PreCurve));
     grow(coefs_, coefs_cap_, hk.size() * sizeof(pre::PreCoef));
-    // pageable sources: the copies complete before these calls return
+    // pageable sources: they are read before these calls return
     if (!hc.empty())
         check_cuda(cudaMemcpyAsync(curves_, hc.data(), hc.size() * sizeof(pre::PreCurve), cudaMemcpyHostToDevice,
                                    stream),
                    "upload pre-verification tables");
     check_cuda(cudaMemcpyAsync(coefs_, hk.data(), hk.size() * sizeof(pre::PreCoef), cudaMemcpyHostToDevice, stream),
                "upload pre-verification tables");
-    check_cuda(cudaStreamSynchronize(stream), "upload pre-verification tables");
     upload_bytes_ = hc.size() * sizeof(pre::PreCurve) + hk.size() * sizeof(pre::PreCoef);
     if (!blocks_) {
         int device = 0, sms = 0;

@@ -17,6 +17,7 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -30,8 +31,13 @@ public:
     Preverifier &operator=(const Preverifier &) = delete;
 
     // Coefficient residues of each curve (curve i = survivors tagged i),
-    // uploaded on `stream`; device buffers grow and are kept across calls.
-    void prepare(const std::vector<const std::vector<std::string> *> &curves, cudaStream_t stream);
+    // uploaded on `stream` (other streams wait for it); device buffers grow and
+    // are kept across calls.
+    // `parallel` (optional) runs its second argument for every index below the
+    // first.
+    using Parallel = std::function<void(std::size_t, const std::function<void(std::size_t)> &)>;
+    void prepare(const std::vector<const std::vector<std::string> *> &curves, cudaStream_t stream,
+                 const Parallel &parallel = nullptr);
 
     // Filter survivors [0, min(*count, capacity)) of the device arrays a, d
     // (and curve, or nullptr for curve 0) into out_a, out_d (out_curve), whose

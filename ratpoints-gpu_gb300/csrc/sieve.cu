@@ -11,6 +11,7 @@
 // lists, candidate primes) are built once per search on the device, and each
 // denominator batch is one persistent launch.
 #include "sieve.hpp"
+#include "batch.hpp"
 #include "tune.hpp"
 
 #include <algorithm>
@@ -18,7 +19,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <deque>
-#include <future>
 #include <mutex>
 #include <tuple>
 #include <utility>
@@ -34,6 +34,20 @@ void check_cuda(cudaError_t status, const char *what) {
         throw CudaError(std::string(what) + ": " + cudaGetErrorString(status));
 }
 
+void *device_malloc(std::size_t bytes, const char *what) {
+    void *p = nullptr;
+    cudaError_t status = cudaMalloc(&p, bytes);
+    if (status == cudaErrorMemoryAllocation) {
+        // the memory that finished searches left for reuse may be what is missing
+        cudaGetLastError();
+        release_pooled_pipelines(-1);
+        release_pooled_engines(-1);
+        status = cudaMalloc(&p, bytes);
+    }
+    check_cuda(status, what);
+    return p;
+}
+
 // ---------------------------------------------------------------------------
 
 namespace {
@@ -45,18 +59,18 @@ double ms_since(Clock::time_point t0) {
 
 template <typename T>
 T *device_alloc(std::size_t count, const char *what) {
-    void *p = nullptr;
-    check_cuda(cudaMalloc(&p, std::max<std::size_t>(count, 1) * sizeof(T)), what);
-    return static_cast<T *>(p);
+    return static_cast<T *>(device_malloc(std::max<std::size_t>(count, 1) * sizeof(T), what));
 }
 
 constexpr long long kInitialSurvivors = 1 << 16;  // survivors per buffer before any growth
 
-// The streams, events, survivor buffers and pinned staging of a finished
-// search, kept for the next search on the same device so that it does not
-// create and allocate them again.  Nothing in them outlives a search as
-// content: every launch resets its counter words first, survivor arrays are
-// written before they are read, and every table is built anew per search.
+// The streams, events, survivor buffers, pinned staging and table memory of a
+// finished search, kept for the next search on the same device so that it does
+// not create and allocate them again (a search of a small box spent 0.16 of
+// 0.6 ms allocating and freeing its tables).  Nothing in them outlives a
+// search as content: every launch resets its counter words first, survivor
+// arrays are written before they are read, and every table is built anew per
+// search.
 struct PooledPipeline {
     struct Buf {
         long long *a = nullptr, *pa = nullptr;
@@ -67,8 +81,11 @@ struct PooledPipeline {
     };
     int device = -1;
     cudaStream_t streams[4] = {};
-    cudaEvent_t events[3] = {};
+    cudaEvent_t events[5] = {};
     Buf buf[2];
+    unsigned char *arena = nullptr;
+    std::size_t arena_bytes = 0;
+    Preverifier *preverifier = nullptr;
     unsigned long long *h_count = nullptr;
     long long *h_a = nullptr;
     int *h_d = nullptr;
@@ -76,6 +93,7 @@ struct PooledPipeline {
 };
 constexpr std::size_t kPooledPipelines = 4;                   // per process
 constexpr long long kPooledSurvivors = 4 * kInitialSurvivors;  // larger buffers are freed
+constexpr std::size_t kPooledTables = std::size_t(64) << 20;  // bytes; larger tables are freed
 
 // Never destroyed: static destructors may run after the CUDA runtime is gone.
 std::mutex &pipeline_pool_mutex() {
@@ -92,36 +110,15 @@ std::vector<PooledPipeline> &pipeline_pool() {
 // Most admissible numerator classes of any denominator under the fast plan:
 // 2-adic classes (by d mod 64) times residues mod the class prime q (by d mod q).
 int max_admissible_classes(const std::vector<std::string> &coefficients, int q) {
-    const int n = int(coefficients.size()) - 1;
-    std::vector<int> c64(coefficients.size());
-    for (std::size_t i = 0; i < coefficients.size(); ++i) c64[i] = decimal_mod(coefficients[i], 64);
-    bool square64[64] = {};
-    for (int v = 0; v < 64; ++v) square64[(v * v) & 63] = true;
+    std::uint64_t classes[64];
+    two_adic_classes(coefficients, classes);
     int most2 = 0;
-    for (int dd = 0; dd < 64; ++dd) {
-        int count = 0;
-        for (int r = 0; r < 64; ++r) {
-            if (dd % 2 == 0 && r % 2 == 0) continue;
-            int value = c64[n], power = 1;
-            for (int i = n - 1; i >= 0; --i) {
-                value = (value * r) & 63;
-                power = (power * dd) & 63;
-                value = (value + c64[i] * power) & 63;
-            }
-            if (n % 2 == 1) value = (value * dd) & 63;
-            count += square64[value];
-        }
-        most2 = std::max(most2, count);
-    }
+    for (auto mask : classes) most2 = std::max(most2, __builtin_popcountll(mask));
     if (q <= 1) return std::max(1, most2);
-    const auto aff = affine_mask(q, coefficients);
-    int most_q = 0;
-    for (int dq = 0; dq < q; ++dq) {
-        int count = 0;
-        for (int r = 0; r < q; ++r) count += dq == 0 ? (r != 0) : aff[(r * mod_inverse(dq, q)) % q];
-        most_q = std::max(most_q, count);
-    }
-    return std::max(1, most2 * std::max(1, most_q));
+    // d = 0 mod q: every r but 0; otherwise the residues r with f(r / d) a
+    // square mod q, as many for every d
+    const int most_q = std::max(q - 1, admitted_residues(q, coefficients));
+    return std::max(1, most2 * most_q);
 }
 
 constexpr int kFastRowSlots = 3;  // most row sets the fast planner divides the budget by
@@ -186,8 +183,15 @@ struct Sieve::Impl {
     // batch's end, both measured from an origin recorded at start().
     cudaEvent_t origin = nullptr;
     float last_end_ms = 0;
+    // Around the table build on `stream`.  Nothing waits for it on the host:
+    // stream2 waits on the device, and its time is read when the first
+    // launch's results are there.
+    cudaEvent_t tables_begin = nullptr, tables_end = nullptr;
+    bool tables_timed = false;
     std::unique_ptr<SweepCurve> curve;
     unsigned char *arena = nullptr;  // its tables
+    std::size_t arena_bytes = 0;
+    mutable bool lent = false;       // launched on a caller's stream: the arena is freed, not pooled
     FastPlan fast_plan;
     long long capacity = 0;       // most survivors a buffer may grow to hold
     long long host_capacity = 0;  // entries of the pinned host arrays
@@ -207,10 +211,12 @@ struct Sieve::Impl {
         bool busy = false;
     };
     Buffer buf[2];
-    Preverifier preverifier;
+    std::unique_ptr<Preverifier> preverifier;
     unsigned long long *h_count = nullptr;  // pinned, 4 words per buffer
     long long *h_a = nullptr;
     int *h_d = nullptr;
+
+    bool in_flight = false;  // launched since the streams were last waited for
 
     // Batch queue.
     long long q_next = 0, q_last = -1, q_batch = 1;
@@ -244,6 +250,11 @@ struct Sieve::Impl {
         fork_event = p.events[0];
         join_event = p.events[1];
         origin = p.events[2];
+        tables_begin = p.events[3];
+        tables_end = p.events[4];
+        arena = p.arena;
+        arena_bytes = p.arena_bytes;
+        preverifier.reset(p.preverifier);
         for (int i = 0; i < 2; ++i) {
             Buffer &b = buf[i];
             const PooledPipeline::Buf &q = p.buf[i];
@@ -268,7 +279,7 @@ struct Sieve::Impl {
     // and the pool has room; release() then frees only what was not handed on.
     void offer_pipeline() {
         if (device < 0 || !stream || !stream2 || !copy_stream || !count_stream || !fork_event ||
-            !join_event || !origin || !h_count)
+            !join_event || !origin || !tables_begin || !tables_end || !h_count)
             return;
         for (cudaStream_t s : {stream, stream2, copy_stream, count_stream})
             if (cudaStreamSynchronize(s) != cudaSuccess) return;
@@ -295,6 +306,11 @@ struct Sieve::Impl {
             h_d = nullptr;
             host_capacity = 0;
         }
+        if (lent || arena_bytes > kPooledTables) {
+            cudaFree(arena);
+            arena = nullptr;
+            arena_bytes = 0;
+        }
         PooledPipeline p;
         p.device = device;
         p.streams[0] = stream;
@@ -304,6 +320,11 @@ struct Sieve::Impl {
         p.events[0] = fork_event;
         p.events[1] = join_event;
         p.events[2] = origin;
+        p.events[3] = tables_begin;
+        p.events[4] = tables_end;
+        p.arena = arena;
+        p.arena_bytes = arena_bytes;
+        p.preverifier = preverifier.get();
         for (int i = 0; i < 2; ++i) {
             const Buffer &b = buf[i];
             PooledPipeline::Buf &q = p.buf[i];
@@ -327,7 +348,10 @@ struct Sieve::Impl {
             pipeline_pool().push_back(p);
         }
         stream = stream2 = copy_stream = count_stream = nullptr;
-        fork_event = join_event = origin = nullptr;
+        fork_event = join_event = origin = tables_begin = tables_end = nullptr;
+        arena = nullptr;
+        arena_bytes = 0;
+        (void)preverifier.release();
         for (auto &b : buf) b = Buffer{};
         h_count = nullptr;
         h_a = nullptr;
@@ -350,6 +374,8 @@ struct Sieve::Impl {
         }
         cudaFree(arena);
         arena = nullptr;
+        arena_bytes = 0;
+        preverifier.reset();
         if (h_count) cudaFreeHost(h_count);
         if (h_a) cudaFreeHost(h_a);
         if (h_d) cudaFreeHost(h_d);
@@ -362,25 +388,15 @@ struct Sieve::Impl {
         if (stream2) cudaStreamDestroy(stream2);
         if (fork_event) cudaEventDestroy(fork_event);
         if (join_event) cudaEventDestroy(join_event);
-        if (origin) cudaEventDestroy(origin);
-        origin = nullptr;
+        for (cudaEvent_t e : {origin, tables_begin, tables_end})
+            if (e) cudaEventDestroy(e);
+        origin = tables_begin = tables_end = nullptr;
         stream = stream2 = copy_stream = count_stream = nullptr;
         fork_event = join_event = nullptr;
     }
 
     void init(const std::vector<std::string> &coefficients) {
         auto t0 = Clock::now();
-        // The fast plan needs only the coefficients and the bound: choose it
-        // on a host thread while the streams and buffers are created.
-        PlannedRows planned;
-        if (opt.plan == PlanKind::fast)
-            planned = std::async(std::launch::async, [&coefficients, h = bound, forced = opt.fast_shape] {
-                int max_classes = 0;
-                FastShape shape = forced;
-                if (shape.rows <= 0) shape = tuned_fast_shape(coefficients, h);
-                FastPlan p = single_curve_plan(coefficients, h, &max_classes, shape);
-                return std::make_pair(std::move(p), max_classes);
-            });
         if (opt.device >= 0) check_cuda(cudaSetDevice(opt.device), "cudaSetDevice");
         check_cuda(cudaGetDevice(&device), "cudaGetDevice");
         if (!adopt_pipeline()) {
@@ -391,6 +407,8 @@ struct Sieve::Impl {
             check_cuda(cudaEventCreateWithFlags(&fork_event, cudaEventDisableTiming), "cudaEventCreate");
             check_cuda(cudaEventCreateWithFlags(&join_event, cudaEventDisableTiming), "cudaEventCreate");
             check_cuda(cudaEventCreate(&origin), "cudaEventCreate");
+            check_cuda(cudaEventCreate(&tables_begin), "cudaEventCreate");
+            check_cuda(cudaEventCreate(&tables_end), "cudaEventCreate");
         }
         // Survivor buffers start small (most searches have few survivors) and
         // grow on overflow up to the per-buffer capacity; past it a batch is
@@ -443,43 +461,53 @@ struct Sieve::Impl {
             host_capacity = initial;
         }
         timings.workspace_ms += ms_since(t0);
-        build_tables(coefficients, planned);
-        if (opt.preverify) {
-            preverifier.prepare({&coefficients}, stream);
-            timings.h2d_bytes += preverifier.upload_bytes();
-        }
+        build_tables(coefficients);
     }
 
-    using PlannedRows = std::future<std::pair<FastPlan, int>>;
-
-    // The curve's sweep plan and its tables on the device.
-    void build_tables(const std::vector<std::string> &coefficients, PlannedRows &planned) {
+    // The curve's sweep plan, and its tables on the device.
+    void build_tables(const std::vector<std::string> &coefficients) {
         auto t0 = Clock::now();
         const bool fast = opt.plan == PlanKind::fast;
-        // the plan was started on a host thread while the buffers were set up
-        if (fast) fast_plan = planned.get().first;
+        if (fast) {
+            FastShape shape = opt.fast_shape;
+            if (shape.rows <= 0) shape = tuned_fast_shape(coefficients, bound);
+            fast_plan = single_curve_plan(coefficients, bound, nullptr, shape);
+        }
         curve.reset(new SweepCurve(coefficients, bound, opt.square, fast ? &fast_plan : nullptr, opt.denominators));
         SweepBuilder builder;
         builder.add(*curve);
         timings.plan_ms += ms_since(t0);
         auto t1 = Clock::now();
-        arena = device_alloc<unsigned char>(builder.bytes(), "cudaMalloc(sieve tables)");
+        if (arena_bytes < builder.bytes()) {
+            cudaFree(arena);
+            arena = nullptr;
+            arena_bytes = 0;
+            arena = device_alloc<unsigned char>(builder.bytes(), "cudaMalloc(sieve tables)");
+            arena_bytes = builder.bytes();
+        }
         timings.workspace_ms += ms_since(t1);
-        cudaEvent_t e0, e1;
-        check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
-        check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
-        check_cuda(cudaEventRecord(e0, stream), "cudaEventRecord");
+        check_cuda(cudaEventRecord(tables_begin, stream), "cudaEventRecord");
         builder.place(arena, stream);
         timings.h2d_bytes += builder.upload_bytes();
         builder.enqueue(stream);
-        check_cuda(cudaEventRecord(e1, stream), "cudaEventRecord");
-        check_cuda(cudaEventSynchronize(e1), "class table build");
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        timings.table_ms += ms;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        if (opt.preverify) {
+            if (!preverifier) preverifier.reset(new Preverifier());
+            preverifier->prepare({&coefficients}, stream);
+            timings.h2d_bytes += preverifier->upload_bytes();
+        }
+        check_cuda(cudaEventRecord(tables_end, stream), "cudaEventRecord");
+        check_cuda(cudaStreamWaitEvent(stream2, tables_end, 0), "cudaStreamWaitEvent");
+        tables_timed = false;
         timings.table_wall_ms += ms_since(t0);
+    }
+
+    // Once a launch on the tables has completed: the device time of their build.
+    void time_tables() {
+        if (tables_timed) return;
+        tables_timed = true;
+        float ms = 0;
+        cudaEventElapsedTime(&ms, tables_begin, tables_end);
+        timings.table_ms += ms;
     }
 
     void launch_sweep(long long first, long long last, long long a_lo, long long a_hi, long long *out_a, int *out_d,
@@ -520,13 +548,14 @@ struct Sieve::Impl {
         b.first = first;
         b.last = last;
         b.busy = true;
+        in_flight = true;
         const cudaStream_t st = launch_stream(which);
         check_cuda(cudaMemsetAsync(b.count, 0, 4 * sizeof(unsigned long long), st), "cudaMemsetAsync");
         check_cuda(cudaEventRecord(b.begin, st), "cudaEventRecord");
         launch_sweep(first, last, a_lo, a_hi, b.a, b.d, (unsigned long long)b.cap, b.count, b.count + 1, b.count + 2,
                      st);
         if (opt.preverify) {
-            preverifier.launch(b.a, b.d, nullptr, b.count, (unsigned long long)b.cap, b.pa, b.pd, nullptr,
+            preverifier->launch(b.a, b.d, nullptr, b.count, (unsigned long long)b.cap, b.pa, b.pd, nullptr,
                                b.count + 3, nullptr, st);
             ++timings.launches;
         }
@@ -567,6 +596,7 @@ struct Sieve::Impl {
 
     // Device time a completed batch adds (see origin).
     float elapsed(const Buffer &b) {
+        time_tables();
         float t0 = 0, t1 = 0;
         cudaEventElapsedTime(&t0, origin, b.begin);
         cudaEventElapsedTime(&t1, origin, b.end);
@@ -602,6 +632,14 @@ struct Sieve::Impl {
         out.modular = n;
         out.kernel_ms = ms;
         out.complete = complete;
+    }
+
+    // Wait until no launch of this search is on its way.
+    void drain() {
+        check_cuda(cudaStreamSynchronize(stream), "sieve stream");
+        check_cuda(cudaStreamSynchronize(stream2), "sieve stream");
+        for (auto &b : buf) b.busy = false;
+        in_flight = false;
     }
 
     // Grow buffer `which` (idle) to hold n survivors if the capacity allows;
@@ -779,6 +817,8 @@ void release_pooled_pipelines(int device) {
             if (b.end) cudaEventDestroy(b.end);
             if (b.copied) cudaEventDestroy(b.copied);
         }
+        cudaFree(p.arena);
+        delete p.preverifier;
         if (p.h_count) cudaFreeHost(p.h_count);
         if (p.h_a) cudaFreeHost(p.h_a);
         if (p.h_d) cudaFreeHost(p.h_d);
@@ -804,16 +844,23 @@ void Sieve::start(long long first, long long last, long long batch_size) {
 bool Sieve::next(BatchView &out) { return impl_->next(out); }
 
 void Sieve::cancel() {
-    check_cuda(cudaStreamSynchronize(impl_->stream), "sieve stream");
-    check_cuda(cudaStreamSynchronize(impl_->stream2), "sieve stream");
-    for (auto &b : impl_->buf) b.busy = false;
+    if (impl_->in_flight) impl_->drain();
     impl_->order.clear();
     impl_->pieces.clear();
     impl_->q_next = 0;
     impl_->q_last = -1;
 }
 
-const SieveTimings &Sieve::timings() const { return impl_->timings; }
+const SieveTimings &Sieve::timings() const {
+    wait_tables();
+    return impl_->timings;
+}
+
+void Sieve::wait_tables() const {
+    if (impl_->tables_timed) return;
+    check_cuda(cudaEventSynchronize(impl_->tables_end), "class table build");
+    impl_->time_tables();
+}
 
 unsigned long long Sieve::swept_words(long long first, long long last) const {
     return impl_->curve->swept_words(first, last);
@@ -848,6 +895,7 @@ bool Sieve::launch_into(long long first, long long last, long long *out_a, int *
                         unsigned long long *work, unsigned long long *error, cudaStream_t stream) {
     const auto &I = *impl_;
     if (!fits_one_launch() || last < first || last - first + 1 > (1 << 16)) return false;
+    I.lent = true;
     I.launch_sweep(first, last, -I.bound, I.bound, out_a, out_d, capacity, out_count, work, error, stream);
     return true;
 }
@@ -885,6 +933,7 @@ unsigned long long Sieve::count_only(long long first, long long last, long long 
     check_cuda(cudaMemcpyAsync(&total, b.count, sizeof total, cudaMemcpyDeviceToHost, I.stream),
                "download survivor count");
     check_cuda(cudaStreamSynchronize(I.stream), "sieve kernel");
+    I.time_tables();
     I.check_error_word(0);
     return total;
 }

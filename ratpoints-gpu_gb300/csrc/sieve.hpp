@@ -81,8 +81,12 @@ struct SieveTimings {
     unsigned long long d2h_bytes = 0;
 };
 
+// cudaMalloc; before it fails for want of memory, what finished searches left
+// for reuse is freed.
+void *device_malloc(std::size_t bytes, const char *what);
+
 // Frees the idle search pipelines (streams, events, survivor buffers, pinned
-// staging) that finished sieves left for reuse on `device` (-1: every
+// staging, table memory) that finished sieves left for reuse on `device` (-1: every
 // device).  A process that resets a device must call it first.
 void release_pooled_pipelines(int device);
 
@@ -111,6 +115,9 @@ public:
 
     // Queue parameters [first, last] as consecutive batches of batch_size.
     void start(long long first, long long last, long long batch_size);
+    // Waits for the table build, which runs on the sieve's own stream beside
+    // the host; needed before launches on any other stream.
+    void wait_tables() const;
     // Next piece in parameter order; false when every queued batch is delivered.
     bool next(BatchView &out);
     // Drop queued and in-flight work (e.g. after a first-point stop).

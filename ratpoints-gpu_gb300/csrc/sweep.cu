@@ -258,6 +258,16 @@ const std::vector<OddPrime> &odd_primes() {
     return primes;
 }
 
+// 64^-1 modulo candidate i.
+int inverse64(int i) {
+    static const std::vector<int> inverses = [] {
+        std::vector<int> out;
+        for (int p : candidate_primes()) out.push_back(int(mod_inverse(64 % p, p)));
+        return out;
+    }();
+    return inverses[std::size_t(i)];
+}
+
 }  // namespace
 
 SweepCurve::~SweepCurve() = default;
@@ -268,20 +278,8 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
     dev::SweepTables &T = *tables_;
     dev::ListJob &L = *list_;
     const int n = int(coefficients.size()) - 1;
-    // the primes the plan tests before stage 2
-    std::vector<int> plan_primes;
-    if (fast) {
-        for (const auto &f : fast->slots)
-            for (int p : f) plan_primes.push_back(p);
-        if (fast->class_prime > 1) plan_primes.push_back(fast->class_prime);
-    }
     auto lead_of = [&](int p) {
         return n % 2 == 1 || square_mod(decimal_mod(coefficients.back(), p), p) ? 1 : 0;
-    };
-    auto admitted = [&](int p) {
-        int count = 0;
-        for (auto v : affine_mask(p, coefficients)) count += v;
-        return count;
     };
     std::vector<char> strict(kMaximumPrime, 0);
     SweepInput in;
@@ -309,16 +307,18 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
         const unsigned long long product = need_ * (unsigned long long)p;
         need_ = product > 0xFFFFFFFFull ? 0xFFFFFFFFull : product;
     };
-    for (int p : plan_primes) {
-        strict[std::size_t(p)] = 1;
-        const int count = admitted(p);
-        if (count == 0) {
-            needed(p);
-            late_primes.push_back(p);
-        } else {
-            in.primes.push_back({p, count, lead_of(p) ? p - 1 : 0, false});
+    if (fast)
+        for (const auto &known : fast->admitted) {
+            const int p = known.first;
+            const int count = known.second >= 0 ? known.second : admitted_residues(p, coefficients);
+            strict[std::size_t(p)] = 1;
+            if (count == 0) {
+                needed(p);
+                late_primes.push_back(p);
+            } else {
+                in.primes.push_back({p, count, lead_of(p) ? p - 1 : 0, false});
+            }
         }
-    }
     // The 32 largest candidates are always selected where they do not divide
     // d, so stage 1 may test them as well: all of the reference plan's, and
     // those of a fast plan whose own rows filter weakly (13 bits are usual) or
@@ -328,7 +328,7 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
     if (!fast || fast->bits < 12.5 || bound >= 4'000'000 || in.primes.size() < 4)
         for (int i = kCandidatePrimes - kSelectedPrimes; i < kCandidatePrimes; ++i)
             if (!strict[std::size_t(cands[i])]) {
-                const int count = admitted(cands[i]);
+                const int count = admitted_residues(cands[i], coefficients);
                 if (count == 0) needed(cands[i]);
                 in.primes.push_back({cands[i], std::max(1, count), cands[i], true});
             }
@@ -419,8 +419,8 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
         const dev::PatternJob &J = pattern_of(p, strict[std::size_t(p)] ? lead_of(p) : 2);
         P.pattern = (long long)(J.out / 8);
         P.words = J.words;
-        P.inv_stride = dev::u32(mod_inverse(S % p, p));
         P.inv_mod = dev::u32(mod_inverse(M % p, p));
+        P.inv_stride = dev::u32((long long)P.inv_mod * inverse64(i) % p);  // S = 64 M
         if (T.tabled && i >= kCandidatePrimes - dev::kFStage2Group) {
             dev::TableJob K{};
             K.m = K.length = p;

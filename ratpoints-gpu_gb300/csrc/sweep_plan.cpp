@@ -83,8 +83,8 @@ SweepPlan plan_sweep(const SweepInput &in) {
     });
     const int n = int(primes.size());
 
-    // ---- class primes: the few cheapest choices at eight rows of 12 bits ----
-    constexpr int kKeep = 3;
+    // ---- class primes: the two cheapest choices at eight rows of 12 bits ----
+    constexpr int kKeep = 2;
     ClassChoice best[kKeep];
     int kept = 0;
     auto offer = [&](ClassChoice c) {
@@ -140,7 +140,7 @@ SweepPlan plan_sweep(const SweepInput &in) {
     // ---- rows: primes in order of bits per bit of size, packed into products
     // below a cap (each into the row with the most headroom that takes it,
     // else a new row); every cap and row count is priced ----
-    static const int caps[] = {1500, 1050, 740, 512, 360, 250, 170, 110, 64};
+    static const int caps[] = {1500, 1050, 740, 512, 360, 250, 170, 110};
     struct Packing {
         int count = 0;
         int modulus[kSweepRows];
@@ -154,8 +154,11 @@ SweepPlan plan_sweep(const SweepInput &in) {
         const ClassChoice &c = best[k];
         bool used[512] = {};
         for (int i = 0; i < c.count; ++i) used[primes[std::size_t(c.index[i])].p] = true;
-        for (int cap : caps)
-            for (int rows = 1; rows <= kSweepRows; ++rows) {
+        int largest = caps[0] + 1;  // of the moduli packed at the previous cap
+        for (int cap : caps) {
+            if (largest <= cap) continue;  // the same packings
+            largest = 0;
+            for (int rows = std::min(3, n); rows <= kSweepRows; ++rows) {
                 Packing p;
                 for (const auto &w : primes) {
                     if (used[w.p] || w.p > cap || w.bits < 0.25) continue;
@@ -178,7 +181,9 @@ SweepPlan plan_sweep(const SweepInput &in) {
                     p.factor[target][p.factors[target]++] = w.p;
                     p.bits += w.bits;
                 }
-                if (p.count < rows) break;  // no more primes for another row
+                if (p.count < rows && rows > 3) break;  // no more primes for another row
+                if (p.count == 0) continue;
+                for (int i = 0; i < p.count; ++i) largest = std::max(largest, p.modulus[i]);
                 long long words = 0;
                 for (int i = 0; i < p.count; ++i) words += sweep_row_words(p.modulus[i]);
                 const long long slot = sweep_slot_bytes(words, c.two_max, c.q_max);
@@ -221,6 +226,7 @@ SweepPlan plan_sweep(const SweepInput &in) {
                 out.slots = slots;
                 choose_items(c, out);
             }
+        }
     }
     if (!found) {  // no prime filters: one row of a small prime all the same
         const ClassChoice &c = best[0];
