@@ -300,14 +300,18 @@ __device__ __forceinline__ void lds_u32x4(u32 a, u32 (&v)[4]) {
 // The row terms of N rows: 16-bit values two to a word.
 template <int N>
 __device__ __forceinline__ void load_starts16(u32 a, u32 (&v)[N]) {
+    u32 x[6];
+    if (N > 4) {
+        u32 y[4];
+        lds_u32x4(a, y);
 #pragma unroll
-    for (int r = 0; r < N; r += 8) {
-        u32 x[4];
-        lds_u32x4(a + 2 * r, x);
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (r + i < N) v[r + i < N ? r + i : 0] = i % 2 ? x[i / 2] >> 16 : x[i / 2] & 0xFFFFu;
+        for (int i = 0; i < 4; ++i) x[i] = y[i];
+    } else {
+        lds_u64(a, x[0], x[1]);
     }
+    if (N > 8) lds_u64(a + 16, x[4], x[5]);
+#pragma unroll
+    for (int r = 0; r < N; ++r) v[r] = r % 2 ? x[r / 2] >> 16 : x[r / 2] & 0xFFFFu;
 }
 
 // Warp-specialized persistent CTAs.  Warp 0 produces: it takes work units from
@@ -330,10 +334,15 @@ __device__ __forceinline__ void load_starts16(u32 a, u32 (&v)[N]) {
 //     m needs no wrap: 61 instead of 115 instructions per step of ten rows,
 //     1.95 instead of 2.49 ms per 65,536 denominators of a curve of degree 6
 //     at H = 5e6, 98 instead of 71 % of the pipe busy;
-//   - a broadcast 128-bit shared read takes two cycles: the terms of a residue
-//     are packed to 16 bits (two reads for eight rows, three for twelve) and
-//     shared by U = 2 pairs (1.81 -> 1.75 ms); read from kernel parameters
-//     instead, they cost more instructions than they saved cycles (2.07 ms);
+//   - a broadcast 128-bit shared read takes two cycles, a 64-bit one one: the
+//     terms of a residue are packed to 16 bits (two cycles for eight rows,
+//     three for twelve) and shared by U = 2 pairs (1.81 -> 1.75 ms); read from
+//     kernel parameters instead, they cost more instructions than they saved
+//     cycles (2.07 ms);
+//   - a unit without a partner is split over both half-warps by residues: at
+//     H = 20,000, where a class is one unit, 400,000 denominators of four
+//     curves take 0.42, 0.25, 0.48 and 0.81 ms instead of 0.53, 0.28, 0.66 and
+//     1.10;
 //   - the 24 warps of an SM form two, three or four CTAs: with four, a curve of
 //     240 words per denominator (H = 3e5) takes 0.22 instead of 0.29 ms per
 //     131,072 denominators, each CTA's producer being serial.
@@ -411,54 +420,56 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
 #pragma unroll 4
             for (int i = 0; i < T.nbad; ++i) hit |= u32(k) * T.bad[i].x <= T.bad[i].y;
             if (hit || du * T.need.x > T.need.y) nq = 0;
-            u32 live = __ballot_sync(kFullMask, n2 > 0 && nq > 0);
+            const int units = nq * A.segs;
+            const int all = ((units + 2 * U - 1) / (2 * U)) << A.split;
+            const int part = int(idx) & ((1 << A.part_shift) - 1);
+            const int first = int((long long)all * part >> A.part_shift);
+            const int items = int((long long)all * (part + 1) >> A.part_shift);  // first: fewer items than parts
+            const int turn = int(unsigned(items - first) % unsigned(consumers));
+            const bool mine = n2 > 0 && nq > 0 && first < items;
+            if (mine && part == 0) swept += (unsigned long long)units * unsigned(n2) * kSweepUnit;
+            u32 live = __ballot_sync(kFullMask, mine);
             while (live) {
                 const int j = __ffs(live) - 1;
                 live &= live - 1;
                 const u32 d = __shfl_sync(kFullMask, du, j);
+                const u32 full = smem_addr(&s_full[b]);
+                const u32 at8 = smem_addr(smem) + u32(b) * slot_bytes;
+                const u32 rho = mod_u32(d, R.m, R.magic);
+                const u64 *const row = T.rows + R.offset + (long long)rho * R.length;
+                const u32 bytes2 = __shfl_sync(kFullMask, u32(n2) * u32(sizeof(SweepClass)), j);
+                const u32 bytesq = __shfl_sync(kFullMask, u32(nq) * u32(sizeof(SweepClass)), j);
                 const u32 dq_j = __shfl_sync(kFullMask, dq, j);
-                const int n2_j = __shfl_sync(kFullMask, n2, j);
-                const int nq_j = __shfl_sync(kFullMask, nq, j);
+                const int turn_j = __shfl_sync(kFullMask, turn, j);
                 if (!acquire_slot()) {
                     failed = true;
                     break;
                 }
-                const u32 full = smem_addr(&s_full[b]);
-                const u32 at8 = smem_addr(smem) + u32(b) * slot_bytes;
-                const int units = nq_j * A.segs;
-                const int all = ((units + 2 * U - 1) / (2 * U)) << A.split;
-                const int part = int(chunk + j) & ((1 << A.part_shift) - 1);
-                const int first = int((long long)all * part >> A.part_shift);
-                const int items = int((long long)all * (part + 1) >> A.part_shift);
-                if (first == items) continue;  // fewer items than parts
-                if (lane == 0) {
+                if (lane == j) {
                     FastSlot &S = slot[b];
                     S.d = d;
                     S.units = units;
-                    S.n2 = n2_j;
+                    S.n2 = n2;
                     S.first = first;
                     S.items = items;
                     S.rot = rot;
-                    S.list = T.listq + (long long)dq_j * T.q_max;
-                    if (part == 0) swept += (unsigned long long)units * unsigned(n2_j) * kSweepUnit;
-                    mbar_arrive_expect_tx(full, u32(T.row_words) * 8u + u32(n2_j) * u32(sizeof(SweepClass)) +
-                                                    (listq_staged ? u32(nq_j) * u32(sizeof(SweepClass)) : 0u));
+                    S.list = T.listq + (long long)dq * T.q_max;
+                    mbar_arrive_expect_tx(full, u32(T.row_words) * 8u + bytes2 + (listq_staged ? bytesq : 0u));
                 }
-                rot = int(unsigned(rot + items - first) % unsigned(consumers));
+                rot += turn_j;
+                if (rot >= consumers) rot -= consumers;
                 // the consumers' reads of this slot's previous contents are
                 // ordered before the asynchronous copies that overwrite them
                 fence_proxy_async_shared();
                 __syncwarp();
                 if (lane < NS) {
-                    const u32 rho = mod_u32(d, R.m, R.magic);
-                    bulk_copy_to_shared(at8 + R.soff8, T.rows + R.offset + (long long)rho * R.length,
-                                        R.length * 8u, full);
+                    bulk_copy_to_shared(at8 + R.soff8, row, R.length * 8u, full);
                 } else if (lane == 30) {
                     bulk_copy_to_shared(at8 + list2_at, T.list2 + (long long)(d & u32(T.two_mask)) * T.two_max,
-                                        u32(n2_j) * u32(sizeof(SweepClass)), full);
+                                        bytes2, full);
                 } else if (lane == 31 && listq_staged) {
                     bulk_copy_to_shared(at8 + listq_at, T.listq + (long long)dq_j * T.q_max,
-                                        u32(nq_j) * u32(sizeof(SweepClass)), full);
+                                        bytesq, full);
                 }
                 if (++b == slots) {
                     b = 0;
@@ -467,9 +478,12 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
             }
             if (failed) break;
         }
-        if (A.swept && lane == 0) {
-            atomicAdd(A.swept, swept);
-            atomicAdd(A.swept + 1, swept * 8ull * NS);
+        if (A.swept) {
+            for (int o = 16; o > 0; o >>= 1) swept += __shfl_xor_sync(kFullMask, swept, o);
+            if (lane == 0) {
+                atomicAdd(A.swept, swept);
+                atomicAdd(A.swept + 1, swept * 8ull * NS);
+            }
         }
         if (!failed) {
             // no more work: an empty slot fill tells the consumers to finish
@@ -530,7 +544,12 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
                 const int group = item >> A.split;
                 const int range = (n2 + (1 << A.split) - 1) >> A.split;
                 const int e0 = (item & ((1 << A.split) - 1)) * range;
-                const int steps = min(range, n2 - e0);
+                int steps = min(range, n2 - e0);
+                // A last group that is at most half full (of short classes the
+                // only one): both half-warps take each of its units, with half
+                // of the residues each.
+                const bool alone = units - 2 * U * group <= U;
+                const int half = lane >> 4;
                 // this half-warp's units, 16 words of one residue mod Q each:
                 // the addresses of their first words in the staged rows
                 u32 o[U][NS];
@@ -538,7 +557,7 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
                 bool valid[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    int unit = 2 * (U * group + u) + (lane >> 4);
+                    int unit = 2 * U * group + (alone ? u : 2 * u + half);
                     valid[u] = unit < units;
                     if (!valid[u]) unit = 0;
                     int s = unit, seg = 0;
@@ -580,53 +599,72 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
                     pos0[u] = u64(xq) + u64(T.stride) * u64(kSweepUnit * seg + (lane & (kSweepUnit - 1)));
                 }
                 u32 a_addr = slot_addr + list2_at + u32(e0) * u32(sizeof(SweepClass));
+                int i = 0, end = steps;
+                int own = valid[0] ? steps : 0;  // U == 1: steps in which this lane's words count
+                if (alone && steps > 0) {
+                    // of an odd number the middle one is both halves' and
+                    // counts in the second, which has it first
+                    const int low = steps >> 1;
+                    steps -= low;
+                    end = U == 1 ? steps : low;
+                    own = half ? steps : low;
+                    if (half) a_addr += u32(low) * u32(sizeof(SweepClass));
+                }
+                // U == 2: the steps in which both halves count, then the middle
+                // residue's; with U == 1 a comparison with own is cheaper
+                for (;;) {
 #pragma unroll 1
-                for (int i = 0; i < steps; ++i, a_addr += u32(sizeof(SweepClass))) {
-                    u32 t[NS];
-                    load_starts16<NS>(a_addr, t);
-                    u32 al[U], ah[U];
-                    bool hit[U];
-                    u32 bb[U];
+                    for (; i < end; ++i, a_addr += u32(sizeof(SweepClass))) {
+                        u32 t[NS];
+                        load_starts16<NS>(a_addr, t);
+                        u32 al[U], ah[U];
+                        bool hit[U];
+                        u32 bb[U];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        u32 lo[NS], hi[NS];
+                        for (int u = 0; u < U; ++u) {
+                            u32 lo[NS], hi[NS];
 #pragma unroll
-                        for (int r = 0; r < NS; ++r) lds_u64(o[u][r] + t[r], lo[r], hi[r]);
-                        al[u] = lo[0];
-                        ah[u] = hi[0];
+                            for (int r = 0; r < NS; ++r) lds_u64(o[u][r] + t[r], lo[r], hi[r]);
+                            al[u] = lo[0];
+                            ah[u] = hi[0];
 #pragma unroll
-                        for (int r = 1; r + 1 < NS; r += 2) {
-                            al[u] = and3(al[u], lo[r], lo[r + 1]);
-                            ah[u] = and3(ah[u], hi[r], hi[r + 1]);
+                            for (int r = 1; r + 1 < NS; r += 2) {
+                                al[u] = and3(al[u], lo[r], lo[r + 1]);
+                                ah[u] = and3(ah[u], hi[r], hi[r + 1]);
+                            }
+                            if (NS % 2 == 0) {
+                                al[u] &= lo[NS - 1];
+                                ah[u] &= hi[NS - 1];
+                            }
+                            hit[u] = (al[u] | ah[u]) != 0 && (U == 1 ? i < own : valid[u]);
+                            bb[u] = __ballot_sync(kFullMask, hit[u]);
                         }
-                        if (NS % 2 == 0) {
-                            al[u] &= lo[NS - 1];
-                            ah[u] &= hi[NS - 1];
+                        u32 any = bb[0];
+                        if (U > 1) any |= bb[U - 1];
+                        if (!any) continue;
+                        u32 x2, pad;
+                        lds_u64(a_addr + 2 * kSweepRows, x2, pad);
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            if (!bb[u]) continue;
+                            const int to = qn + __popc(bb[u] & lanemask_lt());
+                            if (hit[u]) {
+                                wq_mask[to] = (u64(ah[u]) << 32) | al[u];
+                                wq_pos[to] = pos0[u] + x2;
+                                wq_d[to] = d;
+                            }
+                            qn += __popc(bb[u]);
+                            if (qn >= 32) {
+                                __syncwarp();
+                                fast_drain(wq_mask, wq_pos, wq_d, qn - 32, 32, T, A);
+                                qn -= 32;
+                            }
                         }
-                        hit[u] = (al[u] | ah[u]) != 0 && valid[u];
-                        bb[u] = __ballot_sync(kFullMask, hit[u]);
                     }
-                    u32 any = bb[0];
-                    if (U > 1) any |= bb[U - 1];
-                    if (!any) continue;
-                    u32 x2, pad;
-                    lds_u64(a_addr + 2 * kSweepRows, x2, pad);
+                    if (U == 1 || end >= steps) break;
+                    end = steps;
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        if (!bb[u]) continue;
-                        const int to = qn + __popc(bb[u] & lanemask_lt());
-                        if (hit[u]) {
-                            wq_mask[to] = (u64(ah[u]) << 32) | al[u];
-                            wq_pos[to] = pos0[u] + x2;
-                            wq_d[to] = d;
-                        }
-                        qn += __popc(bb[u]);
-                        if (qn >= 32) {
-                            __syncwarp();
-                            fast_drain(wq_mask, wq_pos, wq_d, qn - 32, 32, T, A);
-                            qn -= 32;
-                        }
-                    }
+                    for (int u = 0; u < U; ++u) valid[u] = valid[u] && half;
                 }
             }
         }

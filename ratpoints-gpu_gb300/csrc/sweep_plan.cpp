@@ -41,7 +41,7 @@ double cost_of(const ClassChoice &c, int rows, double bits, double staged_bytes,
     const double live = c.steps * 32.0 * c.fill * (1.0 - std::pow(1.0 - std::exp2(-bits), 64.0));
     const double a_reads = (rows <= 8 ? 2.0 : 3.0) / (c.pairs >= 6.0 ? 2.0 : 1.0);
     const double smem = (c.steps * (2.0 * rows + a_reads) + staged_bytes / 80.0 + live * 5.0) / 0.95;
-    const double issue = (c.steps * (kStepIssue + kRowIssue * rows) + live * kLiveIssue + c.pairs * kItemIssue +
+    const double issue = (c.steps * (kStepIssue + kRowIssue * rows) + live * kLiveIssue + std::max(1.0, c.pairs) * kItemIssue +
                           kVisitIssue * (kSweepWarps / ctas - 1) + kFillIssue) /
                          4.0 / 0.8;
     const double l2 = staged_bytes / 50.0;
@@ -51,18 +51,22 @@ double cost_of(const ClassChoice &c, int rows, double bits, double staged_bytes,
 
 // How items are cut: pairs of units side by side (1 or 2) and ranges of the
 // residues mod two.  More items keep more consumer warps busy on the slots in
-// flight, each costs a set-up (about 2.5 steps of one pair).
+// flight, each costs a set-up (about 2.5 steps of one pair).  Two pairs share
+// the residue's terms but a set-up and a part-filled last group weigh double:
+// with 23 residues and 3 pairs a denominator one pair takes 2.08 ms where two
+// took 2.28, with 40 and 16 two take 9.9 ms where one takes 10.5.
 void choose_items(const ClassChoice &c, SweepPlan &plan) {
     const int consumers = kSweepWarps / plan.ctas - 1;
     double best = 0;
     for (int pairs = 1; pairs <= 2; ++pairs)
         for (int split = 0; split <= 3 && (1 << split) <= c.two; ++split) {
-            const double groups = std::max(1.0, c.pairs / pairs);
-            const double items = groups * double(1 << split);
+            const double ranges = double(1 << split);
+            // a denominator's last group of two pairs is often not full
+            const double groups = std::max(1.0, pairs == 1 ? c.pairs : (c.pairs + 0.6) / 2.0);
+            const double items = groups * ranges;
             const double busy = std::min(double(consumers), std::max(1.0, double(plan.slots - 1)) * items);
-            const double per_item = pairs == 1 ? c.two_classes / double(1 << split) + 2.5
-                                               : 1.9 * c.two_classes / double(1 << split) + 3.5;
-            const double cost = items * per_item / busy;
+            const double steps = (pairs == 1 ? c.pairs : 1.95 * (c.pairs + 0.25) / 2.0) * c.two_classes;
+            const double cost = (steps + items * (pairs == 1 ? 2.5 : 3.5)) / busy;
             if (best > 0 && cost >= best) continue;
             best = cost;
             plan.pairs = pairs;
@@ -91,8 +95,9 @@ SweepPlan plan_sweep(const SweepInput &in) {
         const long long mod = (long long)c.two * c.q;
         const double words = double(sweep_words(in.bound, mod));
         const double segs = std::ceil(words / kSweepUnit);
-        // consecutive units pair up, also across residues
-        c.pairs = std::max(1.0, c.q_mean * segs / 2.0);
+        // consecutive units pair up, also across residues; one left over
+        // takes half the steps of a pair
+        c.pairs = std::max(0.5, c.q_mean * segs / 2.0);
         c.steps = c.pairs * c.two_classes;
         c.fill = words / (segs * kSweepUnit);
         c.rough = cost_of(c, 8, 12.0, 16384.0 + kSweepListBytes * c.q_mean, 2);
