@@ -46,6 +46,7 @@ constexpr int kAdmQ = 16;                               // residue words for cla
 constexpr int kNarrowSlots = 8;
 constexpr int kNK = 4;                                  // consecutive row words per lane (long ranges)
 constexpr int kNShortWords = 96;                        // ranges up to this many words: one word per lane
+constexpr int kNarrowMore = 12;                         // words of a drain with several sites, at most (see there)
 constexpr int kNarrowQueue = 64;                        // queued words per warp
 constexpr int kNWarps = 8;
 constexpr int kNThreads = kNWarps * kWarpSize;
@@ -828,10 +829,16 @@ __global__ void __launch_bounds__(kWThreads, 2)
 
 // Stage 2 and emission for up to 32 queued words of one curve, each with its
 // denominator: the 32 largest of the 36 candidates that do not divide it,
-// largest first, until every word has met 32 or is empty.
-__device__ __forceinline__ void narrow_drain(const u64 *qmask, const u32 *qword, const u32 *qd, int start, int n,
-                                             const NarrowCurve &C, const Candidates &cand, const u64 *s_aff,
-                                             const unsigned short *inv_table, const BatchOut &out) {
+// largest first.  Returns how many of the words it put back, from `start` on.
+// Most words have one site, and one site per lane is what a candidate tests in
+// one go: the words take their lowest, four candidates at a time with all their
+// loads in flight, and those with more go back to the queue.  With a loop over
+// each word's bits per candidate, which is left for words full of sites, a drain
+// took 840 instructions and 60 % of the time of a batch of high-degree curves
+// in intervals.
+__device__ __forceinline__ int narrow_drain(u64 *qmask, u32 *qword, u32 *qd, int start, int n,
+                                            const NarrowCurve &C, const Candidates &cand, const u64 *s_aff,
+                                            const unsigned short *inv_table, const BatchOut &out) {
     const int lane = threadIdx.x & 31;
     u64 m = 0;
     u32 w = 0, d = 1;
@@ -841,6 +848,42 @@ __device__ __forceinline__ void narrow_drain(const u64 *qmask, const u32 *qword,
         d = qd[start + lane];
     }
     __syncwarp();
+    const u32 more = __ballot_sync(kFullMask, (m & (m - 1)) != 0);
+    if (__popc(more) <= kNarrowMore) {
+        constexpr int kGroup = 4;
+        static_assert(kCandidatePrimes % kGroup == 0, "whole groups");
+        const u64 rest = m & (m - 1);
+        if (rest) {
+            const int at = start + __popc(more & lanemask_lt());
+            qmask[at] = rest;
+            qword[at] = w;
+            qd[at] = d;
+        }
+        const u32 site = 64u * w + (m ? u32(__ffsll((long long)m) - 1) : 0u);  // a + H
+        bool alive = m != 0;
+        int tested = 0;
+#pragma unroll 1
+        for (int ci = kCandidatePrimes - 1; ci >= 0; ci -= kGroup) {
+            if (!__any_sync(kFullMask, alive && tested < kSelectedPrimes)) break;
+            bool ok = true;
+#pragma unroll
+            for (int t = 0; t < kGroup; ++t) {
+                const u32 p = u32(cand.p[ci - t]), magic = cand.magic[ci - t];
+                const u32 rho = mod_small(d, p, magic);
+                const bool meets = alive && tested < kSelectedPrimes && rho != 0;
+                const u32 dinv = meets ? __ldg(inv_table + p * kMaximumPrime + rho) : 0;
+                u32 r = C.neg_h[ci - t] + mod_small(site, p, magic);  // a mod p
+                if (r >= p) r -= p;
+                const u32 x = mod_small(r * dinv, p, magic);
+                tested += meets ? 1 : 0;
+                ok &= !meets || ((s_aff[(ci - t) * kRefWords + (x >> 6)] >> (x & 63)) & 1) != 0;
+            }
+            alive = alive && ok;
+        }
+        emit(alive ? u64(1) : 0, -C.bound + (long long)site, 1, (long long)d, C.index, out);
+        __syncwarp();
+        return __popc(more);
+    }
     int tested = 0;
     for (int ci = kCandidatePrimes - 1; ci >= 0; --ci) {
         if (!__any_sync(kFullMask, m != 0 && tested < kSelectedPrimes)) break;
@@ -863,6 +906,7 @@ __device__ __forceinline__ void narrow_drain(const u64 *qmask, const u32 *qword,
         }
     }
     emit(m, -C.bound + 64LL * w, 1, (long long)d, C.index, out);
+    return 0;
 }
 
 // A CTA takes items (curve, parameters; all numerator ranges) and keeps the curve's
@@ -871,14 +915,16 @@ __device__ __forceinline__ void narrow_drain(const u64 *qmask, const u32 *qword,
 // then sweeps the live ones in turn; live words of all of them share its
 // queue, so that stage 2 runs with full warps.
 //
-// What bounds it is what a denominator costs besides its words: with the range
-// of x (fp64, 16 cycles an instruction on this chip), the denominator primes
-// and the selection of stage 2's primes worked out by a whole warp per
-// denominator, 96 curves of degree 12 to 40, 1e5 denominators in three
-// intervals each, took 41.5 ms, now 20.1 (470 instructions for a denominator
-// and interval of 90 words, 58 % of the issue slots); 400,000 denominators of
-// sextics 0.20 -> 0.08 ms at H = 1,000, 0.35 -> 0.27 at 5,000.  The curve's
-// constants stay in shared memory: held in registers they spill (+10 %).
+// What bounds it is instruction issue (72 % of the slots): with the range of x
+// (fp64, 16 cycles an instruction on this chip), the denominator primes and the
+// selection of stage 2's primes worked out by a whole warp per denominator, 96
+// curves of degree 12 to 40, 1e5 denominators in three intervals each, took 41.5
+// ms; classified by lanes 21.4 (60 % of it stage 2: a range of 347 words sends
+// 43 there), with stage 2 by sites 19.0; 384 quartics and cubics up to H =
+// 30,000 2.10 and 1.84.  The curve's constants stay in shared memory: held in
+// registers they spill (+10 %).  Rows long enough to sweep 64 words without a
+// wrap, one CTA of 24 warps per SM, have no bank conflicts (a quarter of the
+// reads here) but wait for each other at an item's end: 22.4 and 2.25 ms.
 __global__ void __launch_bounds__(kNThreads, 3)
     narrow_kernel(const NarrowCurve *__restrict__ curves, const BatchItem *__restrict__ items,
                   int nitems, const u64 *__restrict__ pool, const u64 *__restrict__ affine,
@@ -1019,58 +1065,21 @@ __global__ void __launch_bounds__(kNThreads, 3)
                         base[s] = v & 0xFFFFu;
                         at[s] = v >> 16;
                     }
-                    // queues the live words of a 32-lane step
-                    auto push = [&](u64 word, int w) {
-                        const u32 b = __ballot_sync(kFullMask, word != 0);
-                        if (!b) return;
-                        const int pos = qn + __popc(b & lanemask_lt());
-                        if (word) {
-                            wq_mask[pos] = word;
-                            wq_word[pos] = u32(w);
-                            wq_d[pos] = d;
-                        }
-                        qn += __popc(b);
-                        if (qn >= 32) {
-                            __syncwarp();
-                            narrow_drain(wq_mask, wq_word, wq_d, qn - 32, 32, C, cand, s_aff, inv_table, out);
-                            qn -= 32;
-                        }
-                    };
-                    if (w_hi - w_lo < kNShortWords) {
-                        // lane l takes word w0 + l of each 32-word step
+                    // Short ranges: lane l takes word w0 + l of each 32-word step.
+                    // Others: words w0 + kNK l .. w0 + kNK l + kNK - 1 of each
+                    // 128-word step: rows repeat their first kNK - 1 words, so the
+                    // kNK words of a lane never wrap and one index per modulus
+                    // advances.
+                    const bool wide = w_hi - w_lo >= kNShortWords;
 #pragma unroll
-                        for (int s = 0; s < kNarrowSlots; ++s) {
-                            const u32 t = at[s] + u32(s_lane1[s][lane]);
-                            at[s] = min(t, t - u32(C.m[s]));
-                        }
-                        for (int w0 = w_lo;;) {
-                            u64 acc = mask2;
-#pragma unroll
-                            for (int s = 0; s < kNarrowSlots; ++s) acc &= tab[base[s] + at[s]];
-                            const int w = w0 + lane;
-                            if (w > w_hi) acc = 0;
-                            if (w == w_lo) acc &= first_mask;
-                            if (w == w_hi) acc &= last_mask;
-                            push(acc, w);
-                            w0 += kWarpSize;
-                            if (w0 > w_hi) break;
-#pragma unroll
-                            for (int s = 0; s < kNarrowSlots; ++s) {
-                                const u32 t = at[s] + s_step32[s];
-                                at[s] = min(t, t - u32(C.m[s]));
-                            }
-                        }
-                    } else {
-                        // lane l takes words w0 + kNK l .. w0 + kNK l + kNK - 1 of each
-                        // 128-word step: rows repeat their first kNK - 1 words, so the
-                        // kNK words of a lane never wrap and one index per modulus advances
-#pragma unroll
-                        for (int s = 0; s < kNarrowSlots; ++s) {
-                            const u32 t = at[s] + u32(s_lane4[s][lane]);
-                            at[s] = min(t, t - u32(C.m[s]));
-                        }
-                        for (int w0 = w_lo; w0 <= w_hi; w0 += kWarpSize * kNK) {
-                            u64 acc[kNK];
+                    for (int s = 0; s < kNarrowSlots; ++s) {
+                        const u32 t = at[s] + u32(wide ? s_lane4[s][lane] : s_lane1[s][lane]);
+                        at[s] = min(t, t - u32(C.m[s]));
+                    }
+                    for (int w0 = w_lo;;) {
+                        u64 acc[kNK];
+                        int w = w0 + lane;
+                        if (wide) {
 #pragma unroll
                             for (int k4 = 0; k4 < kNK; ++k4) acc[k4] = mask2;
 #pragma unroll
@@ -1081,27 +1090,69 @@ __global__ void __launch_bounds__(kNThreads, 3)
                                 const u32 t = at[s] + C.step[s];
                                 at[s] = min(t, t - u32(C.m[s]));
                             }
-                            const int wl = w0 + kNK * lane;
+                            w = w0 + kNK * lane;
                             if (w0 == w_lo || w0 + kWarpSize * kNK - 1 > w_hi) {  // the range's first or last step
 #pragma unroll
                                 for (int k4 = 0; k4 < kNK; ++k4) {
-                                    if (wl + k4 > w_hi) acc[k4] = 0;
-                                    if (wl + k4 == w_lo) acc[k4] &= first_mask;
-                                    if (wl + k4 == w_hi) acc[k4] &= last_mask;
+                                    if (w + k4 > w_hi) acc[k4] = 0;
+                                    if (w + k4 == w_lo) acc[k4] &= first_mask;
+                                    if (w + k4 == w_hi) acc[k4] &= last_mask;
                                 }
                             }
-                            if (!__ballot_sync(kFullMask, (acc[0] | acc[1] | acc[2] | acc[3]) != 0)) continue;
+                        } else {
+                            acc[0] = mask2;
 #pragma unroll
-                            for (int k4 = 0; k4 < kNK; ++k4) push(acc[k4], wl + k4);
+                            for (int k4 = 1; k4 < kNK; ++k4) acc[k4] = 0;
+#pragma unroll
+                            for (int s = 0; s < kNarrowSlots; ++s) {
+                                acc[0] &= tab[base[s] + at[s]];
+                                const u32 t = at[s] + s_step32[s];
+                                at[s] = min(t, t - u32(C.m[s]));
+                            }
+                            if (w > w_hi) acc[0] = 0;
+                            if (w == w_lo) acc[0] &= first_mask;
+                            if (w == w_hi) acc[0] &= last_mask;
                         }
+                        // queue the live words, those of one k4 after another: one
+                        // copy of stage 2, or the kernel outgrows the instruction cache
+                        int left = wide ? kNK : 1;
+                        if (wide && !__any_sync(kFullMask, (acc[0] | acc[1] | acc[2] | acc[3]) != 0)) left = 0;
+#pragma unroll 1
+                        for (; left; --left) {
+                            const u64 word = acc[0];
+                            const u32 b = __ballot_sync(kFullMask, word != 0);
+                            if (word) {
+                                const int pos = qn + __popc(b & lanemask_lt());
+                                wq_mask[pos] = word;
+                                wq_word[pos] = u32(w);
+                                wq_d[pos] = d;
+                            }
+                            qn += __popc(b);
+                            while (qn >= 32) {
+                                __syncwarp();
+                                qn -= 32;
+                                qn += narrow_drain(wq_mask, wq_word, wq_d, qn, 32, C, cand, s_aff, inv_table, out);
+                            }
+                            acc[0] = acc[1];
+                            acc[1] = acc[2];
+                            acc[2] = acc[3];
+                            acc[3] = 0;
+                            ++w;
+                        }
+                        w0 += wide ? kWarpSize * kNK : kWarpSize;
+                        if (w0 > w_hi) break;
                     }
                 }
                 if (C.nint == 0) break;
             }
         }
         // the queue's words are this curve's: stage 2 before the next item
-        __syncwarp();
-        if (qn) narrow_drain(wq_mask, wq_word, wq_d, 0, qn, C, cand, s_aff, inv_table, out);
+        while (qn) {
+            __syncwarp();
+            const int n = min(qn, kWarpSize);
+            qn -= n;
+            qn += narrow_drain(wq_mask, wq_word, wq_d, qn, n, C, cand, s_aff, inv_table, out);
+        }
         swept_bytes += 8ull * u32(C.rows) * (swept_words - counted);
         counted = swept_words;
         __syncthreads();
