@@ -139,13 +139,16 @@ __global__ void __launch_bounds__(kTableThreads) class_table_kernel(unsigned cha
 
 // The class lists: block b < Q writes the entries of denominators d = b
 // (mod Q), block Q + b those of d = b (mod two).  A residue r mod Q is
-// admissible if every class prime admits it: byte (d mod p) p + r mod p of its
-// map; a residue mod two if bit r of adm2[d mod two] is set.
+// admissible if every class prime p admits it: byte r d^-1 mod p of its map of
+// the x with f(x) a square, or, where p | d, by `divided`; a residue mod two if
+// bit r of adm2[d mod two] is set.  (A map by d mod p and r mod p, p^2 bytes
+// made on the host, took 0.4 ms for a prime of 331.)
 struct ListJob {
-    std::size_t adm[kSweepClassPrimes], adm2;
+    std::size_t adm[kSweepClassPrimes], inverses[kSweepClassPrimes], adm2;
     std::size_t list2, listq, count2, countq;
     int two, q, two_max, q_max, nprimes, nrows;
     int p[kSweepClassPrimes];
+    int divided[kSweepClassPrimes];  // p | d: 0 admits none, 1 all but 0, 2 all
     u32 lift2, liftq;              // 1 mod two and 0 mod Q; 0 mod two and 1 mod Q (below M)
     u32 h2, hq;                    // H mod two, H mod Q
     u32 m[kSweepRows], inv_stride[kSweepRows], base[kSweepRows];  // base: (-H - M) mod m
@@ -172,7 +175,12 @@ __global__ void __launch_bounds__(kBuildThreads) class_list_kernel(unsigned char
     const u32 M = u32(S.two) * u32(S.q);
     SweepClass *out = reinterpret_cast<SweepClass *>(arena + (second ? S.list2 : S.listq)) + (long long)dres * room;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ u32 s_inverse[kSweepClassPrimes];  // d^-1 mod p, 0 where p | d
     if (threadIdx.x == 0) s_base = 0;
+    if (!second && int(threadIdx.x) < S.nprimes) {
+        const int i = int(threadIdx.x);
+        s_inverse[i] = reinterpret_cast<const unsigned short *>(arena + S.inverses[i])[dres % S.p[i]];
+    }
     __syncthreads();
     for (int r0 = 0; r0 < n; r0 += kBuildThreads) {
         const int r = r0 + int(threadIdx.x);
@@ -181,8 +189,9 @@ __global__ void __launch_bounds__(kBuildThreads) class_list_kernel(unsigned char
             ok = ok && ((reinterpret_cast<const u64 *>(arena + S.adm2)[dres] >> (r & 63)) & 1);
         } else {
             for (int i = 0; i < S.nprimes && ok; ++i) {
-                const int p = S.p[i];
-                ok = arena[S.adm[i] + std::size_t((dres % p) * p + r % p)] != 0;
+                const u32 p = u32(S.p[i]), rp = u32(r) % p, inverse = s_inverse[i];
+                ok = inverse ? arena[S.adm[i] + rp * inverse % p] != 0
+                             : S.divided[i] > (rp == 0 ? 1 : 0);
             }
         }
         const u32 vote = __ballot_sync(kFullMask, ok);
@@ -446,18 +455,12 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
         const auto aff = affine_mask(p, coefficients);
         std::vector<unsigned short> inv(static_cast<std::size_t>(p));
         modular_inverses(p, inv.data());
-        const bool is_strict = strict[std::size_t(p)] != 0;
-        const bool lead = lead_of(p) != 0;
-        std::vector<unsigned char> map;
-        std::vector<int> counts(std::size_t(p), 0);
-        for (int dq = 0; dq < p; ++dq)
-            for (int r = 0; r < p; ++r) {
-                const bool ok = dq == 0 ? (is_strict ? r != 0 && lead : true) : aff[std::size_t(r * inv[std::size_t(dq)] % p)] != 0;
-                map.push_back(ok);
-                counts[std::size_t(dq)] += ok;
-            }
         L.p[i] = p;
-        L.adm[i] = put(map.data(), map.size());
+        L.divided[i] = !strict[std::size_t(p)] ? 2 : lead_of(p) ? 1 : 0;
+        L.adm[i] = put(aff.data(), aff.size());
+        L.inverses[i] = put(inv.data(), inv.size() * sizeof(unsigned short));
+        std::vector<int> counts(std::size_t(p), int(std::count_if(aff.begin(), aff.end(), [](auto v) { return v != 0; })));
+        counts[0] = L.divided[i] == 2 ? p : L.divided[i] * (p - 1);
         countq_.push_back(std::move(counts));
     }
     const dev::u64 two_bits = plan_.two == 64 ? ~dev::u64(0) : (dev::u64(1) << plan_.two) - 1;
@@ -631,7 +634,10 @@ void SweepBuilder::place(unsigned char *arena, cudaStream_t stream) {
             tables.push_back(J);
         }
         dev::ListJob L = *c.list_;
-        for (int k = 0; k < L.nprimes; ++k) L.adm[k] += input;
+        for (int k = 0; k < L.nprimes; ++k) {
+            L.adm[k] += input;
+            L.inverses[k] += input;
+        }
         L.adm2 += input;
         L.list2 += block;
         L.listq += block;
