@@ -278,7 +278,8 @@ rpg_status rpg_session_sieve_noalloc(rpg_session *session, int32_t first, int32_
  * (as a single search stops).  curve_status[i] (optional) receives
  * RPG_OK, RPG_E_ARG or RPG_E_NOT_SQUAREFREE for curve i; a failing curve
  * gets no points and does not fail the call.  curve_survivors[i] (optional)
- * receives the modular survivors of curve i.  The call fails only for a NULL
+ * receives the modular survivors of curve i (of the plan the batch chose for
+ * it).  The call fails only for a NULL
  * argument, a negative count, or a device error.
  */
 #define RPG_BATCH_NO_GRAPH 1u /* launch the batch's kernels directly, not as a CUDA graph */
@@ -415,9 +416,9 @@ rpg_status rpg_smem_read_probe(int32_t device, int32_t iterations, double *gbs,
                                double *bytes_per_clock_per_sm, double *ms);
 
 /* A finished rpg_sieve_run or rpg_point_search leaves its streams, events,
- * survivor buffers (up to 262,144 survivors), pinned staging and table memory
+ * survivor buffers (up to 1,048,576 survivors), pinned staging and table memory
  * for the next search on the same device (at most four such sets per process,
- * up to 80 MB each; mostly 20), and a finished rpg_batch_search or server the
+ * up to 120 MB each; mostly 50), and a finished rpg_batch_search or server the
  * resources of its engines (at most four, up to 512 MB of device memory each).
  * An allocation that finds no memory frees them all and is tried again.  This
  * call frees them for `device` (-1: every device); a caller that resets a

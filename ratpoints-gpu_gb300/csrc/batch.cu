@@ -2552,7 +2552,9 @@ BatchEngine::BatchEngine(int device) {
     check_cuda(cudaGetDevice(&current), "cudaGetDevice");
     impl_ = BatchEnginePool::get().take(current);
     if (!impl_) impl_.reset(new Impl());
+    // a pooled engine keeps the room that an earlier run grew to
     impl_->capacity = Impl::first_capacity();
+    if (!std::getenv("RPG_BATCH_CAPACITY")) impl_->capacity = std::max<unsigned long long>(impl_->capacity, impl_->d_a.cap);
 }
 
 BatchEngine::~BatchEngine() {

@@ -1,23 +1,28 @@
 // Batched many-curve search: every curve's tables resident on the device at
-// once and two persistent kernels over device work queues of
-// (curve, denominator range) items, captured in one CUDA graph.
+// once, persistent kernels over device work queues of (curve, denominator
+// range) items and one sieve launch per curve with much work, all captured in
+// one CUDA graph.
 //
 // No counterpart in the reference, which searches one curve per process
 // (src/main.cpp:48-85); each curve's result here is the result of a
 // single-curve PointSearch of that curve (src/point_search.cpp:171-240): same
 // points, same order, the point at infinity first.
 //
-// Two shapes, chosen per curve by its row length W = ceil((2H + 1) / 64):
-//   - wide rows (W >= kBatchWideWords): the class-strided layout of the
-//     single-curve fast kernel (numerator classes mod 64 q, one CTA per
-//     denominator, stage-1 rows of up to six composite moduli staged into
-//     shared memory by TMA bulk copies), with per-curve descriptors;
-//   - narrow rows: one warp per denominator over dense 64-site words, the
-//     curve's whole stage-1 tables (moduli <= kBatchNarrowModulus, m x m
-//     words each) loaded into shared memory once per work item.
-// Both kernels finish with the reference's 32 selected primes tested bit by
-// bit against per-curve bitmasks of f(x) mod p, then the host verifies each
-// survivor exactly.
+// Three ways, chosen per curve by its row length W = ceil((2H + 1) / 64), its
+// denominators and its x intervals:
+//   - launches of the single-curve kernel (sweep.hpp) for curves without
+//     intervals that have wide rows (W >= kBatchWideWords) or shorter ones
+//     with many denominators, side by side on eight streams;
+//   - the wide kernel for wide rows of curves with intervals: the class-strided
+//     layout (numerator classes mod 64 q, one CTA per denominator, stage-1 rows
+//     of up to six composite moduli staged into shared memory by TMA bulk
+//     copies), with per-curve descriptors;
+//   - the narrow kernel for the rest: one warp per denominator over dense
+//     64-site words, the curve's whole stage-1 tables (moduli <=
+//     kBatchNarrowModulus, m x m words each) loaded into shared memory once per
+//     work item.
+// All finish with the reference's 32 selected primes, then the host verifies
+// each survivor exactly.
 #pragma once
 
 #include <memory>
@@ -51,8 +56,10 @@ struct BatchCurveResult {
     int status = 0;                    // rpg_status code (0 = ok)
     std::string error;
     std::vector<PointPair> points;     // the order of a single-curve search
-    unsigned long long survivors = 0;  // modular survivors of the batched sieve
-    bool wide = false;                 // which kernel swept the curve
+    // modular survivors: the sites that the plan chosen for the curve lets
+    // through (a single search's plan for curves with launches of their own)
+    unsigned long long survivors = 0;
+    bool wide = false;                 // rows of at least kBatchWideWords words
     bool solo = false;                 // huge rows: searched alone by the single-curve kernel
     int class_prime = 1;
     std::vector<int> moduli;           // stage-1 moduli the autotuner chose

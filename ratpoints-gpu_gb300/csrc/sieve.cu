@@ -62,7 +62,12 @@ T *device_alloc(std::size_t count, const char *what) {
     return static_cast<T *>(device_malloc(std::max<std::size_t>(count, 1) * sizeof(T), what));
 }
 
-constexpr long long kInitialSurvivors = 1 << 16;  // survivors per buffer before any growth
+// Survivors per buffer before any growth.  A batch that overflows its buffer is
+// run again, and dense curves leave 10^5 to 10^6 a batch (mostly multiples of
+// points, which no estimate foresees): with 65,536, every search of one at H =
+// 1e7, d <= 1e5 ran its first batch twice (49 instead of 29 ms).
+constexpr long long kInitialSurvivors = 1 << 20;
+constexpr long long kInitialHostSurvivors = 1 << 16;  // entries of the pinned host arrays
 
 // The streams, events, survivor buffers, pinned staging and table memory of a
 // finished search, kept for the next search on the same device so that it does
@@ -92,7 +97,7 @@ struct PooledPipeline {
     long long host_capacity = 0;
 };
 constexpr std::size_t kPooledPipelines = 4;                   // per process
-constexpr long long kPooledSurvivors = 4 * kInitialSurvivors;  // larger buffers are freed
+constexpr long long kPooledSurvivors = kInitialSurvivors;  // larger buffers are freed
 constexpr std::size_t kPooledTables = std::size_t(64) << 20;  // bytes; larger tables are freed
 
 // Never destroyed: static destructors may run after the CUDA runtime is gone.
@@ -136,13 +141,10 @@ long long fast_row_budget(int max_classes, int slots) {
 
 FastPlan single_curve_plan(const std::vector<std::string> &coefficients, long long bound, int *max_classes,
                            FastShape shape) {
-    // the staged row sets of a CTA, its queues and its slots' class runs must
-    // fit shared memory at 2 CTAs/SM.  Three slots stage a denominator ahead
-    // further with less shared memory per row set: they pay when sweeping a
-    // denominator is short against copying its rows (rows of at most 2^20
-    // words) and their plan filters within a quarter bit of the two-slot plan
-    // (the C2 curve: 13.22 bits either way, 30.4 ms against 31.4 ms per step;
-    // cubics with 31 M-word rows: 2 slots).
+    // The choice fixes the set of primes that survivors pass, not the rows that
+    // the kernel stages (those are the sweep plan's): rows for two or three
+    // row sets within the budget, three for rows of at most 2^20 words when
+    // their primes filter within a quarter bit of the two-set plan's.
     const FastPlanner planner(coefficients, bound);
     const int classes = max_admissible_classes(coefficients, planner.class_prime());
     if (max_classes) *max_classes = classes;
@@ -450,15 +452,16 @@ struct Sieve::Impl {
             b.busy = false;
         }
         if (!h_count) check_cuda(cudaMallocHost(&h_count, 8 * sizeof(unsigned long long)), "cudaMallocHost");
-        if (!h_a || !h_d || host_capacity < initial) {
+        if (!h_a || !h_d) {
+            const long long room = std::min(initial, kInitialHostSurvivors);
             if (h_a) cudaFreeHost(h_a);
             if (h_d) cudaFreeHost(h_d);
             h_a = nullptr;
             h_d = nullptr;
             host_capacity = 0;
-            check_cuda(cudaMallocHost(&h_a, std::size_t(initial) * sizeof(long long)), "cudaMallocHost");
-            check_cuda(cudaMallocHost(&h_d, std::size_t(initial) * sizeof(int)), "cudaMallocHost");
-            host_capacity = initial;
+            check_cuda(cudaMallocHost(&h_a, std::size_t(room) * sizeof(long long)), "cudaMallocHost");
+            check_cuda(cudaMallocHost(&h_d, std::size_t(room) * sizeof(int)), "cudaMallocHost");
+            host_capacity = room;
         }
         timings.workspace_ms += ms_since(t0);
         build_tables(coefficients);
@@ -623,6 +626,7 @@ struct Sieve::Impl {
     void deliver(BatchView &out, int which, std::size_t n, std::size_t kept, float ms, long long first,
                  long long last, bool complete) {
         if (!opt.preverify) kept = n;
+        host_room(kept);
         copy_out(which, kept);
         out.first = first;
         out.last = last;
@@ -665,18 +669,25 @@ struct Sieve::Impl {
             b.pd = device_alloc<int>(std::size_t(cap), "cudaMalloc(survivors)");
         }
         b.cap = cap;
-        if (host_capacity < cap) {
-            cudaFreeHost(h_a);
-            cudaFreeHost(h_d);
-            h_a = nullptr;
-            h_d = nullptr;
-            host_capacity = 0;
-            check_cuda(cudaMallocHost(&h_a, std::size_t(cap) * sizeof(long long)), "cudaMallocHost");
-            check_cuda(cudaMallocHost(&h_d, std::size_t(cap) * sizeof(int)), "cudaMallocHost");
-            host_capacity = cap;
-        }
         timings.workspace_ms += ms_since(t0);
         return true;
+    }
+
+    // Room in the pinned host arrays for n survivors (those that pass
+    // pre-verification are far fewer than a buffer holds).
+    void host_room(std::size_t n) {
+        if (host_capacity >= (long long)n) return;
+        const auto t0 = Clock::now();
+        const long long room = (long long)(n + n / 4 + 1024);
+        cudaFreeHost(h_a);
+        cudaFreeHost(h_d);
+        h_a = nullptr;
+        h_d = nullptr;
+        host_capacity = 0;
+        check_cuda(cudaMallocHost(&h_a, std::size_t(room) * sizeof(long long)), "cudaMallocHost");
+        check_cuda(cudaMallocHost(&h_d, std::size_t(room) * sizeof(int)), "cudaMallocHost");
+        host_capacity = room;
+        timings.workspace_ms += ms_since(t0);
     }
 
     // Queue a batch as pieces of at most a tile of numerators.
