@@ -1444,9 +1444,11 @@ long long swept_row_words(const BatchCurveSpec &c, long long first, long long la
 // do; shorter ones when the narrow kernel's time for them, about 0.1 ns per
 // denominator and 2.8e-3 ns per row word, exceeds the sweep's (1 ns per
 // denominator up to H = 65,504) by more than building the curve's tables takes
-// (400,000 denominators of sextics, narrow and sweep: H = 5,000 0.28 and 0.40
-// ms, 10,000 0.40 and 0.38; with the narrow kernel before it shared stage 2
-// among denominators, 20,000 0.66 and 0.38, 65,000 1.7 and 0.40).
+// (400,000 denominators of sextics, narrow and sweep: H = 5,000 0.28 and 0.34
+// ms, 10,000 0.38 and 0.32, and before the narrow kernel shared stage 2 among
+// denominators 20,000 0.66 and 0.38, 65,000 1.7 and 0.40).  The line is flat:
+// with 0.7 for 0.9 or 8,000 for 20,000, bursts of requests and batches change
+// by 4 % at most, either way.
 // Curves with x intervals stay in the kernels that sweep only those.
 bool swept_alone(const BatchCurveSpec &c, const CurveWork &cw) {
     if (!c.intervals.empty() && c.intervals.size() <= std::size_t(dev::kMaxIntervals)) return false;
