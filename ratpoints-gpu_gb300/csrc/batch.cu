@@ -46,7 +46,11 @@ constexpr int kAdmQ = 16;                               // residue words for cla
 constexpr int kNarrowSlots = 8;
 constexpr int kNK = 4;                                  // consecutive row words per lane (long ranges)
 constexpr int kNShortWords = 96;                        // ranges up to this many words: one word per lane
-constexpr int kNarrowMore = 12;                         // words of a drain with several sites, at most (see there)
+// Words with several sites that a drain of stage 2 puts back; with more it loops
+// over their sites.  6, 12, 18, 31: high-degree batch 19.9, 19.0, 18.9, 18.8 ms,
+// 384 small curves 1.95, 1.85, 1.82, 1.81, a curve with sites everywhere 5.55,
+// 5.56, 5.59, 6.05.
+constexpr int kNarrowMore = 18;
 constexpr int kNarrowQueue = 64;                        // queued words per warp
 constexpr int kNWarps = 8;
 constexpr int kNThreads = kNWarps * kWarpSize;
@@ -920,8 +924,8 @@ __device__ __forceinline__ int narrow_drain(u64 *qmask, u32 *qword, u32 *qd, int
 // selection of stage 2's primes worked out by a whole warp per denominator, 96
 // curves of degree 12 to 40, 1e5 denominators in three intervals each, took 41.5
 // ms; classified by lanes 21.4 (60 % of it stage 2: a range of 347 words sends
-// 43 there), with stage 2 by sites 19.0; 384 quartics and cubics up to H =
-// 30,000 2.10 and 1.84.  The curve's constants stay in shared memory: held in
+// 43 there), with stage 2 by sites 18.9; 384 quartics and cubics up to H =
+// 30,000 2.10 and 1.82.  The curve's constants stay in shared memory: held in
 // registers they spill (+10 %).  Rows long enough to sweep 64 words without a
 // wrap, one CTA of 24 warps per SM, have no bank conflicts (a quarter of the
 // reads here) but wait for each other at an item's end: 22.4 and 2.25 ms.
