@@ -207,8 +207,10 @@ FastPlanner::FastPlanner(const std::vector<std::string> &coefficients, long long
             bool prime = q > 2;
             for (int f = 3; f * f <= q; f += 2) prime = prime && q % f;
             if (!prime) continue;
-            const double rate = pass_rate(q, coefficients);
+            const int count = admitted_residues(q, coefficients);
+            const double rate = double(count) / q;
             strength_.push_back({rate > 0 ? -std::log2(rate) : 8.0, q});
+            admitted_[std::size_t(q)] = count;
         }
     };
     add_primes(3, prime_limit_);
@@ -368,15 +370,9 @@ FastPlan FastPlanner::plan(int max_modulus, int max_slots, long long row_budget,
         plan.moduli.push_back(pair[0] * pair[1]);
         plan.slots.push_back(pair);
     }
-    // counts back from the strengths (8 bits stand for none)
-    auto count_of = [&](int q) {
-        for (const auto &s : strength_)
-            if (s.second == q) return s.first >= 8.0 ? 0 : int(std::lround(std::exp2(-s.first) * q));
-        return -1;  // not a prime of the planner: left to the caller
-    };
     for (const auto &f : plan.slots)
-        for (int q : f) plan.admitted.push_back({q, count_of(q)});
-    if (plan.class_prime > 1) plan.admitted.push_back({plan.class_prime, count_of(plan.class_prime)});
+        for (int q : f) plan.admitted.push_back({q, admitted_[std::size_t(q)]});
+    if (plan.class_prime > 1) plan.admitted.push_back({plan.class_prime, admitted_[std::size_t(plan.class_prime)]});
     return plan;
 }
 

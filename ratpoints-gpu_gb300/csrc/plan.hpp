@@ -111,7 +111,9 @@ public:
     int class_prime() const { return class_prime_; }
 
 private:
-    std::vector<std::pair<double, int>> strength_;  // (bits, prime) of the odd primes below the limit
+    std::vector<std::pair<double, int>> strength_;  // (bits, prime) of the odd primes below the limit; 8 bits rank
+                                                    // a prime without admitted residues (one residue of 257 has more)
+    std::array<int, kMaximumPrime> admitted_{};     // by prime: admitted residues, exact
     int class_prime_ = 1;
     int prime_limit_ = kStagePrimeLimit;
 };

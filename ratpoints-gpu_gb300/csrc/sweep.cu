@@ -318,8 +318,7 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
     };
     if (fast)
         for (const auto &known : fast->admitted) {
-            const int p = known.first;
-            const int count = known.second >= 0 ? known.second : admitted_residues(p, coefficients);
+            const int p = known.first, count = known.second;
             strict[std::size_t(p)] = 1;
             if (count == 0) {
                 needed(p);

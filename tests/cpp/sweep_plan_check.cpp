@@ -1,0 +1,41 @@
+// Host checks of the single-curve kernel's plans (csrc/plan.hpp, csrc/sweep.hpp),
+// run by tests/test_sweep_plan_host.py.  Each argument is one check:
+//   admitted H c0 c1 ..   the residue counts that a fast plan carries are those
+//                         of its primes; prints the plan's primes and the
+//                         swept words of denominators 1 .. 256
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "plan.hpp"
+#include "sieve.hpp"
+#include "sweep.hpp"
+
+using namespace rpg;
+using Coefficients = std::vector<std::string>;
+
+static int admitted(long long bound, const Coefficients &f) {
+    const FastPlan plan = single_curve_plan(f, bound, nullptr);
+    int wrong = 0;
+    for (const auto &a : plan.admitted) {
+        std::printf("%d ", a.first);
+        if (a.second != admitted_residues(a.first, f)) {
+            std::fprintf(stderr, "prime %d: %d residues in the plan, %d admitted\n", a.first, a.second,
+                         admitted_residues(a.first, f));
+            ++wrong;
+        }
+    }
+    const SweepCurve curve(f, bound, false, &plan, 0);
+    std::printf("swept %llu\n", curve.swept_words(1, 256));
+    return wrong;
+}
+
+int main(int argc, char **argv) {
+    if (argc < 5) return 2;
+    const long long bound = std::atoll(argv[2]);
+    const Coefficients f(argv + 3, argv + argc);
+    if (!std::strcmp(argv[1], "admitted")) return admitted(bound, f) ? 1 : 0;
+    return 2;
+}
