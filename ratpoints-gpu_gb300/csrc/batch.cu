@@ -2043,6 +2043,7 @@ struct BatchEngine::Impl {
     DeviceArray<int> d_d, d_c, d_pd, d_pc;
     DeviceArray<unsigned long long> d_curve_modular;  // per-curve modular survivors
     Preverifier pre;
+    std::unique_ptr<SweepBuilder> sweep_tables;  // of the run: its upload's source
 
     Impl() {  // on the current device
         check_cuda(cudaGetDevice(&device), "cudaGetDevice");
@@ -2079,19 +2080,21 @@ struct BatchEngine::Impl {
         return 1ull << 20;
     }
 
-    // True if nothing of it is in flight and every stream finished without error.
-    bool idle() {
-        if (failed) return false;
-        for (cudaStream_t s : {stream, side})
-            if (cudaStreamSynchronize(s) != cudaSuccess) return false;
-        for (cudaStream_t s : sweep_stream)
-            if (cudaStreamSynchronize(s) != cudaSuccess) return false;
-        return true;
+    // Waits for every stream; true if all finished without error.
+    bool wait() {
+        bool ok = true;
+        for (cudaStream_t s : {stream, side}) ok = cudaStreamSynchronize(s) == cudaSuccess && ok;
+        for (cudaStream_t s : sweep_stream) ok = cudaStreamSynchronize(s) == cudaSuccess && ok;
+        return ok;
     }
+
+    // True if nothing of it is in flight and every stream finished without error.
+    bool idle() { return !failed && wait(); }
 
     // Frees the largest arrays until at most `limit` bytes are held on the
     // device, and the host's plan if it holds more than an eighth of that.
     void trim(std::size_t limit) {
+        sweep_tables.reset();
         plan.clear();
         if (plan.bytes() > limit / 8) plan = BatchPlan{};
         std::vector<std::pair<std::size_t, std::function<void()>>> arrays;
@@ -2156,6 +2159,8 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
     stats.items_per_kernel = items_per_kernel;
     std::vector<BatchCurveResult> results(curves.size());
     check_cuda(cudaSetDevice(device), "cudaSetDevice");
+    // what a run that failed left on its way reads the plan's arrays
+    if (failed) wait();
     failed = true;  // until the end
     // Curves with huge rows fill the device on their own: batching gains them
     // nothing, and the single-curve kernel (row count compiled in, stage 2
@@ -2231,12 +2236,12 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
         d_aff.ensure(std::size_t(P.aff_words), "cudaMalloc(batch bitmasks)");
         d_patterns.ensure(std::size_t(P.pattern_words), "cudaMalloc(batch patterns)");
         d_rows.ensure(std::size_t(P.row_words), "cudaMalloc(batch tables)");
-        SweepBuilder sweep_tables;
-        for (std::size_t i : P.sweeps) sweep_tables.add(*work[i].sweep);
+        sweep_tables.reset(new SweepBuilder);
+        for (std::size_t i : P.sweeps) sweep_tables->add(*work[i].sweep);
         if (!P.sweeps.empty()) {
-            d_sweep_tables.ensure(sweep_tables.bytes(), "cudaMalloc(sieve tables)");
-            sweep_tables.place(d_sweep_tables.p, stream);
-            stats.h2d_bytes += sweep_tables.upload_bytes();
+            d_sweep_tables.ensure(sweep_tables->bytes(), "cudaMalloc(sieve tables)");
+            sweep_tables->place(d_sweep_tables.p, stream);
+            stats.h2d_bytes += sweep_tables->upload_bytes();
         }
         ensure_output(capacity);
         d_counters.ensure(kCounters + P.sweeps.size(), "cudaMalloc(batch counters)");
@@ -2372,7 +2377,7 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
                     d_cspecs.p, int(P.cspecs.size()), d_patterns.p, d_rows.p, P.row_words);
                 check_cuda(cudaGetLastError(), "composite_kernel launch");
             }
-            if (!P.sweeps.empty()) sweep_tables.enqueue(stream);
+            if (!P.sweeps.empty()) sweep_tables->enqueue(stream);
             record(ev[1], stream);
             enqueue_sieve();
         };

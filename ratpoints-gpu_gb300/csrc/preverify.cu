@@ -273,6 +273,7 @@ PreCoef coef_residues(const std::string &text) {
 
 }  // namespace pre
 
+Preverifier::Preverifier() = default;
 Preverifier::~Preverifier() { release(); }
 
 void Preverifier::release() {
@@ -284,14 +285,16 @@ void Preverifier::release() {
 
 void Preverifier::prepare(const std::vector<const std::vector<std::string> *> &curves, cudaStream_t stream,
                           const Parallel &parallel) {
-    std::vector<pre::PreCurve> hc(curves.size());
+    auto &hc = host_curves_;
+    auto &hk = host_coefs_;
+    hc.assign(curves.size(), {});
     std::size_t total = 0;
     for (std::size_t i = 0; i < curves.size(); ++i) {
         hc[i].coef = (long long)total;
         hc[i].n = curves[i] ? int(curves[i]->size()) : 0;
         total += std::size_t(hc[i].n);
     }
-    std::vector<pre::PreCoef> hk(std::max<std::size_t>(total, 1));
+    hk.assign(std::max<std::size_t>(total, 1), {});
     auto reduce = [&](std::size_t i) {
         for (int j = 0; j < hc[i].n; ++j)
             hk[std::size_t(hc[i].coef + j)] = pre::coef_residues((*curves[i])[std::size_t(j)]);
@@ -311,7 +314,6 @@ void Preverifier::prepare(const std::vector<const std::vector<std::string> *> &c
     };
     grow(curves_, curves_cap_, std::max<std::size_t>(1, hc.size()) * sizeof(pre::PreCurve));
     grow(coefs_, coefs_cap_, hk.size() * sizeof(pre::PreCoef));
-    // pageable sources: they are read before these calls return
     if (!hc.empty())
         check_cuda(cudaMemcpyAsync(curves_, hc.data(), hc.size() * sizeof(pre::PreCurve), cudaMemcpyHostToDevice,
                                    stream),

@@ -23,16 +23,22 @@
 
 namespace rpg {
 
+namespace pre {
+struct PreCurve;
+struct PreCoef;
+}  // namespace pre
+
 class Preverifier {
 public:
-    Preverifier() = default;
+    Preverifier();
     ~Preverifier();
     Preverifier(const Preverifier &) = delete;
     Preverifier &operator=(const Preverifier &) = delete;
 
     // Coefficient residues of each curve (curve i = survivors tagged i),
     // uploaded on `stream` (other streams wait for it); device buffers grow and
-    // are kept across calls.
+    // are kept across calls.  The uploads read this object's arrays when the
+    // stream gets to them: the next call, and the end of the object, come after.
     // `parallel` (optional) runs its second argument for every index below the
     // first.
     using Parallel = std::function<void(std::size_t, const std::function<void(std::size_t)> &)>;
@@ -58,6 +64,8 @@ private:
     std::size_t curves_cap_ = 0, coefs_cap_ = 0;
     int blocks_ = 0;
     unsigned long long upload_bytes_ = 0;
+    std::vector<pre::PreCurve> host_curves_;  // sources of the uploads
+    std::vector<pre::PreCoef> host_coefs_;
 };
 
 // Host restatement of the device test for one survivor (CPU tests compare it

@@ -191,6 +191,7 @@ struct Sieve::Impl {
     cudaEvent_t tables_begin = nullptr, tables_end = nullptr;
     bool tables_timed = false;
     std::unique_ptr<SweepCurve> curve;
+    std::unique_ptr<SweepBuilder> builder;  // its upload's source, until the tables are there
     unsigned char *arena = nullptr;  // its tables
     std::size_t arena_bytes = 0;
     mutable bool lent = false;       // launched on a caller's stream: the arena is freed, not pooled
@@ -362,6 +363,7 @@ struct Sieve::Impl {
     }
 
     void release() {
+        if (stream) cudaStreamSynchronize(stream);  // uploads read arrays of this object
         offer_pipeline();
         for (auto &b : buf) {
             cudaFree(b.a);
@@ -477,22 +479,22 @@ struct Sieve::Impl {
             fast_plan = single_curve_plan(coefficients, bound, nullptr, shape);
         }
         curve.reset(new SweepCurve(coefficients, bound, opt.square, fast ? &fast_plan : nullptr, opt.denominators));
-        SweepBuilder builder;
-        builder.add(*curve);
+        builder.reset(new SweepBuilder);
+        builder->add(*curve);
         timings.plan_ms += ms_since(t0);
         auto t1 = Clock::now();
-        if (arena_bytes < builder.bytes()) {
+        if (arena_bytes < builder->bytes()) {
             cudaFree(arena);
             arena = nullptr;
             arena_bytes = 0;
-            arena = device_alloc<unsigned char>(builder.bytes(), "cudaMalloc(sieve tables)");
-            arena_bytes = builder.bytes();
+            arena = device_alloc<unsigned char>(builder->bytes(), "cudaMalloc(sieve tables)");
+            arena_bytes = builder->bytes();
         }
         timings.workspace_ms += ms_since(t1);
         check_cuda(cudaEventRecord(tables_begin, stream), "cudaEventRecord");
-        builder.place(arena, stream);
-        timings.h2d_bytes += builder.upload_bytes();
-        builder.enqueue(stream);
+        builder->place(arena, stream);
+        timings.h2d_bytes += builder->upload_bytes();
+        builder->enqueue(stream);
         if (opt.preverify) {
             if (!preverifier) preverifier.reset(new Preverifier());
             preverifier->prepare({&coefficients}, stream);
@@ -508,6 +510,7 @@ struct Sieve::Impl {
     void time_tables() {
         if (tables_timed) return;
         tables_timed = true;
+        builder.reset();
         float ms = 0;
         cudaEventElapsedTime(&ms, tables_begin, tables_end);
         timings.table_ms += ms;

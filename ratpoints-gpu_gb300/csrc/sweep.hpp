@@ -92,7 +92,8 @@ public:
     std::size_t bytes() const;
     std::size_t upload_bytes() const { return blob_.size(); }
     // Sets the curves' table addresses in the allocation at `arena`, uploads
-    // the inputs and, in enqueue, launches the builds.
+    // the inputs and, in enqueue, launches the builds.  The upload reads this
+    // object's array when the stream gets to it: the object outlives that.
     void place(unsigned char *arena, cudaStream_t stream);
     void enqueue(cudaStream_t stream) const;
     bool empty() const { return curves_.empty(); }
