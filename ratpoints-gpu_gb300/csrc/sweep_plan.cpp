@@ -240,13 +240,17 @@ SweepPlan plan_sweep(const SweepInput &in) {
         out.q = c.q;
         out.q_max = c.q_max;
         for (int i = 0; i < c.count; ++i) out.class_primes.push_back(primes[std::size_t(c.index[i])].p);
+        double bits = 0;
         for (const auto &w : primes)
             if (out.moduli.empty() &&
                 std::find(out.class_primes.begin(), out.class_primes.end(), w.p) == out.class_primes.end()) {
                 out.moduli.push_back(w.p);
                 out.rows.push_back({w.p});
+                bits = w.bits;
             }
         out.slots = 2;
+        out.cost = cost_of(c, 1, bits, double(sweep_row_words(out.moduli[0])) * 8.0 +
+                           kSweepListBytes * (c.q_mean + c.two_classes), out.ctas);
     }
     bool placed[512] = {};
     for (int p : out.class_primes) placed[p] = true;

@@ -3,6 +3,8 @@
 //   admitted H c0 c1 ..   the residue counts that a fast plan carries are those
 //                         of its primes; prints the plan's primes and the
 //                         swept words of denominators 1 .. 256
+//   cost H c0 c1 ..       prints the modelled cost of the fast and the reference
+//                         plan's sweep (SM cycles per denominator)
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -32,10 +34,18 @@ static int admitted(long long bound, const Coefficients &f) {
     return wrong;
 }
 
+static int cost(long long bound, const Coefficients &f) {
+    const FastPlan plan = single_curve_plan(f, bound, nullptr);
+    std::printf("%.6g %.6g\n", SweepCurve(f, bound, false, &plan, 1000).plan().cost,
+                SweepCurve(f, bound, false, nullptr, 1000).plan().cost);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     if (argc < 5) return 2;
     const long long bound = std::atoll(argv[2]);
     const Coefficients f(argv + 3, argv + argc);
     if (!std::strcmp(argv[1], "admitted")) return admitted(bound, f) ? 1 : 0;
+    if (!std::strcmp(argv[1], "cost")) return cost(bound, f);
     return 2;
 }

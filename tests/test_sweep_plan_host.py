@@ -63,6 +63,34 @@ def test_plans_carry_their_primes_residue_counts(check, coefficients):
         check("admitted", bound, coefficients)
 
 
+# a square at every x modulo every odd prime below 512: no row filters
+EVERYTHING = [1, math.prod(primes(3, 512))]
+
+
+@pytest.mark.parametrize("bound", [1_000, 100_000, 10 ** 8])
+def test_a_curve_that_nothing_filters_has_a_cost(check, bound):
+    # launches are cut by it, and a batch's ordered: not less than a curve
+    # whose words mostly end in the rows
+    for everything, sparse in zip(check("cost", bound, EVERYTHING).split(), check("cost", bound, [2, -3, 0, 5]).split()):
+        assert float(everything) >= float(sparse) > 0
+
+
+@pytest.mark.gpu
+def test_survivors_of_a_curve_that_nothing_filters(rpg):
+    # reference plan: every site; fast plan: those that are squares mod 64
+    a, d, _ = rpg.sieve(EVERYTHING, 70_000, 11, 12)
+    assert sorted(zip(d.tolist(), a.tolist())) == [(k, x) for k in (11, 12) for x in range(-70_000, 70_001)]
+    # and not multiples of a row prime (5 and 7) that divides d: F(a, d) = d (d + P a)
+    squares = {v * v % 64 for v in range(64)}
+    expected = [(k, x) for k in (11, 12) for x in range(-70_000, 70_001)
+                if (k % 2 or x % 2) and k * (k + EVERYTHING[1] * x) % 64 in squares]
+    a, d, _ = rpg.sieve(EVERYTHING, 70_000, 11, 12, plan="fast")
+    assert sorted(zip(d.tolist(), a.tolist())) == expected
+    points, status, survivors, _ = rpg.batch_search([{"coefficients": EVERYTHING, "bound": 70_000, "first": 11, "last": 12}])
+    assert status == [0] and survivors == [len(expected)]
+    assert points[0] == rpg.point_search(EVERYTHING, 70_000, 11, 12)[0]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("q", [257, 331, 509])
 def test_the_point_of_a_curve_with_one_admitted_residue(rpg, q):
