@@ -249,8 +249,8 @@ void rpg_session_destroy(rpg_session *session);
  * before the GPU runs.  The calling thread's current device is left as it was.
  *
  * Limits, each rejected with RPG_E_ARG: at most 16,777,216 denominators (256
- * launches of 65536) per call; and each row must fit one launch, which fails
- * only for very large numerator bounds (above about 1.7e10 times the class
+ * launches of 65536) per call; and rows that are not too long for it, which
+ * very large numerator bounds alone make them (above about 1.7e10 times the class
  * prime for a fast-plan session, above about 3.4e10 for a reference-plan one;
  * rpg_sieve_run has no such limit).
  * The error word and the launches' scheduling counters live in one fixed

@@ -82,7 +82,7 @@ extern "C" rpg_status rpg_session_sieve_noalloc(rpg_session *session, int32_t fi
             return fail(RPG_E_ARG,
                         "rpg_session_sieve_noalloc handles at most 16777216 denominators "
                         "(256 launches of 65536) per call; split the range");
-        if (!session->sieve->fits_one_launch())
+        if (!session->sieve->allocation_free_rows())
             return fail(RPG_E_ARG,
                         "rpg_session_sieve_noalloc needs each row in one launch: the session's "
                         "numerator bound is too large (use rpg_sieve_run)");

@@ -892,26 +892,29 @@ FastPlanInfo Sieve::fast_plan_info() const {
 
 int Sieve::device() const { return impl_->device; }
 
-// The limits of an allocation-free launch are those of the interface (2^23
-// words of a class mod 64 q under the fast plan, 2^30 words of consecutive
-// numerators under the reference plan); the kernel's tile is never smaller.
-bool Sieve::fits_one_launch() const {
+bool Sieve::allocation_free_rows() const {
     const long long sites = 2 * impl_->bound + 1;
-    if (impl_->opt.plan == PlanKind::fast) {
-        const long long words = (sites / (64LL * impl_->fast_plan.class_prime) + 1 + 63) / 64;
-        return words <= (1LL << 23) && impl_->one_launch();
-    }
-    return word_count64(impl_->bound) <= (1LL << 30) && impl_->one_launch();
+    if (impl_->opt.plan == PlanKind::fast)
+        return (sites / (64LL * impl_->fast_plan.class_prime) + 1 + 63) / 64 <= (1LL << 23);
+    return word_count64(impl_->bound) <= (1LL << 30);
 }
 
 bool Sieve::launch_into(long long first, long long last, long long *out_a, int *out_d,
                         unsigned long long capacity, unsigned long long *out_count,
                         unsigned long long *work, unsigned long long *error, cudaStream_t stream) {
     const auto &I = *impl_;
-    if (!fits_one_launch() || last < first || last - first + 1 > (1 << 16)) return false;
+    if (!allocation_free_rows() || last < first || last - first + 1 > (1 << 16)) return false;
     I.lent = true;
-    I.launch_sweep(first, last, -I.bound, I.bound, out_a, out_d, capacity, out_count, work, error, stream);
-    return true;
+    // A launch per tile of numerators: one, but for curves that few primes
+    // filter, whose classes are long.
+    const long long tile = I.curve->tile();
+    for (long long a = -I.bound;; a += tile) {
+        const bool end = I.bound - a < tile;
+        I.launch_sweep(first, last, a, end ? I.bound : a + tile - 1, out_a, out_d, capacity, out_count, work, error,
+                       stream);
+        if (end) return true;
+        check_cuda(cudaMemsetAsync(work, 0, sizeof *work, stream), "cudaMemsetAsync");
+    }
 }
 
 unsigned Sieve::smem_bytes_per_word() const { return unsigned(8 * impl_->curve->plan().moduli.size()); }
