@@ -1454,10 +1454,10 @@ long long swept_row_words(const BatchCurveSpec &c, long long first, long long la
 // with 0.7 for 0.9 or 8,000 for 20,000, bursts of requests and batches change
 // by 4 % at most, either way.
 // Curves with x intervals stay in the kernels that sweep only those.
-bool swept_alone(const BatchCurveSpec &c, const CurveWork &cw) {
+bool swept_alone(const BatchCurveSpec &c, bool wide, long long words, long long count) {
     if (!c.intervals.empty() && c.intervals.size() <= std::size_t(dev::kMaxIntervals)) return false;
-    if (cw.wide) return true;
-    return double(cw.count) * (2.8e-3 * double(cw.words) - 0.9) > 20000.0;
+    if (wide) return true;
+    return double(count) * (2.8e-3 * double(words) - 0.9) > 20000.0;
 }
 
 // Narrow plan: every odd prime up to kBatchNarrowModulus that filters at
@@ -1637,9 +1637,8 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, const std::vector<cha
             cw.count = last >= first ? last - first + 1 : 0;
             cw.swept = swept_row_words(c, first, last, cw.words);
             cw.wide = cw.swept >= kBatchWideWords;
-            if (cw.count > 0 && swept_alone(c, cw)) {
-                cw.plan = single_curve_plan(c.coefficients, c.bound, nullptr);
-                cw.sweep.reset(new SweepCurve(c.coefficients, c.bound, c.square, &cw.plan, double(cw.count)));
+            if (cw.count > 0 && swept_alone(c, cw.wide, cw.words, cw.count)) {
+                cw.sweep = batch_sweep_curve(c, &cw.plan);
                 cw.ok = true;
                 return;
             }
@@ -2590,11 +2589,25 @@ std::vector<BatchCurveResult> BatchEngine::run(const std::vector<BatchCurveSpec>
     return impl_->run(curves, stats, use_graph, preverify, items_per_kernel);
 }
 
+std::unique_ptr<SweepCurve> batch_sweep_curve(const BatchCurveSpec &c, FastPlan *plan) {
+    FastPlan own = single_curve_plan(c.coefficients, c.bound, nullptr);
+    std::unique_ptr<SweepCurve> sweep(new SweepCurve(c.coefficients, c.bound, c.square, &own,
+                                                     double(c.last) - double(c.first) + 1.0, kBatchRowBytes));
+    if (plan) *plan = std::move(own);
+    return sweep;
+}
+
 int BatchEngine::device() const { return impl_->device; }
 
 unsigned long long BatchEngine::estimate_bytes(const BatchCurveSpec &c) {
     const long long words = word_count64(std::max(1LL, c.bound));
     const long long count = c.last >= c.first ? c.last - c.first + 1 : 0;
+    // a search of its own beside the batch (huge rows), with its survivor
+    // buffers, or launches of its own
+    if (words >= kBatchSoloWords)
+        return SweepCurve::most_bytes(c.bound, c.coefficients.size(), 0) + (50ull << 20);
+    if (count > 0 && swept_alone(c, words >= kBatchWideWords, words, count))
+        return SweepCurve::most_bytes(c.bound, c.coefficients.size(), kBatchRowBytes);
     long long table;
     if (words >= kBatchWideWords) {
         const double cap = std::min<double>(kMaxModulus, std::max(64.0, std::sqrt(double(words) * count / 48.0)));
@@ -2602,8 +2615,6 @@ unsigned long long BatchEngine::estimate_bytes(const BatchCurveSpec &c) {
     } else {
         table = dev::kNarrowTableWords;
     }
-    // curves with launches of their own: pattern rows and candidate tables
-    if (words >= 512 && c.intervals.empty()) table = std::max(table, 1700000LL);
     // tables, bitmasks, patterns, descriptor and items (8-byte words)
     return (unsigned long long)(table + 2 * dev::kAffWords + 6 * 127 * 127 + 1024 +
                                 std::max(1LL, count * std::max(1LL, (long long)c.intervals.size()) /

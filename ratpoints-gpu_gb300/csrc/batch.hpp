@@ -120,6 +120,14 @@ private:
 // device).
 void release_pooled_engines(int device);
 
+// A curve's sweep, when it has launches of its own in a batch (plan: its fast
+// plan, optional).  The row tables of such a curve are limited to
+// kBatchRowBytes, so that a batch's memory can be foreseen; of 9,939 random,
+// dense and half dense curves without a limit none had more than 39 MB.
+constexpr long long kBatchRowBytes = 40LL << 20;
+class SweepCurve;
+std::unique_ptr<SweepCurve> batch_sweep_curve(const BatchCurveSpec &curve, FastPlan *plan = nullptr);
+
 // One batched pass on an engine on `device` (-1: current).
 std::vector<BatchCurveResult> batch_search(const std::vector<BatchCurveSpec> &curves, int device,
                                            BatchStats *stats, bool use_graph = true, bool preverify = true);

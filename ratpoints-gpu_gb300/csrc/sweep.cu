@@ -282,7 +282,7 @@ int inverse64(int i) {
 SweepCurve::~SweepCurve() = default;
 
 SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long bound, bool square, const FastPlan *fast,
-                       double denominators)
+                       double denominators, long long row_bytes)
     : bound_(bound), square_(square), tables_(new dev::SweepTables{}), list_(new dev::ListJob{}) {
     dev::SweepTables &T = *tables_;
     dev::ListJob &L = *list_;
@@ -294,6 +294,7 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
     SweepInput in;
     in.bound = bound;
     in.denominators = denominators;
+    in.row_bytes = row_bytes;
     dev::u64 adm2[64];
     for (auto &v : adm2) v = ~dev::u64(0);
     if (fast) {
@@ -498,6 +499,25 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
             std::size_t(kSweepQueueBytes) * std::size_t(kSweepWarps / plan_.ctas - 1);
     // queued positions stay below 2^46 and class words below 2^23
     tile_ = S * std::min<long long>(1LL << 23, (1LL << 45) / S);
+}
+
+unsigned long long SweepCurve::most_bytes(long long bound, std::size_t coefficients, long long row_bytes) {
+    // rows as wide as two slots' worth of a CTA allow, by the plan's largest modulus
+    if (row_bytes <= 0) row_bytes = sweep_cta_bytes(2) * kMaxModulus;
+    // pattern rows of every odd prime below 512, the six largest candidates'
+    // tables, and a job and the coefficients' residues for each of them
+    unsigned long long bytes = (unsigned long long)row_bytes;
+    for (const auto &o : odd_primes())
+        bytes += std::size_t(o.p) * std::size_t((o.p + 64 + 63) / 64 + 1) * 8 + 256 + sizeof(dev::PatternJob) +
+                 sizeof(dev::TableJob) + coefficients * sizeof(unsigned short) + 16;
+    const auto &cands = candidate_primes();
+    for (int i = kCandidatePrimes - dev::kFStage2Group; i < kCandidatePrimes; ++i)
+        bytes += (unsigned long long)cands[std::size_t(i)] * (unsigned long long)cands[std::size_t(i)] * 8 + 256;
+    // class lists: Q at most 8,192, and small enough for classes of ten words
+    const long long q = std::max(1LL, std::min<long long>(8192, bound / (320 * 64) + 1));
+    bytes += (unsigned long long)std::min(32LL << 20, q * std::min<long long>(q, kSweepMaxClasses) * kSweepListBytes);
+    bytes += 64 * 64 * kSweepListBytes + 65536;  // the list mod two, counts, maps, alignment
+    return bytes;
 }
 
 unsigned long long SweepCurve::swept_words(long long first, long long last) const {

@@ -43,9 +43,12 @@ struct SweepLaunch {
 class SweepCurve {
 public:
     // fast null: the reference plan.  denominators: about how many the search
-    // has (0: not known), weighed against the tables' build.  Host only.
+    // has (0: not known), weighed against the tables' build.  row_bytes: most
+    // bytes of the rows' tables (0: no limit).  Host only.
     SweepCurve(const std::vector<std::string> &coefficients, long long bound, bool square, const FastPlan *fast,
-               double denominators);
+               double denominators, long long row_bytes = 0);
+    // What SweepBuilder::bytes() says of a curve under the fast plan, at most.
+    static unsigned long long most_bytes(long long bound, std::size_t coefficients, long long row_bytes);
     ~SweepCurve();
     SweepCurve(const SweepCurve &) = delete;
     SweepCurve &operator=(const SweepCurve &) = delete;

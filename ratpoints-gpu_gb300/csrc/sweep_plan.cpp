@@ -208,13 +208,12 @@ SweepPlan plan_sweep(const SweepInput &in) {
                     slots = int(std::min<long long>(kSweepSlots, room / slot));
                 }
                 if (!ctas) continue;
-                // the rows' build, about three words per SM cycle over the
+                double build = 0;  // words of the rows' tables
+                for (int i = 0; i < p.count; ++i) build += double(p.modulus[i]) * sweep_row_words(p.modulus[i]);
+                if (in.row_bytes > 0 && build * 8.0 > double(in.row_bytes)) continue;
+                // their build, about three words per SM cycle over the
                 // device, shared by the denominators
-                if (in.denominators > 0) {
-                    double build = 0;
-                    for (int i = 0; i < p.count; ++i) build += double(p.modulus[i]) * sweep_row_words(p.modulus[i]);
-                    cost += build / 3.0 / in.denominators;
-                }
+                if (in.denominators > 0) cost += build / 3.0 / in.denominators;
                 if (found && cost >= out.cost) continue;
                 found = true;
                 out.cost = cost;

@@ -38,6 +38,7 @@ struct SweepInput {
     double two_classes = 1; // mean classes mod two of a denominator that has any
     int two_max = 1;        // most of them
     std::vector<SweepPrime> primes;
+    long long row_bytes = 0;  // most bytes of the rows' tables (0: no limit)
 };
 
 struct SweepPlan {

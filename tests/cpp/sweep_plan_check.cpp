@@ -5,12 +5,15 @@
 //                         swept words of denominators 1 .. 256
 //   cost H c0 c1 ..       prints the modelled cost of the fast and the reference
 //                         plan's sweep (SM cycles per denominator)
+//   memory H c0 c1 ..     a batch's admission estimate and table bytes for curves
+//                         with launches of their own, by last denominator
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <string>
 #include <vector>
 
+#include "batch.hpp"
 #include "plan.hpp"
 #include "sieve.hpp"
 #include "sweep.hpp"
@@ -41,11 +44,35 @@ static int cost(long long bound, const Coefficients &f) {
     return 0;
 }
 
+static int memory(long long bound, const Coefficients &f) {
+    BatchCurveSpec c;
+    c.coefficients = f;
+    c.bound = bound;
+    const double words = double(word_count64(bound));
+    for (long long last : {1LL, 20LL, 1'000LL, 30'000LL, 400'000LL, 5'000'000LL, 2'000'000'000LL}) {
+        c.last = last;
+        // the batch's rule: rows of 2,048 words, or shorter ones with much work
+        if (words < double(kBatchWideWords) && double(last) * (2.8e-3 * words - 0.9) <= 20000.0) continue;
+        std::unique_ptr<SweepCurve> curve = batch_sweep_curve(c);
+        SweepBuilder builder;
+        builder.add(*curve);
+        std::printf("%lld %llu ", last, (unsigned long long)builder.bytes());
+        c.intervals.clear();
+        std::printf("%llu ", BatchEngine::estimate_bytes(c));
+        c.intervals.resize(9);  // more than the device takes: the whole row
+        for (auto &i : c.intervals) i.lower_infinite = i.upper_infinite = true;
+        std::printf("%llu\n", BatchEngine::estimate_bytes(c));
+        c.intervals.clear();
+    }
+    return 0;
+}
+
 int main(int argc, char **argv) {
     if (argc < 5) return 2;
     const long long bound = std::atoll(argv[2]);
     const Coefficients f(argv + 3, argv + argc);
     if (!std::strcmp(argv[1], "admitted")) return admitted(bound, f) ? 1 : 0;
+    if (!std::strcmp(argv[1], "memory")) return memory(bound, f);
     if (!std::strcmp(argv[1], "cost")) return cost(bound, f);
     return 2;
 }

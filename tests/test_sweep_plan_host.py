@@ -75,6 +75,18 @@ def test_a_curve_that_nothing_filters_has_a_cost(check, bound):
         assert float(everything) >= float(sparse) > 0
 
 
+@pytest.mark.parametrize("bound", [10_400, 12_000, 16_383, 60_000, 65_503, 65_504, 300_000, 1_000_000, 4_000_000])
+@pytest.mark.parametrize("coefficients", [RECORD, [2, -3, 0, 5], [-533746463, 2318474698, 1819918790, -3268433658,
+                                                                  1978982371, 1087269120, -559365050], EVERYTHING])
+def test_a_batch_admits_what_its_curves_take(check, coefficients, bound):
+    # curves with launches of their own: not less than their tables, nor much more
+    # than the largest
+    rows = [list(map(int, line.split())) for line in check("memory", bound, coefficients).splitlines()]
+    assert rows
+    for last, tables, *estimates in rows:
+        assert all(tables <= estimate <= 64 << 20 for estimate in estimates), (last, tables, estimates)
+
+
 @pytest.mark.gpu
 def test_survivors_of_a_curve_that_nothing_filters(rpg):
     # reference plan: every site; fast plan: those that are squares mod 64
