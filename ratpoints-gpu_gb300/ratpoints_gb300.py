@@ -379,9 +379,9 @@ def _batch_options(curves):
     rows["last"] = [_wrapped(c["last"], 32) for c in curves]
     rows["intervals"] = ends.ctypes.data + 16 * (np.cumsum(spans) - spans)
     rows["interval_count"] = spans
-    rows["include_infinity"] = [int(c.get("include_infinity", True)) for c in curves]
+    rows["include_infinity"] = [_wrapped(c.get("include_infinity", True), 32) for c in curves]
     rows["batch_size"] = 1 << 16
-    rows["square_denominators"] = [int(c.get("square", False)) for c in curves]
+    rows["square_denominators"] = [_wrapped(c.get("square", False), 32) for c in curves]
     rows["plan"] = RPG_PLAN_FAST
     rows["device"] = -1
     return arr, buffers
