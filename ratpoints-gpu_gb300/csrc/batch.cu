@@ -2042,7 +2042,13 @@ struct BatchEngine::Impl {
     DeviceArray<int> d_d, d_c, d_pd, d_pc;
     DeviceArray<unsigned long long> d_curve_modular;  // per-curve modular survivors
     Preverifier pre;
-    std::unique_ptr<SweepBuilder> sweep_tables;  // of the run: its upload's source
+    // Curves with launches of their own (of plan.sweeps), whose tables share
+    // d_sweep_tables; the builders hold the uploads' sources.
+    struct SweepGroup {
+        std::size_t begin = 0, end = 0;
+        std::unique_ptr<SweepBuilder> tables;
+    };
+    std::vector<SweepGroup> sweep_groups;
 
     Impl() {  // on the current device
         check_cuda(cudaGetDevice(&device), "cudaGetDevice");
@@ -2093,7 +2099,7 @@ struct BatchEngine::Impl {
     // Frees the largest arrays until at most `limit` bytes are held on the
     // device, and the host's plan if it holds more than an eighth of that.
     void trim(std::size_t limit) {
-        sweep_tables.reset();
+        sweep_groups.clear();
         plan.clear();
         if (plan.bytes() > limit / 8) plan = BatchPlan{};
         std::vector<std::pair<std::size_t, std::function<void()>>> arrays;
@@ -2130,6 +2136,46 @@ struct BatchEngine::Impl {
         if (h_counters) cudaFreeHost(h_counters);
         if (stream) cudaStreamDestroy(stream);
         if (side) cudaStreamDestroy(side);
+    }
+
+    // Groups the plan's sweeps, in their order, so that the tables of a group
+    // take at most `limit` bytes (or are one curve's); the bytes of the largest.
+    std::size_t group_sweeps(std::size_t limit) {
+        sweep_groups.clear();
+        std::size_t largest = 0, used = 0;
+        for (std::size_t j = 0; j < plan.sweeps.size(); ++j) {
+            SweepCurve &curve = *plan.work[plan.sweeps[j]].sweep;
+            if (sweep_groups.empty() || used + curve.bytes() > limit) {
+                sweep_groups.push_back({j, j, std::unique_ptr<SweepBuilder>(new SweepBuilder)});
+                used = 0;
+            }
+            used += curve.bytes();
+            sweep_groups.back().tables->add(curve);
+            sweep_groups.back().end = j + 1;
+        }
+        for (const auto &g : sweep_groups) largest = std::max(largest, g.tables->bytes());
+        return largest;
+    }
+
+    // Groups the sweeps and gets the memory for their tables: nearly always one
+    // group.  Tables of 13 to 40 MB a curve (searches long enough to gain from
+    // them) fill the device with 7,000 to 20,000 curves, so there is a limit,
+    // and a lower one if that much is not to be had.  RPG_BATCH_TABLE_BYTES sets
+    // it (tests use a small one).
+    void ensure_sweep_tables() {
+        std::size_t limit = std::size_t(64) << 30;
+        if (const char *env = std::getenv("RPG_BATCH_TABLE_BYTES")) limit = std::size_t(std::max(1LL, std::atoll(env)));
+        for (;;) {
+            const std::size_t bytes = group_sweeps(limit);
+            try {
+                if (bytes) d_sweep_tables.ensure(bytes, "cudaMalloc(sieve tables)");
+                return;
+            } catch (const CudaError &) {
+                if (sweep_groups.size() == plan.sweeps.size()) throw;
+                cudaGetLastError();
+                limit = std::min(limit, bytes) / 2;
+            }
+        }
     }
 
     void ensure_output(unsigned long long cap) {
@@ -2235,13 +2281,6 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
         d_aff.ensure(std::size_t(P.aff_words), "cudaMalloc(batch bitmasks)");
         d_patterns.ensure(std::size_t(P.pattern_words), "cudaMalloc(batch patterns)");
         d_rows.ensure(std::size_t(P.row_words), "cudaMalloc(batch tables)");
-        sweep_tables.reset(new SweepBuilder);
-        for (std::size_t i : P.sweeps) sweep_tables->add(*work[i].sweep);
-        if (!P.sweeps.empty()) {
-            d_sweep_tables.ensure(sweep_tables->bytes(), "cudaMalloc(sieve tables)");
-            sweep_tables->place(d_sweep_tables.p, stream);
-            stats.h2d_bytes += sweep_tables->upload_bytes();
-        }
         ensure_output(capacity);
         d_counters.ensure(kCounters + P.sweeps.size(), "cudaMalloc(batch counters)");
         if (preverify) {
@@ -2254,6 +2293,14 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
             stats.h2d_bytes += pre.upload_bytes();
             d_curve_modular.ensure(std::max<std::size_t>(1, curves.size()), "cudaMalloc(batch counters)");
         }
+        ensure_sweep_tables();  // last: it may do with less
+        // more groups than one: their tables are uploaded and built in turn
+        const bool in_turn = sweep_groups.size() > 1;
+        auto upload_tables = [&](const SweepGroup &g) {
+            g.tables->place(d_sweep_tables.p, stream);
+            stats.h2d_bytes += g.tables->upload_bytes();
+        };
+        if (sweep_groups.size() == 1) upload_tables(sweep_groups[0]);
 
         const int wide_smem_words = P.wide_smem_words;
         const int wide_max_classes = P.wide_max_classes;
@@ -2310,31 +2357,38 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
                     d_counters.p + 1, d_counters.p + 5);
                 check_cuda(cudaGetLastError(), "wide_kernel launch");
             }
-            const int streams = int(std::min<std::size_t>(kSweepStreams, P.sweeps.size()));
-            for (int k = 0; k < streams; ++k)
-                check_cuda(cudaStreamWaitEvent(sweep_stream[k], fork, 0), "cudaStreamWaitEvent");
-            for (std::size_t j = 0; j < P.sweeps.size(); ++j) {
-                const std::size_t i = P.sweeps[j];
-                SweepLaunch l;
-                l.first = curves[i].first;
-                l.last = curves[i].last;
-                l.a_lo = -curves[i].bound;
-                l.a_hi = curves[i].bound;
-                l.out_a = d_a.p;
-                l.out_d = d_d.p;
-                l.out_curve = d_c.p;
-                l.curve = int(i);
-                l.capacity = capacity;
-                l.out_count = d_counters.p;
-                l.work = d_counters.p + kCounters + j;
-                l.error = d_counters.p + 3;
-                l.swept = d_counters.p + 5;
-                const int k = int(j % std::size_t(kSweepStreams + 1));
-                work[i].sweep->launch(l, k < streams ? sweep_stream[k] : stream);
-            }
-            for (int k = 0; k < streams; ++k) {
-                check_cuda(cudaEventRecord(sweep_join[k], sweep_stream[k]), "cudaEventRecord");
-                check_cuda(cudaStreamWaitEvent(stream, sweep_join[k], 0), "cudaStreamWaitEvent");
+            for (const SweepGroup &g : sweep_groups) {
+                if (in_turn) {  // after the launches of the group before
+                    upload_tables(g);
+                    g.tables->enqueue(stream);
+                    check_cuda(cudaEventRecord(fork, stream), "cudaEventRecord");
+                }
+                const int streams = int(std::min<std::size_t>(kSweepStreams, g.end - g.begin));
+                for (int k = 0; k < streams; ++k)
+                    check_cuda(cudaStreamWaitEvent(sweep_stream[k], fork, 0), "cudaStreamWaitEvent");
+                for (std::size_t j = g.begin; j < g.end; ++j) {
+                    const std::size_t i = P.sweeps[j];
+                    SweepLaunch l;
+                    l.first = curves[i].first;
+                    l.last = curves[i].last;
+                    l.a_lo = -curves[i].bound;
+                    l.a_hi = curves[i].bound;
+                    l.out_a = d_a.p;
+                    l.out_d = d_d.p;
+                    l.out_curve = d_c.p;
+                    l.curve = int(i);
+                    l.capacity = capacity;
+                    l.out_count = d_counters.p;
+                    l.work = d_counters.p + kCounters + j;
+                    l.error = d_counters.p + 3;
+                    l.swept = d_counters.p + 5;
+                    const int k = int((j - g.begin) % std::size_t(kSweepStreams + 1));
+                    work[i].sweep->launch(l, k < streams ? sweep_stream[k] : stream);
+                }
+                for (int k = 0; k < streams; ++k) {
+                    check_cuda(cudaEventRecord(sweep_join[k], sweep_stream[k]), "cudaEventRecord");
+                    check_cuda(cudaStreamWaitEvent(stream, sweep_join[k], 0), "cudaStreamWaitEvent");
+                }
             }
             record(ev[3], stream);
             record(ev[4], side);
@@ -2376,11 +2430,11 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
                     d_cspecs.p, int(P.cspecs.size()), d_patterns.p, d_rows.p, P.row_words);
                 check_cuda(cudaGetLastError(), "composite_kernel launch");
             }
-            if (!P.sweeps.empty()) sweep_tables->enqueue(stream);
+            if (sweep_groups.size() == 1) sweep_groups[0].tables->enqueue(stream);
             record(ev[1], stream);
             enqueue_sieve();
         };
-        if (use_graph) {
+        if (use_graph && !in_turn) {  // a graph has no uploads in it
             cudaGraph_t graph = nullptr;
             cudaGraphExec_t exec = nullptr;
             check_cuda(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal),
@@ -2411,7 +2465,7 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
         }
         stats.launches += (P.aspecs.empty() ? 0 : 1) + (P.pattern_words ? 1 : 0) + (P.row_words ? 1 : 0) +
                           (wide_grid ? 1 : 0) + (narrow_grid ? 1 : 0) + (preverify ? 1 : 0) +
-                          (P.sweeps.empty() ? 0 : 3 + P.sweeps.size());
+                          3 * sweep_groups.size() + P.sweeps.size();
         auto elapsed = [&](int a, int b) {
             float ms = 0;
             cudaEventElapsedTime(&ms, ev[a], ev[b]);
@@ -2428,7 +2482,8 @@ std::vector<BatchCurveResult> BatchEngine::Impl::run(const std::vector<BatchCurv
             enqueue_sieve();
             check_cuda(cudaStreamSynchronize(stream), "batch sieve");
             stats.sieve_ms += std::max(elapsed(2, 3), elapsed(2, 5));
-            stats.launches += (wide_grid ? 1 : 0) + (narrow_grid ? 1 : 0) + (preverify ? 1 : 0) + P.sweeps.size();
+            stats.launches += (wide_grid ? 1 : 0) + (narrow_grid ? 1 : 0) + (preverify ? 1 : 0) +
+                              (in_turn ? 3 * sweep_groups.size() : 0) + P.sweeps.size();
             if (h_counters[3]) throw DeviceTimeout("batched sieve: a bounded wait timed out");
         }
         stats.survivors = h_counters[0];

@@ -501,6 +501,11 @@ SweepCurve::SweepCurve(const std::vector<std::string> &coefficients, long long b
     tile_ = S * std::min<long long>(1LL << 23, (1LL << 45) / S);
 }
 
+std::size_t SweepCurve::bytes() const {
+    return table_bytes_ + input_.size() + patterns_.size() * sizeof(dev::PatternJob) + jobs_.size() * sizeof(dev::TableJob) +
+           sizeof(dev::ListJob) + 1024;  // alignment
+}
+
 unsigned long long SweepCurve::most_bytes(long long bound, std::size_t coefficients, long long row_bytes) {
     // rows as wide as two slots' worth of a CTA allow, by the plan's largest modulus
     if (row_bytes <= 0) row_bytes = sweep_cta_bytes(2) * kMaxModulus;

@@ -47,7 +47,9 @@ public:
     // bytes of the rows' tables (0: no limit).  Host only.
     SweepCurve(const std::vector<std::string> &coefficients, long long bound, bool square, const FastPlan *fast,
                double denominators, long long row_bytes = 0);
-    // What SweepBuilder::bytes() says of a curve under the fast plan, at most.
+    // What the curve adds to SweepBuilder::bytes(), at most, and the most that any
+    // curve adds under the fast plan.
+    std::size_t bytes() const;
     static unsigned long long most_bytes(long long bound, std::size_t coefficients, long long row_bytes);
     ~SweepCurve();
     SweepCurve(const SweepCurve &) = delete;

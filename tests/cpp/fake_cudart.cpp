@@ -27,6 +27,7 @@ namespace {
 std::recursive_mutex mutex;
 std::vector<std::function<void()>> queue;
 long long stale = 0, launched = 0, fail_in = 0;
+unsigned long long largest_allocation = ~0ull;
 
 using Lock = std::lock_guard<std::recursive_mutex>;
 
@@ -69,6 +70,7 @@ void run_queued() {
 long long stale_sources() { return stale; }
 void fail_launch(long long n) { fail_in = n; }
 long long launches() { return launched; }
+void limit_allocations(unsigned long long bytes) { largest_allocation = bytes; }
 
 }  // namespace fake
 
@@ -123,8 +125,11 @@ cudaError_t cudaGetSymbolAddress(void **p, const void *) {
     return *p = scratch, cudaSuccess;
 }
 
-cudaError_t cudaMalloc(void **p, size_t n) { return *p = std::calloc(n ? n : 1, 1), cudaSuccess; }
-cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return cudaMalloc(p, n); }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return *p = std::calloc(n ? n : 1, 1), cudaSuccess; }
+cudaError_t cudaMalloc(void **p, size_t n) {
+    if (n > largest_allocation) return last = cudaErrorMemoryAllocation;
+    return cudaHostAlloc(p, n, 0);
+}
 // memory that queued work may still name is not handed out again
 cudaError_t cudaFree(void *) { return cudaSuccess; }
 cudaError_t cudaFreeHost(void *) { return cudaSuccess; }

@@ -14,5 +14,7 @@ long long stale_sources();
 // The n-th call from now that launches a kernel fails (n = 0: none does).
 void fail_launch(long long n);
 long long launches();  // kernel launches so far
+// Device allocations above this many bytes fail for want of memory.
+void limit_allocations(unsigned long long bytes);
 
 }  // namespace fake
