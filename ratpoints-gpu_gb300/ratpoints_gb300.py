@@ -332,6 +332,14 @@ def _wrapped(value, bits):
     return value if -half <= value < half else (value + half) % (2 * half) - half
 
 
+def _flags(values):
+    """A column of 32-bit fields (0 and 1, but what wraps is taken)."""
+    try:
+        return np.array(values, dtype=np.int32)
+    except OverflowError:
+        return [_wrapped(v, 32) for v in values]
+
+
 # SearchOptions and Interval as numpy records, to fill a batch's by column
 _OPTIONS_RECORD = np.dtype({
     "names": [f[0] for f in SearchOptions._fields_],
@@ -379,9 +387,9 @@ def _batch_options(curves):
     rows["last"] = [_wrapped(c["last"], 32) for c in curves]
     rows["intervals"] = ends.ctypes.data + 16 * (np.cumsum(spans) - spans)
     rows["interval_count"] = spans
-    rows["include_infinity"] = [_wrapped(c.get("include_infinity", True), 32) for c in curves]
+    rows["include_infinity"] = _flags([int(c.get("include_infinity", True)) for c in curves])
     rows["batch_size"] = 1 << 16
-    rows["square_denominators"] = [_wrapped(c.get("square", False), 32) for c in curves]
+    rows["square_denominators"] = _flags([int(c.get("square", False)) for c in curves])
     rows["plan"] = RPG_PLAN_FAST
     rows["device"] = -1
     return arr, buffers
