@@ -66,8 +66,10 @@ bool coefficients_from(const char *const *c, int32_t n, std::vector<std::string>
         }
         std::string s(c[i]);
         if (!s.empty() && s.front() == '+') s.erase(0, 1);
-        const std::size_t digits = s.find_first_not_of("+-") == 0 ? 0 : 1;  // after at most one sign
-        if (s.size() <= digits || s.find_first_not_of("0123456789", digits) != std::string::npos) {
+        const std::size_t digits = !s.empty() && s[0] != '+' && s[0] != '-' ? 0 : 1;  // after at most one sign
+        bool number = s.size() > digits;
+        for (std::size_t k = digits; k < s.size(); ++k) number = number && s[k] >= '0' && s[k] <= '9';
+        if (!number) {
             error = "coefficients must be decimal integers";
             return false;
         }
