@@ -294,7 +294,8 @@ typedef struct rpg_batch_stats {
     uint64_t launches;         /* kernel launches (table build and sieve) */
     uint64_t words;            /* 64-site row words of all denominators */
     uint64_t table_words;      /* stage-1 table words resident on the device */
-    uint64_t swept_words;      /* 64-site words the sieve kernels sweep (counted by them) */
+    uint64_t swept_words;      /* 64-site words the sieve kernels sweep (counted by them; launches of
+                                * a curve's own sweep 16 words at a time and count the last whole) */
     uint64_t smem_bytes;       /* stage-1 shared-memory bytes those sweeps read */
     double rectangle_sites;    /* sum over curves of (2H + 1) x denominators */
     double plan_ms;            /* host: validation, plans, descriptors */

@@ -427,7 +427,8 @@ __global__ void __launch_bounds__(kFThreads, 2) fast_sieve_kernel(const __grid_c
             const int items = int((long long)all * (part + 1) >> A.part_shift);  // first: fewer items than parts
             const int turn = int(unsigned(items - first) % unsigned(consumers));
             const bool mine = n2 > 0 && nq > 0 && first < items;
-            if (mine && part == 0) swept += (unsigned long long)units * unsigned(n2) * kSweepUnit;
+            if (valid && n2 > 0 && nq > 0 && part == 0)  // the whole denominator's; this share may be empty
+                swept += (unsigned long long)units * unsigned(n2) * kSweepUnit;
             u32 live = __ballot_sync(kFullMask, mine);
             while (live) {
                 const int j = __ffs(live) - 1;

@@ -5,6 +5,8 @@
 //                         swept words of denominators 1 .. 256
 //   cost H c0 c1 ..       prints the modelled cost of the fast and the reference
 //                         plan's sweep (SM cycles per denominator)
+//   swept H last c0 ..    the words a batch's launch for denominators 1 .. last
+//                         sweeps, in units of 16 words
 //   memory H c0 c1 ..     a batch's admission estimate and table bytes for curves
 //                         with launches of their own, by last denominator
 #include <cstdio>
@@ -67,12 +69,25 @@ static int memory(long long bound, const Coefficients &f) {
     return 0;
 }
 
+static int swept(long long bound, long long last, const Coefficients &f) {
+    BatchCurveSpec c;
+    c.coefficients = f;
+    c.bound = bound;
+    c.last = last;
+    const std::unique_ptr<SweepCurve> curve = batch_sweep_curve(c);
+    const long long words = sweep_words(bound, (long long)curve->plan().two * curve->plan().q);
+    std::printf("%llu\n", curve->swept_words(1, last) / (unsigned long long)words *
+                              (unsigned long long)((words + kSweepUnit - 1) / kSweepUnit * kSweepUnit));
+    return 0;
+}
+
 int main(int argc, char **argv) {
     if (argc < 5) return 2;
     const long long bound = std::atoll(argv[2]);
     const Coefficients f(argv + 3, argv + argc);
     if (!std::strcmp(argv[1], "admitted")) return admitted(bound, f) ? 1 : 0;
     if (!std::strcmp(argv[1], "memory")) return memory(bound, f);
+    if (!std::strcmp(argv[1], "swept")) return swept(bound, std::atoll(argv[3]), Coefficients(argv + 4, argv + argc));
     if (!std::strcmp(argv[1], "cost")) return cost(bound, f);
     return 2;
 }

@@ -111,3 +111,14 @@ def test_the_point_of_a_curve_with_one_admitted_residue(rpg, q):
     assert (5, q, 1) in points
     batch, status, _, _ = rpg.batch_search([{"coefficients": curve, "bound": 100_000, "first": 1, "last": 256}])
     assert status == [0] and batch[0] == points
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("last", [1, 2, 50, 3_000])
+@pytest.mark.parametrize("bound", [70_000, 1_000_003, 4_000_000])
+@pytest.mark.parametrize("coefficients", [RECORD, ["2", "-3", "0", "5"]])
+def test_launches_count_the_words_they_sweep(rpg, check, coefficients, bound, last):
+    # also those of a denominator with fewer sweep items than it has shares
+    _, status, _, stats = rpg.batch_search([{"coefficients": coefficients, "bound": bound, "first": 1, "last": last}])
+    expected = int(check("swept", bound, [last, *coefficients]))
+    assert status == [0] and stats["swept_words"] == expected > 0
