@@ -301,8 +301,16 @@ ShapeCache &cache() {
     return c;
 }
 
+// Whether a sieve tests the same primes under both: the sweep plan made of them,
+// and so the kernel, is the same then.
 bool same_plan(const FastPlan &a, const FastPlan &b) {
-    return a.class_prime == b.class_prime && a.moduli == b.moduli && a.row_slots == b.row_slots;
+    auto primes = [](const FastPlan &p) {
+        std::vector<int> out;
+        for (const auto &f : p.slots) out.insert(out.end(), f.begin(), f.end());
+        std::sort(out.begin(), out.end());
+        return out;
+    };
+    return a.class_prime == b.class_prime && primes(a) == primes(b);
 }
 
 }  // namespace
