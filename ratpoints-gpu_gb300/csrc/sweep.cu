@@ -511,13 +511,18 @@ unsigned long long SweepCurve::most_bytes(long long bound, std::size_t coefficie
     if (row_bytes <= 0) row_bytes = sweep_cta_bytes(2) * kMaxModulus;
     // pattern rows of every odd prime below 512, the six largest candidates'
     // tables, and a job and the coefficients' residues for each of them
-    unsigned long long bytes = (unsigned long long)row_bytes;
-    for (const auto &o : odd_primes())
-        bytes += std::size_t(o.p) * std::size_t((o.p + 64 + 63) / 64 + 1) * 8 + 256 + sizeof(dev::PatternJob) +
-                 sizeof(dev::TableJob) + coefficients * sizeof(unsigned short) + 16;
-    const auto &cands = candidate_primes();
-    for (int i = kCandidatePrimes - dev::kFStage2Group; i < kCandidatePrimes; ++i)
-        bytes += (unsigned long long)cands[std::size_t(i)] * (unsigned long long)cands[std::size_t(i)] * 8 + 256;
+    static const unsigned long long tables = [] {
+        unsigned long long sum = 0;
+        for (const auto &o : odd_primes())
+            sum += std::size_t(o.p) * std::size_t((o.p + 64 + 63) / 64 + 1) * 8 + 256 + sizeof(dev::PatternJob) +
+                   sizeof(dev::TableJob) + 16;
+        const auto &cands = candidate_primes();
+        for (int i = kCandidatePrimes - dev::kFStage2Group; i < kCandidatePrimes; ++i)
+            sum += (unsigned long long)cands[std::size_t(i)] * (unsigned long long)cands[std::size_t(i)] * 8 + 256;
+        return sum;
+    }();
+    unsigned long long bytes =
+        (unsigned long long)row_bytes + tables + odd_primes().size() * coefficients * sizeof(unsigned short);
     // class lists: Q at most 8,192, and small enough for classes of ten words
     const long long q = std::max(1LL, std::min<long long>(8192, bound / (320 * 64) + 1));
     bytes += (unsigned long long)std::min(32LL << 20, q * std::min<long long>(q, kSweepMaxClasses) * kSweepListBytes);
