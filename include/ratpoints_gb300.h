@@ -146,26 +146,29 @@ rpg_status rpg_square_root(const char *const *coefficients, int32_t coefficient_
                            int64_t numerator, int64_t denominator, char *ordinate,
                            size_t ordinate_capacity, int32_t *is_point);
 
-/* The fast plan a single-curve search uses (host only, no device needed):
- * numerator classes modulo 64 * class_prime, and the stage-1 row moduli with
- * their prime factors (factors[i][0..3], 0-padded) and filtering bits.  No
- * counterpart in the reference, whose prime set is fixed. */
+/* The fast plan a single-curve search uses (host only, no device needed): the
+ * primes that its survivors pass, as a class prime (1: none) and row moduli
+ * with their prime factors (factors[i][0..3], 0-padded) and filtering bits.
+ * The kernel splits these primes anew between numerator classes, rows and
+ * later tests, which changes no survivor.  No counterpart in the reference,
+ * whose prime set is fixed. */
 typedef struct rpg_fast_plan_info {
     int32_t class_prime;
     int32_t modulus_count;
     int32_t moduli[16];
     int32_t factors[16][4];
     double bits;
-    int32_t slots;             /* denominators staged per CTA by the single-curve kernel (2 or 3) */
+    int32_t slots;             /* row sets whose shared memory the rows were fitted to (2 or 3) */
 } rpg_fast_plan_info;
 rpg_status rpg_fast_plan(const char *const *coefficients, int32_t coefficient_count, int64_t numerator_bound,
                          rpg_fast_plan_info *plan);
 
 /*
- * Measured choice of the fast plan's shape: the number of stage-1 rows and
- * the row slots (2 or 3) per CTA of the single-curve kernel.  Builds the sieve
- * with the cost model's shape and its neighbours (the other slot count, one
- * and two rows fewer or more), times each with CUDA events on parameters
+ * Measured choice of the fast plan's shape: the number of rows, and of row
+ * sets (slots: 2 or 3) whose shared memory they were fitted to, which together
+ * select its primes.  Builds the sieve with the cost model's shape and its
+ * neighbours (the other number of sets, one and two rows fewer or more; shapes
+ * that select the same primes once), times each with CUDA events on parameters
  * [first, first + sample) (clipped to last; flags: RPG_SIEVE_SQUARE_DENOMINATORS),
  * and reports them with the fastest.  When the environment variable
  * RPG_TUNE_CACHE names a file, the choice is stored there as JSON, keyed by

@@ -92,26 +92,22 @@ struct WideCurve {
     int count_r;
     int class_prime;               // q (1: 2-adic classes only)
     int class_mod;                 // M = 64 q
-    int h_mod_m;                   // H mod M
-    int inv64_q;                   // 64^-1 mod q (CRT)
     int smem_words;
     int square;
     int index;                     // position in the caller's curve list
     int rows;                      // stage-1 moduli in use (the others are padding)
     u64 denom_primes[2];           // bit i: odd prime i of the OddPrime table is a denominator prime
     unsigned short neg_h[kCandidatePrimes];   // (-H) mod p
-    unsigned short s_mod[kCandidatePrimes];   // S mod p
     unsigned short m_mod[kCandidatePrimes];   // M mod p
     unsigned char crt[13 * 13];    // [r64 mod q][rq] -> t with r = r64 + 64 t (mod 64 q)
     unsigned char mod_q[64];       // r64 mod q
-    int nint;                      // x intervals (0: the whole row)
+    int nint;                      // x intervals (at least one)
     double lo[kMaxIntervals];      // ascending lower bounds (-inf: none)
     double hi[kMaxIntervals];      // upper bounds (+inf: none)
 };
 
 struct NarrowCurve {
     long long bound;
-    long long words;               // W: dense 64-site words per denominator row
     long long tables;              // word offset of the curve's table block (even)
     long long aff;
     unsigned long long magic[kNarrowSlots];
@@ -170,14 +166,9 @@ __device__ __forceinline__ bool next_x_range(const double *lo, const double *hi,
     return any;
 }
 
-// The want-th of them.  Without intervals the one range is [-H, H].
+// The want-th of them.
 __device__ __forceinline__ bool x_range(const double *lo, const double *hi, int nint, long long H,
                                         long long d, int want, long long &L, long long &U) {
-    if (nint == 0) {
-        L = -H;
-        U = H;
-        return want == 0;
-    }
     for (int i = 0, n = 0; next_x_range(lo, hi, nint, H, double(d), i, L, U); ++n)
         if (n == want) return true;
     return false;
@@ -479,8 +470,8 @@ __device__ __forceinline__ int wide_layout(const WideCurve &C, const ClassStart 
     const u64 classesq = q > 1 ? C.admissible[64 + int(du % u32(q))] : u64(1);
     const int nq = __popcll(classesq);
     const int nclass = __popcll(classes2) * nq;
-    long long lo_a = -C.bound, hi_a = C.bound;
-    if (C.nint > 0) x_range(C.lo, C.hi, C.nint, C.bound, d, range, lo_a, hi_a);
+    long long lo_a = 0, hi_a = -1;
+    x_range(C.lo, C.hi, C.nint, C.bound, d, range, lo_a, hi_a);
     int carry = 0;
     for (int base = 0; base < nclass; base += 32) {
         const int c = base + lane;
@@ -1762,8 +1753,7 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, const std::vector<cha
             if (cw.wide) {
                 if ((2 * curves[i].bound) / (64LL * cw.plan.class_prime) / 64 + 2 >= dev::kMaxClassWords)
                     throw std::invalid_argument("numerator bound too large for the batched search");
-                const std::size_t n = curves[i].intervals.size();
-                wide_items += parts * (n > 0 && n <= std::size_t(dev::kMaxIntervals) ? n : 1);
+                wide_items += parts * curves[i].intervals.size();  // at most kMaxIntervals: swept_alone
                 cls += 64 * std::size_t(cw.plan.class_prime);
                 ++wide;
             } else {
@@ -1857,8 +1847,6 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, const std::vector<cha
             C.count_r = int((2 * H) % M);
             C.class_prime = q;
             C.class_mod = int(M);
-            C.h_mod_m = int(H % M);
-            C.inv64_q = q > 1 ? int(mod_inverse(64 % q, q)) : 0;
             C.square = c.square ? 1 : 0;
             C.index = int(i);
             C.rows = int(plan.moduli.size());
@@ -1885,9 +1873,10 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, const std::vector<cha
             std::copy(cw.adm2, cw.adm2 + 64, C.admissible);
             if (q > 1) {
                 class_prime_residues(c.coefficients, q, C.admissible + 64);
+                const int inv64 = int(mod_inverse(64 % q, q));
                 for (int a = 0; a < q; ++a)
                     for (int rq = 0; rq < q; ++rq)
-                        C.crt[a * 13 + rq] = (unsigned char)(((rq - a + q) % q) * C.inv64_q % q);
+                        C.crt[a * 13 + rq] = (unsigned char)(((rq - a + q) % q) * inv64 % q);
             }
             for (int r64 = 0; r64 < 64; ++r64) C.mod_q[r64] = (unsigned char)(q > 1 ? r64 % q : 0);
             // class starts for every residue r mod M: ofs = (r + H) mod M, and per
@@ -1907,19 +1896,17 @@ void build_plan(const std::vector<BatchCurveSpec> &curves, const std::vector<cha
             for (int ci = 0; ci < kCandidatePrimes; ++ci) {
                 const int p = cands[ci];
                 C.neg_h[ci] = (unsigned short)((p - H % p) % p);
-                C.s_mod[ci] = (unsigned short)(S % p);
                 C.m_mod[ci] = (unsigned short)(M % p);
             }
             device_intervals(c.intervals, C.nint, C.lo, C.hi);
             const long long chunk = item_chunk(cw);
-            for (int range = 0; range < std::max(1, C.nint); ++range)
+            for (int range = 0; range < C.nint; ++range)
                 for (long long f = c.first; f <= c.last; f += chunk)
                     P.wide_items[at.item++] = {f, int(at.descriptor), int(std::min(chunk, c.last - f + 1)), range, 0};
             P.wide[at.descriptor] = C;
         } else {
             dev::NarrowCurve &C = P.narrow[at.descriptor];
             C.bound = H;
-            C.words = cw.words;
             C.square = c.square ? 1 : 0;
             C.index = int(i);
             C.rows = int(plan.moduli.size());

@@ -88,7 +88,7 @@ struct FastPlan {
     double bits = 0;                       // expected filtering of the stage-1 rows (bits)
     // (p, residues x with f(x) a square mod p) of the plan's primes, class prime included
     std::vector<std::pair<int, int>> admitted;
-    int row_slots = 2;                     // single-curve kernel: denominators staged per CTA (2 or 3)
+    int row_slots = 2;                     // row sets whose shared memory the rows were fitted to (2 or 3)
 };
 // max_modulus caps each stage-1 modulus (table size grows as its square);
 // class_prime false keeps the plan to 2-adic classes (the dense layout of the

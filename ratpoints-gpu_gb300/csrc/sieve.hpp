@@ -33,8 +33,10 @@ public:
 
 void check_cuda(cudaError_t status, const char *what);
 
-// Shape of a fast plan: the number of stage-1 rows and the row slots (2 or 3)
-// each CTA of the single-curve kernel stages.  rows 0: the cost model's choice.
+// Shape of a fast plan: how many rows its primes are packed into, and whether
+// within the shared memory of two or three sets of them.  It selects the primes
+// that survivors pass; which rows the kernel stages, and in how many slots, is
+// the sweep plan's choice (sweep_plan.hpp).  rows 0: the cost model's choice.
 struct FastShape {
     int rows = 0;
     int slots = 0;
@@ -91,19 +93,20 @@ void *device_malloc(std::size_t bytes, const char *what);
 void release_pooled_pipelines(int device);
 
 // The fast plan a single-curve sieve uses for a curve and numerator bound
-// (host only): the autotuner's choice under the fast kernel's shared-memory
-// budget; *max_classes (optional) receives the most classes of one denominator.
+// (host only): the autotuner's choice of primes; *max_classes (optional)
+// receives the most classes of one denominator mod 64 times the class prime.
 // A shape with rows > 0 fixes the row count (the rows filtering most) and the
-// row slots instead of the cost model.
+// row sets instead of the cost model.
 struct FastPlan;
 FastPlan single_curve_plan(const std::vector<std::string> &coefficients, long long bound, int *max_classes,
                            FastShape shape = FastShape{});
 
-// The fast plan a sieve chose for its curve (empty for the reference plan).
+// The fast plan a sieve chose for its curve (empty for the reference plan): the
+// primes its survivors pass, wherever the sweep plan has them tested.
 struct FastPlanInfo {
-    int class_prime = 0;           // numerator classes are taken mod 64 * class_prime
-    std::vector<int> primes;       // small primes tested by the stage-1 rows
-    std::vector<int> moduli;       // the stage-1 row moduli (products of those primes)
+    int class_prime = 0;           // 1: none
+    std::vector<int> primes;       // the others
+    std::vector<int> moduli;       // their products that the planner packed them into
 };
 
 class Sieve {

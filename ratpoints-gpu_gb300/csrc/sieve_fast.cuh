@@ -14,9 +14,9 @@
 // A class is a pair: residue r2 mod two and residue rq mod Q.  Its a0 is
 // abase + x2 + xq with x2, xq in [0, M) the CRT lifts (abase = -H - M for a
 // whole row), so its row index is the sum of one term per residue, and the
-// terms are few enough to be tabled once per search.  x2 + xq is not reduced modulo M: a class may start a step
-// before the numerator range, and ends up to a step after it; emission drops
-// those sites, the sweep needs no masks.
+// terms are few enough to be tabled once per search.  x2 + xq is not reduced
+// modulo M: a class may start a step before the numerator range, and ends up to
+// a step after it; emission drops those sites, the sweep needs no masks.
 #pragma once
 
 #include "plan.hpp"
@@ -333,7 +333,7 @@ __device__ __forceinline__ void load_starts16(u32 a, u32 (&v)[N]) {
 //   - rows are staged as two periods, so that the sum of two row offsets below
 //     m needs no wrap: 61 instead of 115 instructions per step of ten rows,
 //     1.95 instead of 2.49 ms per 65,536 denominators of a curve of degree 6
-//     at H = 5e6, 98 instead of 71 % of the pipe busy;
+//     at H = 5e6, the pipe busy in 93 instead of 71 % of its cycles;
 //   - a broadcast 128-bit shared read takes two cycles, a 64-bit one one: the
 //     terms of a residue are packed to 16 bits (two cycles for eight rows,
 //     three for twelve) and shared by U = 2 pairs (1.81 -> 1.75 ms); read from

@@ -21,7 +21,7 @@ struct TableJob;
 struct ListJob;
 }  // namespace dev
 
-// One launch: parameters first .. last (at most 2^31 / 64), numerators
+// One launch: parameters first .. last (below 2^31), numerators
 // a_lo .. a_hi (at most SweepCurve::tile() of them).  Device pointers: the
 // survivor arrays (curve tags only with out_curve), their count, a zeroed work
 // counter, the error word, and (optional) the counts of swept words and of the

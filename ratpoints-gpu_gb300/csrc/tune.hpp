@@ -1,12 +1,13 @@
 // Measured tuning of the single-curve fast plan's shape.
 //
-// The cost model of the planner (plan.hpp) picks how many stage-1 rows a
-// curve gets and whether each CTA stages two or three denominators.  The tuner
-// measures instead: for a curve it builds the sieve with the cost model's
-// shape and with its neighbours (one and two rows fewer or more, the other
-// slot count), times each on a sample of the search's denominators with CUDA
-// events, and keeps the fastest.  Choices persist in a JSON file, keyed by
-// the kind of curve (degree, class prime, row length, small- or large-prime
+// The cost model of the planner (plan.hpp) packs a curve's primes into some
+// number of rows that fit two or three sets into shared memory: its shape, which
+// selects the primes that survivors pass.  The tuner measures instead: for a
+// curve it builds the sieve with the cost model's shape and with its neighbours
+// (one and two rows fewer or more, the other number of sets; shapes that select
+// the same primes once), times each on a sample of the search's denominators
+// with CUDA events, and keeps the fastest.  Choices persist in a JSON file,
+// keyed by the kind of curve (degree, class prime, row length, small- or large-prime
 // rows), and every later sieve of a curve of that kind uses the stored shape.
 // The file is named by the RPG_TUNE_CACHE environment variable; without it no
 // shape is read or stored and sieves use the cost model.  No counterpart in
