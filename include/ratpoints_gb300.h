@@ -269,10 +269,12 @@ rpg_status rpg_session_sieve_noalloc(rpg_session *session, int32_t first, int32_
 
 /*
  * Batched search of many curves in one pass: every curve's tables resident on
- * the device, two persistent sieve kernels over device work queues, one
- * captured CUDA graph.  No counterpart in the reference, which searches one
- * curve per process (src/main.cpp:48-85); each curve's points are exactly
- * what rpg_point_search reports for the same options, in the same order.
+ * the device, persistent sieve kernels over device work queues and a launch of
+ * the single-curve kernel per curve with much work, in one captured CUDA graph
+ * (beyond 64 GB of tables: those curves in groups, by direct launches).  No
+ * counterpart in the reference, which searches one curve per process
+ * (src/main.cpp:48-85); each curve's points are exactly what rpg_point_search
+ * reports for the same options, in the same order.
  *
  * Each curves[i] is read as by rpg_point_search; batch_size, plan, device
  * and verify_threads are ignored (the batch has its own plan and uses

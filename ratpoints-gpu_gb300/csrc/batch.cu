@@ -1436,14 +1436,14 @@ long long swept_row_words(const BatchCurveSpec &c, long long first, long long la
 
 // Whether a curve gets sieve launches of its own (sweep.hpp) instead of work
 // items of the batched kernels.  Rows of at least kBatchWideWords words always
-// do; shorter ones when the narrow kernel's time for them, about 0.1 ns per
-// denominator and 2.8e-3 ns per row word, exceeds the sweep's (1 ns per
-// denominator up to H = 65,504) by more than building the curve's tables takes
-// (400,000 denominators of sextics, narrow and sweep: H = 5,000 0.28 and 0.34
-// ms, 10,000 0.38 and 0.32, and before the narrow kernel shared stage 2 among
-// denominators 20,000 0.66 and 0.38, 65,000 1.7 and 0.40).  The line is flat:
-// with 0.7 for 0.9 or 8,000 for 20,000, bursts of requests and batches change
-// by 4 % at most, either way.
+// do; shorter ones from 322 words on, with denominators enough.  Kernel time of
+// 400,000 denominators, mean of six random sextics, narrow kernel and sweep: H =
+// 5,000 0.21 and 0.22 ms, 10,000 0.28 and 0.21, 20,000 0.40 and 0.21, 65,000
+// 1.04 and 0.23; of 40,000 at H = 20,000 0.10 and 0.04, of 4,000 at 65,000 0.045
+// and 0.025.  A launch of a curve's own needs its sweep plan (some 0.1 ms of a
+// host core) and tables (0.03 ms), which the narrow kernel shares better among
+// many small curves.  The line is flat: with 0.7 for 0.9 or 8,000 for 20,000,
+// bursts of requests and batches change by 4 % at most, either way.
 // Curves with x intervals stay in the kernels that sweep only those.
 bool swept_alone(const BatchCurveSpec &c, bool wide, long long words, long long count) {
     if (!c.intervals.empty() && c.intervals.size() <= std::size_t(dev::kMaxIntervals)) return false;
